@@ -1,0 +1,46 @@
+"""The quotient of csrc/vxb_common.cuh (divBy): x * r corrected twice by its
+remainder, r the rounded reciprocal, equals the correctly rounded x / d
+(Markstein 1990).  Evaluated in exact rational arithmetic with one rounding
+per operation, as the fused operations round."""
+
+import random
+from fractions import Fraction
+
+import pytest
+
+
+def _fma(a, b, c):
+    return float(Fraction(a) * Fraction(b) + Fraction(c))   # one correct rounding
+
+
+def _div_by(x, d):
+    r = 1.0 / d
+    q = x * r
+    q = _fma(_fma(-q, d, x), r, q)
+    return _fma(_fma(-q, d, x), r, q)
+
+
+def _mantissas(rng, n):
+    # Mantissas at the ends of the binade, with few and with many set bits.
+    for k in range(n):
+        kind = k % 4
+        if kind == 0:
+            yield 1.0 + rng.getrandbits(52) * 2.0 ** -52
+        elif kind == 1:
+            yield 1.0 + rng.getrandbits(8) * 2.0 ** -52
+        elif kind == 2:
+            yield 2.0 - (1 + rng.getrandbits(8)) * 2.0 ** -52
+        else:
+            yield 1.0 + sum(2.0 ** -rng.randint(1, 52) for _ in range(3)) % 1.0
+
+
+@pytest.mark.parametrize("scale", [0, -7, 300, -300])
+def test_quotient_is_correctly_rounded(scale):
+    rng = random.Random(scale)
+    xs, ds = list(_mantissas(rng, 160)), list(_mantissas(rng, 160))
+    for d in ds:
+        d = d * 2.0 ** -scale
+        for x in rng.sample(xs, 24):
+            for s in (x, -x * 2.0 ** scale):
+                assert _div_by(s, d) == s / d
+    assert _div_by(0.0, ds[0]) == 0.0

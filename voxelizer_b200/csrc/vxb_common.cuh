@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace vxb {
@@ -56,12 +57,47 @@ __device__ __forceinline__ uint32_t warpFindOwner(const uint32_t* __restrict__ o
     return lo;
 }
 
+// Exact conversion of a 32-bit unsigned integer: 2^52 + x as a bit pattern,
+// less 2^52 (the conversion instruction runs at a quarter of the FP64 rate).
+__device__ __forceinline__ double toDouble(uint32_t x) {
+    return __dsub_rn(__hiloint2double(0x43300000, (int)x), 4503599627370496.0);
+}
+
+// Whether |x| lies in [2^-400, 2^400) (not zero, infinite or NaN).
+__host__ __device__ __forceinline__ bool divScale(double x) {
+#ifdef __CUDA_ARCH__
+    const uint32_t h = (uint32_t)__double2hiint(x);
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    const uint32_t h = (uint32_t)(u >> 32);
+#endif
+    return (h & 0x7FFFFFFFu) - 0x26F00000u < 0x32000000u;
+}
+
+// The correctly rounded x / d for operands with divExact(x) and r = 1 / d
+// rounded to nearest with divScale(d).  Two corrections of x * r by its
+// remainder: the first brings the quotient within one ulp, and the second
+// then rounds it correctly (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
+// 1990, theorem 7).  With both operands within 2^+-400 no intermediate
+// leaves the normal range; x = +-0 gives a zero (of either sign).
+__device__ __forceinline__ bool divExact(double x) { return divScale(x) || x == 0.0; }
+__device__ __forceinline__ double divBy(double x, double d, double r) {
+    double q = __dmul_rn(x, r);
+    q = __fma_rn(__fma_rn(-q, d, x), r, q);
+    return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
 // Blocks for `work` items at `threads` per block, capped (grid-stride loops).
 inline uint32_t gridFor(uint64_t work, uint32_t threads, uint32_t cap = 148u * 32u) {
     uint64_t b = (work + threads - 1) / threads;
     if (b == 0) b = 1;
     return (uint32_t)(b < cap ? b : cap);
 }
+
+// 1 / d for divBy.
+inline double divReciprocal(double d) { return divScale(d) ? 1.0 / d : 0.0; }
 
 }  // namespace detail
 }  // namespace vxb

@@ -20,6 +20,7 @@ namespace vxb {
 struct PassGeom {
     double mn[3];        // minimum corner (FP64, as the reference's extMinVertex)
     double d;            // voxel length
+    double rd;           // 1 / d, or 0 (divBy)
     float mnf[3];        // float(mn) for the FP32 surface path
     float df;            // float(d)
     uint32_t X;          // voxels along x (padded and rounded to 32 * xSplits)
@@ -74,15 +75,20 @@ void launch_scan(const uint32_t* in, uint32_t* offsets, uint32_t n, uint32_t* bl
                  uint32_t* overflow, cudaStream_t s, uint32_t* launches);
 
 // ---- Solid (parity) voxelization: src/voxelizer.cu:840-1617 ----
-// Candidates per work triangle, the toggles of the listed candidates into
-// the `fill` arena, then the row prefix XOR over all rows of the batch.
-void launch_solid_count(const Batch& b, uint32_t nWork, uint32_t* counts, cudaStream_t s, uint32_t* launches);
+// The toggles of every candidate into the `fill` arena, then the row prefix
+// XOR over all rows of the batch.  *total (zero on entry) receives the number
+// of candidates.  `big` holds the listed chunks of batches with very many
+// candidates (bigCap entries, *bigCount zero on entry); it may be NULL where
+// solid_may_list answers false for every unit, and the call then takes one
+// launch instead of two.
 // blocksPerSm: launch shape (the autotuner's choice; results do not depend
 // on it), here and in the launchers below that take one.  queue: NULL for
 // a fixed grid-stride order, else a device word the launcher zeroes and the
-// kernel's persistent blocks take batches of work from.
-void launch_solid_toggle(const Batch& b, uint32_t nWork, const uint32_t* offsets, const uint32_t* total,
-                         uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue, cudaStream_t s, uint32_t* launches);
+// kernel's warps take batches of work from.
+bool solid_may_list(const PassGeom& g, uint64_t nSplits, uint32_t nWork);
+void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, unsigned long long* big,
+                         uint32_t* bigCount, uint32_t bigCap, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
+                         cudaStream_t s, uint32_t* launches);
 void launch_row_fill(const Batch& b, uint64_t nRows, uint32_t* fill, cudaStream_t s, uint32_t* launches);
 
 // ---- Surface voxelization: src/voxelizer.cu:2358-2989, 3040-4201 ----

@@ -6,9 +6,9 @@
 // times cudaMalloc) synchronizes the whole device, which a caller that keeps
 // several streams busy cannot afford in the middle of a time step.  The
 // caller passes the mesh and the output already in device memory; the work
-// lists this path needs (a range-checked copy of the indices, per-triangle
-// candidate counts, their scan, the yz subspace table and the unit table)
-// live in a fixed, statically sized array in device memory instead of
+// lists this path needs (a range-checked copy of the indices, the chunks of
+// triangles with very many candidates, the yz subspace table and the unit
+// table) live in a fixed, statically sized array in device memory instead of
 // buffers allocated per call.  The call itself allocates nothing, on the
 // device or on the host; its tables are passed to a set-up kernel by value,
 // so it copies nothing from host memory either.  The array is placed by the
@@ -34,6 +34,7 @@
 // race on the array and give undefined results: serialize them.
 
 #include "vxb.h"
+#include "vxb_common.cuh"
 #include "vxb_kernels.cuh"
 #include "vxb_plan.h"
 
@@ -53,7 +54,7 @@ namespace {
 
 constexpr uint32_t kMaxTriangles = 1u << 20;  // 1,048,576
 constexpr uint32_t kMaxSubspaces = 1024;
-constexpr uint32_t kScanTile = 4096;          // items per tile of launch_scan
+constexpr uint32_t kBigChunks = 1u << 20;     // chunks of big triangles (launch_solid_toggle)
 constexpr int kMaxDevices = 64;
 
 constexpr size_t roundUp(size_t v) { return (v + 255) / 256 * 256; }
@@ -68,14 +69,12 @@ struct UnitTables {
 };
 
 // Layout of the scratch array (byte offsets).
-constexpr size_t kStatusOff = 0;  // [0] candidate total, [1] overflow flag, [2] index out of range
+constexpr size_t kStatusOff = 0;  // [0, 1] candidate total, [2] index out of range, [3] big chunks
 constexpr size_t kTablesOff = kStatusOff + 256;
 constexpr size_t kSubspaceOff = kTablesOff + 768;
 static_assert(sizeof(UnitTables) <= 768, "tables region");
-constexpr size_t kTileOff = kSubspaceOff + roundUp(kMaxSubspaces * sizeof(vxb::SplitYZ));
-constexpr size_t kCountOff = kTileOff + roundUp(4 * (kMaxTriangles / kScanTile + 2));
-constexpr size_t kOffsetOff = kCountOff + roundUp(4 * ((size_t)kMaxTriangles + 1));
-constexpr size_t kIndexOff = kOffsetOff + roundUp(4 * ((size_t)kMaxTriangles + 2));
+constexpr size_t kBigOff = kSubspaceOff + roundUp(kMaxSubspaces * sizeof(vxb::SplitYZ));
+constexpr size_t kIndexOff = kBigOff + roundUp(8 * (size_t)kBigChunks + 1792);
 constexpr size_t kScratchBytes = kIndexOff + roundUp(12 * (size_t)kMaxTriangles);
 static_assert(kScratchBytes == 20990720, "scratch layout changed: update the stated size");
 
@@ -126,7 +125,7 @@ __global__ void noallocSetupKernel(UnitTables tab, uint32_t resY, uint32_t resZ,
                                    UnitTables* dtab, vxb::SplitYZ* dsub, uint32_t* status) {
     if (threadIdx.x == 0) {
         *dtab = tab;
-        status[0] = status[1] = status[2] = 0u;
+        status[0] = status[1] = status[2] = status[3] = 0u;
     }
     const uint32_t ny = (resY + splitY - 1) / splitY, nz = (resZ + splitZ - 1) / splitZ;
     for (uint32_t k = threadIdx.x; k < ny * nz; k += blockDim.x) {
@@ -180,7 +179,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
                      (unsigned long long)ny * nz, kMaxSubspaces);
     // A triangle is a candidate at most once per (subspace, 4x4 tile) pair
     // it overlaps, and a subspace cut adds at most one partial tile per
-    // axis: keep the scan of candidate counts below 2^32.
+    // axis: keep the candidate count below 2^32.
     const double bound = (double)n_triangles * (double)((bg.res[1] + 3) / 4 + ny) * (double)((bg.res[2] + 3) / 4 + nz);
     if (bound >= 4294967295.0)
         return failf(VXB_EINVAL,
@@ -224,6 +223,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
         g.mnf[a] = (float)min_vertex[a];
     }
     g.d = bg.d;
+    g.rd = vxb::detail::divReciprocal(bg.d);
     g.df = (float)bg.d;
     g.X = bg.res[0];
     g.resY = bg.res[1];
@@ -248,9 +248,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     uint32_t* status = reinterpret_cast<uint32_t*>(scratch + kStatusOff);
     UnitTables* dtab = reinterpret_cast<UnitTables*>(scratch + kTablesOff);
     vxb::SplitYZ* dsub = reinterpret_cast<vxb::SplitYZ*>(scratch + kSubspaceOff);
-    uint32_t* tiles = reinterpret_cast<uint32_t*>(scratch + kTileOff);
-    uint32_t* counts = reinterpret_cast<uint32_t*>(scratch + kCountOff);
-    uint32_t* offsets = reinterpret_cast<uint32_t*>(scratch + kOffsetOff);
+    unsigned long long* big = reinterpret_cast<unsigned long long*>(scratch + kBigOff);
     uint32_t* grid = static_cast<uint32_t*>(dev_out);
     vxb::Batch b;
     memset(&b, 0, sizeof(b));
@@ -272,9 +270,9 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     noallocIndexKernel<<<(nIdx + 255) / 256 < 148u * 8u ? (nIdx + 255) / 256 : 148u * 8u, 256, 0, s>>>(
         dev_indices, nIdx, n_vertices, checkedIdx, status);
     launches += 2;
-    vxb::launch_solid_count(b, n_triangles, counts, s, &launches);
-    vxb::launch_scan(counts, offsets, n_triangles, tiles, status, status + 1, s, &launches);
-    vxb::launch_solid_toggle(b, n_triangles, offsets, status, grid, 3, nullptr, s, &launches);
+    vxb::launch_solid_toggle(b, n_triangles, reinterpret_cast<unsigned long long*>(status),
+                             vxb::solid_may_list(g, nSub, n_triangles) ? big : nullptr, status + 3, kBigChunks, grid, 3, nullptr,
+                             s, &launches);
     vxb::launch_row_fill(b, tab.rowBase[1], grid, s, &launches);
     e = cudaGetLastError();
     if (e != cudaSuccess) return failf(VXB_ECUDA, "%s", cudaGetErrorString(e));
@@ -295,6 +293,6 @@ extern "C" vxb_status vxb_noalloc_status(void) {
         return failf(VXB_ECUDA, "reading the status words: %s", cudaGetErrorString(e));
     }
     if (st[2]) return failf(VXB_EINVAL, "the last call's mesh has an index >= n_vertices; its bit array is undefined");
-    if (st[1]) return failf(VXB_EOVERFLOW, "the last call's candidate count overflowed; its bit array is undefined");
+    if (st[1] || st[0] == 0xFFFFFFFFu) return failf(VXB_EOVERFLOW, "the last call's candidate count overflowed; its bit array is undefined");
     return VXB_OK;
 }

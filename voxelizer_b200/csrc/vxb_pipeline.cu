@@ -10,6 +10,8 @@
 
 #include "vxb_pipeline.h"
 
+#include "vxb_common.cuh"
+
 #include <algorithm>
 #include <cstring>
 
@@ -18,8 +20,12 @@ namespace vxb {
 namespace {
 
 // Slots of the status buffer; pruning flags follow at kFlags.
-enum : int { kSolidTotal = 0, kSolidOverflow = 1, kSurfTotal = 2, kSurfOverflow = 3, kHitCount = 4,
-             kSurfaceVoxels = 5, kSurfQueue = 6, kToggleQueue = 7, kFlags = 8 };
+// kSolidTotal and kSolidHigh are the low and high word of one 64-bit count.
+enum : int { kSolidTotal = 0, kSolidHigh = 1, kSurfTotal = 2, kSurfOverflow = 3, kHitCount = 4,
+             kSurfaceVoxels = 5, kSurfQueue = 6, kToggleQueue = 7, kBigCount = 8, kFlags = 10 };
+
+// The work counts take 32 bits: totals of 2^32 - 1 or more are refused.
+bool solidOverflow(const uint32_t* h) { return h[kSolidHigh] || h[kSolidTotal] == 0xFFFFFFFFu; }
 
 const uint32_t kNodeBytes[5] = {1, 2, 8, 2, 4};
 
@@ -87,6 +93,7 @@ PassGeom makeGeom(const Plan& p, int lattice, bool turned) {
         g.mnf[a] = (float)g.mn[a];
     }
     g.d = p.d;
+    g.rd = detail::divReciprocal(p.d);
     g.df = (float)p.d;
     g.X = p.res[0];
     g.resY = p.res[1];
@@ -276,9 +283,9 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     const size_t wordBytes = 4 * (size_t)totalWords_;
     if ((rc = tables.ensure(blob_.size() + 64))) return rc;
     if ((rc = status.ensure(4 * (kFlags + (size_t)nRegions_ * kPasses) + 256))) return rc;
-    if ((rc = counts.ensure(4 * ((size_t)nWork_ + 1)))) return rc;
-    if ((rc = offsets.ensure(4 * ((size_t)nWork_ + 2)))) return rc;
-    if ((rc = tileSums.ensure(4 * ((size_t)nWork_ / 4096 + 2)))) return rc;
+    mayList_ = false;
+    for (const Unit& u : units_) mayList_ |= solid_may_list(u.g, u.nSplits, nWork_);
+    if (mayList_ && (rc = bigList.ensure(8 * (size_t)kBigCap))) return rc;
     if (!aliasFill_ && (rc = fill.ensure(wordBytes))) return rc;
     if (anyCartesian_ && (rc = fin.ensure(wordBytes))) return rc;
     // Change lists of the pruning passes: the first pass lists every word it
@@ -358,6 +365,8 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     bucket_ = tuneBucket(nWork_, totalWords_, nodeKind_, anyMaterials_);
     shape = tunePick(bucket_, &trial_, cap == cudaStreamCaptureStatusNone);
     for (bool& u : tuneUsed_) u = false;
+    // Work counts, hit count and pruning flags.
+    VXB_CUDA(cudaMemsetAsync(st, 0, 4 * (kFlags + (size_t)nRegions_ * kPasses), s));
     // Surface voxelization, hit list and surface ranks on the side stream,
     // beside the solid pass (they share no buffer).
     cudaStream_t ss = s;
@@ -372,7 +381,6 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         VXB_CUDA(cudaMemsetAsync(surf.p, 0, 4 * (size_t)totalWords_, ss));
         VXB_CUDA(cudaMemsetAsync(buckets.p, 0, 4 * 2 * kSurfaceBuckets, ss));
         VXB_CUDA(cudaMemsetAsync(sCounts.p, 0, 4 * ((size_t)nWork_ + 1), ss));
-        VXB_CUDA(cudaMemsetAsync(st + kHitCount, 0, 4, ss));
         launch_surface_prepare(b, nWork_, codes.as<uint32_t>(), unitCounts.as<uint32_t>(), buckets.as<uint32_t>(),
                                sCounts.as<uint32_t>(), recs.p, ovl.p, ss, &launches);
         launch_scan(sCounts.as<uint32_t>(), sOffsets.as<uint32_t>(), nWork_, sTileSums.as<uint32_t>(),
@@ -413,12 +421,10 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     // Solid voxelization.
     mark(0, false);
     VXB_CUDA(cudaMemsetAsync(fillP, 0, wordBytes, s));
-    launch_solid_count(b, nWork_, counts.as<uint32_t>(), s, &launches);
-    launch_scan(counts.as<uint32_t>(), offsets.as<uint32_t>(), nWork_, tileSums.as<uint32_t>(), st + kSolidTotal,
-                st + kSolidOverflow, s, &launches);
     tuneMark(kKnobToggle, false, s);
-    launch_solid_toggle(b, nWork_, offsets.as<uint32_t>(), st + kSolidTotal, fillP, shape.toggleBlocksPerSm,
-                        shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
+    launch_solid_toggle(b, nWork_, reinterpret_cast<unsigned long long*>(st + kSolidTotal),
+                        mayList_ ? bigList.as<unsigned long long>() : nullptr, st + kBigCount, kBigCap, fillP,
+                        shape.toggleBlocksPerSm, shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
     tuneMark(kKnobToggle, true, s);
     launch_row_fill(b, totalRows_, fillP, s, &launches);
     mark(0, true);
@@ -451,7 +457,6 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
             launch_combine(fillP, surf.as<uint32_t>(), fin.as<uint32_t>(), totalWords_, ps, &launches);
         else
             VXB_CUDA(cudaMemcpyAsync(fin.p, fillP, 4 * (size_t)totalWords_, cudaMemcpyDeviceToDevice, ps));
-        VXB_CUDA(cudaMemsetAsync(st + kFlags, 0, 4 * (size_t)nRegions_ * kPasses, ps));
         // Per subspace index and pass: the count of its change list; the
         // last word is the list overflow flag.
         uint32_t* counts = pruneScratch.as<uint32_t>();
@@ -600,7 +605,7 @@ int Pipeline::finish(cudaStream_t s) {
         tuneFinish();
         uint32_t h[2];
         VXB_CUDA(cudaMemcpy(h, status.p, sizeof(h), cudaMemcpyDeviceToHost));
-        if (h[kSolidOverflow]) return failf(VXB_EOVERFLOW, "solid work list exceeds 2^32 entries");
+        if (solidOverflow(h)) return failf(VXB_EOVERFLOW, "solid work list exceeds 2^32 entries");
         return 0;
     }
     std::vector<uint32_t> h(kFlags + (size_t)nRegions_ * kPasses);
@@ -618,7 +623,7 @@ int Pipeline::finish(cudaStream_t s) {
     stats.surface_voxels = anyMaterials_ ? h[kSurfaceVoxels] : 0;
     for (uint32_t k = 0; k < kSurfaceBuckets; ++k) stats.surface_triangles[k / 3] += bk[k];
     stats.grid_words = totalWords_;
-    if (h[kSolidOverflow] || (anyMaterials_ && h[kSurfOverflow]))
+    if (solidOverflow(h.data()) || (anyMaterials_ && h[kSurfOverflow]))
         return failf(VXB_EOVERFLOW, "work list exceeds 2^32 entries");
     bool reemit = false;
     const Batch b = batch();

@@ -94,6 +94,7 @@ public:
 
     static constexpr uint32_t kPasses = 8;   // pruning passes queued per subspace
     static constexpr uint32_t kLoopListMax = 32768;   // longest list the one-block passes take
+    static constexpr uint32_t kBigCap = 1u << 19;       // candidate chunks listed by the solid pass
     static constexpr uint32_t kOutChunks = 4;         // emit / host-copy ranges of streamed output
 
     // Launch shape of the last enqueue (the autotuner's choice).
@@ -127,19 +128,19 @@ private:
     uint32_t nWork_ = 0, nRegions_ = 0, nFcc_ = 0;
     uint64_t totalWords_ = 0, totalRows_ = 0, totalGroups_ = 0;
     int nodeKind_ = 0, nodes_ = 1;
-    bool anyMaterials_ = false, anyCartesian_ = false, wide_ = false, aliasFill_ = false, raw_ = false;
+    bool anyMaterials_ = false, anyCartesian_ = false, wide_ = false, aliasFill_ = false, raw_ = false,
+         mayList_ = false;
     uint32_t listCap_ = 0, keysCap_ = 0, pruneCap_ = 0, mergeEntries_ = 0;
     // table offsets (bytes) in `tables`
     size_t oUnits_ = 0, oWork_ = 0, oRow_ = 0, oWord_ = 0, oSplits_ = 0, oSlices_ = 0, oLater_ = 0, oRegions_ = 0,
            oFcc_ = 0, oGroupBase_ = 0;
     std::vector<uint8_t> blob_;   // host copy of the tables (alive while the upload runs)
 
-    DevBuf tables, status, counts, offsets, tileSums;
+    DevBuf tables, status, bigList;
     DevBuf fill, surf, fin, ranks, rankTiles, pruneScratch, pruneLists;
     DevBuf codes, unitCounts, buckets, recs, ovl, hitList, keys;
-    // The surface pass runs on a second stream beside the solid pass (its
-    // own work-list scan buffers), joined before pruning (surface bits) and
-    // before emission (merged keys).
+    // The surface pass runs on a second stream beside the solid pass, joined
+    // before pruning (surface bits) and before emission (merged keys).
     DevBuf sCounts, sOffsets, sTileSums;
     cudaStream_t side_ = nullptr, hi_ = nullptr;
     cudaEvent_t evFork_ = nullptr, evSurfBits_ = nullptr, evSurfDone_ = nullptr, evSolid_ = nullptr,

@@ -3,17 +3,32 @@
 // FP64 as in the reference.
 //
 // The reference sorts (tile, triangle) pairs and voxelizes one tile per
-// block.  Here the work list is the flat set of (work triangle, yz subspace,
-// 4x4 tile) candidates of every unit of the batch over an exclusive scan of
-// per-triangle candidate counts;
-// a candidate is a member of the tile's list iff one voxel centre of the
-// tile inside the triangle's clipped bounding box passes the binning test,
-// and a member toggles, for each centre of the tile inside the subspace that
-// passes the strict generation test, the bit of its x-intercept voxel in the
-// centre's row.  Toggles commute (XOR), so no sort is needed; a row prefix
-// XOR then turns toggles into solid runs.  A block stages its candidates'
-// triangles (vertices, tN, voxel box, both edge-function sets, the normal)
-// in shared memory once.
+// block.  Here the work is the flat set of (work triangle, yz subspace, 4x4
+// tile) candidates of every unit of the batch; a candidate is a member of
+// the tile's list iff one voxel centre of the tile inside the triangle's
+// clipped bounding box passes the binning test, and a member toggles, for
+// each centre of the tile inside the subspace that passes the strict
+// generation test, the bit of its x-intercept voxel in the centre's row.
+// Toggles commute (XOR), so no sort is needed; a row prefix XOR then turns
+// toggles into solid runs.
+//
+// No work list is built.  A warp takes a batch of up to 32 consecutive work
+// triangles, sets them up one per lane in shared memory (count of candidates
+// included) and walks their candidates 32 at a time over a prefix of those
+// counts, so nothing is counted, scanned or searched in global memory first
+// and no block-wide barrier holds a warp.  A batch with more than kSplit
+// candidates keeps its first chunk and lists the others, which a second
+// launch spreads over all warps (a box wall alone has tens of thousands).
+//
+// Bounds: FP64 issue at half rate (48 edge values a candidate) and the latency
+// of its chains.  Solid pass alone on a B200 (memset, toggles, row fill), with
+// a candidate list staged per block and with this split: room of 1,049,868
+// triangles at 1024 voxels 364 -> 196 us, 81,920 triangles at 701 voxels
+// 87 -> 52 us, 576 triangles at 32 voxels 48 -> 17 us.  Chunks of 32 / 64 /
+// 128 candidates on the room: 204 / 196 / 232 us; 32 costs scenes with many
+// medium triangles (stress mesh 54 against 45 us) because every chunk sets
+// its batch up again.  Five resident blocks of 96 registers: six (80) and
+// seven (72) spill and are equal or up to 8% slower.
 
 #include "vxb_common.cuh"
 #include "vxb_device.cuh"
@@ -26,8 +41,11 @@ using namespace detail;
 namespace {
 
 constexpr double kDblMin = 2.2250738585072014e-308;  // DBL_MIN, src/voxelizer.cu:1443
-constexpr int kBlock = 256;
-constexpr uint32_t kSlots = 160;   // 160 staged triangles: 44 KB of static shared memory
+constexpr int kWarps = 4;                     // warps per block of the toggle kernels
+constexpr int kBlocks = 5;                    // resident blocks per SM
+constexpr uint32_t kSplit = 256;              // candidates of a batch before its chunks are listed
+constexpr uint32_t kChunk = 64;               // candidates of one listed chunk
+constexpr uint32_t kFull = 0xffffffffu;
 
 __device__ __forceinline__ void loadTriD(const float* __restrict__ V, const uint32_t* __restrict__ I, uint32_t t,
                                          D3* v) {
@@ -37,6 +55,9 @@ __device__ __forceinline__ void loadTriD(const float* __restrict__ V, const uint
         v[k] = D3{(double)__ldg(V + 3 * a), (double)__ldg(V + 3 * a + 1), (double)__ldg(V + 3 * a + 2)};
     }
 }
+
+// The division where divBy does not apply.
+__device__ __noinline__ double divide(double x, double d) { return __ddiv_rn(x, d); }
 
 // Per-triangle binning setup: calculateTileOverlap / constructWorkQueue,
 // src/voxelizer.cu:861-945 and 1086-1144 (getTriangleBounds 2397-2418,
@@ -58,8 +79,20 @@ __device__ __forceinline__ void binSetup(const float* V, const uint32_t* I, uint
         zmax = b.v[i].z > zmax ? b.v[i].z : zmax;
     }
     const double d = g.d;
-    double a0 = __ddiv_rn(__dsub_rn(ymin, g.mn[1]), d), a1 = __ddiv_rn(__dsub_rn(zmin, g.mn[2]), d);
-    double b0 = __ddiv_rn(__dsub_rn(ymax, g.mn[1]), d), b1 = __ddiv_rn(__dsub_rn(zmax, g.mn[2]), d);
+    const double rd = g.rd;
+    double a0 = __dsub_rn(ymin, g.mn[1]), a1 = __dsub_rn(zmin, g.mn[2]);
+    double b0 = __dsub_rn(ymax, g.mn[1]), b1 = __dsub_rn(zmax, g.mn[2]);
+    if (rd != 0.0 && divExact(a0) && divExact(a1) && divExact(b0) && divExact(b1)) {
+        a0 = divBy(a0, d, rd);
+        a1 = divBy(a1, d, rd);
+        b0 = divBy(b0, d, rd);
+        b1 = divBy(b1, d, rd);
+    } else {
+        a0 = divide(a0, d);
+        a1 = divide(a1, d);
+        b0 = divide(b0, d);
+        b1 = divide(b1, d);
+    }
     b.vlo[0] = __double2int_rz(ceil(a0));
     b.vlo[1] = __double2int_rz(ceil(a1));
     b.vhi[0] = __double2int_rz(__dadd_rn(floor(b0), 1.0));
@@ -91,220 +124,365 @@ __device__ __forceinline__ uint32_t workUnit(const Batch& b, uint32_t wt, uint32
     return u;
 }
 
-__global__ void solidCountKernel(Batch b, uint32_t nWork, uint32_t* __restrict__ counts) {
-    for (uint32_t wt = blockIdx.x * blockDim.x + threadIdx.x; wt < nWork; wt += gridDim.x * blockDim.x) {
-        uint32_t t;
-        const Unit& U = b.units[workUnit(b, wt, &t)];
-        const PassGeom g = U.g;
-        BinTri bt;
-        binSetup(U.V, U.I, t, g, bt);
-        uint32_t c = 0;
-        if (!binRejected(bt)) {
-            const SplitYZ* splits = b.splits + U.splitBase;
-            for (uint32_t s = 0; s < U.nSplits; ++s) {
-                uint32_t lo[2], hi[2];
-                if (!commonSpace(bt, splits[s], lo, hi)) continue;
-                c += ((hi[0] - 1) / 4 - lo[0] / 4 + 1) * ((hi[1] - 1) / 4 - lo[1] / 4 + 1);
-            }
-        }
-        counts[wt] = c;
-    }
+// The centres of a 4x4 tile starting at (ty, tz) that lie in [y0, y1) x
+// [z0, z1), as bits 4 * cz + cy.
+__device__ __forceinline__ uint32_t clipTile(uint32_t ty, uint32_t tz, uint32_t y0, uint32_t y1, uint32_t z0,
+                                             uint32_t z1) {
+    auto clip = [](uint32_t t, uint32_t lo, uint32_t hi) {
+        const uint32_t l = lo > t ? min(lo - t, 4u) : 0u, h = hi > t ? min(hi - t, 4u) : 0u;
+        return ((1u << h) - 1u) & ~((1u << l) - 1u);
+    };
+    const uint32_t y = clip(ty, y0, y1), z = clip(tz, z0, z1);
+    return (y * 0x1111u) & (((z & 1u) | (z & 2u) << 3 | (z & 4u) << 6 | (z & 8u) << 9) * 15u);
 }
 
-// Staged triangle: binning data plus the generation edge functions.
-struct SolidStage {
-    BinTri b;
-    double bnx[3], bny[3], bd[3];   // binning edges (oriented by tN)
-    D3 n;                           // cross(v0 - v2, v1 - v0)
-    double ex[3], ey[3], ed[3];     // generation edges (oriented by n.x)
-    uint32_t tl;                    // top-left flags of the generation edges
-    uint32_t unit;
+// The triangles of one warp that have candidates, one slot each, and the
+// warp's queue of toggles (lane of the candidate << 4 | centre).
+// Field-major, so that lanes reading one field of different slots do not
+// conflict.
+struct SolidSlots {
+    double v0[3][32];
+    double n[3][32];                           // cross(v0 - v2, v1 - v0)
+    double rn[32];                             // 1 / n.x (0: divide)
+    double ex[3][32], ey[3][32], ed[3][32];    // generation edges (oriented by n.x)
+    int lo[2][32], hi[2][32];                  // voxel box
+    uint32_t wt[32], unit[32];
+    uint32_t flags[32];   // bits 0-2: top-left generation edges; bit 3: binning edges are the same
+    uint32_t off[32];     // first candidate
+    uint16_t queue[512];
 };
 
-__device__ __forceinline__ void stageSolid(SolidStage& st, const Batch& b, uint32_t wt) {
+// Candidates of work triangle wt.
+__device__ __forceinline__ uint32_t solidCount(const Batch& b, uint32_t wt, BinTri& bt, uint32_t* unit) {
     uint32_t t;
-    st.unit = workUnit(b, wt, &t);
-    const Unit& unit = b.units[st.unit];
-    binSetup(unit.V, unit.I, t, unit.g, st.b);
-    const D3* v = st.b.v;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const D3& p = v[i];
-        const D3& q = v[(i + 1) % 3];
-        if (st.b.tN > 0.0) { st.bnx[i] = __dsub_rn(p.z, q.z); st.bny[i] = __dsub_rn(q.y, p.y); }
-        else { st.bnx[i] = __dsub_rn(q.z, p.z); st.bny[i] = __dsub_rn(p.y, q.y); }
-        st.bd[i] = -sum2<site::D_BIN>(st.bnx[i], p.y, st.bny[i], p.z);
+    *unit = workUnit(b, wt, &t);
+    const Unit& U = b.units[*unit];
+    binSetup(U.V, U.I, t, U.g, bt);
+    if (binRejected(bt)) return 0u;
+    uint32_t c = 0;
+    const SplitYZ* __restrict__ splits = b.splits + U.splitBase;
+    for (uint32_t s = 0; s < U.nSplits; ++s) {
+        uint32_t lo[2], hi[2];
+        if (!commonSpace(bt, splits[s], lo, hi)) continue;
+        c += ((hi[0] - 1) / 4 - lo[0] / 4 + 1) * ((hi[1] - 1) / 4 - lo[1] / 4 + 1);
     }
-    const D3 U{__dsub_rn(v[0].x, v[2].x), __dsub_rn(v[0].y, v[2].y), __dsub_rn(v[0].z, v[2].z)};
-    const D3 W{__dsub_rn(v[1].x, v[0].x), __dsub_rn(v[1].y, v[0].y), __dsub_rn(v[1].z, v[0].z)};
-    st.n = D3{diff2<site::CR_GEN>(U.y, W.z, U.z, W.y), diff2<site::CR_GEN>(U.z, W.x, U.x, W.z),
-              diff2<site::CR_GEN>(U.x, W.y, U.y, W.x)};
-    st.tl = 0;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const D3& p = v[i];
-        const D3& q = v[(i + 1) % 3];
-        if (st.n.x > 0.0) { st.ex[i] = __dsub_rn(p.z, q.z); st.ey[i] = __dsub_rn(q.y, p.y); }
-        else { st.ex[i] = __dsub_rn(q.z, p.z); st.ey[i] = __dsub_rn(p.y, q.y); }
-        st.ed[i] = -sum2<site::D_GEN>(st.ex[i], p.y, st.ey[i], p.z);
-        if (st.ex[i] > 0.0 || (st.ex[i] == 0.0 && st.ey[i] < 0.0)) st.tl |= 1u << i;
-    }
+    return c;
 }
 
-// One (triangle, subspace, tile) candidate: binning membership
-// (traverseTilesForOverlaps, src/voxelizer.cu:980-1033), then
-// generateVoxelization's per-centre work (1344-1462) for the tile's centres
-// inside the subspace.
-__device__ __forceinline__ void solidCandidate(const SolidStage& st, const Batch& b, uint32_t local,
-                                               uint32_t* __restrict__ fill) {
-    const Unit& U = b.units[st.unit];
+__device__ __forceinline__ void solidStage(SolidSlots& st, uint32_t slot, const BinTri& bt, uint32_t unit,
+                                           uint32_t wt) {
+    const D3* v = bt.v;
+    st.v0[0][slot] = v[0].x;
+    st.v0[1][slot] = v[0].y;
+    st.v0[2][slot] = v[0].z;
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        st.lo[a][slot] = bt.vlo[a];
+        st.hi[a][slot] = bt.vhi[a];
+    }
+    st.wt[slot] = wt;
+    st.unit[slot] = unit;
+    const D3 A{__dsub_rn(v[0].x, v[2].x), __dsub_rn(v[0].y, v[2].y), __dsub_rn(v[0].z, v[2].z)};
+    const D3 W{__dsub_rn(v[1].x, v[0].x), __dsub_rn(v[1].y, v[0].y), __dsub_rn(v[1].z, v[0].z)};
+    const D3 n{diff2<site::CR_GEN>(A.y, W.z, A.z, W.y), diff2<site::CR_GEN>(A.z, W.x, A.x, W.z),
+               diff2<site::CR_GEN>(A.x, W.y, A.y, W.x)};
+    st.n[0][slot] = n.x;
+    st.n[1][slot] = n.y;
+    st.n[2][slot] = n.z;
+    st.rn[slot] = divScale(n.x) ? __drcp_rn(n.x) : 0.0;
+    uint32_t flags = (bt.tN > 0.0) == (n.x > 0.0) ? 8u : 0u;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const D3& p = v[i];
+        const D3& q = v[(i + 1) % 3];
+        double ex, ey;
+        if (n.x > 0.0) { ex = __dsub_rn(p.z, q.z); ey = __dsub_rn(q.y, p.y); }
+        else { ex = __dsub_rn(q.z, p.z); ey = __dsub_rn(p.y, q.y); }
+        st.ex[i][slot] = ex;
+        st.ey[i][slot] = ey;
+        st.ed[i][slot] = -sum2<site::D_GEN>(ex, p.y, ey, p.z);
+        if (ex > 0.0 || (ex == 0.0 && ey < 0.0)) flags |= 1u << i;
+    }
+    st.flags[slot] = flags;
+}
+
+// Sets up batch `batch` (whole warp): the slots of its triangles with
+// candidates in order, *off the first candidate of slot `lane` (~0 past the
+// last one).  Returns the number of candidates.
+__device__ __forceinline__ uint32_t solidBatch(SolidSlots& st, const Batch& b, uint32_t batch, uint32_t perWarp,
+                                               uint32_t nWork, uint32_t lane, unsigned long long* mine, uint32_t* off) {
+    const uint32_t wt = batch * perWarp + lane;
+    BinTri bt;
+    uint32_t unit = 0;
+    const uint32_t c = lane < perWarp && wt < nWork ? solidCount(b, wt, bt, &unit) : 0u;
+    *mine += c;
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= (uint32_t)o) incl += t;
+    }
+    const uint32_t used = __ballot_sync(kFull, c != 0u);
+    if (c) {
+        const uint32_t slot = __popc(used & laneMaskLt());
+        st.off[slot] = incl - c;
+        solidStage(st, slot, bt, unit, wt);
+    }
+    __syncwarp();
+    *off = lane < __popc(used) ? st.off[lane] : 0xFFFFFFFFu;
+    return __shfl_sync(kFull, incl, 31);
+}
+
+// Binning membership of a candidate evaluated from the triangle
+// (traverseTilesForOverlaps, src/voxelizer.cu:980-1033): some centre of the
+// tile inside the clipped box passes all three binning edges.
+__device__ __noinline__ bool binMember(const Batch& b, uint32_t unit, uint32_t wt, uint32_t ty, uint32_t tz,
+                                       uint32_t y0, uint32_t y1, uint32_t z0, uint32_t z1) {
+    const Unit& U = b.units[unit];
     const PassGeom& g = U.g;
-    const SplitYZ* __restrict__ splits = b.splits + U.splitBase;
-    const uint32_t nSplits = U.nSplits;
-    uint32_t* __restrict__ toggles = fill + U.wordBase;
+    BinTri bt;
+    binSetup(U.V, U.I, wt - __ldg(b.workBase + unit), g, bt);
     const double d = g.d;
-    uint32_t lo[2] = {0, 0}, hi[2] = {0, 0};
-    SplitYZ sp = splits[0];
-    for (uint32_t s = 0; s < nSplits; ++s) {
-        if (!commonSpace(st.b, splits[s], lo, hi)) continue;
-        const uint32_t nty = (hi[0] - 1) / 4 - lo[0] / 4 + 1, ntz = (hi[1] - 1) / 4 - lo[1] / 4 + 1;
-        if (local < nty * ntz) { sp = splits[s]; break; }
-        local -= nty * ntz;
-    }
-    const uint32_t nty = (hi[0] - 1) / 4 - lo[0] / 4 + 1;
-    const uint32_t tileY = lo[0] / 4 + local % nty, tileZ = lo[1] / 4 + local / nty;
-    // Unfused edge functions (the pinned forms of E_BIN and E_GEN) keep the
-    // product of the row's coordinate across the row: the same operations
-    // in the same order as evaluating each centre from scratch.
-    static_assert(site::E_BIN == 0 && site::E_GEN == 0, "row products assume the unfused edge forms");
-    static_assert(site::P_BIN == 0, "corner test assumes the unfused centre form");
-    // Every operation of an unfused binning edge function is monotone in the
-    // centre's row and column (d > 0), so its largest value over the tile's
-    // centres is at the corner its normal points to: a tile where one edge
-    // is negative even there has no member centre.
-    {
-        const uint32_t y0 = max(tileY * 4, lo[0]), y1 = min(tileY * 4 + 4, hi[0]);
-        const uint32_t z0 = max(tileZ * 4, lo[1]), z1 = min(tileZ * 4 + 4, hi[1]);
+    double ex[3], ey[3], ed[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const double py = lin<site::P_BIN>((double)(st.bnx[k] > 0.0 ? y1 - 1 : y0), d, g.mn[1]);
-            const double pz = lin<site::P_BIN>((double)(st.bny[k] > 0.0 ? z1 - 1 : z0), d, g.mn[2]);
-            if (__dadd_rn(__dadd_rn(__dmul_rn(st.bnx[k], py), __dmul_rn(st.bny[k], pz)), st.bd[k]) < 0.0) return;
-        }
+    for (int i = 0; i < 3; ++i) {
+        const D3& p = bt.v[i];
+        const D3& q = bt.v[(i + 1) % 3];
+        if (bt.tN > 0.0) { ex[i] = __dsub_rn(p.z, q.z); ey[i] = __dsub_rn(q.y, p.y); }
+        else { ex[i] = __dsub_rn(q.z, p.z); ey[i] = __dsub_rn(p.y, q.y); }
+        ed[i] = -sum2<site::D_BIN>(ex[i], p.y, ey[i], p.z);
     }
-    bool member = false;
-    for (uint32_t iy = tileY * 4; iy < tileY * 4 + 4 && iy < hi[0] && !member; ++iy) {
-        if (iy < lo[0]) continue;
-        const double py = lin<site::P_BIN>((double)iy, d, g.mn[1]);
-        double ry[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ry[k] = __dmul_rn(st.bnx[k], py);
-        for (uint32_t iz = tileZ * 4; iz < tileZ * 4 + 4 && iz < hi[1]; ++iz) {
-            if (iz < lo[1]) continue;
-            const double pz = lin<site::P_BIN>((double)iz, d, g.mn[2]);
+    for (uint32_t iz = max(tz, z0); iz < min(tz + 4u, z1); ++iz) {
+        const double pz = lin<site::P_BIN>((double)iz, d, g.mn[2]);
+        for (uint32_t iy = max(ty, y0); iy < min(ty + 4u, y1); ++iy) {
+            const double py = lin<site::P_BIN>((double)iy, d, g.mn[1]);
             bool ok = true;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) ok &= __dadd_rn(__dadd_rn(ry[k], __dmul_rn(st.bny[k], pz)), st.bd[k]) >= 0.0;
-            if (ok) { member = true; break; }
+            for (int i = 0; i < 3; ++i) ok &= sum2p1<site::E_BIN>(ex[i], py, ey[i], pz, ed[i]) >= 0.0;
+            if (ok) return true;
         }
     }
-    if (!member) return;
-    const D3* v = st.b.v;
-    for (uint32_t cz = 0; cz < 4; ++cz) {
-        const uint32_t vz = tileZ * 4 + cz;
-        if (vz < sp.z0 || vz >= sp.z1) continue;
-        const double pz = lin<site::P_GEN>((double)vz, d, g.mn[2]);
+    return false;
+}
+
+// Candidate `local` of a slot: the centres it toggles (bits 4 * cz + cy of
+// the tile at *ty, *tz; generateVoxelization, src/voxelizer.cu:1344-1440).
+//
+// The generation edges r > 0 (top-left: r + DBL_MIN > 0, i.e. r > -DBL_MIN)
+// imply the binning edges r >= 0 where both sets have the same orientation,
+// so a generating centre inside the clipped box makes the candidate a
+// member, and a candidate without generating centres needs no membership.
+// Only the rest (rounding at degenerate triangles) evaluates the binning
+// edges.
+__device__ __forceinline__ uint32_t solidCandidate(const SolidSlots& st, uint32_t slot, const Batch& b, uint32_t local,
+                                                   uint32_t* ty, uint32_t* tz) {
+    const Unit& U = b.units[st.unit[slot]];
+    const PassGeom& g = U.g;
+    const SplitYZ* __restrict__ splits = b.splits + U.splitBase;
+    BinTri box;
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        box.vlo[a] = st.lo[a][slot];
+        box.vhi[a] = st.hi[a][slot];
+    }
+    uint32_t lo[2] = {0, 0}, hi[2] = {1, 1};
+    SplitYZ sp = splits[0];
+    for (uint32_t s = 0; s < U.nSplits; ++s) {
+        const SplitYZ q = splits[s];
+        if (!commonSpace(box, q, lo, hi)) continue;
+        const uint32_t n = ((hi[0] - 1) / 4 - lo[0] / 4 + 1) * ((hi[1] - 1) / 4 - lo[1] / 4 + 1);
+        sp = q;
+        if (local < n) break;
+        local -= n;
+    }
+    const uint32_t nty = (hi[0] - 1) / 4 - lo[0] / 4 + 1;
+    const uint32_t row = local / nty;
+    const uint32_t y = (lo[0] / 4 + (local - row * nty)) * 4, z = (lo[1] / 4 + row) * 4;
+    *ty = y;
+    *tz = z;
+    static_assert(site::E_BIN == 0 && site::E_GEN == 0, "row products assume the unfused edge forms");
+    static_assert(site::P_BIN == site::P_GEN && site::D_BIN == site::D_GEN, "shared edges assume the same forms");
+    const double d = g.d, my = g.mn[1], mz = g.mn[2];
+    const uint32_t flags = st.flags[slot];
+    // The products of the edges with the four columns' coordinates are kept
+    // (the same unfused operations as from scratch).
+    double least[3], ed[3], ry[3][4];
+    {
+        double py[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) py[c] = lin<site::P_GEN>(toDouble(y + c), d, my);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double ex = st.ex[i][slot];
+            ed[i] = st.ed[i][slot];
+            least[i] = (flags >> i) & 1u ? -kDblMin : 0.0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ry[i][c] = __dmul_rn(ex, py[c]);
+        }
+    }
+    uint32_t gen = 0;
+#pragma unroll
+    for (int cz = 0; cz < 4; ++cz) {
+        const double pz = lin<site::P_GEN>(toDouble(z + cz), d, mz);
         double rz[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) rz[i] = __dmul_rn(st.ey[i], pz);
-        for (uint32_t cy = 0; cy < 4; ++cy) {
-            const uint32_t vy = tileY * 4 + cy;
-            if (vy < sp.y0 || vy >= sp.y1) continue;
-            const double py = lin<site::P_GEN>((double)vy, d, g.mn[1]);
-            int pass = 0;
+        for (int i = 0; i < 3; ++i) rz[i] = __dmul_rn(st.ey[i][slot], pz);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                double r = __dadd_rn(__dadd_rn(__dmul_rn(st.ex[i], py), rz[i]), st.ed[i]);
-                if ((st.tl >> i) & 1u) r = __dadd_rn(r, kDblMin);
-                pass += r > 0.0;
-            }
-            if (pass != 3) continue;
-            const double ax = __dsub_rn(v[0].x, g.mn[0]), ay = __dsub_rn(v[0].y, py), az = __dsub_rn(v[0].z, pz);
-            const double B = sum3<site::B_GEN>(ax, st.n.x, ay, st.n.y, az, st.n.z);
-            double px = __ddiv_rn(B, st.n.x);
-            px = px < 0.0 ? 0.0 : px;
-            const uint32_t vx = __double2uint_rz(ceil(__ddiv_rn(px, d))) + 1u;
-            if (vx >= g.X) continue;
-            const uint32_t row = (vz + g.padZ) * g.AY + (vy + g.padY);
-            atomicXor(toggles + (size_t)row * g.ipx + (vx >> 5), 0x80000000u >> (vx & 31u));
+        for (int cy = 0; cy < 4; ++cy) {
+            bool in = true;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) in &= __dadd_rn(__dadd_rn(ry[i][cy], rz[i]), ed[i]) > least[i];
+            if (in) gen |= 1u << (4 * cz + cy);
         }
+    }
+    gen &= clipTile(y, z, sp.y0, sp.y1, sp.z0, sp.z1);
+    if (gen && !((flags & 8u) && (gen & clipTile(y, z, lo[0], hi[0], lo[1], hi[1]))) &&
+        !binMember(b, st.unit[slot], st.wt[slot], y, z, lo[0], hi[0], lo[1], hi[1]))
+        gen = 0u;
+    return gen;
+}
+
+// The grid word and bit that centre (vy, vz) toggles for a slot's triangle
+// (src/voxelizer.cu:1441-1462); a zero bit past the grid.  Straight-line but
+// for operands divBy does not take, so that two toggles of a lane overlap.
+struct Toggle {
+    uint32_t* word;
+    uint32_t bit;
+};
+__device__ __forceinline__ Toggle solidToggle(const SolidSlots& st, uint32_t slot, const Batch& b, uint32_t vy,
+                                              uint32_t vz, uint32_t* __restrict__ fill) {
+    const Unit& U = b.units[st.unit[slot]];
+    const PassGeom& g = U.g;
+    const double d = g.d, rd = g.rd;
+    const double py = lin<site::P_GEN>(toDouble(vy), d, g.mn[1]), pz = lin<site::P_GEN>(toDouble(vz), d, g.mn[2]);
+    const double nx = st.n[0][slot], rn = st.rn[slot];
+    const double ax = __dsub_rn(st.v0[0][slot], g.mn[0]), ay = __dsub_rn(st.v0[1][slot], py),
+                 az = __dsub_rn(st.v0[2][slot], pz);
+    const double B = sum3<site::B_GEN>(ax, nx, ay, st.n[1][slot], az, st.n[2][slot]);
+    double px = divBy(B, nx, rn);
+    px = px < 0.0 ? 0.0 : px;
+    double x = divBy(px, d, rd);
+    if (rn == 0.0 || rd == 0.0 || !divExact(B) || !divExact(px)) {
+        px = divide(B, nx);
+        px = px < 0.0 ? 0.0 : px;
+        x = divide(px, d);
+    }
+    const uint32_t vx = __double2uint_rz(ceil(x)) + 1u;
+    const uint32_t row = (vz + g.padZ) * g.AY + (vy + g.padY);
+    return Toggle{fill + U.wordBase + (size_t)row * g.ipx + (vx >> 5), vx < g.X ? 0x80000000u >> (vx & 31u) : 0u};
+}
+
+// Candidates [first, last) of a warp's slots (whole warp; `off` as
+// solidBatch leaves it).  Each step tests the tiles of 32 candidates, queues
+// the centres that toggle and then works the queue 32 centres at a time, so
+// that the divisions of the intercept run in full warps although a tile
+// toggles 2-3 of its 16 centres on average.
+__device__ __forceinline__ void solidCandidates(SolidSlots& st, const Batch& b, uint32_t off, uint32_t first,
+                                                uint32_t last, uint32_t lane, uint32_t* __restrict__ fill) {
+    for (uint32_t base = first; base < last; base += 32u) {
+        // Every slot has a candidate, so the slots that start inside the
+        // window are consecutive.
+        const uint32_t s0 = __popc(__ballot_sync(kFull, off <= base)) - 1u;
+        const uint32_t starts = __reduce_or_sync(kFull, off > base && off - base < 32u ? 1u << (off - base) : 0u);
+        uint32_t slot = s0 + __popc(starts & ((2u << lane) - 1u));
+        const uint32_t o = __shfl_sync(kFull, off, slot);
+        const uint32_t item = base + lane;
+        uint32_t gen = 0, ty = 0, tz = 0;
+        if (item < last) gen = solidCandidate(st, slot, b, item - o, &ty, &tz);
+        // Queue positions: exclusive prefix of the lanes' centre counts.
+        uint32_t n = __popc(gen), incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= (uint32_t)o) incl += t;
+        }
+        const uint32_t total = __shfl_sync(kFull, incl, 31);
+        uint32_t at = incl - n;
+        while (gen) {
+            st.queue[at++] = (uint16_t)((lane << 4) | (__ffs(gen) - 1));
+            gen &= gen - 1u;
+        }
+        __syncwarp();
+        for (uint32_t q = 0; q < total; q += 64u) {
+            const bool in0 = q + lane < total, in1 = q + 32u + lane < total;
+            const uint32_t e0 = st.queue[in0 ? q + lane : 0u], e1 = st.queue[in1 ? q + 32u + lane : 0u];
+            const uint32_t s0 = __shfl_sync(kFull, slot, e0 >> 4), s1 = __shfl_sync(kFull, slot, e1 >> 4);
+            const uint32_t y0 = __shfl_sync(kFull, ty, e0 >> 4), y1 = __shfl_sync(kFull, ty, e1 >> 4);
+            const uint32_t z0 = __shfl_sync(kFull, tz, e0 >> 4), z1 = __shfl_sync(kFull, tz, e1 >> 4);
+            const Toggle t0 = solidToggle(st, s0, b, y0 + (e0 & 3u), z0 + ((e0 >> 2) & 3u), fill);
+            if (q + 32u < total) {
+                const Toggle t1 = solidToggle(st, s1, b, y1 + (e1 & 3u), z1 + ((e1 >> 2) & 3u), fill);
+                if (in1 && t1.bit) atomicXor(t1.word, t1.bit);
+            }
+            if (in0 && t0.bit) atomicXor(t0.word, t0.bit);
+        }
+        __syncwarp();
     }
 }
 
-__global__ void __launch_bounds__(kBlock, 3) solidToggleKernel(Batch b, uint32_t nWork,
-                                                               const uint32_t* __restrict__ offsets,
-                                                               const uint32_t* __restrict__ totalPtr,
-                                                               uint32_t* __restrict__ fill, uint32_t* queue) {
-    __shared__ SolidStage stage[kSlots];
-    __shared__ uint32_t stOff[kSlots + 1];
-    __shared__ uint32_t tFirst, tLast, nextBase;
-    const uint32_t total = *totalPtr;
-    // Batches of kBlock candidates in a fixed grid-stride order, or
-    // (queue != NULL) taken from a device work queue, one atomic per batch.
-    uint32_t base = blockIdx.x * kBlock;
-    if (queue) {
-        if (threadIdx.x == 0) nextBase = atomicAdd(queue, kBlock);
-        __syncthreads();
-        base = nextBase;
+// Toggles of every work triangle.  A warp takes batches of `perWarp` (a
+// power of two up to 32) triangles in a fixed grid-stride order or (queue !=
+// NULL) from a device work queue, one atomic per batch.  The chunks after the
+// first of a batch with more than kSplit candidates are appended to `big`
+// (batch << 32 | chunk).  *total counts the candidates.
+__global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch b, uint32_t nWork, uint32_t perWarp,
+                                                                          unsigned long long* total,
+                                                                          unsigned long long* big, uint32_t* bigCount,
+                                                                          uint32_t bigCap, uint32_t* __restrict__ fill,
+                                                                          uint32_t* queue) {
+    __shared__ SolidSlots slots[kWarps];
+    const uint32_t lane = threadIdx.x & 31u;
+    SolidSlots& st = slots[threadIdx.x >> 5];
+    const uint32_t batches = (nWork + perWarp - 1) / perWarp;
+    const uint32_t nWarps = gridDim.x * kWarps;
+    unsigned long long mine = 0;
+    uint32_t bt = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    auto take = [&]() {
+        uint32_t v = 0;
+        if (lane == 0) v = atomicAdd(queue, 1u);
+        return __shfl_sync(kFull, v, 0);
+    };
+    if (queue) bt = take();
+    while (bt < batches) {
+        uint32_t off;
+        uint32_t n = solidBatch(st, b, bt, perWarp, nWork, lane, &mine, &off);
+        if (n > kSplit && big) {
+            const uint32_t more = (n - 1u) / kChunk;   // chunks 1 .. more
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(bigCount, more);
+            at = __shfl_sync(kFull, at, 0);
+            // A list without room for all of them leaves the batch to this
+            // warp; the entries it reserved are marked as empty.
+            const bool fits = at < bigCap && more <= bigCap - at;
+            for (uint32_t k = lane; k < more && at < bigCap && k < bigCap - at; k += 32u)
+                big[at + k] = fits ? ((unsigned long long)bt << 32) | (k + 1u) : ~0ull;
+            if (fits) n = kChunk;
+        }
+        solidCandidates(st, b, off, 0u, n, lane, fill);
+        bt = queue ? take() : bt + nWarps;
     }
-    while (base < total) {
-        const uint32_t last = min(base + kBlock, total) - 1;
-        // Owners of the batch's first and last items, one warp each.
-        if (threadIdx.x < 64) {
-            const uint32_t t = warpFindOwner(offsets, nWork, threadIdx.x < 32 ? base : last, threadIdx.x & 31u);
-            if (threadIdx.x == 0) tFirst = t;
-            if (threadIdx.x == 32) tLast = t;
-        }
-        __syncthreads();
-        const uint32_t t0 = tFirst, t1 = tLast, ns = min(t1 - t0 + 1, kSlots);
-        // Triangles without candidates between them are never selected
-        // (their offset equals the next one) and are not staged.
-        if (threadIdx.x < ns) {
-            const uint32_t o = __ldg(offsets + t0 + threadIdx.x);
-            stOff[threadIdx.x] = o;
-            if (__ldg(offsets + t0 + threadIdx.x + 1) > o) stageSolid(stage[threadIdx.x], b, t0 + threadIdx.x);
-        }
-        if (threadIdx.x == 0) stOff[ns] = __ldg(offsets + t0 + ns);
-        __syncthreads();
-        const uint32_t item = base + threadIdx.x;
-        if (item <= last) {
-            if (item < stOff[ns]) {
-                uint32_t lo = 0, hi = ns;  // stOff[lo] <= item < stOff[hi]
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (stOff[mid] <= item) lo = mid;
-                    else hi = mid;
-                }
-                solidCandidate(stage[lo], b, item - stOff[lo], fill);
-            } else {
-                // The owner lies past the staged triangles and at most at
-                // the batch's last owner: offsets[t0 + ns] <= item <
-                // offsets[t1 + 1].
-                uint32_t lo = t0 + ns, hi = t1 + 1;
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (__ldg(offsets + mid) <= item) lo = mid;
-                    else hi = mid;
-                }
-                const uint32_t wt = lo;
-                SolidStage st;
-                stageSolid(st, b, wt);
-                solidCandidate(st, b, item - __ldg(offsets + wt), fill);
-            }
-        }
-        if (queue && threadIdx.x == 0) nextBase = atomicAdd(queue, kBlock);
-        __syncthreads();
-        base = queue ? nextBase : base + gridDim.x * kBlock;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mine += __shfl_down_sync(kFull, mine, o);
+    if (lane == 0 && mine) atomicAdd(total, mine);
+}
+
+// The listed chunks, one warp each.
+__global__ void __launch_bounds__(kWarps * 32, kBlocks) solidBigKernel(Batch b, uint32_t nWork, uint32_t perWarp,
+                                                                       const unsigned long long* __restrict__ big,
+                                                                       const uint32_t* __restrict__ bigCount,
+                                                                       uint32_t bigCap, uint32_t* __restrict__ fill) {
+    __shared__ SolidSlots slots[kWarps];
+    const uint32_t lane = threadIdx.x & 31u;
+    SolidSlots& st = slots[threadIdx.x >> 5];
+    const uint32_t entries = min(*bigCount, bigCap);
+    for (uint32_t e = blockIdx.x * kWarps + (threadIdx.x >> 5); e < entries; e += gridDim.x * kWarps) {
+        const unsigned long long ent = big[e];
+        if (ent == ~0ull) continue;
+        unsigned long long mine = 0;
+        uint32_t off;
+        const uint32_t n = solidBatch(st, b, (uint32_t)(ent >> 32), perWarp, nWork, lane, &mine, &off);
+        const uint32_t first = (uint32_t)ent * kChunk;
+        solidCandidates(st, b, off, first, min(n - first, kChunk) + first, lane, fill);
     }
 }
 
@@ -362,16 +540,32 @@ __global__ void rowFillKernel(Batch b, uint64_t nRows, uint32_t* __restrict__ fi
 
 }  // namespace
 
-void launch_solid_count(const Batch& b, uint32_t nWork, uint32_t* counts, cudaStream_t s, uint32_t* launches) {
-    solidCountKernel<<<gridFor(nWork, 256), 256, 0, s>>>(b, nWork, counts);
-    *launches += 1;
+// Triangles per batch: 32 lanes set up 32, but a small mesh is spread over 8
+// warps per SM first (one triangle per warp at the least).
+static uint32_t solidPerWarp(uint32_t nWork) {
+    uint32_t n = 1;
+    while (n < 32u && nWork / (2u * n) >= 148u * 8u) n *= 2u;
+    return n;
 }
 
-void launch_solid_toggle(const Batch& b, uint32_t nWork, const uint32_t* offsets, const uint32_t* total,
-                         uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue, cudaStream_t s, uint32_t* launches) {
+bool solid_may_list(const PassGeom& g, uint64_t nSplits, uint32_t nWork) {
+    // A triangle has at most one candidate per 4x4 tile and one more row and
+    // column of partial tiles per subspace cut.
+    return ((g.resY + 3ull) / 4 + nSplits) * ((g.resZ + 3ull) / 4 + nSplits) * solidPerWarp(nWork) > kSplit;
+}
+
+void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, unsigned long long* big,
+                         uint32_t* bigCount, uint32_t bigCap, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
+                         cudaStream_t s, uint32_t* launches) {
+    const uint32_t perWarp = solidPerWarp(nWork), batches = (nWork + perWarp - 1) / perWarp;
     if (queue) cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
-    solidToggleKernel<<<148u * blocksPerSm, kBlock, 0, s>>>(b, nWork, offsets, total, fill, queue);
+    const uint32_t grid = gridFor(batches, kWarps, 148u * 8u * blocksPerSm);
+    solidToggleKernel<<<grid, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, big, bigCount, bigCap, fill, queue);
     *launches += 1;
+    if (big) {
+        solidBigKernel<<<148 * kBlocks, kWarps * 32, 0, s>>>(b, nWork, perWarp, big, bigCount, bigCap, fill);
+        *launches += 1;
+    }
 }
 
 void launch_row_fill(const Batch& b, uint64_t nRows, uint32_t* fill, cudaStream_t s, uint32_t* launches) {
