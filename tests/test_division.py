@@ -6,6 +6,7 @@ per operation, as the fused operations round."""
 import random
 from fractions import Fraction
 
+import numpy as np
 import pytest
 
 
@@ -44,3 +45,22 @@ def test_quotient_is_correctly_rounded(scale):
             for s in (x, -x * 2.0 ** scale):
                 assert _div_by(s, d) == s / d
     assert _div_by(0.0, ds[0]) == 0.0
+
+
+def test_division_by_multiplication():
+    """FastDiv (csrc/vxb_kernels.cuh) restated: n * m >> (27 + L) is n // d for
+    every n below 2^27, with m << 4 in 32 bits."""
+    rng = np.random.default_rng(1)
+    ds = np.unique(np.concatenate([np.arange(2, 300), 2 ** np.arange(1, 27), 2 ** np.arange(2, 27) + 1,
+                                   2 ** np.arange(2, 27) - 1, rng.integers(2, 1 << 27, 500)]))
+    for d in (int(x) for x in ds):
+        L = 1
+        while L < 27 and (1 << L) < d:
+            L += 1
+        mul = ((1 << (27 + L)) // d + 1) << 4
+        assert mul < 1 << 32
+        top = (1 << 27) - 1
+        q = top // d
+        for n in {0, 1, d - 1, d, d + 1, top, q * d - 1, q * d, *(int(x) for x in rng.integers(0, 1 << 27, 20))}:
+            if 0 <= n <= top:
+                assert ((n * mul) >> 32) >> (L - 1) == n // d

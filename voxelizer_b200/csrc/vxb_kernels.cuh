@@ -15,6 +15,27 @@
 
 namespace vxb {
 
+// Division of word and row numbers below 2^27 (a grid holds fewer than 2^32
+// voxels) by a constant d: with 2^L >= d, m = floor(2^(27 + L) / d) + 1
+// exceeds the exact reciprocal by less than 2^-27 of itself, so n * m >> (27 +
+// L) is n / d for n < 2^27 (Granlund and Montgomery 1994).  mul holds m << 4,
+// which leaves a shift of L - 1 after the high word; d = 1 has mul 0.
+struct FastDiv {
+    uint32_t mul, shift;
+    static FastDiv of(uint32_t d) {
+        FastDiv f{0u, 0u};
+        if (d <= 1u) return f;
+        uint32_t L = 1;
+        while (L < 27u && (1u << L) < d) ++L;
+        f.mul = (uint32_t)(((1ull << (27 + L)) / d + 1ull) << 4);
+        f.shift = L - 1u;
+        return f;
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ uint32_t div(uint32_t n) const { return mul ? __umulhi(n, mul) >> shift : n; }
+#endif
+};
+
 // Geometry of one unit.  For FCC lattices each of the four sub-lattices has
 // its own shifted minimum corner.
 struct PassGeom {
@@ -30,6 +51,7 @@ struct PassGeom {
     uint32_t padY, padZ; // allocation row / plane of local voxel row / plane 0 (1, or 0 next to a neighbour)
     uint32_t border;     // zero the allocation's faces in the node output (a device space with neighbours)
     uint32_t pad0;
+    FastDiv divX, divY;  // by ipx and by AY
 };
 
 struct SplitYZ { uint32_t y0, y1, z0, z1; };
@@ -140,42 +162,24 @@ int meshCheck(const float* dV, uint32_t nV, const uint32_t* dI, uint64_t nIdx, u
               unsigned long long* hostOut, cudaStream_t s);
 
 // ---- Node classification: src/voxelizer.cu:1626-2048 ----
-void launch_combine(const uint32_t* a, const uint32_t* b, uint32_t* out, uint64_t n, cudaStream_t s,
-                    uint32_t* launches);
-
-// One pruning region: subspace `split` of unit `unit`.  wordStart is the
-// exclusive prefix of region words within one launch.
-struct PruneRegion {
-    uint32_t unit;
-    SplitYZ split;
-    uint32_t wordStart;
-};
-// Pruning of one subspace index.  launch_prune: the first pass over every
-// word of its `n` regions (groupWords words in all), appending each changed
-// word to `list`; launch_prune_list: a later pass over the words next to the
-// changes listed in `in`, appending its own changes to `out`.  Lists hold
-// (region << 32 | word) entries, at most `cap`; past it *overflow is set and
-// the passes are no longer complete.  A region that changed in pass p sets
-// flags[(flagBase + region) * passes + p].  Neighbours in later subspaces
-// are read from fill | surf (surf may be NULL).
-void launch_prune(const Batch& b, const PruneRegion* regions, uint32_t n, uint32_t groupWords, uint32_t* solid,
-                  const uint32_t* fill, const uint32_t* surf, uint32_t* flags, uint32_t flagBase, uint32_t passes,
-                  unsigned long long* list, uint32_t* count, uint32_t cap, uint32_t* overflow, cudaStream_t s,
-                  uint32_t* launches);
-// Passes firstPass .. passes - 1 of one subspace index in one block-sized
-// launch (lists alternating between list0 and list1, counts[p] the count of
-// pass p); it stops at an empty list, and a list longer than escapeAt marks
-// all nRegions regions as changed in the last pass (the host then runs full
-// passes until stable).
-void launch_prune_list_loop(const Batch& b, const PruneRegion* regions, uint32_t nRegions, uint32_t* solid,
-                            const uint32_t* fill, const uint32_t* surf, uint32_t* flags, uint32_t flagBase,
-                            uint32_t passes, uint32_t firstPass, unsigned long long* list0, unsigned long long* list1,
-                            uint32_t* counts, uint32_t cap, uint32_t escapeAt, uint32_t* overflow, cudaStream_t s,
-                            uint32_t* launches);
-void launch_prune_list(const Batch& b, const PruneRegion* regions, uint32_t* solid, const uint32_t* fill,
-                       const uint32_t* surf, uint32_t* flags, uint32_t flagBase, uint32_t passes, uint32_t pass,
-                       const unsigned long long* in, const uint32_t* inCount, unsigned long long* out,
-                       uint32_t* outCount, uint32_t cap, uint32_t* overflow, cudaStream_t s, uint32_t* launches);
+// Pruning of every unit (Cartesian node grids): `solid` from fill | surf
+// (surf may be NULL).  counts[p], p < passes, is the length of pass p's
+// change list and *overflow a flag, all zero on entry.  Pass 0 goes over all
+// words, pass 1 over the words it changed (list0), the others in one block
+// with alternating lists of at most `cap` (unit << 32 | word) entries.  The
+// blockBase: exclusive prefix over the units of prune_blocks (nUnits + 1
+// entries) for `planes` = prune_planes(totalWords); `blocks` is their sum.  The
+// grid is pruned unless counts[passes - 1] or *overflow is set (a list longer
+// than cap or, after pass 1, than escapeAt): then launch_prune_full passes,
+// which set *changed, finish it.
+uint32_t prune_planes(uint64_t totalWords);
+uint32_t prune_blocks(const PassGeom& g, uint32_t planes);
+void launch_prune(const Batch& b, uint64_t totalWords, const uint32_t* blockBase, uint32_t blocks, uint32_t planes,
+                  uint32_t* solid, const uint32_t* fill, const uint32_t* surf, uint32_t passes,
+                  unsigned long long* list0, unsigned long long* list1, uint32_t* counts, uint32_t cap,
+                  uint32_t escapeAt, uint32_t* overflow, cudaStream_t s, uint32_t* launches);
+void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, const uint32_t* fill,
+                       const uint32_t* surf, uint32_t* changed, cudaStream_t s, uint32_t* launches);
 // Slices along x (vxb_xslice.cu): vertex rotation, the node array before
 // the boundary ids, un-rotation, one in-place boundary-id pass over a yz
 // subspace (sets *changed when a node loses its id) and face zeroing.  The

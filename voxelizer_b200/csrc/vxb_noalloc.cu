@@ -234,6 +234,8 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     g.padY = 1;
     g.padZ = 1;
     g.border = 0;
+    g.divX = vxb::FastDiv::of(g.ipx);
+    g.divY = vxb::FastDiv::of(g.AY);
     uint32_t* checkedIdx = reinterpret_cast<uint32_t*>(scratch + kIndexOff);
     tab.unit.V = dev_vertices;
     tab.unit.I = checkedIdx;

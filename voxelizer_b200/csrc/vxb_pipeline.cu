@@ -2,11 +2,10 @@
 //
 // All units of a batch go through each stage in one launch: solid
 // voxelization, surface voxelization with its hit list and ranks,
-// split-ordered pruning, material merge and node emission.  Pruning runs
-// kPasses speculative passes per subspace index (for all units at once,
-// each region skipping passes once it stops changing); the host checks the
-// flags after the batch and adds passes only where a region had not
-// converged.
+// split-ordered pruning, material merge and node emission.  Pruning queues
+// kPasses passes (the later ones over lists of changed words, ending with an
+// empty list); the host checks their counts after the batch and adds passes
+// only where they had not converged.
 
 #include "vxb_pipeline.h"
 
@@ -22,7 +21,8 @@ namespace {
 // Slots of the status buffer; pruning flags follow at kFlags.
 // kSolidTotal and kSolidHigh are the low and high word of one 64-bit count.
 enum : int { kSolidTotal = 0, kSolidHigh = 1, kSurfTotal = 2, kSurfOverflow = 3, kHitCount = 4,
-             kSurfaceVoxels = 5, kSurfQueue = 6, kToggleQueue = 7, kBigCount = 8, kFlags = 10 };
+             kSurfaceVoxels = 5, kSurfQueue = 6, kToggleQueue = 7, kBigCount = 8, kPruneOverflow = 9,
+             kPruneCounts = 10 };
 
 // The work counts take 32 bits: totals of 2^32 - 1 or more are refused.
 bool solidOverflow(const uint32_t* h) { return h[kSolidHigh] || h[kSolidTotal] == 0xFFFFFFFFu; }
@@ -105,6 +105,8 @@ PassGeom makeGeom(const Plan& p, int lattice, bool turned) {
     g.padZ = p.padZ;
     g.border = p.border ? 1u : 0u;
     g.pad0 = 0;
+    g.divX = FastDiv::of(g.ipx);
+    g.divY = FastDiv::of(g.AY);
     return g;
 }
 
@@ -150,13 +152,11 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
         if ((j.raw != 0) != raw_ || (raw_ && !j.nodes))
             return failf(VXB_EINVAL, "raw node output is for node grids of a whole batch");
     units_.clear();
-    groups_.clear();
     std::vector<uint32_t> workBase{0};
     std::vector<uint64_t> rowBase{0}, wordBase{0};
     std::vector<SplitYZ> splits;
     std::vector<uint32_t> slices;
     std::vector<uint8_t> later;
-    std::vector<std::vector<PruneRegion>> regionsBySplit;
     std::vector<FccMesh> fccMeshes;
     std::vector<uint64_t> groupBase{0};
     anyMaterials_ = false;
@@ -220,19 +220,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
                 return failf(VXB_EOVERFLOW, "batch of more than 2^32 work triangles");
             workBase.push_back(workBase.back() + j.nT);
             units_.push_back(u);
-            if (j.nodes && !fcc) {
-                anyCartesian_ = true;
-                size_t k = 0;
-                for (const auto& z : p.zSplitsAlloc)
-                    for (const auto& y : p.ySplitsAlloc) {
-                        if (regionsBySplit.size() <= k) regionsBySplit.resize(k + 1);
-                        PruneRegion r;
-                        r.unit = firstUnit + (uint32_t)l;
-                        r.split = SplitYZ{y.lo, y.hi, z.lo, z.hi};
-                        r.wordStart = 0;
-                        regionsBySplit[k++].push_back(r);
-                    }
-            }
+            anyCartesian_ |= j.nodes && !fcc;
         }
         if (j.nodes && fcc) {
             fccMeshes.push_back(FccMesh{firstUnit, j.out});
@@ -244,25 +232,16 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     totalRows_ = rowBase.back();
     nFcc_ = (uint32_t)fccMeshes.size();
     totalGroups_ = groupBase.back();
-    // Pruning regions, grouped by subspace index.
-    std::vector<PruneRegion> regions;
-    for (auto& grp : regionsBySplit) {
-        Group gr;
-        gr.first = (uint32_t)regions.size();
-        gr.count = (uint32_t)grp.size();
-        gr.flagBase = gr.first;
-        uint64_t words = 0;
-        for (PruneRegion& r : grp) {
-            r.wordStart = (uint32_t)words;
-            const Unit& u = units_[r.unit];
-            words += (uint64_t)(r.split.y1 - r.split.y0) * (r.split.z1 - r.split.z0) * u.g.ipx;
-            regions.push_back(r);
+    // Blocks of the first pruning pass.
+    std::vector<uint32_t> pruneBase{0};
+    prunePlanes_ = prune_planes(totalWords_);
+    if (anyCartesian_)
+        for (const Unit& u : units_) {
+            const uint64_t blocks = (uint64_t)pruneBase.back() + prune_blocks(u.g, prunePlanes_);
+            if (blocks > 0x7FFFFFFFull) return failf(VXB_EOVERFLOW, "pruning launch of more than 2^31 blocks");
+            pruneBase.push_back((uint32_t)blocks);
         }
-        if (words > 0xFFFFFFFFull) return failf(VXB_EOVERFLOW, "pruning launch of more than 2^32 words");
-        gr.words = (uint32_t)words;
-        groups_.push_back(gr);
-    }
-    nRegions_ = (uint32_t)regions.size();
+    pruneBlocks_ = pruneBase.back();
     // A single plain voxelization writes its solid grid straight into the
     // caller's buffer.
     aliasFill_ = !nodes_ && jobs.size() == 1;
@@ -275,14 +254,14 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     oSplits_ = append(blob_, splits);
     oSlices_ = append(blob_, slices);
     oLater_ = append(blob_, later);
-    oRegions_ = append(blob_, regions);
+    oPrune_ = append(blob_, pruneBase);
     oFcc_ = append(blob_, fccMeshes);
     oGroupBase_ = append(blob_, groupBase);
     // Buffers.
     int rc;
     const size_t wordBytes = 4 * (size_t)totalWords_;
     if ((rc = tables.ensure(blob_.size() + 64))) return rc;
-    if ((rc = status.ensure(4 * (kFlags + (size_t)nRegions_ * kPasses) + 256))) return rc;
+    if ((rc = status.ensure(4 * (kPruneCounts + (size_t)kPasses)))) return rc;
     mayList_ = false;
     for (const Unit& u : units_) mayList_ |= solid_may_list(u.g, u.nSplits, nWork_);
     if (mayList_ && (rc = bigList.ensure(8 * (size_t)kBigCap))) return rc;
@@ -291,10 +270,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     // Change lists of the pruning passes: the first pass lists every word it
     // changes (a fraction of the boundary words); past the cap the host
     // finishes pruning with full passes.
-    uint32_t maxGroupWords = 0;
-    for (const Group& gr : groups_) maxGroupWords = std::max(maxGroupWords, gr.words);
-    pruneCap_ = std::max<uint32_t>(4u << 20, maxGroupWords / 4);
-    if (anyCartesian_ && (rc = pruneScratch.ensure(4 * (groups_.size() * kPasses + 1)))) return rc;
+    pruneCap_ = (uint32_t)std::max<uint64_t>(1u << 16, std::min<uint64_t>(totalWords_ / 4, 0x7FFFFFFFull));
     if (anyCartesian_ && (rc = pruneLists.ensure(2 * 8 * (size_t)pruneCap_))) return rc;
     listCap_ = 0;
     mergeEntries_ = 0;
@@ -365,8 +341,8 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     bucket_ = tuneBucket(nWork_, totalWords_, nodeKind_, anyMaterials_);
     shape = tunePick(bucket_, &trial_, cap == cudaStreamCaptureStatusNone);
     for (bool& u : tuneUsed_) u = false;
-    // Work counts, hit count and pruning flags.
-    VXB_CUDA(cudaMemsetAsync(st, 0, 4 * (kFlags + (size_t)nRegions_ * kPasses), s));
+    // Work counts, hit count and pruning counts.
+    VXB_CUDA(cudaMemsetAsync(st, 0, 4 * (kPruneCounts + (size_t)kPasses), s));
     // Surface voxelization, hit list and surface ranks on the side stream,
     // beside the solid pass (they share no buffer).
     cudaStream_t ss = s;
@@ -453,32 +429,10 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
             mergeSpan = true;
         }
         mark(2, false);
-        if (anyMaterials_)
-            launch_combine(fillP, surf.as<uint32_t>(), fin.as<uint32_t>(), totalWords_, ps, &launches);
-        else
-            VXB_CUDA(cudaMemcpyAsync(fin.p, fillP, 4 * (size_t)totalWords_, cudaMemcpyDeviceToDevice, ps));
-        // Per subspace index and pass: the count of its change list; the
-        // last word is the list overflow flag.
-        uint32_t* counts = pruneScratch.as<uint32_t>();
-        uint32_t* overflow = counts + groups_.size() * kPasses;
-        VXB_CUDA(cudaMemsetAsync(counts, 0, 4 * (groups_.size() * kPasses + 1), ps));
-        const PruneRegion* regions = reinterpret_cast<const PruneRegion*>(tables.as<uint8_t>() + oRegions_);
-        unsigned long long* lists[2] = {pruneLists.as<unsigned long long>(),
-                                        pruneLists.as<unsigned long long>() + pruneCap_};
-        const uint32_t* surfP = anyMaterials_ ? surf.as<uint32_t>() : nullptr;
-        for (size_t gi = 0; gi < groups_.size(); ++gi) {
-            const Group& gr = groups_[gi];
-            uint32_t* c = counts + gi * kPasses;
-            launch_prune(b, regions + gr.first, gr.count, gr.words, fin.as<uint32_t>(), fillP, surfP, st + kFlags,
-                         gr.flagBase, kPasses, lists[0], c, pruneCap_, overflow, ps, &launches);
-            // Pass 1 over the whole device; later lists are short (usually
-            // empty), so passes 2 .. kPasses - 1 run in one block.
-            launch_prune_list(b, regions + gr.first, fin.as<uint32_t>(), fillP, surfP, st + kFlags, gr.flagBase,
-                              kPasses, 1, lists[0], c, lists[1], c + 1, pruneCap_, overflow, ps, &launches);
-            launch_prune_list_loop(b, regions + gr.first, gr.count, fin.as<uint32_t>(), fillP, surfP, st + kFlags,
-                                   gr.flagBase, kPasses, 2, lists[0], lists[1], c, pruneCap_, kLoopListMax, overflow, ps,
-                                   &launches);
-        }
+        launch_prune(b, totalWords_, reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oPrune_), pruneBlocks_,
+                     prunePlanes_, fin.as<uint32_t>(), fillP, anyMaterials_ ? surf.as<uint32_t>() : nullptr, kPasses,
+                     pruneLists.as<unsigned long long>(), pruneLists.as<unsigned long long>() + pruneCap_,
+                     st + kPruneCounts, pruneCap_, kLoopListMax, st + kPruneOverflow, ps, &launches);
         mark(2, true);
     }
     // Join: emission reads the merged keys.
@@ -534,29 +488,19 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     return 0;
 }
 
-// More passes over one subspace index until no region changes, one full
-// pass at a time with a host check in between.
-int Pipeline::pruneGroupUntilStable(const Group& gr, cudaStream_t s) {
+// Full passes until nothing changes, with a host check after each.
+int Pipeline::pruneUntilStable(cudaStream_t s) {
     const Batch b = batch();
-    uint32_t* st = status.as<uint32_t>();
-    uint32_t* fillP = aliasFill_ ? static_cast<uint32_t*>(jobs_[0].out) : fill.as<uint32_t>();
-    const PruneRegion* regions = reinterpret_cast<const PruneRegion*>(tables.as<uint8_t>() + oRegions_);
-    uint32_t* counts = pruneScratch.as<uint32_t>();
-    uint32_t* overflow = counts + groups_.size() * kPasses;
-    std::vector<uint32_t> h((size_t)gr.count * kPasses);
+    uint32_t* changed = status.as<uint32_t>() + kPruneOverflow;
     for (uint64_t round = 0;; ++round) {
         if (round > (1u << 24)) return failf(VXB_ETIMEDOUT, "pruning did not converge");
-        VXB_CUDA(cudaMemsetAsync(st + kFlags + (size_t)gr.flagBase * kPasses, 0, 4 * h.size(), s));
-        VXB_CUDA(cudaMemsetAsync(counts, 0, 4, s));
-        launch_prune(b, regions + gr.first, gr.count, gr.words, fin.as<uint32_t>(), fillP,
-                     anyMaterials_ ? surf.as<uint32_t>() : nullptr, st + kFlags, gr.flagBase, kPasses,
-                     pruneLists.as<unsigned long long>(), counts, pruneCap_, overflow, s, &launches);
-        VXB_CUDA(cudaMemcpyAsync(h.data(), st + kFlags + (size_t)gr.flagBase * kPasses, 4 * h.size(),
-                                 cudaMemcpyDeviceToHost, s));
+        uint32_t h = 0;
+        VXB_CUDA(cudaMemsetAsync(changed, 0, 4, s));
+        launch_prune_full(b, totalWords_, fin.as<uint32_t>(), fill.as<uint32_t>(),
+                          anyMaterials_ ? surf.as<uint32_t>() : nullptr, changed, s, &launches);
+        VXB_CUDA(cudaMemcpyAsync(&h, changed, 4, cudaMemcpyDeviceToHost, s));
         VXB_CUDA(cudaStreamSynchronize(s));
-        bool changed = false;
-        for (uint32_t r = 0; r < gr.count; ++r) changed |= h[(size_t)r * kPasses] != 0;
-        if (!changed) return 0;
+        if (!h) return 0;
     }
 }
 
@@ -608,8 +552,8 @@ int Pipeline::finish(cudaStream_t s) {
         if (solidOverflow(h)) return failf(VXB_EOVERFLOW, "solid work list exceeds 2^32 entries");
         return 0;
     }
-    std::vector<uint32_t> h(kFlags + (size_t)nRegions_ * kPasses);
-    VXB_CUDA(cudaMemcpyAsync(h.data(), status.p, 4 * h.size(), cudaMemcpyDeviceToHost, s));
+    uint32_t h[kPruneCounts + kPasses];
+    VXB_CUDA(cudaMemcpyAsync(h, status.p, sizeof(h), cudaMemcpyDeviceToHost, s));
     uint32_t bk[kSurfaceBuckets] = {0};
     if (anyMaterials_) VXB_CUDA(cudaMemcpyAsync(bk, buckets.p, sizeof(bk), cudaMemcpyDeviceToHost, s));
     VXB_CUDA(cudaStreamSynchronize(s));
@@ -623,7 +567,7 @@ int Pipeline::finish(cudaStream_t s) {
     stats.surface_voxels = anyMaterials_ ? h[kSurfaceVoxels] : 0;
     for (uint32_t k = 0; k < kSurfaceBuckets; ++k) stats.surface_triangles[k / 3] += bk[k];
     stats.grid_words = totalWords_;
-    if (solidOverflow(h.data()) || (anyMaterials_ && h[kSurfOverflow]))
+    if (solidOverflow(h) || (anyMaterials_ && h[kSurfOverflow]))
         return failf(VXB_EOVERFLOW, "work list exceeds 2^32 entries");
     bool reemit = false;
     const Batch b = batch();
@@ -648,21 +592,10 @@ int Pipeline::finish(cudaStream_t s) {
         }
     }
     if (anyCartesian_ && !raw_) {
-        // The first subspace index with a region that changed in its last
-        // queued pass has not converged; it and every later index (pruned
-        // against a superset of its final state) get passes until stable.
-        uint32_t overflow = 0;
-        VXB_CUDA(cudaMemcpy(&overflow, pruneScratch.as<uint32_t>() + groups_.size() * kPasses, 4,
-                            cudaMemcpyDeviceToHost));
-        size_t first = overflow ? 0 : groups_.size();
-        for (size_t gi = 0; gi < groups_.size() && first == groups_.size(); ++gi)
-            for (uint32_t r = 0; r < groups_[gi].count; ++r)
-                if (h[kFlags + ((size_t)groups_[gi].flagBase + r) * kPasses + kPasses - 1]) {
-                    first = gi;
-                    break;
-                }
-        for (size_t gi = first; gi < groups_.size(); ++gi) {
-            if (int rc = pruneGroupUntilStable(groups_[gi], s)) return rc;
+        // A change list that overflowed, or a last queued pass that still
+        // changed something.
+        if (h[kPruneOverflow] || h[kPruneCounts + kPasses - 1]) {
+            if (int rc = pruneUntilStable(s)) return rc;
             reemit = true;
         }
     }

@@ -92,7 +92,7 @@ public:
     // Counters of the last finish (vxb_last_stats).
     vxb_stats stats{};
 
-    static constexpr uint32_t kPasses = 8;   // pruning passes queued per subspace
+    static constexpr uint32_t kPasses = 16;  // pruning passes queued
     static constexpr uint32_t kLoopListMax = 32768;   // longest list the one-block passes take
     static constexpr uint32_t kBigCap = 1u << 19;       // candidate chunks listed by the solid pass
     static constexpr uint32_t kOutChunks = 4;         // emit / host-copy ranges of streamed output
@@ -116,28 +116,24 @@ private:
     void tuneMark(int knob, bool end, cudaStream_t s);
     void tuneFinish();
 
-    struct Group {            // pruning regions of one subspace index
-        uint32_t first, count, words, flagBase;
-    };
     Batch batch();
-    int pruneGroupUntilStable(const Group& gr, cudaStream_t s);
+    int pruneUntilStable(cudaStream_t s);
 
     std::vector<MeshJob> jobs_;
     std::vector<Unit> units_;
-    std::vector<Group> groups_;
-    uint32_t nWork_ = 0, nRegions_ = 0, nFcc_ = 0;
+    uint32_t nWork_ = 0, nFcc_ = 0, prunePlanes_ = 0, pruneBlocks_ = 0;
     uint64_t totalWords_ = 0, totalRows_ = 0, totalGroups_ = 0;
     int nodeKind_ = 0, nodes_ = 1;
     bool anyMaterials_ = false, anyCartesian_ = false, wide_ = false, aliasFill_ = false, raw_ = false,
          mayList_ = false;
     uint32_t listCap_ = 0, keysCap_ = 0, pruneCap_ = 0, mergeEntries_ = 0;
     // table offsets (bytes) in `tables`
-    size_t oUnits_ = 0, oWork_ = 0, oRow_ = 0, oWord_ = 0, oSplits_ = 0, oSlices_ = 0, oLater_ = 0, oRegions_ = 0,
-           oFcc_ = 0, oGroupBase_ = 0;
+    size_t oUnits_ = 0, oWork_ = 0, oRow_ = 0, oWord_ = 0, oSplits_ = 0, oSlices_ = 0, oLater_ = 0,
+           oPrune_ = 0, oFcc_ = 0, oGroupBase_ = 0;
     std::vector<uint8_t> blob_;   // host copy of the tables (alive while the upload runs)
 
     DevBuf tables, status, bigList;
-    DevBuf fill, surf, fin, ranks, rankTiles, pruneScratch, pruneLists;
+    DevBuf fill, surf, fin, ranks, rankTiles, pruneLists;
     DevBuf codes, unitCounts, buckets, recs, ovl, hitList, keys;
     // The surface pass runs on a second stream beside the solid pass, joined
     // before pruning (surface bits) and before emission (merged keys).
