@@ -131,13 +131,15 @@ void launch_surface_prepare(const Batch& b, uint32_t nWork, uint32_t* codes, uin
 // entries), one thread per column.  mode 0: set bits in the `surf` arena and
 // append (bit position << 24 | key) to `list` (entries past listCap are
 // counted, not stored); mode 1: merge every hit's key at its rank (needs
-// complete bits and their `ranks`).  wide: 64-bit keys (PartialNode).  kind: the
+// complete bits and their `ranks`) and, where `positions` is not NULL, store
+// its arena position there too (PartialNode).  wide: 64-bit keys (PartialNode).  kind: the
 // node type, whose instantiation of the class kernels the arithmetic
 // follows.  queue: as for launch_solid_toggle, per warp.
 void launch_surface_work(int kind, int mode, int wide, const Batch& b, const void* recs, const void* ovl,
                          const uint32_t* offsets, uint32_t nWork, const uint32_t* total, const uint32_t* buckets,
                          uint32_t* surf, const WordRank* ranks, void* keys, uint32_t keysCap,
-                         unsigned long long* list, uint32_t* listCount, uint32_t listCap, uint32_t blocksPerSm,
+                         unsigned long long* positions, unsigned long long* list, uint32_t* listCount, uint32_t listCap,
+                         uint32_t blocksPerSm,
                          uint32_t batch, uint32_t* queue, cudaStream_t s, uint32_t* launches);
 // Exclusive popcount prefix over `words` surface words, stored beside each
 // word; *total = surface voxels.
@@ -188,7 +190,8 @@ void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, con
 void launch_rotate_vertices(const float* V, float* R, uint32_t n, double a, double b, cudaStream_t s,
                             uint32_t* launches);
 void launch_emit_raw(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* fill, const uint32_t* surf,
-                     const WordRank* ranks, const void* keys, uint32_t keysCap, cudaStream_t s, uint32_t* launches);
+                     const WordRank* ranks, const void* keys, uint32_t keysCap, const unsigned long long* values,
+                     cudaStream_t s, uint32_t* launches);
 void launch_unrotate(const void* in, void* out, uint32_t X, uint32_t Y, uint32_t Z, uint32_t nodeBytes,
                      cudaStream_t s, uint32_t* launches);
 void launch_id_pass(void* nodes, uint32_t X, uint32_t Y, uint32_t Z, uint32_t nodeBytes, uint32_t idMask,
@@ -202,12 +205,17 @@ void launch_unrotate_fcc(const void* in, void* out, uint32_t X, uint32_t Y, uint
                          cudaStream_t s, uint32_t* launches);
 void launch_fcc_boundaries(void* nodes, uint32_t X, uint32_t Y, uint32_t Z, uint32_t nodeBytes, cudaStream_t s,
                            uint32_t* launches);
-// Keys at ranks >= keysCap read as 0.
+// PartialNodes: values[r] (cap entries) from the arena position of surface
+// node r to its node without the id, for r < min(*count, cap).
+void launch_partial_values(const Batch& b, const void* keys, const uint32_t* count, uint32_t cap,
+                           unsigned long long* values, cudaStream_t s, uint32_t* launches);
+// Keys (PartialNodes: values) at ranks >= keysCap read as 0.
 // Words [wordBegin, totalWords) of the arena (wordBegin a multiple of 32).
 void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t wordBegin, uint64_t totalWords,
                            const uint32_t* finalSolid,
                            const uint32_t* fill, const uint32_t* surf, const WordRank* ranks, const void* keys,
-                           uint32_t keysCap, uint32_t blocksPerSm, cudaStream_t s, uint32_t* launches);
+                           uint32_t keysCap, const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s,
+                           uint32_t* launches);
 
 // An FCC mesh: its four sub-lattice units are units [unit0, unit0 + 4).
 struct FccMesh {

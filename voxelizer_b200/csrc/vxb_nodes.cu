@@ -333,6 +333,7 @@ struct EmitArgs {
     const WordRank* ranks;   // surface words with their ranks (arena-wide)
     const void* keys;        // merged material keys by rank
     uint32_t keysCap;        // keys past it read as 0
+    const unsigned long long* values;   // PartialNode surface nodes without their ids, by rank
 };
 
 __device__ __forceinline__ UnitWords unitWords(const EmitArgs& a, const Unit& U) {
@@ -436,11 +437,6 @@ __device__ __forceinline__ void idBytes(const uint32_t P[5], uint32_t N[8]) {
         N[4 + h] = __byte_perm(t1, t3, 0x5410);
         N[6 + h] = __byte_perm(t1, t3, 0x7632);
     }
-}
-
-__device__ __forceinline__ uint32_t permOf(const WordNbrs& n, uint32_t q) {
-    return ((n.L >> q) & 1u) | (((n.R >> q) & 1u) << 1) | (((n.In >> q) & 1u) << 2) | (((n.Out >> q) & 1u) << 3) |
-           (((n.Dn >> q) & 1u) << 4) | (((n.Up >> q) & 1u) << 5);
 }
 
 // 1- and 2-byte nodes.  Each lane owns one word and builds its 32 nodes in
@@ -568,58 +564,96 @@ __global__ void __launch_bounds__(256, 6) emitNarrowKernel(EmitArgs a, uint64_t 
     }
 }
 
-// 8-byte PartialNodes: one lane per word, nodes stored from registers.  The
-// ratio of a node is 1 where the parity fill is set and the node is not a
-// surface node.
+// Values of PartialNode surface nodes by rank (the node without its id): the
+// material of the merged key and the volume ratio cut by its triangle, a few
+// hundred operations that a thread per surface node shares out evenly over
+// the device.  On entry values[r] is the arena position (word * 32 + node) of
+// surface node r.
+__global__ void __launch_bounds__(128) partialValuesKernel(Batch b, const unsigned long long* __restrict__ keys,
+                                                           const uint32_t* __restrict__ countPtr, uint32_t cap,
+                                                           unsigned long long* __restrict__ values) {
+    const uint32_t n = min(*countPtr, cap);
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        const unsigned long long key = keys[r], at = values[r];
+        const uint32_t u = b.nUnits > 1 ? unitOf(b.wordBase, b.nUnits, (uint64_t)(at >> 5)) : 0u;
+        const Unit& U = b.units[u];
+        const PassGeom& g = U.g;
+        const uint32_t w = (uint32_t)((at >> 5) - U.wordBase), bt = (uint32_t)at & 31u;
+        const uint32_t row = g.divX.div(w), z = g.divY.div(row);
+        const float ratio = ratio::nodeRatio(U.V, U.I, (uint32_t)key, (uint32_t)(key >> 40),
+                                             (int)((w - row * g.ipx) * 32u + bt), (int)(row - z * g.AY), (int)z,
+                                             detail::F3{g.mnf[0], g.mnf[1], g.mnf[2]}, g.df);
+        values[r] = NodeT<kPartial>::pack(0u, NodeT<kPartial>::keyMat(key), ratio);
+    }
+}
+
+// 8-byte PartialNodes.  Each lane forms the ids of one word (bit-sliced, as
+// for the narrow nodes); the warp's 1,024 nodes are then stored in order, two
+// nodes (16 bytes) a lane, with the values of surface nodes loaded by rank.
+// The ratio of any other node is 1 where the parity fill is set.
+//
+// With one thread per word that computed the ratios of its surface nodes, 2-3
+// lanes of a warp worked at a time: 4.5 M nodes (36 MB) with 118,463 surface
+// nodes took 395 us; now 27 us of values and 14 us of emission.  Sharing the
+// ratios out inside blocks of 128 words instead took 75 us (64 words: 90).
 __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t wordBegin, uint64_t totalWords) {
     typedef NodeT<kPartial> NT;
-    __shared__ uint8_t lut[64];
-    if (threadIdx.x < 64) lut[threadIdx.x] = kOrientTable[threadIdx.x];
-    __syncthreads();
-    for (uint64_t gw = wordBegin + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; gw < totalWords;
-         gw += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t u = unitOf(a.b.wordBase, a.b.nUnits, gw);
+    __shared__ uint32_t ids[8][32][9];          // 32 ids a word, padded
+    __shared__ uint32_t masks[8][32][4];        // surface, surface less cleared nodes, fill, rank
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint64_t gbase = wordBegin + ((uint64_t)blockIdx.x * 8u + warp) * 32u; gbase < totalWords;
+         gbase += (uint64_t)gridDim.x * 8u * 32u) {
+        const uint32_t u = a.b.nUnits > 1 ? unitOf(a.b.wordBase, a.b.nUnits, gbase) : 0u;
         const Unit& U = a.b.units[u];
-        const uint32_t w = (uint32_t)(gw - U.wordBase);
-        if (w >= U.g.ipx * U.g.AY * U.g.AZ) continue;
-        const UnitWords uw = unitWords(a, U);
-        const WordNbrs n = loadNbrs<kPartial>(uw, w);
-        const uint32_t zero = borderMask(uw, w);
-        uint4* out = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(U.out) + (size_t)w * 32 * 8);
-        if (((n.c | n.s0 | n.f0) & ~zero) == 0u) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) out[i] = make_uint4(0, 0, 0, 0);
+        const uint32_t nWords = U.g.ipx * U.g.AY * U.g.AZ, wbase = (uint32_t)(gbase - U.wordBase);
+        if (wbase >= nWords) continue;          // padding after the unit's grid (whole warp)
+        const uint32_t w = wbase + lane;
+        WordNbrs n{};
+        uint32_t zero = 0u;
+        if (w < nWords) {
+            const UnitWords uw = unitWords(a, U);
+            n = loadNbrs<kPartial>(uw, w);
+            zero = borderMask(uw, w);
+        }
+        const uint32_t cm = n.c & ~zero, sm = n.s0 & ~zero, fm = n.f0 & ~zero;
+        uint4* out = reinterpret_cast<uint4*>(U.out) + (size_t)wbase * 16u;
+        const uint32_t wend = min(nWords - wbase, 32u);
+        if (!__any_sync(0xffffffffu, (cm | sm | fm) != 0u)) {
+            for (uint32_t i = lane; i < wend * 16u; i += 32u) out[i] = make_uint4(0u, 0u, 0u, 0u);
             continue;
         }
-        uint32_t matRank = n.s0 ? a.ranks[U.wordBase + w].rank : 0u;
-        // Node coordinates of the word's first node (ratio of surface nodes).
-        const int x0 = (int)(w % U.g.ipx) * 32, y0 = (int)(w / U.g.ipx % U.g.AY), z0 = (int)(w / U.g.ipx / U.g.AY);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            uint32_t v32[4];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint32_t bt = 2 * i + j, q = 31u - bt;
-                uint32_t bid = 0, mat = 0;
-                if ((n.c >> q) & 1u) bid = lut[permOf(n, q)];
-                // constructNodeList2 writes float(solid); processVoxel<PartialNode>
-                // overwrites surface nodes with the winning triangle's ratio.
-                float r = ((n.f0 >> q) & 1u) ? 1.0f : 0.0f;
-                if ((n.s0 >> q) & 1u) {
-                    if (matRank < a.keysCap && !((zero >> q) & 1u)) {
-                        const uint64_t key = reinterpret_cast<const unsigned long long*>(a.keys)[matRank];
-                        mat = NT::keyMat(key);
-                        r = ratio::nodeRatio(U.V, U.I, (uint32_t)key, (uint32_t)(key >> 40), x0 + (int)bt, y0, z0,
-                                             detail::F3{U.g.mnf[0], U.g.mnf[1], U.g.mnf[2]}, U.g.df);
-                    }
-                    ++matRank;
-                }
-                const uint64_t nv = (zero >> q) & 1u ? 0ull : NT::pack(bid, mat, r);
-                v32[2 * j] = (uint32_t)nv;
-                v32[2 * j + 1] = (uint32_t)(nv >> 32);
+        {
+            uint32_t N[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+            if (cm) {
+                uint32_t P[5];
+                idPlanes(n, cm, P);
+                idBytes(P, N);
             }
-            out[i] = make_uint4(v32[0], v32[1], v32[2], v32[3]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ids[warp][lane][i] = N[i];
         }
+        *reinterpret_cast<uint4*>(masks[warp][lane]) =
+            make_uint4(n.s0, sm, fm, sm ? a.ranks[U.wordBase + w].rank : 0u);
+        __syncwarp();
+#pragma unroll 4
+        for (uint32_t i = lane; i < wend * 16u; i += 32u) {
+            const uint32_t l = i >> 4, p = (i & 15u) * 2u;   // word and its first node
+            const uint32_t id2 = reinterpret_cast<const uint16_t*>(ids[warp][l])[p >> 1];
+            const uint4 m = *reinterpret_cast<const uint4*>(masks[warp][l]);
+            uint64_t v[2];
+#pragma unroll
+            for (uint32_t j = 0; j < 2; ++j) {
+                const uint32_t t = p + j;
+                // Ranks count every surface node of the word, cleared ones
+                // included; ranks past the key array have no value.
+                const uint32_t r = m.w + (t ? __popc(m.x >> (32u - t)) : 0u);
+                v[j] = NT::pack(0u, 0u, (m.z << t) & 0x80000000u ? 1.0f : 0.0f);
+                if (((m.y << t) & 0x80000000u) && r < a.keysCap) v[j] = __ldg(a.values + r);
+                v[j] |= (id2 >> (8u * j)) & 255u;
+            }
+            out[i] = make_uint4((uint32_t)v[0], (uint32_t)(v[0] >> 32), (uint32_t)v[1], (uint32_t)(v[1] >> 32));
+        }
+        __syncwarp();
     }
 }
 
@@ -770,7 +804,7 @@ void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, con
 void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t wordBegin, uint64_t totalWords,
                            const uint32_t* finalSolid,
                            const uint32_t* fill, const uint32_t* surf, const WordRank* ranks, const void* keys,
-                           uint32_t keysCap, uint32_t blocksPerSm, cudaStream_t s, uint32_t* launches) {
+                           uint32_t keysCap, const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s, uint32_t* launches) {
     EmitArgs a;
     a.keysCap = keysCap;
     a.b = b;
@@ -779,13 +813,20 @@ void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t wordBegin, uin
     a.surf = surf;
     a.ranks = ranks;
     a.keys = keys;
+    a.values = values;
     const uint64_t words = totalWords - wordBegin;
     const uint32_t grid = gridFor(words, 256, 148u * blocksPerSm);
     switch (nodeKind) {
     case kShort: emitNarrowKernel<kShort><<<grid, 256, 0, s>>>(a, wordBegin, totalWords); break;
     case kLong: emitNarrowKernel<kLong><<<grid, 256, 0, s>>>(a, wordBegin, totalWords); break;
-    default: emitPartialKernel<<<gridFor(words, 256, 148u * 8u), 256, 0, s>>>(a, wordBegin, totalWords); break;
+    default: emitPartialKernel<<<gridFor(words, 256, 148u * 64u), 256, 0, s>>>(a, wordBegin, totalWords); break;
     }
+    *launches += 1;
+}
+
+void launch_partial_values(const Batch& b, const void* keys, const uint32_t* count, uint32_t cap,
+                           unsigned long long* values, cudaStream_t s, uint32_t* launches) {
+    partialValuesKernel<<<148 * 16, 128, 0, s>>>(b, static_cast<const unsigned long long*>(keys), count, cap, values);
     *launches += 1;
 }
 

@@ -316,6 +316,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
                                                      std::max<uint64_t>(1u << 20, totalWords_ * 32 / 16));
         }
         if ((rc = keys.ensure((size_t)keysCap_ * (wide_ ? 8 : 4)))) return rc;
+        if (wide_ && (rc = values.ensure((size_t)keysCap_ * 8))) return rc;
     }
     VXB_CUDA(cudaMemcpyAsync(tables.p, blob_.data(), blob_.size(), cudaMemcpyHostToDevice, s));
     return 0;
@@ -370,7 +371,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         tuneMark(kKnobSurface, false, ss);
         launch_surface_work(nodeKind_, retraverse ? 2 : 0, wide_ ? 1 : 0, b, recs.p, ovl.p, sOffsets.as<uint32_t>(), nWork_,
                             st + kSurfTotal, buckets.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(),
-                            keys.p, keysCap_, hitList.as<unsigned long long>(), st + kHitCount, listCap_,
+                            keys.p, keysCap_, nullptr, hitList.as<unsigned long long>(), st + kHitCount, listCap_,
                             shape.surfBlocksPerSm, shape.surfBatch, shape.surfQueue ? st + kSurfQueue : nullptr, ss,
                             &launches);
         tuneMark(kKnobSurface, true, ss);
@@ -388,8 +389,11 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         else
             launch_surface_work(nodeKind_, 1, wide_ ? 1 : 0, b, recs.p, ovl.p, sOffsets.as<uint32_t>(), nWork_,
                                 st + kSurfTotal, buckets.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(),
-                                keys.p, keysCap_, nullptr, st + kHitCount, 0, shape.surfBlocksPerSm, shape.surfBatch,
+                                keys.p, keysCap_, values.as<unsigned long long>(), nullptr, st + kHitCount, 0, shape.surfBlocksPerSm, shape.surfBatch,
                                 shape.surfQueue ? st + kSurfQueue : nullptr, ss, &launches);
+        if (wide_)
+            launch_partial_values(b, keys.p, st + kSurfaceVoxels, keysCap_, values.as<unsigned long long>(), ss,
+                                  &launches);
         tuneMark(kKnobSurfaceSpan, true, ss);
         if (timer) timer->mark(4, true, ss);
         VXB_CUDA(cudaEventRecord(evSurfDone_, ss));
@@ -445,7 +449,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     mark(3, false);
     if (raw_ && anyCartesian_)
         launch_emit_raw(nodeKind_, b, totalWords_, fillP, surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p, keysCap_,
-                        ps, &launches);
+                        values.as<unsigned long long>(), ps, &launches);
     else if (anyCartesian_) {
         tuneMark(kKnobEmit, false, ps);
         if (hostOut_ && units_.size() == 1) {
@@ -460,7 +464,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
                 const uint64_t w1 = k + 1 == kOutChunks ? words : (words * (k + 1) / kOutChunks) & ~uint64_t(31);
                 if (w1 <= w0) continue;
                 launch_emit_cartesian(nodeKind_, b, w0, w1, fin.as<uint32_t>(), fillP, surf.as<uint32_t>(),
-                                      ranks.as<WordRank>(), keys.p, keysCap_, shape.emitBlocksPerSm, ps, &launches);
+                                      ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, ps, &launches);
                 if (!outEv_[k]) VXB_CUDA(cudaEventCreateWithFlags(&outEv_[k], cudaEventDisableTiming));
                 VXB_CUDA(cudaEventRecord(outEv_[k], ps));
                 VXB_CUDA(cudaStreamWaitEvent(copyStream_, outEv_[k], 0));
@@ -471,7 +475,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
             hostCopied_ = true;
         } else {
             launch_emit_cartesian(nodeKind_, b, 0, totalWords_, fin.as<uint32_t>(), fillP, surf.as<uint32_t>(),
-                                  ranks.as<WordRank>(), keys.p, keysCap_, shape.emitBlocksPerSm, ps, &launches);
+                                  ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, ps, &launches);
         }
         tuneMark(kKnobEmit, true, ps);
     }
@@ -581,13 +585,17 @@ int Pipeline::finish(cudaStream_t s) {
             int rc;
             if ((uint64_t)surfaceVoxels + 1 > keysCap_) {
                 if ((rc = keys.ensure(((size_t)surfaceVoxels + 1) * (wide_ ? 8 : 4)))) return rc;
+                if (wide_ && (rc = values.ensure(((size_t)surfaceVoxels + 1) * 8))) return rc;
                 keysCap_ = surfaceVoxels + 1;
             }
             launch_surface_keys_zero(keys.p, st + kSurfaceVoxels, keysCap_, wide_ ? 1 : 0, s, &launches);
             launch_surface_work(nodeKind_, 1, wide_ ? 1 : 0, b, recs.p, ovl.p, sOffsets.as<uint32_t>(), nWork_,
                                 st + kSurfTotal, buckets.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(),
-                                keys.p, keysCap_, nullptr, st + kHitCount, 0, shape.surfBlocksPerSm, shape.surfBatch,
+                                keys.p, keysCap_, values.as<unsigned long long>(), nullptr, st + kHitCount, 0, shape.surfBlocksPerSm, shape.surfBatch,
                                 shape.surfQueue ? st + kSurfQueue : nullptr, s, &launches);
+            if (wide_)
+                launch_partial_values(b, keys.p, st + kSurfaceVoxels, keysCap_, values.as<unsigned long long>(), s,
+                                      &launches);
             reemit = true;
         }
     }
@@ -602,10 +610,10 @@ int Pipeline::finish(cudaStream_t s) {
     if (reemit) {
         if (raw_ && anyCartesian_)
             launch_emit_raw(nodeKind_, b, totalWords_, fillP, surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p,
-                            keysCap_, s, &launches);
+                            keysCap_, values.as<unsigned long long>(), s, &launches);
         else if (anyCartesian_)
             launch_emit_cartesian(nodeKind_, b, 0, totalWords_, fin.as<uint32_t>(), fillP, surf.as<uint32_t>(),
-                                  ranks.as<WordRank>(), keys.p, keysCap_, shape.emitBlocksPerSm, s, &launches);
+                                  ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, s, &launches);
         if (nFcc_)
             launch_emit_fcc(nodeKind_, b, reinterpret_cast<const FccMesh*>(tables.as<uint8_t>() + oFcc_),
                             reinterpret_cast<const uint64_t*>(tables.as<uint8_t>() + oGroupBase_), nFcc_,

@@ -134,7 +134,7 @@ private:
 
     DevBuf tables, status, bigList;
     DevBuf fill, surf, fin, ranks, rankTiles, pruneLists;
-    DevBuf codes, unitCounts, buckets, recs, ovl, hitList, keys;
+    DevBuf codes, unitCounts, buckets, recs, ovl, hitList, keys, values;
     // The surface pass runs on a second stream beside the solid pass, joined
     // before pruning (surface bits) and before emission (merged keys).
     DevBuf sCounts, sOffsets, sTileSums;

@@ -374,6 +374,7 @@ struct Sink {
     const WordRank* wordRank;  // complete surface words with their ranks (mode 1)
     void* keys;                // compact key array (mode 1)
     uint32_t keysCap;          // keys at ranks past it are dropped
+    unsigned long long* positions;   // arena position of each rank (wide keys)
     unsigned long long* list;
     uint32_t* listCount;
     uint32_t listCap;
@@ -403,8 +404,12 @@ struct Sink {
             const WordRank wr = wordRank[w];
             const uint32_t r = wr.rank + (b ? __popc(wr.bits >> (32 - b)) : 0u);
             if (r >= keysCap) return;
-            if (wide) atomicMax(reinterpret_cast<unsigned long long*>(keys) + r, (unsigned long long)key);
-            else atomicMax(reinterpret_cast<uint32_t*>(keys) + r, (uint32_t)key);
+            if (wide) {
+                atomicMax(reinterpret_cast<unsigned long long*>(keys) + r, (unsigned long long)key);
+                positions[r] = w * 32u + b;   // every hit of a voxel stores the same
+            } else {
+                atomicMax(reinterpret_cast<uint32_t*>(keys) + r, (uint32_t)key);
+            }
         }
     }
     // Moves the warp's staged hits to the global list (whole warp, converged).
@@ -828,14 +833,16 @@ static void launchSurfaceWorkKind(uint32_t batch, uint32_t grid, const Sink& sin
 void launch_surface_work(int kind, int mode, int wide, const Batch& b, const void* recs, const void* ovl,
                          const uint32_t* offsets, uint32_t nWork, const uint32_t* total, const uint32_t* buckets,
                          uint32_t* surf, const WordRank* ranks, void* keys, uint32_t keysCap,
-                         unsigned long long* list, uint32_t* listCount, uint32_t listCap, uint32_t blocksPerSm,
-                         uint32_t batch, uint32_t* queue, cudaStream_t s, uint32_t* launches) {
+                         unsigned long long* positions, unsigned long long* list, uint32_t* listCount,
+                         uint32_t listCap, uint32_t blocksPerSm, uint32_t batch, uint32_t* queue, cudaStream_t s,
+                         uint32_t* launches) {
     if (queue) cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
     Sink sink;
     sink.bits = surf;
     sink.wordRank = ranks;
     sink.keys = keys;
     sink.keysCap = keysCap;
+    sink.positions = positions;
     sink.list = list;
     sink.listCount = listCount;
     sink.listCap = listCap;

@@ -18,7 +18,6 @@
 #include "vxb_common.cuh"
 #include "vxb_device.cuh"
 #include "vxb_kernels.cuh"
-#include "vxb_ratio.cuh"
 
 #include <type_traits>
 
@@ -41,7 +40,7 @@ __global__ void rotateKernel(const float* __restrict__ V, float* __restrict__ R,
 template <int K>
 __global__ void emitRawKernel(Batch b, uint64_t totalWords, const uint32_t* __restrict__ fill,
                               const uint32_t* __restrict__ surf, const WordRank* __restrict__ ranks, const void* keys,
-                              uint32_t keysCap) {
+                              uint32_t keysCap, const unsigned long long* __restrict__ values) {
     typedef NodeT<K> NT;
     for (uint64_t gw = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; gw < totalWords;
          gw += (uint64_t)gridDim.x * blockDim.x) {
@@ -52,27 +51,18 @@ __global__ void emitRawKernel(Batch b, uint64_t totalWords, const uint32_t* __re
         const uint32_t f = __ldg(fill + U.wordBase + w);
         const uint32_t s = U.materials ? __ldg(surf + U.wordBase + w) : 0u;
         uint32_t rank = s ? ranks[U.wordBase + w].rank : 0u;
-        const int x0 = (int)(w % U.g.ipx) * 32, y0 = (int)(w / U.g.ipx % U.g.AY), z0 = (int)(w / U.g.ipx / U.g.AY);
         uint8_t* out = static_cast<uint8_t*>(U.out) + (size_t)w * 32 * NT::bytes;
         for (uint32_t bt = 0; bt < 32; ++bt) {
             const uint32_t q = 31u - bt;
             const uint32_t fb = (f >> q) & 1u, sb = (s >> q) & 1u;
-            uint32_t mat = 0;
-            float r = fb ? 1.0f : 0.0f;
+            uint64_t nv = NT::pack(0u, 0u, fb ? 1.0f : 0.0f);
             if (sb) {
-                if (rank < keysCap) {
-                    if (NT::bytes == 8) {
-                        const uint64_t key = reinterpret_cast<const unsigned long long*>(keys)[rank];
-                        mat = NT::keyMat(key);
-                        r = ratio::nodeRatio(U.V, U.I, (uint32_t)key, (uint32_t)(key >> 40), x0 + (int)bt, y0, z0,
-                                             detail::F3{U.g.mnf[0], U.g.mnf[1], U.g.mnf[2]}, U.g.df);
-                    } else {
-                        mat = NT::keyMat(reinterpret_cast<const uint32_t*>(keys)[rank]);
-                    }
-                }
+                if (rank < keysCap)
+                    nv = NT::bytes == 8 ? values[rank]
+                                        : NT::pack(0u, NT::keyMat(reinterpret_cast<const uint32_t*>(keys)[rank]), 0.0f);
                 ++rank;
             }
-            const uint64_t nv = NT::pack((fb | sb) ? 1u : 0u, mat, r);
+            nv |= NT::pack((fb | sb) ? 1u : 0u, 0u, 0.0f);
             for (int k = 0; k < NT::bytes; ++k) out[bt * NT::bytes + k] = (uint8_t)(nv >> (8 * k));
         }
     }
@@ -193,12 +183,13 @@ void launch_rotate_vertices(const float* V, float* R, uint32_t n, double a, doub
 }
 
 void launch_emit_raw(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* fill, const uint32_t* surf,
-                     const WordRank* ranks, const void* keys, uint32_t keysCap, cudaStream_t s, uint32_t* launches) {
+                     const WordRank* ranks, const void* keys, uint32_t keysCap, const unsigned long long* values,
+                     cudaStream_t s, uint32_t* launches) {
     const uint32_t grid = gridFor(totalWords, 128, 148u * 8u);
     switch (nodeKind) {
-    case kShort: emitRawKernel<kShort><<<grid, 128, 0, s>>>(b, totalWords, fill, surf, ranks, keys, keysCap); break;
-    case kLong: emitRawKernel<kLong><<<grid, 128, 0, s>>>(b, totalWords, fill, surf, ranks, keys, keysCap); break;
-    default: emitRawKernel<kPartial><<<grid, 128, 0, s>>>(b, totalWords, fill, surf, ranks, keys, keysCap); break;
+    case kShort: emitRawKernel<kShort><<<grid, 128, 0, s>>>(b, totalWords, fill, surf, ranks, keys, keysCap, values); break;
+    case kLong: emitRawKernel<kLong><<<grid, 128, 0, s>>>(b, totalWords, fill, surf, ranks, keys, keysCap, values); break;
+    default: emitRawKernel<kPartial><<<grid, 128, 0, s>>>(b, totalWords, fill, surf, ranks, keys, keysCap, values); break;
     }
     *launches += 1;
 }
