@@ -222,11 +222,11 @@ struct FccMesh {
     uint32_t unit0;
     void* out;
 };
-// FCC node grids; groupBase[m] is the first 16-byte output group of mesh m
-// (nMeshes + 1 entries).  raw: the nodes before calculateFCCBoundaries (id =
+// FCC node grids; pairBase[m] is the first pair of words (64 nodes of a row)
+// of mesh m, a multiple of 16 (nMeshes + 1 entries).  raw: the nodes before calculateFCCBoundaries (id =
 // solid bit, the surface material), for slices along x.
-void launch_emit_fcc(int nodeKind, const Batch& b, const FccMesh* meshes, const uint64_t* groupBase,
-                     uint32_t nMeshes, uint64_t totalGroups, const uint32_t* fill, const uint32_t* surf,
+void launch_emit_fcc(int nodeKind, const Batch& b, const FccMesh* meshes, const uint64_t* pairBase,
+                     uint32_t nMeshes, uint64_t totalPairs, const uint32_t* fill, const uint32_t* surf,
                      const WordRank* ranks, const void* keys, uint32_t keysCap, bool raw, cudaStream_t s,
                      uint32_t* launches);
 

@@ -5,11 +5,10 @@
 // row): it forms the six neighbour masks of its word with shifts of the word
 // and of the words around it, so a whole word of boundary ids costs a few
 // bitwise operations when the word is uniform (all empty, or all solid with
-// all six neighbours solid: id 27).  For 1- and 2-byte nodes the ids of a
-// mixed word are computed bit-sliced (five planes, one per id bit) and
-// transposed to bytes; PartialNodes and FCC nodes take a per-node table
-// lookup where solid meets empty.  A warp's 32 words are staged in shared
-// memory and stored as contiguous 512-byte rows with 16-byte vector stores.
+// all six neighbours solid: id 27).  The ids of a mixed word are computed
+// bit-sliced (a plane per id bit) and transposed to bytes.  A warp's 32 words
+// are staged in shared memory and stored as contiguous 512-byte rows with
+// 16-byte vector stores.
 //
 // Grids of one unit hold fewer than 2^32 voxels, so word indices inside a
 // unit fit 32 bits; arena offsets (unit word bases) are 64-bit.
@@ -407,15 +406,14 @@ __device__ __forceinline__ void idPlanes(const WordNbrs& n, uint32_t cm, uint32_
     P[4] = ((Y3 & ((Z1 & X3) | (Z2 & R))) | (Z3 & Ya & Xa)) & cm;
 }
 
-// The planes as bytes in node order: N[m] holds the ids of nodes 4m .. 4m+3
-// (node t of a word is bit 31 - t), one per byte.  An 8x8 bit transpose in
-// each byte lane of the bit-reversed planes leaves the id of node 8b + i in
-// byte b of row i; 4x4 byte transposes put the nodes in order.
-__device__ __forceinline__ void idBytes(const uint32_t P[5], uint32_t N[8]) {
+// NP <= 8 bit planes as bytes in node order: N[m] holds the bytes of nodes
+// 4m .. 4m+3 (node t of a word is bit 31 - t), plane k in bit k.  An 8x8 bit
+// transpose in each byte lane of the bit-reversed planes leaves the byte of
+// node 8b + i in byte b of row i; 4x4 byte transposes put the nodes in order.
+template <int NP> __device__ __forceinline__ void planeBytes(const uint32_t* P, uint32_t N[8]) {
     uint32_t r[8];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) r[k] = __brev(P[k]);
-    r[5] = r[6] = r[7] = 0u;
+    for (int k = 0; k < 8; ++k) r[k] = k < NP ? __brev(P[k]) : 0u;
 #pragma unroll
     for (int s = 4; s >= 1; s >>= 1) {
         const uint32_t m = s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
@@ -498,7 +496,7 @@ __global__ void __launch_bounds__(256, 6) emitNarrowKernel(EmitArgs a, uint64_t 
             {
                 uint32_t P[5];
                 idPlanes(n, cm, P);
-                idBytes(P, N);
+                planeBytes<5>(P, N);
             }
 #pragma unroll
             for (int i = 0; i < CH; ++i) {
@@ -627,7 +625,7 @@ __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t wo
             if (cm) {
                 uint32_t P[5];
                 idPlanes(n, cm, P);
-                idBytes(P, N);
+                planeBytes<5>(P, N);
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i) ids[warp][lane][i] = N[i];
@@ -660,7 +658,7 @@ __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t wo
 struct FccArgs {
     Batch b;
     const FccMesh* meshes;
-    const uint64_t* groupBase;
+    const uint64_t* pairBase;
     uint32_t nMeshes;
     const uint32_t* fill;
     const uint32_t* surf;
@@ -670,102 +668,168 @@ struct FccArgs {
     uint32_t raw;   // nodes before the boundaries: id = solid bit, no face clearing
 };
 
-// The four sub-lattice grids of one FCC mesh.
-struct FccGrids {
-    const uint32_t* fill[4];
-    const uint32_t* surf[4];   // NULL without materials
-    uint64_t wordBase[4];      // arena word of each sub-lattice (rank space)
-    uint32_t ipx, AY;
-};
-
 // Node emission, FCC lattices (convertToFCCGrid + calculateFCCBoundaries,
 // src/voxelizer.cu:1710-1776, 1929-2048).  FCC node (X, y, Z) belongs to
-// sub-lattice 1 + (X & 1) + 2 * (Z & 1) at voxel (X / 2, y, Z / 2); its id is
-// the 12-bit mask of solid FCC neighbours.  The neighbour relation is
-// symmetric, so the reference's in-place pass equals this snapshot
-// evaluation.
-__device__ __forceinline__ uint32_t fccSolid(const FccGrids& G, uint32_t X2, uint32_t y, uint32_t Z2) {
-    const int gt = (int)(X2 & 1u) + 2 * (int)(Z2 & 1u);
-    const uint32_t x = X2 >> 1, z = Z2 >> 1;
-    const uint32_t w = (z * G.AY + y) * G.ipx + (x >> 5);
-    uint32_t word = __ldg(G.fill[gt] + w);
-    if (G.surf[gt]) word |= __ldg(G.surf[gt] + w);
-    return (word >> (31u - (x & 31u))) & 1u;
-}
-
+// sub-lattice (X & 1) + 2 * (Z & 1) at voxel (X / 2, y, Z / 2); its id is the
+// 12-bit mask of solid FCC neighbours.  The neighbour relation is symmetric,
+// so the reference's in-place pass equals this snapshot evaluation.
+//
+// All 12 neighbours of a word of one sub-lattice lie in words of the other
+// three, at the same x or one node beside it, so a lane takes one word and
+// forms the 12 bits of its 32 nodes as 12 word planes (24 loads instead of
+// up to 24 per node), which are transposed to 16-bit ids.  A pair of lanes
+// holds the two words whose nodes alternate along X; a warp's 16 pairs are
+// 1,024 consecutive nodes, stored 16 bytes a lane with the materials of
+// surface nodes loaded by rank.
+//
+// Node by node (12 neighbour tests of two loads each, 16 bytes a thread) 8.2 M
+// LongFCC nodes (33 MB) took 115 us and 1.7 M ShortFCC nodes 39 us; now 21 and
+// 13 us.
 template <int K>
-__global__ void emitFccKernel(FccArgs A, uint64_t totalGroups) {
+__global__ void __launch_bounds__(256) emitFccKernel(FccArgs A, uint64_t totalPairs) {
     typedef NodeT<K> NT;
-    constexpr int GN = 16 / NT::bytes;
-    for (uint64_t gg = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; gg < totalGroups;
-         gg += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t m = unitOf(A.groupBase, A.nMeshes, gg);
+    constexpr uint32_t NPC = 16 / NT::bytes;      // nodes of a 16-byte chunk
+    constexpr uint32_t CPP = 64 / NPC;            // chunks of a pair
+    __shared__ __align__(16) uint32_t ids[8][32][18];   // 32 16-bit ids a word, padded
+    __shared__ __align__(16) uint4 masks[8][32];        // surface nodes, those not cleared, rank
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t px = lane & 1u;
+    for (uint64_t g0 = ((uint64_t)blockIdx.x * 8u + warp) * 16u; g0 < totalPairs; g0 += (uint64_t)gridDim.x * 8u * 16u) {
+        // Mesh pair bases are multiples of 16.
+        const uint32_t m = A.nMeshes > 1 ? unitOf(A.pairBase, A.nMeshes, g0) : 0u;
         const FccMesh M = A.meshes[m];
-        FccGrids G;
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const Unit& U = A.b.units[M.unit0 + l];
-            G.fill[l] = A.fill + U.wordBase;
-            G.surf[l] = U.materials ? A.surf + U.wordBase : nullptr;
-            G.wordBase[l] = U.wordBase;
-        }
         const PassGeom& g = A.b.units[M.unit0].g;
-        G.ipx = g.ipx;
-        G.AY = g.AY;
-        const uint32_t NX = 2 * g.X, NY = g.AY, NZ = 2 * g.AZ;
-        const uint32_t groupsPerRow = NX / GN;
-        const uint32_t gi = (uint32_t)(gg - __ldg(A.groupBase + m));
-        const uint32_t row = gi / groupsPerRow;
-        const uint32_t X0 = (gi - row * groupsPerRow) * GN;
-        const uint32_t Z2 = row / NY, y = row - Z2 * NY;
-        uint4 outv = make_uint4(0, 0, 0, 0);
+        const uint32_t ipx = g.ipx, AY = g.AY, AZ = g.AZ;
+        const uint32_t p0 = (uint32_t)(g0 - __ldg(A.pairBase + m)), nPairs = 2u * AZ * AY * ipx;
+        if (p0 >= nPairs) continue;               // padding after the mesh (whole warp)
+        const uint32_t pair = p0 + (lane >> 1), last = min(nPairs - p0, 16u);
+        uint32_t c = 0u, s0 = 0u, zero = 0u, rank = 0u;
+        uint32_t N[16];
 #pragma unroll
-        for (int n = 0; n < GN; ++n) {
-            const uint32_t X2 = X0 + n;
-            const int gt = (int)(X2 & 1u) + 2 * (int)(Z2 & 1u);
-            const uint32_t x = X2 >> 1, z = Z2 >> 1;
-            const uint32_t w = (z * G.AY + y) * G.ipx + (x >> 5);
-            const uint32_t q = 31u - (x & 31u);
-            const uint32_t fb = (__ldg(G.fill[gt] + w) >> q) & 1u;
-            const uint32_t sw = G.surf[gt] ? __ldg(G.surf[gt] + w) : 0u;
-            const uint32_t sb = (sw >> q) & 1u;
-            uint32_t bid = 0;
-            if ((fb | sb) && A.raw) {
-                bid = 1;
-            } else if (fb | sb) {
-                const bool left = X2 > 0, right = X2 < NX - 1, in = y > 0, out = y < NY - 1;
-                const bool down = Z2 > 0, up = Z2 < NZ - 1, xe = ((X2 + Z2) & 1u) == 0;
-                const uint32_t ym = xe ? y - 1 : y;   // y - xEven
-                const uint32_t yp = xe ? y : y + 1;   // y + !xEven
-                const bool cIn = (xe && in) || !xe, cOut = (!xe && out) || xe;
-                if (down && cIn && fccSolid(G, X2, ym, Z2 - 1)) bid |= 1u;
-                if (down && left && fccSolid(G, X2 - 1, y, Z2 - 1)) bid |= 2u;
-                if (down && right && fccSolid(G, X2 + 1, y, Z2 - 1)) bid |= 4u;
-                if (down && cOut && fccSolid(G, X2, yp, Z2 - 1)) bid |= 8u;
-                if (left && cIn && fccSolid(G, X2 - 1, ym, Z2)) bid |= 16u;
-                if (right && cIn && fccSolid(G, X2 + 1, ym, Z2)) bid |= 32u;
-                if (left && cOut && fccSolid(G, X2 - 1, yp, Z2)) bid |= 64u;
-                if (right && cOut && fccSolid(G, X2 + 1, yp, Z2)) bid |= 128u;
-                if (up && cIn && fccSolid(G, X2, ym, Z2 + 1)) bid |= 256u;
-                if (up && left && fccSolid(G, X2 - 1, y, Z2 + 1)) bid |= 512u;
-                if (up && right && fccSolid(G, X2 + 1, y, Z2 + 1)) bid |= 1024u;
-                if (up && cOut && fccSolid(G, X2, yp, Z2 + 1)) bid |= 2048u;
+        for (int i = 0; i < 16; ++i) N[i] = 0u;
+        if (pair < nPairs) {
+            const uint32_t row = g.divX.div(pair), k = pair - row * ipx;
+            const uint32_t Z2 = g.divY.div(row), y = row - Z2 * AY, z = Z2 >> 1, pz = Z2 & 1u;
+            auto lattice = [&](uint32_t x1, uint32_t z1) -> const Unit& { return A.b.units[M.unit0 + x1 + 2u * z1]; };
+            const Unit& U = lattice(px, pz);
+            const uint32_t w = (z * AY + y) * ipx + k;
+            s0 = U.materials ? __ldg(A.surf + U.wordBase + w) : 0u;
+            c = __ldg(A.fill + U.wordBase + w) | s0;
+            if (g.border && !A.raw)
+                // zeroPadding of an FCC device space with neighbours
+                // (src/voxelizer.cu:4827-4834): two node layers at the x and
+                // z faces, one at the y faces.
+                zero = y == 0 || y + 1 == AY || z == 0 || z + 1 == AZ
+                           ? 0xFFFFFFFFu
+                           : (k == 0 ? 0x80000000u : 0u) | (k + 1 == ipx ? 1u : 0u);
+            const uint32_t cm = c & ~zero;
+            if (s0 & ~zero) rank = A.ranks[U.wordBase + w].rank;
+            if (cm && A.raw) {
+                const uint32_t P[1] = {cm};
+                uint32_t lo[8];
+                planeBytes<1>(P, lo);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    N[2 * i] = __byte_perm(lo[i], 0u, 0x4140);
+                    N[2 * i + 1] = __byte_perm(lo[i], 0u, 0x4342);
+                }
+            } else if (cm) {
+                const bool xe = px == pz;
+                // Rows before and after along y of the neighbours that differ
+                // in y (y - xe and y + !xe), planes below and above.
+                const bool in = !xe || y > 0, out = xe || y + 1 < AY;
+                const bool down = pz != 0u || z > 0, up = pz == 0u || z + 1 < AZ;
+                const uint32_t ym = xe ? y - 1 : y, yp = xe ? y : y + 1, zd = pz ? z : z - 1, zu = pz ? z + 1 : z;
+                auto word = [&](const Unit& L, bool ok, uint32_t zz, uint32_t yy, uint32_t kk) {
+                    if (!ok) return 0u;
+                    const uint64_t i = L.wordBase + ((zz * AY + yy) * ipx + kk);
+                    return __ldg(A.fill + i) | (L.materials ? __ldg(A.surf + i) : 0u);
+                };
+                const Unit& LA = lattice(px, 1u - pz);
+                const Unit& LB = lattice(1u - px, 1u - pz);
+                const Unit& LC = lattice(1u - px, pz);
+                uint32_t P[12];
+                P[0] = word(LA, down && in, zd, ym, k);
+                P[3] = word(LA, down && out, zd, yp, k);
+                P[8] = word(LA, up && in, zu, ym, k);
+                P[11] = word(LA, up && out, zu, yp, k);
+                // The other x parity: X - 1 and X + 1 are the same voxel and
+                // the one beside it (the previous for even X, the next for
+                // odd X).
+                const bool edge = px ? k + 1 < ipx : k > 0;
+                const uint32_t kn = px ? k + 1 : k - 1;
+                auto sides = [&](const Unit& L, bool ok, uint32_t zz, uint32_t yy, uint32_t& left, uint32_t& right) {
+                    const uint32_t same = word(L, ok, zz, yy, k), beside = word(L, ok && edge, zz, yy, kn);
+                    left = px ? same : (same >> 1) | (beside << 31);
+                    right = px ? (same << 1) | (beside >> 31) : same;
+                };
+                sides(LB, down, zd, y, P[1], P[2]);
+                sides(LC, in, z, ym, P[4], P[5]);
+                sides(LC, out, z, yp, P[6], P[7]);
+                sides(LB, up, zu, y, P[9], P[10]);
+                uint32_t all = cm;
+#pragma unroll
+                for (int i = 0; i < 12; ++i) {
+                    P[i] &= cm;
+                    all &= P[i];
+                }
+                if (all == 0xFFFFFFFFu) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) N[i] = 0x0FFF0FFFu;
+                } else {
+                    uint32_t lo[8], hi[8];
+                    planeBytes<8>(P, lo);
+                    planeBytes<4>(P + 8, hi);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        N[2 * i] = __byte_perm(lo[i], hi[i], 0x5140);
+                        N[2 * i + 1] = __byte_perm(lo[i], hi[i], 0x7362);
+                    }
+                }
             }
-            uint32_t mat = 0;
-            if (sb) {
-                const uint32_t bt = x & 31u;
-                const uint32_t r = A.ranks[G.wordBase[gt] + w].rank + (bt ? __popc(sw >> (32 - bt)) : 0u);
-                mat = r < A.keysCap ? NT::keyMat(reinterpret_cast<const uint32_t*>(A.keys)[r]) : 0u;
-            }
-            // zeroPadding of an FCC device space with neighbours
-            // (src/voxelizer.cu:4827-4834): two node layers at the x and z
-            // faces, one at the y faces.
-            const bool face = g.border && !A.raw && (X2 < 2 || X2 + 2 >= NX || y == 0 || y + 1 == NY || Z2 < 2 || Z2 + 2 >= NZ);
-            const uint64_t val = face ? 0ull : NT::pack(bid, mat, 0.0f);
-            if (NT::bytes == 2) reinterpret_cast<uint16_t*>(&outv)[n] = (uint16_t)val;
-            else reinterpret_cast<uint32_t*>(&outv)[n] = (uint32_t)val;
         }
-        reinterpret_cast<uint4*>(M.out)[gi] = outv;
+        uint4* out = reinterpret_cast<uint4*>(M.out) + (size_t)p0 * CPP;
+        if (!__any_sync(0xffffffffu, (c & ~zero) != 0u)) {
+            for (uint32_t i = lane; i < last * CPP; i += 32u) out[i] = make_uint4(0u, 0u, 0u, 0u);
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i += 2)
+            *reinterpret_cast<uint2*>(&ids[warp][lane][i]) = make_uint2(N[i], N[i + 1]);
+        masks[warp][lane] = make_uint4(s0, s0 & ~zero, rank, 0u);
+        __syncwarp();
+#pragma unroll 2
+        for (uint32_t i = lane; i < last * CPP; i += 32u) {
+            const uint32_t l = (i / CPP) * 2u, t0 = (i % CPP) * (NPC / 2u);   // even word's lane, its first node
+            uint32_t v[4];
+            const uint4 m0 = masks[warp][l], m1 = masks[warp][l + 1];
+            uint32_t mat[NPC];
+#pragma unroll
+            for (uint32_t j = 0; j < NPC; ++j) {
+                const uint4& q = j & 1u ? m1 : m0;
+                const uint32_t t = t0 + j / 2u, r = q.z + (t ? __popc(q.x >> (32u - t)) : 0u);
+                mat[j] = ((q.y << t) & 0x80000000u) && r < A.keysCap
+                             ? NT::keyMat(__ldg(reinterpret_cast<const uint32_t*>(A.keys) + r))
+                             : 0u;
+            }
+            const uint16_t* e = reinterpret_cast<const uint16_t*>(ids[warp][l]) + t0;
+            const uint16_t* o = reinterpret_cast<const uint16_t*>(ids[warp][l + 1]) + t0;
+            if (NT::bytes == 2) {
+                const uint2 a2 = *reinterpret_cast<const uint2*>(e), b2 = *reinterpret_cast<const uint2*>(o);
+                v[0] = __byte_perm(a2.x, b2.x, 0x5410) | (mat[0] << 12) | (mat[1] << 28);
+                v[1] = __byte_perm(a2.x, b2.x, 0x7632) | (mat[2] << 12) | (mat[3] << 28);
+                v[2] = __byte_perm(a2.y, b2.y, 0x5410) | (mat[NPC - 4] << 12) | (mat[NPC - 3] << 28);
+                v[3] = __byte_perm(a2.y, b2.y, 0x7632) | (mat[NPC - 2] << 12) | (mat[NPC - 1] << 28);
+            } else {
+                const uint32_t a1 = *reinterpret_cast<const uint32_t*>(e), b1 = *reinterpret_cast<const uint32_t*>(o);
+                v[0] = (a1 & 0xFFFFu) | (mat[0] << 16);
+                v[1] = (b1 & 0xFFFFu) | (mat[1] << 16);
+                v[2] = (a1 >> 16) | (mat[2] << 16);
+                v[3] = (b1 >> 16) | (mat[3] << 16);
+            }
+            out[i] = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+        __syncwarp();
     }
 }
 
@@ -830,8 +894,8 @@ void launch_partial_values(const Batch& b, const void* keys, const uint32_t* cou
     *launches += 1;
 }
 
-void launch_emit_fcc(int nodeKind, const Batch& b, const FccMesh* meshes, const uint64_t* groupBase,
-                     uint32_t nMeshes, uint64_t totalGroups, const uint32_t* fill, const uint32_t* surf,
+void launch_emit_fcc(int nodeKind, const Batch& b, const FccMesh* meshes, const uint64_t* pairBase,
+                     uint32_t nMeshes, uint64_t totalPairs, const uint32_t* fill, const uint32_t* surf,
                      const WordRank* ranks, const void* keys, uint32_t keysCap, bool raw, cudaStream_t s,
                      uint32_t* launches) {
     FccArgs A;
@@ -839,15 +903,15 @@ void launch_emit_fcc(int nodeKind, const Batch& b, const FccMesh* meshes, const 
     A.raw = raw ? 1u : 0u;
     A.b = b;
     A.meshes = meshes;
-    A.groupBase = groupBase;
+    A.pairBase = pairBase;
     A.nMeshes = nMeshes;
     A.fill = fill;
     A.surf = surf;
     A.ranks = ranks;
     A.keys = keys;
-    const uint32_t grid = gridFor(totalGroups, 256, 148u * 64u);
-    if (nodeKind == kShortFcc) emitFccKernel<kShortFcc><<<grid, 256, 0, s>>>(A, totalGroups);
-    else emitFccKernel<kLongFcc><<<grid, 256, 0, s>>>(A, totalGroups);
+    const uint32_t grid = gridFor(totalPairs, 8u * 16u, 148u * 64u);
+    if (nodeKind == kShortFcc) emitFccKernel<kShortFcc><<<grid, 256, 0, s>>>(A, totalPairs);
+    else emitFccKernel<kLongFcc><<<grid, 256, 0, s>>>(A, totalPairs);
     *launches += 1;
 }
 

@@ -158,7 +158,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     std::vector<uint32_t> slices;
     std::vector<uint8_t> later;
     std::vector<FccMesh> fccMeshes;
-    std::vector<uint64_t> groupBase{0};
+    std::vector<uint64_t> pairBase{0};
     anyMaterials_ = false;
     anyCartesian_ = false;
     uint64_t nodeCount = 0;
@@ -224,14 +224,14 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
         }
         if (j.nodes && fcc) {
             fccMeshes.push_back(FccMesh{firstUnit, j.out});
-            groupBase.push_back(groupBase.back() + gi.bytes / 16);
+            pairBase.push_back(pairBase.back() + ((gi.count / 64 + 15) & ~uint64_t(15)));
         }
     }
     nWork_ = workBase.back();
     totalWords_ = wordBase.back();
     totalRows_ = rowBase.back();
     nFcc_ = (uint32_t)fccMeshes.size();
-    totalGroups_ = groupBase.back();
+    totalPairs_ = pairBase.back();
     // Blocks of the first pruning pass.
     std::vector<uint32_t> pruneBase{0};
     prunePlanes_ = prune_planes(totalWords_);
@@ -256,7 +256,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     oLater_ = append(blob_, later);
     oPrune_ = append(blob_, pruneBase);
     oFcc_ = append(blob_, fccMeshes);
-    oGroupBase_ = append(blob_, groupBase);
+    oPairBase_ = append(blob_, pairBase);
     // Buffers.
     int rc;
     const size_t wordBytes = 4 * (size_t)totalWords_;
@@ -481,7 +481,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     }
     if (nFcc_)
         launch_emit_fcc(nodeKind_, b, reinterpret_cast<const FccMesh*>(tables.as<uint8_t>() + oFcc_),
-                        reinterpret_cast<const uint64_t*>(tables.as<uint8_t>() + oGroupBase_), nFcc_, totalGroups_,
+                        reinterpret_cast<const uint64_t*>(tables.as<uint8_t>() + oPairBase_), nFcc_, totalPairs_,
                         fillP, surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p, keysCap_, raw_, ps, &launches);
     mark(3, true);
     if (ps != s) {
@@ -616,8 +616,8 @@ int Pipeline::finish(cudaStream_t s) {
                                   ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, s, &launches);
         if (nFcc_)
             launch_emit_fcc(nodeKind_, b, reinterpret_cast<const FccMesh*>(tables.as<uint8_t>() + oFcc_),
-                            reinterpret_cast<const uint64_t*>(tables.as<uint8_t>() + oGroupBase_), nFcc_,
-                            totalGroups_, fillP, surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p, keysCap_, raw_, s,
+                            reinterpret_cast<const uint64_t*>(tables.as<uint8_t>() + oPairBase_), nFcc_,
+                            totalPairs_, fillP, surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p, keysCap_, raw_, s,
                             &launches);
         VXB_CUDA(cudaGetLastError());
         VXB_CUDA(cudaStreamSynchronize(s));
