@@ -210,11 +210,13 @@ void launch_fcc_boundaries(void* nodes, uint32_t X, uint32_t Y, uint32_t Z, uint
 void launch_partial_values(const Batch& b, const void* keys, const uint32_t* count, uint32_t cap,
                            unsigned long long* values, cudaStream_t s, uint32_t* launches);
 // Keys (PartialNodes: values) at ranks >= keysCap read as 0.
-// Words [wordBegin, totalWords) of the arena (wordBegin a multiple of 32).
-void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t wordBegin, uint64_t totalWords,
-                           const uint32_t* finalSolid,
-                           const uint32_t* fill, const uint32_t* surf, const WordRank* ranks, const void* keys,
-                           uint32_t keysCap, const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s,
+// Planes [zBegin, zEnd) of every unit.  spanBase: exclusive prefix over the
+// units of emit_spans (nUnits + 1 entries), `spans` their sum.
+uint32_t emit_spans(const PassGeom& g);
+void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* spanBase, uint32_t spans,
+                           uint32_t zBegin, uint32_t zEnd, const uint32_t* finalSolid, const uint32_t* fill,
+                           const uint32_t* surf, const WordRank* ranks, const void* keys, uint32_t keysCap,
+                           const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s,
                            uint32_t* launches);
 
 // An FCC mesh: its four sub-lattice units are units [unit0, unit0 + 4).

@@ -393,12 +393,12 @@ __device__ __forceinline__ WordNbrs loadNbrs(const UnitWords& u, uint32_t w) {
 // kOrientTable[x | y << 2 | z << 4] for those three codes (0 when an axis has
 // none), and each plane is the union of the code combinations whose id has
 // that bit set, evaluated on whole words at once.
-__device__ __forceinline__ void idPlanes(const WordNbrs& n, uint32_t cm, uint32_t P[5]) {
-    const uint32_t L = n.L, R = n.R;
+__device__ __forceinline__ void idPlanes(uint32_t L, uint32_t R, uint32_t In, uint32_t Out, uint32_t Dn, uint32_t Up,
+                                         uint32_t cm, uint32_t P[5]) {
     const uint32_t X1 = L & ~R, X3 = L & R, Xo = L ^ R, Xa = L | R, X2 = R & ~L;
-    const uint32_t Y1 = n.In & ~n.Out, Y2 = n.Out & ~n.In, Y3 = n.In & n.Out, Ya = n.In | n.Out;
-    const uint32_t Z1 = n.Dn & ~n.Up, Z2 = n.Up & ~n.Dn, Z3 = n.Dn & n.Up, Za = n.Dn | n.Up, Zo = n.Dn ^ n.Up;
-    P[0] = ((Za & ((Y1 & L) | (Y2 & X1))) | (Y3 & ((n.Dn & L) | (Z2 & X1)))) & cm;
+    const uint32_t Y1 = In & ~Out, Y2 = Out & ~In, Y3 = In & Out, Ya = In | Out;
+    const uint32_t Z1 = Dn & ~Up, Z2 = Up & ~Dn, Z3 = Dn & Up, Za = Dn | Up, Zo = Dn ^ Up;
+    P[0] = ((Za & ((Y1 & L) | (Y2 & X1))) | (Y3 & ((Dn & L) | (Z2 & X1)))) & cm;
     P[1] = ((Y1 & ((Zo & X2) | (Z3 & R))) | (Za & Y2 & L) | (Y3 & ((Z1 & X1) | (Z2 & L) | (Z3 & X3)))) & cm;
     P[2] = ((Z1 & ((Y2 & X2) | (Y3 & R))) | (Z2 & ((Y1 & Xa) | (Y2 & L) | (Y3 & X1))) | (Z3 & ((Y1 & X3) | (Y2 & R)))) &
            cm;
@@ -437,129 +437,258 @@ template <int NP> __device__ __forceinline__ void planeBytes(const uint32_t* P, 
     }
 }
 
-// 1- and 2-byte nodes.  Each lane owns one word and builds its 32 nodes in
-// its own shared-memory row: the ids of all 32 come from the bit planes of
-// idPlanes (or a constant for empty and all-interior words), the materials
-// of surface nodes from the merged keys, which are consecutive by rank (a
-// word whose 32 nodes are all surface nodes loads its 32 keys without a
-// per-node loop).  The warp's 32 rows are then stored as one contiguous
-// span.  Unit word bases are multiples of 32, so a warp's words belong to
-// one unit.
+// 1- and 2-byte nodes.  A warp takes 32 consecutive words of a plane, a lane
+// one of them, and walks `planes` planes along z: the words of the planes
+// below, at and above the current one stay in registers, positions are
+// divided out once, and a plane's loads are issued a plane ahead.
+//
+// Words of one id without surface nodes (none solid, or every node solid with
+// six solid neighbours: id 27) are stored at once.  The others, 2-26% of the
+// words but spread over a third to all of the chunks, are collected with
+// their neighbour words; once 32 are there, a lane takes each: its ids come
+// from the bit planes of idPlanes, the materials of its surface nodes from
+// the merged keys, which are consecutive by rank.  So the planes, transposes
+// and key loads run in full warps.
+//
+// Bounds: the store of the grid (131 us of the room's 864 MB), then issue of
+// integer instructions.  With every lane forming its own word at once the
+// room took 371 us (materials 126, ids and neighbours 86), 558 MB of a duct
+// 197 us, 143 MB without materials 72 us; with words collected but positions
+// and neighbours found per word 328, 172 and 58 us; now 259, 127 and 52 us.
+// The plane ahead is only in flight with 64 registers (four blocks per SM):
+// with 48 (five) the same code takes 320, 156 and 54 us.
+constexpr int kEmitWarps = 8;
+
+constexpr uint32_t kSparse = 4;   // most surface nodes of a sparse word
+constexpr uint32_t kSlots = 96;
+
+// The collected words of a warp: those with at most kSparse surface nodes
+// from slot 0 on, the others from the last slot down, so that the lanes of a
+// group need about as many key loads.  32 of a kind leave together, and a
+// step collects 32 at the most: 96 slots hold both.
+// a: index | flags << 27, solid, surface, rank of the first surface node;
+// b: the neighbour words In, Out, Dn, Up.
+struct EmitSlots {
+    uint4 a[kSlots], b[kSlots];
+};
+enum : uint32_t {
+    kHasPrev = 1u << 27,    // solid node before the first, after the last
+    kHasNext = 1u << 28,
+    kNoFirst = 1u << 29,    // first, last node cleared (border words)
+    kNoLast = 1u << 30,
+    kIndexMask = (1u << 27) - 1u
+};
+
+// The nodes of the n <= 32 words in slots [from, from + n) (whole warp).
 template <int K>
-__global__ void __launch_bounds__(256, 6) emitNarrowKernel(EmitArgs a, uint64_t wordBegin, uint64_t totalWords) {
+__device__ __forceinline__ void emitWords(const EmitArgs& args, const EmitSlots& slots, uint32_t from, uint32_t n,
+                                          uint32_t* __restrict__ stage, uint8_t* __restrict__ uOut, uint32_t lane) {
+    typedef NodeT<K> NT;
+    constexpr uint32_t NB = NT::bytes;
+    constexpr uint32_t CH = 2 * NB;              // 16-byte chunks of a word
+    constexpr uint32_t PITCH = 8 * NB + 4;       // 32-bit words of a padded row
+    uint32_t* const row = stage + lane * PITCH;
+    uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
+    if (lane < n) {
+        a = slots.a[from + lane];
+        b = slots.b[from + lane];
+    }
+    const uint32_t zero = (a.x & kNoFirst ? 0x80000000u : 0u) | (a.x & kNoLast ? 1u : 0u);
+    const uint32_t c = a.y, s0 = a.z;
+    {
+        uint32_t P[5], N[8];
+        idPlanes((c >> 1) | (a.x & kHasPrev ? 0x80000000u : 0u), (c << 1) | (a.x & kHasNext ? 1u : 0u), b.x, b.y, b.z,
+                 b.w, c & ~zero, P);
+        planeBytes<5>(P, N);
+#pragma unroll
+        for (int q = 0; q < 8; q += 2) {
+            if (NB == 1)
+                *reinterpret_cast<uint2*>(row + q) = make_uint2(N[q], N[q + 1]);
+            else
+                *reinterpret_cast<uint4*>(row + 2 * q) =
+                    make_uint4(__byte_perm(N[q], 0u, 0x4140), __byte_perm(N[q], 0u, 0x4342),
+                               __byte_perm(N[q + 1], 0u, 0x4140), __byte_perm(N[q + 1], 0u, 0x4342));
+        }
+    }
+    // Four surface nodes per step, so that their key loads are in flight
+    // together; keys past keysCap read as 0.
+    const uint32_t* const keys = reinterpret_cast<const uint32_t*>(args.keys);
+    uint8_t* const my = reinterpret_cast<uint8_t*>(row);
+    uint32_t r = a.w + (s0 & zero & 0x80000000u ? 1u : 0u);   // a cleared first node has a key too
+    for (uint32_t rest = s0 & ~zero; rest; r += 4) {
+        uint32_t bt[4], mat[4];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            bt[q] = __clz(rest);                 // node index in the word (32: none left)
+            rest &= ~(0x80000000u >> (bt[q] & 31u));
+            mat[q] = bt[q] < 32u && r + q < args.keysCap ? NT::keyMat(__ldg(keys + r + q)) : 0u;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            if (bt[q] == 32u) break;
+            if (NB == 1) my[bt[q]] |= (uint8_t)(mat[q] << 5);
+            else my[2 * bt[q] + 1] = (uint8_t)mat[q];
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t k = 0; k < CH; ++k) {
+        const uint32_t l = (k * 32u + lane) / CH, q = lane % CH;   // word and 16-byte chunk of it
+        const uint32_t w = __shfl_sync(0xffffffffu, a.x & kIndexMask, l);
+        if (l < n)
+            *reinterpret_cast<uint4*>(uOut + (size_t)w * (32u * NB) + 16u * q) =
+                *reinterpret_cast<const uint4*>(stage + l * PITCH + 4u * q);
+    }
+    __syncwarp();
+}
+
+template <int K>
+__global__ void __launch_bounds__(kEmitWarps * 32, 4) emitNarrowKernel(EmitArgs a, const uint32_t* __restrict__ spanBase,
+                                                                       uint32_t planes, uint32_t zBegin,
+                                                                       uint32_t zEnd) {
     typedef NodeT<K> NT;
     static_assert(NT::bytes <= 2, "narrow nodes only");
-    constexpr int NB = NT::bytes;
-    constexpr int WB = 32 * NB;                  // bytes of one word's nodes
-    constexpr int CH = WB / 16;                  // 16-byte chunks per word
-    constexpr int PITCH = (CH + 1) * 16;         // padded smem row (conflict-free)
-    __shared__ __align__(16) uint8_t stage[8][32 * PITCH];
+    constexpr uint32_t NB = NT::bytes;
+    constexpr uint32_t CH = 2 * NB;
+    constexpr uint32_t kFull = 0xffffffffu;
+    __shared__ __align__(16) uint32_t stageAll[kEmitWarps][32 * (8 * NB + 4)];
+    __shared__ EmitSlots slotsAll[kEmitWarps];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint8_t* my = stage[warp] + lane * PITCH;
-    const uint32_t v27 = (uint32_t)NT::pack(27u, 0u, 0.0f);
-    // Data of the unit last visited (a warp's words belong to one unit).
-    uint32_t cur = 0xFFFFFFFFu, nWords = 0;
-    uint64_t uBase = 0;
-    uint8_t* uOut = nullptr;
-    UnitWords uw{};
-    for (uint64_t gbase = wordBegin + ((uint64_t)blockIdx.x * 8u + warp) * 32u; gbase < totalWords;
-         gbase += (uint64_t)gridDim.x * 8u * 32u) {
-        const uint32_t u = a.b.nUnits > 1 ? unitOf(a.b.wordBase, a.b.nUnits, gbase) : 0u;
-        if (u != cur) {
-            cur = u;
-            const Unit& U = a.b.units[u];
-            nWords = U.g.ipx * U.g.AY * U.g.AZ;
-            uBase = U.wordBase;
-            uOut = static_cast<uint8_t*>(U.out);
-            uw = unitWords(a, U);
-        }
-        const uint32_t wbase = (uint32_t)(gbase - uBase);
-        if (wbase >= nWords) continue;            // padding after the unit's grid (whole warp)
-        const uint32_t w = wbase + lane;
-        WordNbrs n{};
-        uint32_t zero = 0u;
-        if (w < nWords) {
-            n = loadNbrs<K>(uw, w);
-            zero = borderMask(uw, w);
-        }
-        // Ids: none, all 27 (every node solid with six solid neighbours), or
-        // the bit-sliced planes.  Materials of surface nodes follow by rank
-        // (the rank is loaded first, so that its latency overlaps the ids).
-        const uint32_t cm = n.c & ~zero, sm = n.s0 & ~zero;
-        const uint32_t rank0 = sm ? a.ranks[uBase + w].rank : 0u;
-        if (cm == 0u || (cm & n.L & n.R & n.In & n.Out & n.Dn & n.Up) == 0xFFFFFFFFu) {
-            const uint32_t rep = cm == 0u ? 0u : NB == 1 ? v27 * 0x01010101u : v27 * 0x00010001u;
+    const uint32_t u = a.b.nUnits > 1 ? unitOf(spanBase, a.b.nUnits, blockIdx.x) : 0u;
+    const Unit& U = a.b.units[u];
+    const uint32_t ipx = U.g.ipx, AY = U.g.AY, AZ = U.g.AZ, plane = ipx * AY;
+    const uint32_t z0 = zBegin + blockIdx.y * planes, z1 = min(z0 + planes, min(AZ, zEnd));
+    const uint32_t first = ((blockIdx.x - (a.b.nUnits > 1 ? __ldg(spanBase + u) : 0u)) * kEmitWarps + warp) * 32u;
+    if (z0 >= z1 || first >= plane) return;   // whole warp
+    EmitSlots& slots = slotsAll[warp];
+    uint32_t* const stage = stageAll[warp];
+    uint8_t* const uOut = static_cast<uint8_t*>(U.out);
+    const uint32_t* const fin = a.fin + U.wordBase;
+    const uint32_t* const fill = a.fill + U.wordBase;
+    const uint32_t* const surf = U.materials ? a.surf + U.wordBase : nullptr;
+    const WordRank* const ranks = a.ranks + U.wordBase;
+    const uint8_t* const zLater = a.b.later + U.laterBase + AY;
+    const bool border = U.g.border != 0u;
+    // The lane's word (clamped to the plane) and its neighbours: offsets in
+    // the plane, and masks for those that do not exist.  Loads need no
+    // conditions that way; lanes past the plane are left out of every ballot.
+    const uint32_t j = min(first + lane, plane - 1u), y = U.g.divX.div(j), k = j - y * ipx;
+    const uint32_t wend = min(plane - first, 32u);
+    const uint32_t dead = wend < 32u ? kFull << wend : 0u;
+    const uint32_t mPrev = k > 0 ? 1u : 0u, mNext = k + 1 < ipx ? 1u : 0u;   // masks of one bit
+    const uint32_t mIn = y > 0 ? kFull : 0u, mOut = y + 1 < AY ? kFull : 0u;
+    const uint32_t jIn = y > 0 ? j - ipx : j, jOut = y + 1 < AY ? j + ipx : j;
+    const bool outLater = y + 1 < AY && a.b.later[U.laterBase + y];
+    const bool anyLater = __any_sync(kFull, outLater);
+    // Neighbour words along x are in the next lanes; the first and last lane
+    // load theirs.
+    const uint32_t jEdge = lane == 0 && k > 0 ? j - 1u : lane == 31 && k + 1 < ipx ? j + 1u : j;
+    // Planes of [z0, z1) that lie below a later subspace (at most 64).
+    uint64_t later = 0;
 #pragma unroll
-            for (int i = 0; i < CH; ++i) *reinterpret_cast<uint4*>(my + 16 * i) = make_uint4(rep, rep, rep, rep);
-        } else {
-            uint32_t N[8];
-            {
-                uint32_t P[5];
-                idPlanes(n, cm, P);
-                planeBytes<5>(P, N);
-            }
-#pragma unroll
-            for (int i = 0; i < CH; ++i) {
-                uint4 q;
-                if (NB == 1) {
-                    q = make_uint4(N[4 * i], N[4 * i + 1], N[4 * i + 2], N[4 * i + 3]);
-                } else {
-                    q = make_uint4(__byte_perm(N[2 * i], 0u, 0x4140), __byte_perm(N[2 * i], 0u, 0x4342),
-                                   __byte_perm(N[2 * i + 1], 0u, 0x4140), __byte_perm(N[2 * i + 1], 0u, 0x4342));
-                }
-                *reinterpret_cast<uint4*>(my + 16 * i) = q;
-            }
-        }
-        if (sm) {
-            const uint32_t* keys = reinterpret_cast<const uint32_t*>(a.keys);
-            if (sm == 0xFFFFFFFFu && (uint64_t)rank0 + 32u <= a.keysCap) {
-                // 32 surface nodes: their keys are the 32 from rank0 on.
-#pragma unroll 8
-                for (uint32_t j = 0; j < 32u; ++j) {
-                    const uint32_t mat = NT::keyMat(__ldg(keys + rank0 + j));
-                    if (NB == 1) my[j] |= (uint8_t)(mat << 5);
-                    else my[2 * j + 1] = (uint8_t)mat;
-                }
-            } else {
-                // Four surface nodes per step, so that their key loads are
-                // in flight together.
-                constexpr int kKeys = 4;
-                uint32_t rest = sm;
-                do {
-                    uint32_t bt[kKeys], mat[kKeys];
-#pragma unroll
-                    for (int q = 0; q < kKeys; ++q) {
-                        bt[q] = 32u;
-                        if (rest) {
-                            bt[q] = __clz(rest);       // node index in the word
-                            rest &= ~(0x80000000u >> bt[q]);
-                        }
-                    }
-#pragma unroll
-                    for (int q = 0; q < kKeys; ++q) {
-                        const uint32_t r = rank0 + (bt[q] ? __popc(n.s0 >> (32u - bt[q])) : 0u);
-                        mat[q] = bt[q] < 32u && r < a.keysCap ? NT::keyMat(__ldg(keys + r)) : 0u;
-                    }
-#pragma unroll
-                    for (int q = 0; q < kKeys; ++q) {
-                        if (bt[q] == 32u) break;
-                        if (NB == 1) my[bt[q]] |= (uint8_t)(mat[q] << 5);
-                        else my[2 * bt[q] + 1] = (uint8_t)mat[q];
-                    }
-                } while (rest);
-            }
-        }
-        __syncwarp();
-        const uint32_t wend = wbase + 32u <= nWords ? 32u : nWords - wbase;
-        uint4* out = reinterpret_cast<uint4*>(uOut + (size_t)wbase * WB);
-#pragma unroll
-        for (int i = 0; i < CH; ++i) {
-            const uint32_t chunk = i * 32 + lane;       // 16-byte chunk of the warp's span
-            const uint32_t wi = chunk / CH, ci = chunk % CH;
-            if (wi < wend) out[chunk] = *reinterpret_cast<const uint4*>(stage[warp] + wi * PITCH + 16 * ci);
-        }
-        __syncwarp();
+    for (uint32_t h = 0; h < 2; ++h) {
+        const uint32_t z = z0 + 32u * h + lane;
+        later |= (uint64_t)__ballot_sync(kFull, z < z1 && z + 1 < AZ && zLater[z]) << (32u * h);
     }
+    struct Plane {
+        uint32_t In, Out, edge, up;   // `up`: the word of the plane above
+    };
+    auto load = [&](uint32_t z) {
+        const uint32_t* __restrict__ f = fin + (size_t)z * plane;
+        Plane p;
+        p.In = __ldg(f + jIn);
+        p.Out = __ldg(f + jOut);
+        p.edge = __ldg(f + jEdge);
+        p.up = z + 1 < AZ ? __ldg(f + plane + j) : 0u;
+        return p;
+    };
+    const uint32_t v27 = NB == 1 ? 27u * 0x01010101u : 27u * 0x00010001u;
+    uint32_t nSparse = 0, nDense = 0;   // collected words
+    uint32_t Dn = z0 > 0 ? __ldg(fin + (size_t)(z0 - 1) * plane + j) : 0u;
+    uint32_t c = __ldg(fin + (size_t)z0 * plane + j);
+    uint4* out = reinterpret_cast<uint4*>(uOut) + ((size_t)(z0 * plane + first) * CH + lane);
+    Plane next = load(z0);
+    // Surface words are loaded two planes ahead, so that the rank of a word
+    // that has surface nodes can be loaded one plane ahead.
+    auto surfAt = [&](uint32_t z) { return surf && z < z1 ? __ldg(surf + (size_t)z * plane + j) : 0u; };
+    auto rankAt = [&](uint32_t z, uint32_t word) { return word ? __ldg(&ranks[z * plane + j].rank) : 0u; };
+    uint32_t s0 = surfAt(z0), nextS = surfAt(z0 + 1u), rank = rankAt(z0, s0);
+    for (uint32_t z = z0; z < z1; ++z, out += (size_t)plane * CH) {
+        const Plane p = next;
+        const uint32_t w = z * plane + j;
+        next = load(min(z + 1, z1 - 1u));
+        const uint32_t nextRank = rankAt(z + 1u, nextS), afterS = surfAt(z + 2u);
+        uint32_t Out = p.Out & mOut, Up = p.up;
+        const uint32_t In = p.In & mIn;
+        // Rows and planes that start a later pruning subspace are read from
+        // the unpruned grid.
+        if (anyLater && outLater) Out = __ldg(fill + (w + ipx)) | (surf ? __ldg(surf + (w + ipx)) : 0u);
+        if ((later >> (z - z0)) & 1ull) Up = __ldg(fill + (w + plane)) | (surf ? __ldg(surf + (w + plane)) : 0u);
+        uint32_t before = __shfl_up_sync(kFull, c, 1), after = __shfl_down_sync(kFull, c, 1);
+        before = (lane == 0 ? p.edge : before) & mPrev;
+        after = ((lane == 31 ? p.edge : after) >> 31) & mNext;
+        uint32_t zero = 0u, flags = (before ? kHasPrev : 0u) | (after ? kHasNext : 0u);
+        if (border) {
+            // zeroPadding (src/voxelizer.cu:4811-4844).
+            zero = mIn == 0u || mOut == 0u || z == 0 || z + 1 == AZ ? kFull : (mPrev ^ 1u) << 31 | (mNext ^ 1u);
+            flags |= (mPrev ? 0u : kNoFirst) | (mNext ? 0u : kNoLast);
+        }
+        const uint32_t cm = c & ~zero, sm = s0 & ~zero;
+        const bool full = (cm & ((c >> 1) | before << 31) & ((c << 1) | after) & In & Out & Dn & Up) == kFull;
+        const uint32_t rest = __ballot_sync(kFull, sm != 0u || (cm != 0u && !full)) & ~dead;
+        const uint32_t fulls = __ballot_sync(kFull, full);
+        if ((rest | dead) == 0u && (fulls == 0u || fulls == kFull)) {
+            const uint32_t v = fulls ? v27 : 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < CH; ++q) out[q * 32u] = make_uint4(v, v, v, v);
+        } else {
+            // 16-byte chunk q * 32 + lane belongs to word q * (32 / CH) + lane / CH.
+            const uint32_t skip = (rest | dead) >> (lane / CH), ones = fulls >> (lane / CH);
+#pragma unroll
+            for (uint32_t q = 0; q < CH; ++q) {
+                const uint32_t v = (ones >> (q * (32u / CH))) & 1u ? v27 : 0u;
+                if (!((skip >> (q * (32u / CH))) & 1u)) out[q * 32u] = make_uint4(v, v, v, v);
+            }
+            if (rest) {
+                const uint32_t dense = __ballot_sync(kFull, __popc(s0) > (int)kSparse) & rest;
+                if ((rest >> lane) & 1u) {
+                    const uint32_t below = laneMaskLt();
+                    const uint32_t at = (dense >> lane) & 1u ? kSlots - 1u - nDense - __popc(dense & below)
+                                                             : nSparse + __popc(rest & ~dense & below);
+                    slots.a[at] = make_uint4(w | flags, c, s0, rank);
+                    slots.b[at] = make_uint4(In, Out, Dn, Up);
+                }
+                nDense += __popc(dense);
+                nSparse += __popc(rest & ~dense);
+                __syncwarp();
+                if (nSparse >= 32u) {
+                    nSparse -= 32u;
+                    emitWords<K>(a, slots, nSparse, 32u, stage, uOut, lane);
+                }
+                if (nDense >= 32u) {
+                    nDense -= 32u;
+                    emitWords<K>(a, slots, kSlots - 32u - nDense, 32u, stage, uOut, lane);
+                }
+            }
+        }
+        Dn = c;
+        c = p.up;
+        s0 = nextS;
+        nextS = afterS;
+        rank = nextRank;
+    }
+    // The rest, both kinds together where they fit one group.
+    if (nSparse + nDense <= 32u && nDense) {
+        if (lane < nDense) {
+            slots.a[nSparse + lane] = slots.a[kSlots - 1u - lane];
+            slots.b[nSparse + lane] = slots.b[kSlots - 1u - lane];
+        }
+        __syncwarp();
+        nSparse += nDense;
+        nDense = 0u;
+    }
+    if (nSparse) emitWords<K>(a, slots, 0u, nSparse, stage, uOut, lane);
+    if (nDense) emitWords<K>(a, slots, kSlots - nDense, nDense, stage, uOut, lane);
 }
 
 // Values of PartialNode surface nodes by rank (the node without its id): the
@@ -594,21 +723,23 @@ __global__ void __launch_bounds__(128) partialValuesKernel(Batch b, const unsign
 // lanes of a warp worked at a time: 4.5 M nodes (36 MB) with 118,463 surface
 // nodes took 395 us; now 27 us of values and 14 us of emission.  Sharing the
 // ratios out inside blocks of 128 words instead took 75 us (64 words: 90).
-__global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t wordBegin, uint64_t totalWords) {
+__global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t totalWords, uint32_t zBegin, uint32_t zEnd) {
     typedef NodeT<kPartial> NT;
     __shared__ uint32_t ids[8][32][9];          // 32 ids a word, padded
     __shared__ uint32_t masks[8][32][4];        // surface, surface less cleared nodes, fill, rank
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint64_t gbase = wordBegin + ((uint64_t)blockIdx.x * 8u + warp) * 32u; gbase < totalWords;
+    for (uint64_t gbase = ((uint64_t)blockIdx.x * 8u + warp) * 32u; gbase < totalWords;
          gbase += (uint64_t)gridDim.x * 8u * 32u) {
         const uint32_t u = a.b.nUnits > 1 ? unitOf(a.b.wordBase, a.b.nUnits, gbase) : 0u;
         const Unit& U = a.b.units[u];
-        const uint32_t nWords = U.g.ipx * U.g.AY * U.g.AZ, wbase = (uint32_t)(gbase - U.wordBase);
-        if (wbase >= nWords) continue;          // padding after the unit's grid (whole warp)
-        const uint32_t w = wbase + lane;
+        // The words of planes [zBegin, zEnd).
+        const uint32_t plane = U.g.ipx * U.g.AY, wLo = min(zBegin, U.g.AZ) * plane, nWords = min(zEnd, U.g.AZ) * plane;
+        const uint32_t wbase = (uint32_t)(gbase - U.wordBase);
+        if (wbase >= nWords || wbase + 32u <= wLo) continue;   // whole warp
+        const uint32_t w = wbase + lane, wbeg = wLo > wbase ? wLo - wbase : 0u;
         WordNbrs n{};
         uint32_t zero = 0u;
-        if (w < nWords) {
+        if (w >= wLo && w < nWords) {
             const UnitWords uw = unitWords(a, U);
             n = loadNbrs<kPartial>(uw, w);
             zero = borderMask(uw, w);
@@ -617,14 +748,14 @@ __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t wo
         uint4* out = reinterpret_cast<uint4*>(U.out) + (size_t)wbase * 16u;
         const uint32_t wend = min(nWords - wbase, 32u);
         if (!__any_sync(0xffffffffu, (cm | sm | fm) != 0u)) {
-            for (uint32_t i = lane; i < wend * 16u; i += 32u) out[i] = make_uint4(0u, 0u, 0u, 0u);
+            for (uint32_t i = wbeg * 16u + lane; i < wend * 16u; i += 32u) out[i] = make_uint4(0u, 0u, 0u, 0u);
             continue;
         }
         {
             uint32_t N[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
             if (cm) {
                 uint32_t P[5];
-                idPlanes(n, cm, P);
+                idPlanes(n.L, n.R, n.In, n.Out, n.Dn, n.Up, cm, P);
                 planeBytes<5>(P, N);
             }
 #pragma unroll
@@ -634,7 +765,7 @@ __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t wo
             make_uint4(n.s0, sm, fm, sm ? a.ranks[U.wordBase + w].rank : 0u);
         __syncwarp();
 #pragma unroll 4
-        for (uint32_t i = lane; i < wend * 16u; i += 32u) {
+        for (uint32_t i = wbeg * 16u + lane; i < wend * 16u; i += 32u) {
             const uint32_t l = i >> 4, p = (i & 15u) * 2u;   // word and its first node
             const uint32_t id2 = reinterpret_cast<const uint16_t*>(ids[warp][l])[p >> 1];
             const uint4 m = *reinterpret_cast<const uint4*>(masks[warp][l]);
@@ -865,10 +996,13 @@ void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, con
     *launches += 1;
 }
 
-void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t wordBegin, uint64_t totalWords,
-                           const uint32_t* finalSolid,
-                           const uint32_t* fill, const uint32_t* surf, const WordRank* ranks, const void* keys,
-                           uint32_t keysCap, const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s, uint32_t* launches) {
+uint32_t emit_spans(const PassGeom& g) { return (g.ipx * g.AY + kEmitWarps * 32u - 1) / (kEmitWarps * 32u); }
+
+void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* spanBase, uint32_t spans,
+                           uint32_t zBegin, uint32_t zEnd, const uint32_t* finalSolid, const uint32_t* fill,
+                           const uint32_t* surf, const WordRank* ranks, const void* keys, uint32_t keysCap,
+                           const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s,
+                           uint32_t* launches) {
     EmitArgs a;
     a.keysCap = keysCap;
     a.b = b;
@@ -878,12 +1012,19 @@ void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t wordBegin, uin
     a.ranks = ranks;
     a.keys = keys;
     a.values = values;
-    const uint64_t words = totalWords - wordBegin;
-    const uint32_t grid = gridFor(words, 256, 148u * blocksPerSm);
-    switch (nodeKind) {
-    case kShort: emitNarrowKernel<kShort><<<grid, 256, 0, s>>>(a, wordBegin, totalWords); break;
-    case kLong: emitNarrowKernel<kLong><<<grid, 256, 0, s>>>(a, wordBegin, totalWords); break;
-    default: emitPartialKernel<<<gridFor(words, 256, 148u * 64u), 256, 0, s>>>(a, wordBegin, totalWords); break;
+    if (nodeKind == kPartial) {
+        emitPartialKernel<<<gridFor(totalWords, 256, 148u * 64u), 256, 0, s>>>(a, totalWords, zBegin, zEnd);
+    } else {
+        // Planes per warp: 2 * blocksPerSm blocks per SM share the grid (their
+        // work differs, so more of them balance better), but a warp's set-up
+        // pays for 8 planes where 8 blocks per SM remain.
+        const uint64_t chunks = totalWords / (32u * kEmitWarps);
+        const uint64_t share = chunks / (148u * 2u * blocksPerSm), least = std::min<uint64_t>(8, chunks / (148u * 8u));
+        const uint32_t planes = (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(1, std::max(share, least)));
+        const dim3 grid(spans, (zEnd - zBegin + planes - 1) / planes);
+        if (nodeKind == kShort)
+            emitNarrowKernel<kShort><<<grid, kEmitWarps * 32, 0, s>>>(a, spanBase, planes, zBegin, zEnd);
+        else emitNarrowKernel<kLong><<<grid, kEmitWarps * 32, 0, s>>>(a, spanBase, planes, zBegin, zEnd);
     }
     *launches += 1;
 }

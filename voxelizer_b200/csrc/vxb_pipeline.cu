@@ -242,6 +242,14 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
             pruneBase.push_back((uint32_t)blocks);
         }
     pruneBlocks_ = pruneBase.back();
+    // Blocks of a plane and planes of the emission.
+    std::vector<uint32_t> spanBase{0};
+    maxPlanes_ = 0;
+    for (const Unit& u : units_) {
+        spanBase.push_back(spanBase.back() + emit_spans(u.g));
+        maxPlanes_ = std::max(maxPlanes_, u.g.AZ);
+    }
+    emitSpans_ = spanBase.back();
     // A single plain voxelization writes its solid grid straight into the
     // caller's buffer.
     aliasFill_ = !nodes_ && jobs.size() == 1;
@@ -255,6 +263,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     oSlices_ = append(blob_, slices);
     oLater_ = append(blob_, later);
     oPrune_ = append(blob_, pruneBase);
+    oSpans_ = append(blob_, spanBase);
     oFcc_ = append(blob_, fccMeshes);
     oPairBase_ = append(blob_, pairBase);
     // Buffers.
@@ -453,29 +462,26 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     else if (anyCartesian_) {
         tuneMark(kKnobEmit, false, ps);
         if (hostOut_ && units_.size() == 1) {
-            // The node array in kOutChunks word ranges, each copied to the
-            // caller's pinned host buffer on the copy stream as soon as it
+            // The node array in kOutChunks ranges of planes, each copied to
+            // the caller's pinned host buffer on the copy stream as soon as it
             // is written, so the copy of the first ranges overlaps the rest.
             const Unit& u = units_[0];
-            const uint64_t words = (uint64_t)u.g.ipx * u.g.AY * u.g.AZ;
-            const uint64_t wordBytes = hostBytes_ / words;
+            const uint64_t planeBytes = hostBytes_ / u.g.AZ;
             for (uint32_t k = 0; k < kOutChunks; ++k) {
-                const uint64_t w0 = (words * k / kOutChunks) & ~uint64_t(31);
-                const uint64_t w1 = k + 1 == kOutChunks ? words : (words * (k + 1) / kOutChunks) & ~uint64_t(31);
-                if (w1 <= w0) continue;
-                launch_emit_cartesian(nodeKind_, b, w0, w1, fin.as<uint32_t>(), fillP, surf.as<uint32_t>(),
-                                      ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, ps, &launches);
+                const uint32_t p0 = (uint32_t)((uint64_t)u.g.AZ * k / kOutChunks);
+                const uint32_t p1 = (uint32_t)((uint64_t)u.g.AZ * (k + 1) / kOutChunks);
+                if (p1 <= p0) continue;
+                emitCartesian(p0, p1, ps);
                 if (!outEv_[k]) VXB_CUDA(cudaEventCreateWithFlags(&outEv_[k], cudaEventDisableTiming));
                 VXB_CUDA(cudaEventRecord(outEv_[k], ps));
                 VXB_CUDA(cudaStreamWaitEvent(copyStream_, outEv_[k], 0));
-                VXB_CUDA(cudaMemcpyAsync(static_cast<uint8_t*>(hostOut_) + w0 * wordBytes,
-                                         static_cast<const uint8_t*>(u.out) + w0 * wordBytes, (w1 - w0) * wordBytes,
+                VXB_CUDA(cudaMemcpyAsync(static_cast<uint8_t*>(hostOut_) + p0 * planeBytes,
+                                         static_cast<const uint8_t*>(u.out) + p0 * planeBytes, (p1 - p0) * planeBytes,
                                          cudaMemcpyDeviceToHost, copyStream_));
             }
             hostCopied_ = true;
         } else {
-            launch_emit_cartesian(nodeKind_, b, 0, totalWords_, fin.as<uint32_t>(), fillP, surf.as<uint32_t>(),
-                                  ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, ps, &launches);
+            emitCartesian(0, maxPlanes_, ps);
         }
         tuneMark(kKnobEmit, true, ps);
     }
@@ -490,6 +496,13 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     }
     VXB_CUDA(cudaGetLastError());
     return 0;
+}
+
+void Pipeline::emitCartesian(uint32_t zBegin, uint32_t zEnd, cudaStream_t s) {
+    launch_emit_cartesian(nodeKind_, batch(), totalWords_, reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oSpans_),
+                          emitSpans_, zBegin, zEnd, fin.as<uint32_t>(), fill.as<uint32_t>(), surf.as<uint32_t>(),
+                          ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(),
+                          shape.emitBlocksPerSm, s, &launches);
 }
 
 // Full passes until nothing changes, with a host check after each.
@@ -612,8 +625,7 @@ int Pipeline::finish(cudaStream_t s) {
             launch_emit_raw(nodeKind_, b, totalWords_, fillP, surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p,
                             keysCap_, values.as<unsigned long long>(), s, &launches);
         else if (anyCartesian_)
-            launch_emit_cartesian(nodeKind_, b, 0, totalWords_, fin.as<uint32_t>(), fillP, surf.as<uint32_t>(),
-                                  ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(), shape.emitBlocksPerSm, s, &launches);
+            emitCartesian(0, maxPlanes_, s);
         if (nFcc_)
             launch_emit_fcc(nodeKind_, b, reinterpret_cast<const FccMesh*>(tables.as<uint8_t>() + oFcc_),
                             reinterpret_cast<const uint64_t*>(tables.as<uint8_t>() + oPairBase_), nFcc_,
