@@ -89,6 +89,23 @@ __device__ __forceinline__ double divBy(double x, double d, double r) {
     return __fma_rn(__fma_rn(-q, d, x), r, q);
 }
 
+// The same in FP32, for operands within 2^+-60.
+__host__ __device__ __forceinline__ bool divScaleF(float x) {
+#ifdef __CUDA_ARCH__
+    const uint32_t h = __float_as_uint(x);
+#else
+    uint32_t h;
+    memcpy(&h, &x, 4);
+#endif
+    return (h & 0x7FFFFFFFu) - 0x21800000u < 0x3C000000u;
+}
+__device__ __forceinline__ bool divExactF(float x) { return divScaleF(x) || x == 0.0f; }
+__device__ __forceinline__ float divByF(float x, float d, float r) {
+    float q = __fmul_rn(x, r);
+    q = __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+    return __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+}
+
 // Blocks for `work` items at `threads` per block, capped (grid-stride loops).
 inline uint32_t gridFor(uint64_t work, uint32_t threads, uint32_t cap = 148u * 32u) {
     uint64_t b = (work + threads - 1) / threads;
@@ -96,8 +113,9 @@ inline uint32_t gridFor(uint64_t work, uint32_t threads, uint32_t cap = 148u * 3
     return (uint32_t)(b < cap ? b : cap);
 }
 
-// 1 / d for divBy.
+// 1 / d for divBy and divByF.
 inline double divReciprocal(double d) { return divScale(d) ? 1.0 / d : 0.0; }
+inline float divReciprocalF(float d) { return divScaleF(d) ? 1.0f / d : 0.0f; }
 
 }  // namespace detail
 }  // namespace vxb

@@ -44,13 +44,13 @@ struct PassGeom {
     double rd;           // 1 / d, or 0 (divBy)
     float mnf[3];        // float(mn) for the FP32 surface path
     float df;            // float(d)
+    float rdf;           // 1 / df, or 0 (divByF)
     uint32_t X;          // voxels along x (padded and rounded to 32 * xSplits)
     uint32_t resY, resZ; // voxels along y / z before the 1-voxel padding
     uint32_t AY, AZ;     // allocated rows: resY + 2, resZ + 2
     uint32_t ipx;        // 32-bit words per row: X / 32
     uint32_t padY, padZ; // allocation row / plane of local voxel row / plane 0 (1, or 0 next to a neighbour)
     uint32_t border;     // zero the allocation's faces in the node output (a device space with neighbours)
-    uint32_t pad0;
     FastDiv divX, divY;  // by ipx and by AY
 };
 
@@ -114,33 +114,35 @@ void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* tot
 void launch_row_fill(const Batch& b, uint64_t nRows, uint32_t* fill, cudaStream_t s, uint32_t* launches);
 
 // ---- Surface voxelization: src/voxelizer.cu:2358-2989, 3040-4201 ----
-// Triangles with surface work are partitioned into kSurfaceBuckets buckets
-// by (class, axis); each gets a kSurfRecBytes record and a kSurfOvlBytes
-// block of projection edge functions.
+// Triangles with surface work get consecutive positions (ordered by (class,
+// axis) inside each block of the set-up kernel), each with a kSurfRecBytes
+// record and, for 3D boxes, a kSurfDepthBytes one.
 constexpr uint32_t kSurfaceBuckets = 9;
-constexpr size_t kSurfRecBytes = 64;
-constexpr size_t kSurfOvlBytes = 112;
+constexpr size_t kSurfRecBytes = 80;
+constexpr size_t kSurfDepthBytes = 112;
 
-// Classify (codes / units in work-triangle order, per-bucket counts in
-// buckets[0..9)), then partition (unitsP in partitioned order; buckets[9..18)
-// are cursors) and set up (records) the work triangles of units with
-// materials.  buckets and unitsP[0..nWork] must be zero on entry.
-void launch_surface_prepare(const Batch& b, uint32_t nWork, uint32_t* codes, uint32_t* units, uint32_t* buckets,
-                            uint32_t* unitsP, void* recs, void* ovl, cudaStream_t s, uint32_t* launches);
-// Surface work over the exclusive scan `offsets` of unitsP (nWork + 1
-// entries), one thread per column.  mode 0: set bits in the `surf` arena and
-// append (bit position << 24 | key) to `list` (entries past listCap are
-// counted, not stored); mode 1: merge every hit's key at its rank (needs
-// complete bits and their `ranks`) and, where `positions` is not NULL, store
-// its arena position there too (PartialNode).  wide: 64-bit keys (PartialNode).  kind: the
-// node type, whose instantiation of the class kernels the arithmetic
-// follows.  queue: as for launch_solid_toggle, per warp.
-void launch_surface_work(int kind, int mode, int wide, const Batch& b, const void* recs, const void* ovl,
-                         const uint32_t* offsets, uint32_t nWork, const uint32_t* total, const uint32_t* buckets,
+// Classification and set-up of the work triangles of units with materials:
+// records, first work unit per position (offsets), mesh triangle per position
+// (triOf, may be NULL).  *cursor, *total (the exact number of work units) and
+// classes[0..3) (triangles per class) are zero on entry.
+void launch_surface_prepare(const Batch& b, uint32_t nWork, unsigned long long* cursor, unsigned long long* total,
+                            uint32_t* classes, uint32_t* offsets, uint32_t* triOf, void* recs, void* depth,
+                            cudaStream_t s, uint32_t* launches);
+// Surface work over what launch_surface_prepare wrote, one thread per column.
+// mode 0: set bits in the `surf` arena and append (bit position << 24 | key)
+// to `list` (entries past listCap are counted, not stored); mode 1: merge
+// every hit's key at its rank (needs complete bits and their `ranks`) and, for
+// PartialNodes (64-bit keys), store its arena position in `positions`; mode 2:
+// set bits only.  kind: the node type, whose instantiation of the class
+// kernels the arithmetic follows.  batch: 32-item chunks a warp takes at a
+// time.  queue: as for launch_solid_toggle.  Nothing is done when *total is
+// 2^32 - 1 or more.
+void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, const void* depth, const uint32_t* triOf,
+                         const uint32_t* offsets, const unsigned long long* cursor, const unsigned long long* total,
                          uint32_t* surf, const WordRank* ranks, void* keys, uint32_t keysCap,
-                         unsigned long long* positions, unsigned long long* list, uint32_t* listCount, uint32_t listCap,
-                         uint32_t blocksPerSm,
-                         uint32_t batch, uint32_t* queue, cudaStream_t s, uint32_t* launches);
+                         unsigned long long* positions, unsigned long long* list, uint32_t* listCount,
+                         uint32_t listCap, uint32_t blocksPerSm, uint32_t batch, uint32_t* queue, cudaStream_t s,
+                         uint32_t* launches);
 // Exclusive popcount prefix over `words` surface words, stored beside each
 // word; *total = surface voxels.
 void launch_surface_rank(const uint32_t* bits, uint64_t words, WordRank* ranks, uint32_t* tileSums, uint32_t* total,

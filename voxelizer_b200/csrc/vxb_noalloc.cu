@@ -225,6 +225,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     g.d = bg.d;
     g.rd = vxb::detail::divReciprocal(bg.d);
     g.df = (float)bg.d;
+    g.rdf = vxb::detail::divReciprocalF(g.df);
     g.X = bg.res[0];
     g.resY = bg.res[1];
     g.resZ = bg.res[2];

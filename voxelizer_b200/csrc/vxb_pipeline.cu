@@ -20,12 +20,13 @@ namespace {
 
 // Slots of the status buffer; pruning flags follow at kFlags.
 // kSolidTotal and kSolidHigh are the low and high word of one 64-bit count.
-enum : int { kSolidTotal = 0, kSolidHigh = 1, kSurfTotal = 2, kSurfOverflow = 3, kHitCount = 4,
-             kSurfaceVoxels = 5, kSurfQueue = 6, kToggleQueue = 7, kBigCount = 8, kPruneOverflow = 9,
-             kPruneCounts = 10 };
+// kSurfTotal and kSurfHigh likewise; kSurfCursor takes two words.
+enum : int { kSolidTotal = 0, kSolidHigh = 1, kSurfTotal = 2, kSurfHigh = 3, kSurfCursor = 4, kHitCount = 6,
+             kSurfaceVoxels = 7, kSurfQueue = 8, kToggleQueue = 9, kBigCount = 10, kPruneOverflow = 11,
+             kSurfClasses = 12, kPruneCounts = 15 };
 
 // The work counts take 32 bits: totals of 2^32 - 1 or more are refused.
-bool solidOverflow(const uint32_t* h) { return h[kSolidHigh] || h[kSolidTotal] == 0xFFFFFFFFu; }
+bool countOverflow(const uint32_t* h) { return h[1] || h[0] == 0xFFFFFFFFu; }
 
 const uint32_t kNodeBytes[5] = {1, 2, 8, 2, 4};
 
@@ -95,6 +96,7 @@ PassGeom makeGeom(const Plan& p, int lattice, bool turned) {
     g.d = p.d;
     g.rd = detail::divReciprocal(p.d);
     g.df = (float)p.d;
+    g.rdf = detail::divReciprocalF(g.df);
     g.X = p.res[0];
     g.resY = p.res[1];
     g.resZ = p.res[2];
@@ -104,7 +106,6 @@ PassGeom makeGeom(const Plan& p, int lattice, bool turned) {
     g.padY = p.padY;
     g.padZ = p.padZ;
     g.border = p.border ? 1u : 0u;
-    g.pad0 = 0;
     g.divX = FastDiv::of(g.ipx);
     g.divY = FastDiv::of(g.AY);
     return g;
@@ -299,17 +300,13 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
             VXB_CUDA(cudaEventCreateWithFlags(&evSolid_, cudaEventDisableTiming));
             VXB_CUDA(cudaEventCreateWithFlags(&evHiDone_, cudaEventDisableTiming));
         }
-        if ((rc = sCounts.ensure(4 * ((size_t)nWork_ + 2)))) return rc;
-        if ((rc = sOffsets.ensure(4 * ((size_t)nWork_ + 2)))) return rc;
-        if ((rc = sTileSums.ensure(4 * ((size_t)nWork_ / 4096 + 2)))) return rc;
+        if ((rc = sOffsets.ensure(4 * (size_t)nWork_))) return rc;
+        if (wide_ && (rc = triOf.ensure(4 * (size_t)nWork_))) return rc;
         if ((rc = surf.ensure(wordBytes))) return rc;
         if ((rc = ranks.ensure(2 * wordBytes))) return rc;
         if ((rc = rankTiles.ensure(4 * ((size_t)totalWords_ / 2048 + 2)))) return rc;
-        if ((rc = codes.ensure(4 * (size_t)nWork_))) return rc;
-        if ((rc = unitCounts.ensure(4 * (size_t)nWork_))) return rc;
-        if ((rc = buckets.ensure(4 * 2 * kSurfaceBuckets))) return rc;
         if ((rc = recs.ensure(kSurfRecBytes * (size_t)nWork_))) return rc;
-        if ((rc = ovl.ensure(kSurfOvlBytes * (size_t)nWork_))) return rc;
+        if ((rc = depth.ensure(kSurfDepthBytes * (size_t)nWork_))) return rc;
         // Hit list: 8-byte entries (bit position << 24 | key).  PartialNode
         // keys are 64-bit and always take the second traversal.  With the
         // list, the surface voxels are at most its entries.
@@ -365,12 +362,10 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         }
         if (timer) timer->mark(1, false, ss);
         VXB_CUDA(cudaMemsetAsync(surf.p, 0, 4 * (size_t)totalWords_, ss));
-        VXB_CUDA(cudaMemsetAsync(buckets.p, 0, 4 * 2 * kSurfaceBuckets, ss));
-        VXB_CUDA(cudaMemsetAsync(sCounts.p, 0, 4 * ((size_t)nWork_ + 1), ss));
-        launch_surface_prepare(b, nWork_, codes.as<uint32_t>(), unitCounts.as<uint32_t>(), buckets.as<uint32_t>(),
-                               sCounts.as<uint32_t>(), recs.p, ovl.p, ss, &launches);
-        launch_scan(sCounts.as<uint32_t>(), sOffsets.as<uint32_t>(), nWork_, sTileSums.as<uint32_t>(),
-                    st + kSurfTotal, st + kSurfOverflow, ss, &launches);
+        launch_surface_prepare(b, nWork_, reinterpret_cast<unsigned long long*>(st + kSurfCursor),
+                               reinterpret_cast<unsigned long long*>(st + kSurfTotal), st + kSurfClasses,
+                               sOffsets.as<uint32_t>(), wide_ ? triOf.as<uint32_t>() : nullptr, recs.p, depth.p, ss,
+                               &launches);
         // Without a hit list (PartialNode keys, or the tuned strategy) the
         // first traversal sets surface bits only and a second one merges
         // every hit at its rank.
@@ -378,11 +373,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         if (timer) timer->mark(5, false, ss);
         tuneMark(kKnobSurfaceSpan, false, ss);
         tuneMark(kKnobSurface, false, ss);
-        launch_surface_work(nodeKind_, retraverse ? 2 : 0, wide_ ? 1 : 0, b, recs.p, ovl.p, sOffsets.as<uint32_t>(), nWork_,
-                            st + kSurfTotal, buckets.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(),
-                            keys.p, keysCap_, nullptr, hitList.as<unsigned long long>(), st + kHitCount, listCap_,
-                            shape.surfBlocksPerSm, shape.surfBatch, shape.surfQueue ? st + kSurfQueue : nullptr, ss,
-                            &launches);
+        surfaceWork(retraverse ? 2 : 0, ss);
         tuneMark(kKnobSurface, true, ss);
         if (timer) timer->mark(5, true, ss);
         VXB_CUDA(cudaEventRecord(evSurfBits_, ss));
@@ -395,11 +386,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         if (!retraverse)
             launch_surface_merge(hitList.as<unsigned long long>(), st + kHitCount, listCap_, ranks.as<WordRank>(),
                                  keys.as<uint32_t>(), keysCap_, shape.mergeBlocksPerSm, mergeEntries_, ss, &launches);
-        else
-            launch_surface_work(nodeKind_, 1, wide_ ? 1 : 0, b, recs.p, ovl.p, sOffsets.as<uint32_t>(), nWork_,
-                                st + kSurfTotal, buckets.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(),
-                                keys.p, keysCap_, values.as<unsigned long long>(), nullptr, st + kHitCount, 0, shape.surfBlocksPerSm, shape.surfBatch,
-                                shape.surfQueue ? st + kSurfQueue : nullptr, ss, &launches);
+        else surfaceWork(1, ss);
         if (wide_)
             launch_partial_values(b, keys.p, st + kSurfaceVoxels, keysCap_, values.as<unsigned long long>(), ss,
                                   &launches);
@@ -498,6 +485,16 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     return 0;
 }
 
+void Pipeline::surfaceWork(int mode, cudaStream_t s) {
+    uint32_t* st = status.as<uint32_t>();
+    launch_surface_work(nodeKind_, mode, batch(), recs.p, depth.p, triOf.as<uint32_t>(), sOffsets.as<uint32_t>(),
+                        reinterpret_cast<unsigned long long*>(st + kSurfCursor),
+                        reinterpret_cast<unsigned long long*>(st + kSurfTotal), surf.as<uint32_t>(),
+                        ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(),
+                        hitList.as<unsigned long long>(), st + kHitCount, listCap_, shape.surfBlocksPerSm,
+                        shape.surfBatch, shape.surfQueue ? st + kSurfQueue : nullptr, s, &launches);
+}
+
 void Pipeline::emitCartesian(uint32_t zBegin, uint32_t zEnd, cudaStream_t s) {
     launch_emit_cartesian(nodeKind_, batch(), totalWords_, reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oSpans_),
                           emitSpans_, zBegin, zEnd, fin.as<uint32_t>(), fill.as<uint32_t>(), surf.as<uint32_t>(),
@@ -566,13 +563,11 @@ int Pipeline::finish(cudaStream_t s) {
         tuneFinish();
         uint32_t h[2];
         VXB_CUDA(cudaMemcpy(h, status.p, sizeof(h), cudaMemcpyDeviceToHost));
-        if (solidOverflow(h)) return failf(VXB_EOVERFLOW, "solid work list exceeds 2^32 entries");
+        if (countOverflow(h + kSolidTotal)) return failf(VXB_EOVERFLOW, "solid work list exceeds 2^32 entries");
         return 0;
     }
     uint32_t h[kPruneCounts + kPasses];
     VXB_CUDA(cudaMemcpyAsync(h, status.p, sizeof(h), cudaMemcpyDeviceToHost, s));
-    uint32_t bk[kSurfaceBuckets] = {0};
-    if (anyMaterials_) VXB_CUDA(cudaMemcpyAsync(bk, buckets.p, sizeof(bk), cudaMemcpyDeviceToHost, s));
     VXB_CUDA(cudaStreamSynchronize(s));
     tuneFinish();
     memset(&stats, 0, sizeof(stats));
@@ -582,9 +577,9 @@ int Pipeline::finish(cudaStream_t s) {
     stats.surface_columns = anyMaterials_ ? h[kSurfTotal] : 0;
     stats.surface_hits = anyMaterials_ ? h[kHitCount] : 0;
     stats.surface_voxels = anyMaterials_ ? h[kSurfaceVoxels] : 0;
-    for (uint32_t k = 0; k < kSurfaceBuckets; ++k) stats.surface_triangles[k / 3] += bk[k];
+    for (uint32_t k = 0; k < 3; ++k) stats.surface_triangles[k] = h[kSurfClasses + k];
     stats.grid_words = totalWords_;
-    if (solidOverflow(h) || (anyMaterials_ && h[kSurfOverflow]))
+    if (countOverflow(h + kSolidTotal) || countOverflow(h + kSurfTotal))
         return failf(VXB_EOVERFLOW, "work list exceeds 2^32 entries");
     bool reemit = false;
     const Batch b = batch();
@@ -602,10 +597,7 @@ int Pipeline::finish(cudaStream_t s) {
                 keysCap_ = surfaceVoxels + 1;
             }
             launch_surface_keys_zero(keys.p, st + kSurfaceVoxels, keysCap_, wide_ ? 1 : 0, s, &launches);
-            launch_surface_work(nodeKind_, 1, wide_ ? 1 : 0, b, recs.p, ovl.p, sOffsets.as<uint32_t>(), nWork_,
-                                st + kSurfTotal, buckets.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(),
-                                keys.p, keysCap_, values.as<unsigned long long>(), nullptr, st + kHitCount, 0, shape.surfBlocksPerSm, shape.surfBatch,
-                                shape.surfQueue ? st + kSurfQueue : nullptr, s, &launches);
+            surfaceWork(1, s);
             if (wide_)
                 launch_partial_values(b, keys.p, st + kSurfaceVoxels, keysCap_, values.as<unsigned long long>(), s,
                                       &launches);

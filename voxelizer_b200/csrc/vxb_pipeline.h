@@ -118,6 +118,7 @@ private:
 
     Batch batch();
     int pruneUntilStable(cudaStream_t s);
+    void surfaceWork(int mode, cudaStream_t s);
     void emitCartesian(uint32_t zBegin, uint32_t zEnd, cudaStream_t s);
 
     std::vector<MeshJob> jobs_;
@@ -135,10 +136,9 @@ private:
 
     DevBuf tables, status, bigList;
     DevBuf fill, surf, fin, ranks, rankTiles, pruneLists;
-    DevBuf codes, unitCounts, buckets, recs, ovl, hitList, keys, values;
+    DevBuf recs, depth, sOffsets, triOf, hitList, keys, values;
     // The surface pass runs on a second stream beside the solid pass, joined
     // before pruning (surface bits) and before emission (merged keys).
-    DevBuf sCounts, sOffsets, sTileSums;
     cudaStream_t side_ = nullptr, hi_ = nullptr;
     cudaEvent_t evFork_ = nullptr, evSurfBits_ = nullptr, evSurfDone_ = nullptr, evSolid_ = nullptr,
                 evHiDone_ = nullptr;

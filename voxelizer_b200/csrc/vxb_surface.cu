@@ -2,14 +2,14 @@
 // / encodeTriangleType (src/voxelizer.cu:3040-3221) and the 1D / 2D / 3D
 // processing kernels (3306-3955) with processVoxel (2946-2989).
 //
-// Per pass: classify every triangle (class, dominant axis, voxel box clamped
-// to the grid, work units), partition the triangles with work by (class,
-// axis) as the reference's sort by triangle type does, write one set-up
-// record per partitioned triangle (box, normal, the edge functions of the
-// projections it tests), scan the unit counts and run the work list: one
-// thread per column of the dominant projection (per voxel of a 1D line).
-// Warps find the triangle of each of their 32 items with one coalesced load
-// of 32 offsets, so the work kernel has no block-wide barrier.
+// One kernel classifies every triangle (class, dominant axis, voxel box clamped
+// to the grid, work units), gives the triangles with work consecutive
+// positions, ordered by class and axis inside a block, and writes one set-up
+// record per position together with the prefix of its work units.  The work
+// list runs over that prefix: one thread per column of the dominant projection
+// (per voxel of a 1D line).  Warps find the triangle of each of their 32 items
+// with one coalesced load of 32 offsets, so the work kernel has no block-wide
+// barrier.
 //
 // The reference runs the surface kernels once per material subspace on
 // boxes clamped to it.  Subspaces tile the grid, so the columns of the
@@ -136,10 +136,6 @@ __device__ __forceinline__ uint32_t surfUnits(const IBox& b, uint32_t code) {
     return axis == 0 ? ey * ez : axis == 1 ? ex * ez : ex * ey;
 }
 
-__device__ __forceinline__ uint32_t bucketOf(uint32_t code, uint32_t units) {
-    return units ? ((code >> 30) - 1u) * 3u + ((code >> 28) & 3u) : kNone;
-}
-
 // The unit and mesh triangle of work triangle wt.
 __device__ __forceinline__ uint32_t workUnit(const Batch& b, uint32_t wt, uint32_t* t) {
     const uint32_t u = unitOf(b.workBase, b.nUnits, wt);
@@ -147,54 +143,54 @@ __device__ __forceinline__ uint32_t workUnit(const Batch& b, uint32_t wt, uint32
     return u;
 }
 
-// Pass 1 (work-triangle order): code and units per triangle, triangles per
-// bucket.  Units without materials have no surface pass.
-__global__ void surfaceClassifyKernel(Batch b, uint32_t nWork, uint32_t* __restrict__ codes,
-                                      uint32_t* __restrict__ units, uint32_t* __restrict__ bucketCount) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < nWork; base += stride) {
-        const uint32_t wt = base + lane;
-        uint32_t code = 0, u = 0;
-        if (wt < nWork) {
-            uint32_t t;
-            const Unit& U = b.units[workUnit(b, wt, &t)];
-            if (U.materials) {
-                const PassGeom g = U.g;
-                F3 v[3];
-                loadTriF(U.V, U.I, t, v);
-                const IBox full = voxBoundsHalf(v, g);
-                code = classifyTri(v, full);
-                u = surfUnits(gridClamp(full, g), code);
-            }
-            codes[wt] = code;
-            units[wt] = u;
-        }
-        const uint32_t bk = bucketOf(code, u);
-        const uint32_t peers = __match_any_sync(kFull, bk);
-        if (bk != kNone && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(bucketCount + bk, (uint32_t)__popc(peers));
-    }
-}
-
 struct Overlap { float nx[3], ny[3], de[3]; };
 
-// Set-up record of one partitioned triangle (64 bytes) and its projection
-// edge functions (o[axis] for 2D boxes, all three for 3D boxes).
+// Columns are indexed along the inner and the outer axis of the dominant
+// projection and run along the depth axis:
+//   axis 0: inner y, outer z, depth x
+//   axis 1: inner x, outer z, depth y
+//   axis 2: inner x, outer y, depth z
+// First record (80 bytes) of a triangle with work: what every column needs.
 struct __align__(16) SurfRec {
-    int lo[3], hi[3];   // voxel box clamped to the grid
-    uint32_t code;      // class << 30 | axis << 28
-    uint32_t key;       // class << 8 | material
-    uint32_t tri;       // mesh index (PartialNode keys)
-    float v0[3];        // first vertex (3D depth range)
-    float n[3];         // normal (3D depth range)
+    // Edge functions of the dominant projection (not for 1D boxes), as the
+    // coefficients whose products are evaluated unfused and fused.
+    float cu[3], cf[3], de[3];
+    int lo[2];          // voxel box clamped to the grid: first inner, outer
+    uint32_t ext;       // inner extent
+    float rext;         // about 1 / ext
+    uint32_t code;      // class << 30 | axis << 28 | kLongUnits | material
     uint32_t unit;      // unit of the batch
+    int dlo, hi;        // first depth; last depth (3D) or outer (2D)
+    float m[3];         // minimum corner along inner, outer, depth
 };
-struct __align__(16) SurfOvl {
-    Overlap o[3];
-    uint32_t pad;
+constexpr uint32_t kLongUnits = 1u << 27;   // 2^22 or more columns
+// Second record (112 bytes) of 3D boxes, in (inner, outer, depth) order.
+struct __align__(16) SurfDepth {
+    float v0[3], n[3];  // first vertex, normal
+    float rn;           // 1 / the normal's depth component (0: divide)
+    float pad;
+    // The other two projections in the order of their tests: coefficients of
+    // the column's coordinate and of the depth.
+    float cc1[3], cd1[3], de1[3], cc2[3], cd2[3], de2[3];
+    float pad2[2];
 };
 static_assert(sizeof(SurfRec) == kSurfRecBytes, "record size");
-static_assert(sizeof(SurfOvl) == kSurfOvlBytes, "record size");
+static_assert(sizeof(SurfDepth) == kSurfDepthBytes, "record size");
+
+// The sites that the common forms below rely on: the dominant projection of
+// 3D boxes evaluates all edges alike, 2D boxes fuse the outer coordinate, the
+// depth loop tests fuse the depth coordinate in the first projection and the
+// constant one in the second.
+static_assert(site::OT_3D_YZ == 42 && site::OT_3D_ZX == 42 && site::OT_3D_XY == 42, "dominant projection form");
+static_assert(site::OT_2D_YZ == 42 && site::OT_2D_ZX == 21 && site::OT_2D_XY == 42, "2D form");
+static_assert(site::OT_2DP_YZ == 0 && site::OT_2DP_ZX == 0 && site::OT_2DP_XY == 0, "2D prolog form");
+static_assert(site::OT_3DX_ZX == 42 && site::OT_3DY_XY == 42 && site::OT_3DZ_YZ == 42, "first depth test form");
+static_assert(site::OT_3DX_XY == 21 && site::OT_3DY_YZ == 21 && site::OT_3DZ_ZX == 21, "second depth test form");
+static_assert(site::OT_3DYP_XY == 21 && site::OT_3DZP_YZ == 21, "first depth test prolog form");
+static_assert(site::OT_3DXP_XY == 21 && site::OT_3DYP_YZ == 21 && site::OT_3DZP_ZX == 21,
+              "second depth test prolog form");
+static_assert(site::PC_2D == 1 && site::PC_3D == 1 && site::PC_3DL == 1, "voxel corner form");
+static_assert(site::DT_3DY == 3 && site::DT_3DZ == 5, "depth range form");
 
 // Per-edge contraction modes: the three edge expressions of a test are
 // separate (unrolled) expressions in the reference, so a site's mode packs
@@ -202,11 +198,6 @@ static_assert(sizeof(SurfOvl) == kSurfOvlBytes, "record size");
 __device__ __forceinline__ float sum2fm(int m, float a, float b, float c, float d) {
     return m == 0 ? sum2f<0>(a, b, c, d) : m == 1 ? sum2f<1>(a, b, c, d) : sum2f<2>(a, b, c, d);
 }
-__device__ __forceinline__ float sum2p1fm(int m, float a, float b, float c, float d, float e) {
-    return m == 0 ? sum2p1f<0>(a, b, c, d, e) : m == 1 ? sum2p1f<1>(a, b, c, d, e)
-         : m == 2 ? sum2p1f<2>(a, b, c, d, e) : sum2p1f<3>(a, b, c, d, e);
-}
-
 // setupYZ / ZX / XYOverlapTest (src/voxelizer.cu:2675-2757).  A = 0: (y, z)
 // oriented by n.x; A = 1: (z, x) by n.y; A = 2: (x, y) by n.z.
 template <int A, int DE> __device__ __forceinline__ Overlap setupOverlap(const F3* t, F3 n, float d) {
@@ -227,205 +218,235 @@ template <int A, int DE> __device__ __forceinline__ Overlap setupOverlap(const F
     return o;
 }
 
-template <int OT> __device__ __forceinline__ bool overlapTest(const Overlap& o, float a, float b) {
-    bool r = true;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) r &= sum2p1fm((OT >> (2 * i)) & 3, o.nx[i], a, o.ny[i], b, o.de[i]) >= 0.0f;
-    return r;
+// Component of (x, y, z) along the inner, outer or depth axis.
+__device__ __forceinline__ float along(uint32_t axis, int role, float x, float y, float z) {
+    return role == 0 ? (axis == 0 ? y : x) : role == 1 ? (axis == 2 ? y : z) : axis == 0 ? x : axis == 1 ? y : z;
 }
 
-// The set-up record of work triangle wt at partitioned position pos.
-__device__ __forceinline__ void setupRecord(const Batch& b, uint32_t wt, uint32_t code, uint32_t pos,
-                                            SurfRec* __restrict__ recs, SurfOvl* __restrict__ ovl) {
-    uint32_t t;
-    const uint32_t unit = workUnit(b, wt, &t);
-    const Unit& U = b.units[unit];
-    const PassGeom g = U.g;
-    F3 v[3];
-    loadTriF(U.V, U.I, t, v);
+// Set-up records of a triangle at position pos.
+__device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32_t t, const F3* v, const IBox& box,
+                                            uint32_t code, uint32_t units, uint32_t pos, SurfRec* __restrict__ recs,
+                                            SurfDepth* __restrict__ depth) {
     const uint32_t bb = code >> 30, axis = (code >> 28) & 3u;
-    const IBox box = gridClamp(voxBoundsHalf(v, g), g);
+    const float d = U.g.df;
     SurfRec r;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) { r.lo[a] = box.lo[a]; r.hi[a] = box.hi[a]; }
-    r.code = code;
-    r.key = (bb << 8) | (U.M ? __ldg(U.M + t) : 0u);
-    r.tri = t;
-    r.v0[0] = v[0].x; r.v0[1] = v[0].y; r.v0[2] = v[0].z;
-    r.n[0] = r.n[1] = r.n[2] = 0.0f;
+    for (int i = 0; i < 3; ++i) {
+        r.cu[i] = r.cf[i] = r.de[i] = 0.0f;
+        r.m[i] = along(axis, i, U.g.mnf[0], U.g.mnf[1], U.g.mnf[2]);
+    }
+    r.lo[0] = axis == 0 ? box.lo[1] : box.lo[0];
+    r.lo[1] = axis == 2 ? box.lo[1] : box.lo[2];
+    r.dlo = axis == 0 ? box.lo[0] : axis == 1 ? box.lo[1] : box.lo[2];
+    r.hi = 0;
+    r.ext = (uint32_t)((axis == 0 ? box.hi[1] : box.hi[0]) - r.lo[0]) + 1u;
+    r.rext = __fdividef(1.0f, (float)r.ext);
+    r.code = code | (units >= (1u << 22) ? kLongUnits : 0u) | (U.M ? __ldg(U.M + t) : 0u);
     r.unit = unit;
-    const float d = g.df;
-    if (bb == 2) {
-        const F3 n = crossF<site::CRF_2D>(subF(v[0], v[2]), subF(v[1], v[0]));
-        r.n[0] = n.x; r.n[1] = n.y; r.n[2] = n.z;
-        if (axis == 0) ovl[pos].o[0] = setupOverlap<0, site::DE_2D_YZ>(v, n, d);
-        else if (axis == 1) ovl[pos].o[1] = setupOverlap<1, site::DE_2D_ZX>(v, n, d);
-        else ovl[pos].o[2] = setupOverlap<2, site::DE_2D_XY>(v, n, d);
-    } else if (bb == 3) {
-        const F3 n = crossF<site::CRF_3D>(subF(v[0], v[2]), subF(v[1], v[0]));
-        r.n[0] = n.x; r.n[1] = n.y; r.n[2] = n.z;
-        SurfOvl o;
-        o.o[0] = setupOverlap<0, site::DE_3D_YZ>(v, n, d);
-        o.o[1] = setupOverlap<1, site::DE_3D_ZX>(v, n, d);
-        o.o[2] = setupOverlap<2, site::DE_3D_XY>(v, n, d);
-        o.pad = 0;
-        ovl[pos] = o;
+    if (bb >= 2) {
+        const F3 e0 = subF(v[0], v[2]), e1 = subF(v[1], v[0]);
+        const F3 n = bb == 2 ? crossF<site::CRF_2D>(e0, e1) : crossF<site::CRF_3D>(e0, e1);
+        static_assert(site::DE_2D_YZ == site::DE_3D_YZ && site::DE_2D_ZX == site::DE_3D_ZX &&
+                          site::DE_2D_XY == site::DE_3D_XY, "one set-up form");
+        Overlap o[3];
+        o[0] = setupOverlap<0, site::DE_3D_YZ>(v, n, d);
+        o[1] = setupOverlap<1, site::DE_3D_ZX>(v, n, d);
+        o[2] = setupOverlap<2, site::DE_3D_XY>(v, n, d);
+        // 2D boxes: products of the inner coordinate unfused, of the outer one
+        // fused; 3D boxes: products of the first coordinate unfused.  The
+        // first coordinate of the (z, x) projection is the outer one.
+        const bool swap = bb == 2 && axis == 1;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float nx = axis == 0 ? o[0].nx[i] : axis == 1 ? o[1].nx[i] : o[2].nx[i];
+            const float ny = axis == 0 ? o[0].ny[i] : axis == 1 ? o[1].ny[i] : o[2].ny[i];
+            r.cu[i] = swap ? ny : nx;
+            r.cf[i] = swap ? nx : ny;
+            r.de[i] = axis == 0 ? o[0].de[i] : axis == 1 ? o[1].de[i] : o[2].de[i];
+        }
+        if (bb == 2) {
+            r.hi = axis == 2 ? box.hi[1] : box.hi[2];
+        } else {
+            r.hi = axis == 0 ? box.hi[0] : axis == 1 ? box.hi[1] : box.hi[2];
+            SurfDepth s;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                s.v0[i] = along(axis, i, v[0].x, v[0].y, v[0].z);
+                s.n[i] = along(axis, i, n.x, n.y, n.z);
+                // First test: (column, depth) coordinates of zx, xy or yz;
+                // second: (depth, column) coordinates of xy, yz or zx.
+                s.cc1[i] = axis == 0 ? o[1].nx[i] : axis == 1 ? o[2].nx[i] : o[0].nx[i];
+                s.cd1[i] = axis == 0 ? o[1].ny[i] : axis == 1 ? o[2].ny[i] : o[0].ny[i];
+                s.de1[i] = axis == 0 ? o[1].de[i] : axis == 1 ? o[2].de[i] : o[0].de[i];
+                s.cd2[i] = axis == 0 ? o[2].nx[i] : axis == 1 ? o[0].nx[i] : o[1].nx[i];
+                s.cc2[i] = axis == 0 ? o[2].ny[i] : axis == 1 ? o[0].ny[i] : o[1].ny[i];
+                s.de2[i] = axis == 0 ? o[2].de[i] : axis == 1 ? o[0].de[i] : o[1].de[i];
+            }
+            s.rn = divScaleF(s.n[2]) ? __frcp_rn(s.n[2]) : 0.0f;
+            s.pad = s.pad2[0] = s.pad2[1] = 0.0f;
+            depth[pos] = s;
+        }
     }
     recs[pos] = r;
 }
 
-// Pass 2 (work-triangle order): the position of every triangle with work in
-// the partitioned order, its units there (unitsP, zero past the end) and its
-// set-up record.
-__global__ void surfacePartitionKernel(Batch bt, const uint32_t* __restrict__ codes,
-                                       const uint32_t* __restrict__ units, uint32_t nT,
-                                       const uint32_t* __restrict__ bucketCount, uint32_t* __restrict__ bucketCursor,
-                                       uint32_t* __restrict__ unitsP, SurfRec* __restrict__ recs,
-                                       SurfOvl* __restrict__ ovl) {
-    __shared__ uint32_t bucketBase[kSurfaceBuckets];
-    if (threadIdx.x < kSurfaceBuckets) {
-        uint32_t s = 0;
-        for (uint32_t k = 0; k < threadIdx.x; ++k) s += bucketCount[k];
-        bucketBase[threadIdx.x] = s;
-    }
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < nT; base += stride) {
-        const uint32_t t = base + lane;
-        const uint32_t u = t < nT ? __ldg(units + t) : 0u;
-        const uint32_t code = t < nT ? __ldg(codes + t) : 0u;
-        const uint32_t b = t < nT ? bucketOf(code, u) : kNone;
-        const uint32_t peers = __match_any_sync(kFull, b);
-        const uint32_t leader = __ffs(peers) - 1;
-        uint32_t start = 0;
-        if (b != kNone && lane == leader) start = atomicAdd(bucketCursor + b, (uint32_t)__popc(peers));
-        start = __shfl_sync(kFull, start, leader);
-        if (b != kNone) {
-            const uint32_t pos = bucketBase[b] + start + __popc(peers & laneMaskLt());
-            unitsP[pos] = u;
-            setupRecord(bt, t, code, pos, recs, ovl);
+// Classification, positions and set-up.  A block takes kPrepThreads
+// consecutive work triangles, orders those with work by (class, axis), so that
+// the warps of the work kernel rarely mix kinds, and reserves their positions
+// and their work units with one 64-bit atomic: *cursor counts triangles above
+// bit kUnitBits and units below, so that positions and unit offsets of all
+// blocks follow the same order.  offsets[pos] is the first unit of pos.
+// *total is the exact number of units: past 2^32 - 2 of them the cursor may
+// have carried and the work kernel does nothing.  classes[0..3): triangles per
+// class.
+//
+// Bounds: the triangle gathers and the records' stores.  In place of a
+// classification, a partition by global (class, axis) cursors that set up the
+// records and a three-launch scan of the units: PREP_FIGURES
+constexpr int kPrepThreads = 256;
+constexpr uint32_t kUnitBits = 33;
+
+__global__ void __launch_bounds__(kPrepThreads) surfacePrepareKernel(Batch b, uint32_t nWork,
+                                                                     unsigned long long* cursor,
+                                                                     unsigned long long* total, uint32_t* classes,
+                                                                     uint32_t* __restrict__ offsets,
+                                                                     uint32_t* __restrict__ triOf,
+                                                                     SurfRec* __restrict__ recs,
+                                                                     SurfDepth* __restrict__ depth) {
+    constexpr int kW = kPrepThreads / 32;
+    __shared__ uint32_t cnt[kSurfaceBuckets * kW + 1];      // triangles per bucket and warp, then their prefix
+    __shared__ uint32_t sorted[kPrepThreads];               // units in order of position
+    __shared__ unsigned long long warpSum[kW], base;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint64_t b0 = (uint64_t)blockIdx.x * kPrepThreads; b0 < nWork; b0 += (uint64_t)gridDim.x * kPrepThreads) {
+        const uint64_t wt = b0 + threadIdx.x;
+        uint32_t t = 0, unit = 0, code = 0, u = 0;
+        F3 v[3];
+        IBox box;
+        if (wt < nWork) {
+            unit = workUnit(b, (uint32_t)wt, &t);
+            const Unit& U = b.units[unit];
+            if (U.materials) {
+                loadTriF(U.V, U.I, t, v);
+                const IBox full = voxBoundsHalf(v, U.g);
+                code = classifyTri(v, full);
+                box = gridClamp(full, U.g);
+                u = surfUnits(box, code);
+            }
         }
+        const uint32_t bucket = u ? ((code >> 30) - 1u) * 3u + ((code >> 28) & 3u) : kNone;
+        const uint32_t peers = __match_any_sync(kFull, bucket);
+        for (uint32_t i = threadIdx.x; i < kSurfaceBuckets * kW; i += kPrepThreads) cnt[i] = 0u;
+        __syncthreads();
+        if (u && lane == (uint32_t)(__ffs(peers) - 1)) cnt[bucket * kW + warp] = __popc(peers);
+        __syncthreads();
+        // Exclusive prefix over (bucket, warp), by the first warp; sum at the end.
+        if (warp == 0) {
+            uint32_t carry = 0;
+            for (uint32_t i0 = 0; i0 < kSurfaceBuckets * kW; i0 += 32u) {
+                const uint32_t i = i0 + lane, x = i < kSurfaceBuckets * kW ? cnt[i] : 0u;
+                uint32_t incl = x;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t q = __shfl_up_sync(kFull, incl, o);
+                    if (lane >= (uint32_t)o) incl += q;
+                }
+                if (i < kSurfaceBuckets * kW) cnt[i] = carry + incl - x;
+                carry += __shfl_sync(kFull, incl, 31);
+            }
+            if (lane == 0) cnt[kSurfaceBuckets * kW] = carry;
+        }
+        __syncthreads();
+        const uint32_t n = cnt[kSurfaceBuckets * kW];
+        uint32_t at = 0;
+        if (u) {
+            at = cnt[bucket * kW + warp] + __popc(peers & laneMaskLt());
+            sorted[at] = u;
+        }
+        __syncthreads();
+        const unsigned long long x = threadIdx.x < n ? sorted[threadIdx.x] : 0u;
+        unsigned long long incl = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long q = __shfl_up_sync(kFull, incl, o);
+            if (lane >= (uint32_t)o) incl += q;
+        }
+        if (lane == 31) warpSum[warp] = incl;
+        __syncthreads();
+        unsigned long long before = 0, sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kW; ++k) {
+            if (k < warp) before += warpSum[k];
+            sum += warpSum[k];
+        }
+        if (threadIdx.x == 0 && n) {
+            base = atomicAdd(cursor, ((unsigned long long)n << kUnitBits) + sum);
+            atomicAdd(total, sum);
+        }
+        if (threadIdx.x < 3) {
+            const uint32_t c = cnt[(threadIdx.x + 1u) * 3u * kW] - cnt[threadIdx.x * 3u * kW];
+            if (c) atomicAdd(classes + threadIdx.x, c);
+        }
+        __syncthreads();
+        // Positions past the arrays are only possible after a carry.
+        const uint32_t pos0 = (uint32_t)(base >> kUnitBits);
+        if (threadIdx.x < n && pos0 + threadIdx.x < nWork)
+            offsets[pos0 + threadIdx.x] = (uint32_t)(base + before + incl - x);
+        if (u && pos0 + at < nWork) {
+            if (triOf) triOf[pos0 + at] = t;
+            setupRecord(b.units[unit], unit, t, v, box, code, u, pos0 + at, recs, depth);
+        }
+        __syncthreads();
     }
 }
 
 // getSingleVoxelBoundsComponent, src/voxelizer.cu:2575-2586.
-template <int M> __device__ __forceinline__ float vbComp(int c, float m, float d) {
-    return linf<M>(__fsub_rn((float)c, 0.5f), d, m);
+__device__ __forceinline__ float vbComp(int c, float m, float d) {
+    return linf<1>(__fsub_rn((float)c, 0.5f), d, m);
 }
 
 // determineDepthRange{X,Y,Z} (src/voxelizer.cu:3994-4119) with
-// intersectWithPlane* and boundsCheck; t0 is the triangle's first vertex.
-template <int A, int DT> __device__ __forceinline__ void depthRange(F3 t0, F3 p, F3 n, const PassGeom& g, int& lo,
-                                                                    int& hi) {
-    const float d = g.df;
-    F3 pmin, pmax;
-    float a, b;
-    if (A == 0) {
-        const float sy = n.y > 0.0f ? 1.0f : 0.0f, sz = n.z > 0.0f ? 1.0f : 0.0f;
-        pmin = F3{0.0f, __fadd_rn(p.y, __fmul_rn(sy, d)), __fadd_rn(p.z, __fmul_rn(sz, d))};
-        pmax = F3{0.0f, __fadd_rn(p.y, __fmul_rn(1.0f - sy, d)), __fadd_rn(p.z, __fmul_rn(1.0f - sz, d))};
-        const F3 u = subF(t0, pmin), w = subF(t0, pmax);
-        a = __fdiv_rn(sum3f<DT>(u.x, n.x, u.y, n.y, u.z, n.z), n.x);
-        b = __fdiv_rn(sum3f<DT>(w.x, n.x, w.y, n.y, w.z, n.z), n.x);
-    } else if (A == 1) {
-        const float sx = n.x > 0.0f ? 1.0f : 0.0f, sz = n.z > 0.0f ? 1.0f : 0.0f;
-        pmin = F3{__fadd_rn(p.x, __fmul_rn(sx, d)), 0.0f, __fadd_rn(p.z, __fmul_rn(sz, d))};
-        pmax = F3{__fadd_rn(p.x, __fmul_rn(1.0f - sx, d)), 0.0f, __fadd_rn(p.z, __fmul_rn(1.0f - sz, d))};
-        const F3 u = subF(t0, pmin), w = subF(t0, pmax);
-        a = __fdiv_rn(sum3f<DT>(u.x, n.x, u.y, n.y, u.z, n.z), n.y);
-        b = __fdiv_rn(sum3f<DT>(w.x, n.x, w.y, n.y, w.z, n.z), n.y);
-    } else {
-        const float sx = n.x > 0.0f ? 1.0f : 0.0f, sy = n.y > 0.0f ? 1.0f : 0.0f;
-        pmin = F3{__fadd_rn(p.x, __fmul_rn(sx, d)), __fadd_rn(p.y, __fmul_rn(sy, d)), 0.0f};
-        pmax = F3{__fadd_rn(p.x, __fmul_rn(1.0f - sx, d)), __fadd_rn(p.y, __fmul_rn(1.0f - sy, d)), 0.0f};
-        const F3 u = subF(t0, pmin), w = subF(t0, pmax);
-        a = __fdiv_rn(sum3f<DT>(u.x, n.x, u.y, n.y, u.z, n.z), n.z);
-        b = __fdiv_rn(sum3f<DT>(w.x, n.x, w.y, n.y, w.z, n.z), n.z);
-    }
-    if (a > b) { float tmp = a; a = b; b = tmp; }
-    const float m = A == 0 ? g.mnf[0] : A == 1 ? g.mnf[1] : g.mnf[2];
-    lo = __float2int_rz(ceilf(__fsub_rn(__fdiv_rn(__fsub_rn(a, m), d), 0.5f)));
-    hi = __float2int_rz(floorf(__fadd_rn(__fdiv_rn(__fsub_rn(b, m), d), 0.5f)));
+// intersectWithPlane* and boundsCheck, in (inner, outer, depth) coordinates:
+// p the column's corner, t0 the first vertex, n the normal.
+__device__ __noinline__ void depthDivide(float a, float b, float nd, float m, float d, int& lo, int& hi) {
+    a = __fdiv_rn(a, nd);
+    b = __fdiv_rn(b, nd);
+    if (a > b) { const float t = a; a = b; b = t; }
+    lo = __float2int_ru(__fsub_rn(__fdiv_rn(__fsub_rn(a, m), d), 0.5f));
+    hi = __float2int_rd(__fadd_rn(__fdiv_rn(__fsub_rn(b, m), d), 0.5f));
 }
 
-// Hits of one warp staged in shared memory before they go to the global
-// hit list, so that the list takes one atomic per flush instead of one per
-// hit.
-constexpr uint32_t kStageHits = 256;
-constexpr uint32_t kFlushAt = kStageHits - 96;
-struct WarpStage {
-    unsigned long long* buf;
-    uint32_t* count;
-};
-
-// Where a unit's surface bits live.
-struct UnitGrid {
-    uint64_t wordBase;   // first word of the unit in the surface arena
-    uint32_t AY, ipx, padY, padZ;
-};
-
-// processVoxel of the surface pass.
-// mode 0: set the bit and append (bit position << 24 | key) to the hit list;
-// mode 1: merge the key at the voxel's rank (surface bits are complete);
-// mode 2: set the bit only (a mode-1 traversal merges the keys).
-struct Sink {
-    uint32_t* bits;            // surface arena
-    const WordRank* wordRank;  // complete surface words with their ranks (mode 1)
-    void* keys;                // compact key array (mode 1)
-    uint32_t keysCap;          // keys at ranks past it are dropped
-    unsigned long long* positions;   // arena position of each rank (wide keys)
-    unsigned long long* list;
-    uint32_t* listCount;
-    uint32_t listCap;
-    int mode;
-    int wide;                  // 64-bit keys (PartialNode)
-    // (xi, yi, zi): voxel of the unit's voxelized box; the allocation holds
-    // it one column further along x and padY / padZ rows further along y / z.
-    __device__ __forceinline__ void operator()(int xi, int yi, int zi, uint64_t key, const UnitGrid& ug,
-                                               const WarpStage& ws) const {
-        const uint32_t x = (uint32_t)xi + 1u, y = (uint32_t)yi + ug.padY, z = (uint32_t)zi + ug.padZ;
-        const uint64_t w = ug.wordBase + ((uint64_t)z * ug.AY + y) * ug.ipx + (x >> 5);
-        const uint32_t b = x & 31u;
-        const uint32_t bit = 0x80000000u >> b;
-        if (mode == 2) {
-            atomicOr(bits + w, bit);
-        } else if (mode == 0) {
-            atomicOr(bits + w, bit);
-            const unsigned long long e = ((unsigned long long)(w * 32 + b) << 24) | (key & 0xFFFFFFull);
-            const uint32_t at = atomicAdd(ws.count, 1u);
-            if (at < kStageHits) {
-                ws.buf[at] = e;
-            } else {
-                const uint32_t gat = atomicAdd(listCount, 1u);
-                if (gat < listCap) list[gat] = e;
-            }
-        } else {
-            const WordRank wr = wordRank[w];
-            const uint32_t r = wr.rank + (b ? __popc(wr.bits >> (32 - b)) : 0u);
-            if (r >= keysCap) return;
-            if (wide) {
-                atomicMax(reinterpret_cast<unsigned long long*>(keys) + r, (unsigned long long)key);
-                positions[r] = w * 32u + b;   // every hit of a voxel stores the same
-            } else {
-                atomicMax(reinterpret_cast<uint32_t*>(keys) + r, (uint32_t)key);
-            }
-        }
+template <int K>
+__device__ __forceinline__ void depthRange(uint32_t axis, float pi, float po, const float4& q0, const float4& q1,
+                                           float m, float d, float rd, int& lo, int& hi) {
+    // q0: v0 (inner, outer, depth), n inner; q1: n outer, n depth, 1 / n depth.
+    const float ni = q0.w, no = q1.x, nd = q1.y, rn = q1.z;
+    const float ui = __fsub_rn(q0.x, __fadd_rn(pi, ni > 0.0f ? d : 0.0f)),
+                wi = __fsub_rn(q0.x, __fadd_rn(pi, ni > 0.0f ? 0.0f : d));
+    const float uo = __fsub_rn(q0.y, __fadd_rn(po, no > 0.0f ? d : 0.0f)),
+                wo = __fsub_rn(q0.y, __fadd_rn(po, no > 0.0f ? 0.0f : d));
+    float a, b;
+    if (axis == 0) {
+        // (x, y, z) = (depth, inner, outer)
+        a = sum3f<site::DT_3DX[K]>(q0.z, nd, ui, ni, uo, no);
+        b = sum3f<site::DT_3DX[K]>(q0.z, nd, wi, ni, wo, no);
+    } else if (axis == 1) {
+        a = sum3f<site::DT_3DY>(ui, ni, q0.z, nd, uo, no);
+        b = sum3f<site::DT_3DY>(wi, ni, q0.z, nd, wo, no);
+    } else {
+        a = sum3f<site::DT_3DZ>(ui, ni, uo, no, q0.z, nd);
+        b = sum3f<site::DT_3DZ>(wi, ni, wo, no, q0.z, nd);
     }
-    // Moves the warp's staged hits to the global list (whole warp, converged).
-    __device__ __forceinline__ void flush(const WarpStage& ws, uint32_t lane) const {
-        __syncwarp();
-        const uint32_t n = min(*ws.count, kStageHits);
-        uint32_t base = 0;
-        if (lane == 0 && n) base = atomicAdd(listCount, n);
-        base = __shfl_sync(kFull, base, 0);
-        for (uint32_t i = lane; i < n; i += 32u)
-            if (base + i < listCap) list[base + i] = ws.buf[i];
-        __syncwarp();
-        if (lane == 0) *ws.count = 0;
-        __syncwarp();
-    }
-};
+    const float qa = divByF(a, nd, rn), qb = divByF(b, nd, rn);
+    const float x = __fsub_rn(fminf(qa, qb), m), y = __fsub_rn(fmaxf(qa, qb), m);
+    lo = __float2int_ru(__fsub_rn(divByF(x, d, rd), 0.5f));
+    hi = __float2int_rd(__fadd_rn(divByF(y, d, rd), 0.5f));
+    // x and y need no lower bound: a quotient below 2^-30 rounds away against
+    // the half voxel.
+    constexpr float kBig = 1.1529215046068470e18f;   // 2^60
+    if (rn == 0.0f || rd == 0.0f || !divExactF(a) || !divExactF(b) || !(fabsf(x) < kBig) || !(fabsf(y) < kBig))
+        depthDivide(a, b, nd, m, d, lo, hi);
+}
 
 // The loop of the reference over [lo, hi] along one axis runs inside one
 // material subspace (adjustVoxelRange, src/voxelizer.cu:3963-3993): clamps
@@ -446,165 +467,65 @@ __device__ __forceinline__ void subspaceRange(const uint32_t* sl, uint32_t nSl, 
 // n mod U iterations; vxb_sites.inc).
 template <int U> __device__ __forceinline__ bool inProlog(int pos, int n) { return U > 1 && pos < n % U; }
 
-template <int M, int P> __device__ __forceinline__ bool overlapAt(bool prolog, const Overlap& o, float a, float b) {
-    return prolog ? overlapTest<P>(o, a, b) : overlapTest<M>(o, a, b);
-}
+// Where the hits of the surface pass (processVoxel) go.
+struct Sink {
+    uint32_t* bits;            // surface arena
+    const WordRank* wordRank;  // complete surface words with their ranks (mode 1)
+    void* keys;                // compact key array (mode 1)
+    uint32_t keysCap;          // keys at ranks past it are dropped
+    unsigned long long* positions;   // arena position of each rank (mode 1, wide keys)
+    unsigned long long* list;
+    uint32_t* listCount;
+    uint32_t listCap;
+};
 
-// One column (one voxel for 1D boxes) of a partitioned triangle
-// (process1D/2D/3DTriangles, instantiated per node type K as the reference
-// instantiates them).  xr / yr / zr: the material subspace slices along each
-// axis ((lo, hi) pairs).
-template <int K>
-__device__ __forceinline__ void surfaceItem(uint32_t bb, uint32_t axis, const SurfRec& r, const Overlap& od,
-                                            const SurfOvl* __restrict__ ov, uint32_t u, const PassGeom& g,
-                                            const uint32_t* __restrict__ slices, const uint32_t* sliceOff,
-                                            const uint32_t* sliceN, uint64_t key, const Sink& sink,
-                                            const UnitGrid& ug, const WarpStage& ws) {
-    const float d = g.df;
-    const uint32_t ex = (uint32_t)(r.hi[0] - r.lo[0] + 1), ey = (uint32_t)(r.hi[1] - r.lo[1] + 1);
-    if (bb == 1) {
-        // process1DTriangles (3306-3411): every voxel of the line, no test.
-        if (axis == 0) sink(r.lo[0] + (int)u, r.lo[1], r.lo[2], key, ug, ws);
-        else if (axis == 1) sink(r.lo[0], r.lo[1] + (int)u, r.lo[2], key, ug, ws);
-        else sink(r.lo[0], r.lo[1], r.lo[2] + (int)u, key, ug, ws);
-        return;
-    }
-    if (bb == 2) {
-        // process2DTriangles (3418-3596): the dominant projection only; the
-        // inner loop (z for the x and y axes, y for the z axis) evaluates its
-        // prolog iterations in their own forms.
-        constexpr int U = site::UNR_2D[K];
-        if (axis == 0) {
-            const int j = r.lo[1] + (int)(u % ey), k = r.lo[2] + (int)(u / ey);
-            int lo = r.lo[2], hi = r.hi[2];
-            if (U > 1) subspaceRange(slices + 2 * sliceOff[2], sliceN[2], k, lo, hi);
-            if (overlapAt<site::OT_2D_YZ, site::OT_2DP_YZ>(inProlog<U>(k - lo, hi - lo + 1), od,
-                                                           vbComp<site::PC_2D>(j, g.mnf[1], d),
-                                                           vbComp<site::PC_2D>(k, g.mnf[2], d)))
-                sink(r.lo[0], j, k, key, ug, ws);
-        } else if (axis == 1) {
-            const int i = r.lo[0] + (int)(u % ex), k = r.lo[2] + (int)(u / ex);
-            int lo = r.lo[2], hi = r.hi[2];
-            if (U > 1) subspaceRange(slices + 2 * sliceOff[2], sliceN[2], k, lo, hi);
-            if (overlapAt<site::OT_2D_ZX, site::OT_2DP_ZX>(inProlog<U>(k - lo, hi - lo + 1), od,
-                                                           vbComp<site::PC_2D>(k, g.mnf[2], d),
-                                                           vbComp<site::PC_2D>(i, g.mnf[0], d)))
-                sink(i, r.lo[1], k, key, ug, ws);
-        } else {
-            const int i = r.lo[0] + (int)(u % ex), j = r.lo[1] + (int)(u / ex);
-            int lo = r.lo[1], hi = r.hi[1];
-            if (U > 1) subspaceRange(slices + 2 * sliceOff[1], sliceN[1], j, lo, hi);
-            if (overlapAt<site::OT_2D_XY, site::OT_2DP_XY>(inProlog<U>(j - lo, hi - lo + 1), od,
-                                                           vbComp<site::PC_2D>(i, g.mnf[0], d),
-                                                           vbComp<site::PC_2D>(j, g.mnf[1], d)))
-                sink(i, j, r.lo[2], key, ug, ws);
-        }
-        return;
-    }
-    // process3DTriangles (3603-3955): dominant projection, depth range from
-    // the plane, then per subspace slice of the depth axis either the single
-    // voxel or the other two projections per voxel (the depth loop's prolog
-    // iterations in their own forms).
-    constexpr int UL = site::UNR_3DL[K];
-    const F3 n{r.n[0], r.n[1], r.n[2]};
-    const F3 t0{r.v0[0], r.v0[1], r.v0[2]};
-    if (axis == 0) {
-        const int j = r.lo[1] + (int)(u % ey), k = r.lo[2] + (int)(u / ey);
-        F3 p{0.0f, vbComp<site::PC_3D>(j, g.mnf[1], d), vbComp<site::PC_3D>(k, g.mnf[2], d)};
-        if (!overlapTest<site::OT_3D_YZ>(od, p.y, p.z)) return;
-        int d0, d1;
-        depthRange<0, site::DT_3DX[K]>(t0, p, n, g, d0, d1);
-        const uint32_t* sl = slices + 2 * sliceOff[0];
-        for (uint32_t s = 0; s < sliceN[0]; ++s) {
-            const int lo = max(r.lo[0], (int)__ldg(sl + 2 * s)), hi = min(r.hi[0], (int)__ldg(sl + 2 * s + 1) - 1);
-            if (lo > hi || d0 > hi || d1 < lo) continue;
-            const int a = d0 < lo ? lo : d0, c = d1 > hi ? hi : d1;
-            if (a == c) { sink(a, j, k, key, ug, ws); continue; }
-            for (int i = a; i <= c; ++i) {
-                p.x = vbComp<site::PC_3DL>(i, g.mnf[0], d);
-                const bool pro = inProlog<UL>(i - a, c - a + 1);
-                if (overlapAt<site::OT_3DX_ZX, site::OT_3DXP_ZX[K]>(pro, ov->o[1], p.z, p.x) &&
-                    overlapAt<site::OT_3DX_XY, site::OT_3DXP_XY>(pro, ov->o[2], p.x, p.y))
-                    sink(i, j, k, key, ug, ws);
-            }
-        }
-    } else if (axis == 1) {
-        const int i = r.lo[0] + (int)(u % ex), k = r.lo[2] + (int)(u / ex);
-        F3 p{vbComp<site::PC_3D>(i, g.mnf[0], d), 0.0f, vbComp<site::PC_3D>(k, g.mnf[2], d)};
-        if (!overlapTest<site::OT_3D_ZX>(od, p.z, p.x)) return;
-        int d0, d1;
-        depthRange<1, site::DT_3DY>(t0, p, n, g, d0, d1);
-        const uint32_t* sl = slices + 2 * sliceOff[1];
-        for (uint32_t s = 0; s < sliceN[1]; ++s) {
-            const int lo = max(r.lo[1], (int)__ldg(sl + 2 * s)), hi = min(r.hi[1], (int)__ldg(sl + 2 * s + 1) - 1);
-            if (lo > hi || d0 > hi || d1 < lo) continue;
-            const int a = d0 < lo ? lo : d0, c = d1 > hi ? hi : d1;
-            if (a == c) { sink(i, a, k, key, ug, ws); continue; }
-            for (int j = a; j <= c; ++j) {
-                p.y = vbComp<site::PC_3DL>(j, g.mnf[1], d);
-                const bool pro = inProlog<UL>(j - a, c - a + 1);
-                if (overlapAt<site::OT_3DY_XY, site::OT_3DYP_XY>(pro, ov->o[2], p.x, p.y) &&
-                    overlapAt<site::OT_3DY_YZ, site::OT_3DYP_YZ>(pro, ov->o[0], p.y, p.z))
-                    sink(i, j, k, key, ug, ws);
-            }
-        }
-    } else {
-        const int i = r.lo[0] + (int)(u % ex), j = r.lo[1] + (int)(u / ex);
-        F3 p{vbComp<site::PC_3D>(i, g.mnf[0], d), vbComp<site::PC_3D>(j, g.mnf[1], d), 0.0f};
-        if (!overlapTest<site::OT_3D_XY>(od, p.x, p.y)) return;
-        int d0, d1;
-        depthRange<2, site::DT_3DZ>(t0, p, n, g, d0, d1);
-        const uint32_t* sl = slices + 2 * sliceOff[2];
-        for (uint32_t s = 0; s < sliceN[2]; ++s) {
-            const int lo = max(r.lo[2], (int)__ldg(sl + 2 * s)), hi = min(r.hi[2], (int)__ldg(sl + 2 * s + 1) - 1);
-            if (lo > hi || d0 > hi || d1 < lo) continue;
-            const int a = d0 < lo ? lo : d0, c = d1 > hi ? hi : d1;
-            if (a == c) { sink(i, j, a, key, ug, ws); continue; }
-            for (int k = a; k <= c; ++k) {
-                p.z = vbComp<site::PC_3DL>(k, g.mnf[2], d);
-                const bool pro = inProlog<UL>(k - a, c - a + 1);
-                if (overlapAt<site::OT_3DZ_YZ, site::OT_3DZP_YZ>(pro, ov->o[0], p.y, p.z) &&
-                    overlapAt<site::OT_3DZ_ZX, site::OT_3DZP_ZX>(pro, ov->o[1], p.z, p.x))
-                    sink(i, j, k, key, ug, ws);
-            }
-        }
-    }
-}
+// Hits of one warp are staged in shared memory before they go to the global
+// hit list, so that the list takes one atomic per flush.
+constexpr uint32_t kStageHits = 256;
 
-// Pass 4: the work list.  Warps take batches of kBatch (8, 16 or 32, the
-// launch shape) consecutive 32-item
+// The work list.  Warps take batches of `chunksPerBatch` consecutive 32-item
 // chunks; within a batch the owner of each chunk's first item follows from
-// the previous chunk.  Every partitioned triangle has at least one unit, so
-// a chunk's 32 items belong to at most 32 consecutive triangles: lane l
-// loads off[t0 + l] and a bit mask of the triangle starts inside the chunk
-// gives every lane its owner.  The class and axis of a position follow from
-// the bucket bounds, so the projection edge functions load together with
-// the record.
-template <uint32_t kBatch, int K>
-__global__ void __launch_bounds__(kBlock) surfaceWorkKernel(Sink sink, Batch b, const SurfRec* __restrict__ recs,
-                                                            const SurfOvl* __restrict__ ovl,
-                                                            const uint32_t* __restrict__ off, uint32_t n,
-                                                            const uint32_t* __restrict__ totalPtr,
-                                                            const uint32_t* __restrict__ bucketCount,
-                                                            uint32_t* queue) {
-    __shared__ unsigned long long stageBuf[kBlock / 32][kStageHits];
-    __shared__ uint32_t stageCount[kBlock / 32];
-    __shared__ uint32_t bucketEnd[kSurfaceBuckets];
-    const uint32_t total = *totalPtr;
+// the previous chunk.  Every listed triangle has at least one unit, so a
+// chunk's 32 items belong to at most 32 consecutive positions: lane l loads
+// off[t0 + l] and a bit mask of the triangle starts inside the chunk gives
+// every lane its owner.
+//
+// A lane takes one item: a voxel of a 1D line, a column of a 2D box
+// (process2DTriangles, src/voxelizer.cu:3418-3596: the dominant projection
+// only) or of a 3D box (process3DTriangles, 3603-3955: dominant projection,
+// depth range from the plane, then per material subspace slice of the depth
+// axis either the single voxel or the other two projections per voxel).  The
+// products of the column's coordinate do not change along the depth, so a
+// depth voxel costs six fused edge values.  The depth loop only marks hits
+// (32 voxels at a time in a mask); they are recorded afterwards, one per lane
+// and step.  Loops that the reference build unrolled evaluate their first
+// iterations in their own forms (instantiated per node type K as there).
+//
+// Mode 0: set the voxel's bit and append (bit position << 24 | key) to the
+// hit list; mode 1: merge the key at the voxel's rank (surface bits are
+// complete); mode 2: set the bit only.  PartialNodes have 64-bit keys.
+//
+// Bounds: issue.  WORK_FIGURES
+template <int K, int MODE>
+__global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch b, const SurfRec* __restrict__ recs,
+                                                               const SurfDepth* __restrict__ depth,
+                                                               const uint32_t* __restrict__ triOf,
+                                                               const uint32_t* __restrict__ off,
+                                                               const unsigned long long* __restrict__ cursor,
+                                                               const unsigned long long* __restrict__ totalPtr,
+                                                               uint32_t chunksPerBatch, uint32_t* queue) {
+    constexpr bool kWide = K == kPartial;
+    constexpr int kXProlog = site::OT_3DXP_ZX[K];
+    static_assert(kXProlog == site::OT_3DX_ZX || kXProlog == 21, "x-dominant prolog form");
+    __shared__ unsigned long long stage[kBlock / 32][MODE == 0 ? kStageHits : 1];
+    const unsigned long long exact = *totalPtr;
+    if (exact >= 0xFFFFFFFFull) return;   // refused by the host
+    const uint32_t n = (uint32_t)(*cursor >> kUnitBits), total = (uint32_t)exact;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t wib = threadIdx.x >> 5;
-    const WarpStage ws{stageBuf[wib], stageCount + wib};
-    if (lane == 0) stageCount[wib] = 0;
-    if (threadIdx.x == 0) {
-        uint32_t acc = 0;
-        for (uint32_t k = 0; k < kSurfaceBuckets; ++k) {
-            acc += __ldg(bucketCount + k);
-            bucketEnd[k] = acc;
-        }
-    }
-    __syncthreads();
+    unsigned long long* const hits = stage[threadIdx.x >> 5];
+    uint32_t staged = 0;
     const uint32_t chunks = (total + 31u) / 32u;
-    const uint32_t batches = (chunks + kBatch - 1) / kBatch;
+    const uint32_t batches = (chunks + chunksPerBatch - 1) / chunksPerBatch;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
     // Batches in a fixed grid-stride order, or (queue != NULL) taken from a
@@ -616,46 +537,251 @@ __global__ void __launch_bounds__(kBlock) surfaceWorkKernel(Sink sink, Batch b, 
         if (lane == 0) v = atomicAdd(queue, 1u);
         return __shfl_sync(kFull, v, 0);
     };
+    auto flush = [&]() {
+        __syncwarp();
+        uint32_t base = 0;
+        if (lane == 0 && staged) base = atomicAdd(sink.listCount, staged);
+        base = __shfl_sync(kFull, base, 0);
+        for (uint32_t i = lane; i < staged; i += 32u)
+            if (base + i < sink.listCap) sink.list[base + i] = hits[i];
+        __syncwarp();
+        staged = 0;
+    };
     for (uint32_t bt = queue ? nextBatch(0) : warp; bt < batches; bt = nextBatch(bt)) {
-        const uint32_t c1 = min((bt + 1) * kBatch, chunks);
-        uint32_t t0 = warpFindOwner(off, n, bt * kBatch * 32u, lane);
-        for (uint32_t c = bt * kBatch; c < c1; ++c) {
+        const uint32_t c1 = min((bt + 1) * chunksPerBatch, chunks);
+        uint32_t t0 = warpFindOwner(off, n, bt * chunksPerBatch * 32u, lane);
+        for (uint32_t c = bt * chunksPerBatch; c < c1; ++c) {
             const uint32_t base = c * 32u;
-            const uint32_t ol = t0 + lane <= n ? __ldg(off + t0 + lane) : 0xFFFFFFFFu;
-            const uint32_t o32 = t0 + 32u <= n ? __ldg(off + t0 + 32u) : 0xFFFFFFFFu;
-            const uint32_t starts = __reduce_or_sync(kFull, (lane >= 1u && ol < base + 32u) ? 1u << (ol - base) : 0u);
+            const uint32_t ol = t0 + lane < n ? __ldg(off + t0 + lane) : total;
+            const uint32_t o32 = t0 + 32u < n ? __ldg(off + t0 + 32u) : total;
+            const uint32_t starts =
+                __reduce_or_sync(kFull, (t0 + lane < n && lane >= 1u && ol < base + 32u) ? 1u << (ol - base) : 0u);
             const uint32_t k = __popc(starts & ((2u << lane) - 1u));
             const uint32_t ok = __shfl_sync(kFull, ol, k);
             const uint32_t k31 = __popc(starts);
             const uint32_t next = __shfl_sync(kFull, ol, (k31 + 1u) & 31u);
             const uint32_t nextOff = k31 < 31u ? next : o32;
-            const uint32_t item = base + lane;
-            if (item < total) {
-                const uint32_t pos = t0 + k;
-                uint32_t bucket = 0;
-#pragma unroll
-                for (uint32_t q = 0; q + 1 < kSurfaceBuckets; ++q) bucket += pos >= bucketEnd[q] ? 1u : 0u;
-                const uint32_t bb = bucket / 3u + 1u, axis = bucket % 3u;
-                Overlap od;
-                if (bb >= 2) od = ovl[pos].o[axis];
-                const SurfRec r = recs[pos];
-                const uint64_t key = sink.wide ? (((uint64_t)bb << 40) | ((uint64_t)(r.key & 255u) << 32) | r.tri)
-                                               : (uint64_t)r.key;
-                const Unit& U = b.units[r.unit];
-                const PassGeom g = U.g;
-                const UnitGrid ug{U.wordBase, g.AY, g.ipx, g.padY, g.padZ};
-                const uint32_t sliceOff[3] = {U.sliceBase, U.sliceBase + U.sliceN[0],
-                                              U.sliceBase + U.sliceN[0] + U.sliceN[1]};
-                const uint32_t sliceN[3] = {U.sliceN[0], U.sliceN[1], U.sliceN[2]};
-                surfaceItem<K>(bb, axis, r, od, ovl + pos, item - ok, g, b.slices, sliceOff, sliceN, key, sink,
-                               ug, ws);
-            }
-            __syncwarp();
-            if (sink.mode == 0 && *ws.count >= kFlushAt) sink.flush(ws, lane);
+            const uint32_t item = base + lane, pos = t0 + k;
             t0 += k31 + (nextOff == base + 32u ? 1u : 0u);
+
+            // The item's column and its depth range [dlo, dhi]; `deep` for
+            // the ranges of 3D boxes, which are clamped to [blo, bhi] and the
+            // slices below.
+            const Unit* U = b.units;
+            uint32_t code = 0, nSlices = 0;
+            int inner = 0, outer = 0, dlo = 0, dhi = -1, blo = 0, bhi = -1;
+            float pi = 0.0f, po = 0.0f, mD = 0.0f, d = 0.0f;
+            bool deep = false;
+            if (item < total) {
+                const SurfRec& rec = recs[pos];
+                const float4 r0 = __ldg(reinterpret_cast<const float4*>(&rec)),
+                             r1 = __ldg(reinterpret_cast<const float4*>(&rec) + 1);
+                const uint4 r2 = __ldg(reinterpret_cast<const uint4*>(&rec) + 2),
+                            r3 = __ldg(reinterpret_cast<const uint4*>(&rec) + 3);
+                const float4 r4 = __ldg(reinterpret_cast<const float4*>(&rec) + 4);
+                const float cu[3] = {r0.x, r0.y, r0.z}, cf[3] = {r0.w, r1.x, r1.y},
+                            de[3] = {r1.z, r1.w, __uint_as_float(r2.x)};
+                const uint32_t ext = r2.w;
+                code = r3.y;
+                U = b.units + r3.z;
+                inner = (int)r2.y;
+                outer = (int)r2.z;
+                dlo = (int)r3.w;
+                const int hi = __float_as_int(r4.x);
+                mD = r4.w;
+                const uint32_t axis = (code >> 28) & 3u, bb = code >> 30;
+                const uint32_t u = item - ok;
+                if (bb == 1) {
+                    dlo += (int)u;
+                    dhi = dlo;
+                } else {
+                    // u / ext by the approximate reciprocal, which is off by
+                    // one at the most below 2^22 columns.
+                    uint32_t q, m;
+                    if (code & kLongUnits) {
+                        q = u / ext;
+                        m = u - q * ext;
+                    } else {
+                        q = (uint32_t)((float)u * __uint_as_float(r3.x));
+                        m = u - q * ext;
+                        if ((int)m < 0) {
+                            m += ext;
+                            --q;
+                        }
+                        if (m >= ext) {
+                            m -= ext;
+                            ++q;
+                        }
+                    }
+                    const int olo = outer;
+                    inner += (int)m;
+                    outer += (int)q;
+                    d = U->g.df;
+                    pi = vbComp(inner, r4.y, d);
+                    po = vbComp(outer, r4.z, d);
+                    if (bb == 2) {
+                        constexpr int UN = site::UNR_2D[K];
+                        bool pro = false;
+                        if (UN > 1) {
+                            const uint32_t oa = axis == 2 ? 1u : 2u;   // outer axis
+                            int lo = olo, ohi = hi;
+                            if (U->sliceN[oa] > 1u)
+                                subspaceRange(b.slices + 2 * (U->sliceBase + U->sliceN[0] + (oa == 2u ? U->sliceN[1] : 0u)),
+                                              U->sliceN[oa], outer, lo, ohi);
+                            pro = inProlog<UN>(outer - lo, ohi - lo + 1);
+                        }
+                        bool hit = true;
+#pragma unroll
+                        for (int i = 0; i < 3; ++i)
+                            hit &= (pro ? sum2p1f<0>(cu[i], pi, cf[i], po, de[i])
+                                        : sum2p1f<2>(cu[i], pi, cf[i], po, de[i])) >= 0.0f;
+                        dhi = hit ? dlo : dlo - 1;
+                    } else {
+                        const float pu = axis == 1 ? po : pi, pf = axis == 1 ? pi : po;
+                        bool hit = true;
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) hit &= sum2p1f<2>(cu[i], pu, cf[i], pf, de[i]) >= 0.0f;
+                        dhi = dlo - 1;
+                        if (hit) {
+                            const float4* s = reinterpret_cast<const float4*>(depth + pos);
+                            deep = true;
+                            blo = dlo;
+                            bhi = hi;
+                            depthRange<K>(axis, pi, po, __ldg(s), __ldg(s + 1), mD, d, U->g.rdf, dlo, dhi);
+                            nSlices = U->sliceN[axis];
+                        }
+                    }
+                }
+            }
+            const uint32_t axis = (code >> 28) & 3u;
+            // One slice of the depth axis at a time (a single one covers the
+            // grid, and the box is inside the grid).
+            uint32_t s = 0;
+            do {
+                int a = dlo, z = s == 0u ? dhi : dlo - 1;
+                if (deep) {
+                    int lo = blo, hi = bhi;
+                    if (nSlices > 1u) {
+                        const uint32_t* sl = b.slices + 2 * (U->sliceBase + (axis >= 1u ? U->sliceN[0] : 0u) +
+                                                             (axis == 2u ? U->sliceN[1] : 0u));
+                        if (s < nSlices) {
+                            lo = max(lo, (int)__ldg(sl + 2 * s));
+                            hi = min(hi, (int)__ldg(sl + 2 * s + 1) - 1);
+                        } else {
+                            hi = lo - 1;
+                        }
+                    } else if (s > 0u) {
+                        hi = lo - 1;
+                    }
+                    if (lo > hi || dlo > hi || dhi < lo) {
+                        a = 0;
+                        z = -1;
+                    } else {
+                        a = max(dlo, lo);
+                        z = min(dhi, hi);
+                    }
+                }
+                const uint32_t cnt = z >= a ? (uint32_t)(z - a) + 1u : 0u;
+                for (uint32_t w0 = 0; __any_sync(kFull, w0 < cnt); w0 += 32u) {
+                    // Hits of voxels a + w0 .. a + w0 + 31.
+                    uint32_t m = w0 < cnt ? 1u : 0u;
+                    if (deep && cnt > 1u && w0 < cnt) {
+                        float e[20];   // cc1 cd1 de1 cc2 cd2 de2
+                        const float4* f = reinterpret_cast<const float4*>(depth + pos) + 2;
+#pragma unroll
+                        for (int i = 0; i < 5; ++i) {
+                            const float4 q = __ldg(f + i);
+                            e[4 * i] = q.x; e[4 * i + 1] = q.y; e[4 * i + 2] = q.z; e[4 * i + 3] = q.w;
+                        }
+                        const float p1 = axis == 1 ? pi : po, p2 = axis == 1 ? po : pi;
+                        float k1[3], k2[3];
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) {
+                            k1[i] = __fmul_rn(e[i], p1);
+                            k2[i] = __fmul_rn(e[9 + i], p2);
+                        }
+                        const uint32_t last = min(cnt - w0, 32u);
+                        m = 0u;
+                        for (uint32_t v = 0; v < last; ++v) {
+                            const float pd = vbComp(a + (int)(w0 + v), mD, d);
+                            bool hit = true;
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) {
+                                hit &= __fadd_rn(__fmaf_rn(e[3 + i], pd, k1[i]), e[6 + i]) >= 0.0f;
+                                hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
+                            }
+                            m |= hit ? 1u << v : 0u;
+                        }
+                        constexpr int UL = site::UNR_3DL[K];
+                        static_assert(UL == 0 || UL == 2, "at most one prolog iteration");
+                        // The prolog iteration in its own form of the first
+                        // test (the x-dominant one differs by node type).
+                        if (UL == 2 && w0 == 0u && (cnt & 1u) && (kXProlog == 21 || axis != 0u)) {
+                            const float pd = vbComp(a, mD, d);
+                            bool hit = true;
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) {
+                                hit &= __fadd_rn(__fmaf_rn(e[i], p1, __fmul_rn(e[3 + i], pd)), e[6 + i]) >= 0.0f;
+                                hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
+                            }
+                            m = (m & ~1u) | (hit ? 1u : 0u);
+                        }
+                    }
+                    if (!__any_sync(kFull, m != 0u)) continue;
+                    // Bit position in the unit of the column's voxel at depth
+                    // 0 and its step along the depth.  The allocation holds a
+                    // voxel one column further along x and padY / padZ rows
+                    // further along y / z.
+                    uint32_t at = 0, step = 0;
+                    uint64_t wordBase = 0;
+                    if (m) {
+                        const uint32_t X = U->g.X, AY = U->g.AY, pY = U->g.padY, pZ = U->g.padZ;
+                        wordBase = U->wordBase;
+                        const uint32_t zr = axis == 2 ? pZ : (uint32_t)outer + pZ;
+                        const uint32_t yr = pY + (axis == 0 ? (uint32_t)inner : axis == 2 ? (uint32_t)outer : 0u);
+                        step = axis == 0 ? 1u : axis == 1 ? X : X * AY;
+                        at = (zr * AY + yr) * X + (axis == 0 ? 1u : (uint32_t)inner + 1u) + (uint32_t)(a + (int)w0) * step;
+                    }
+                    const uint32_t cls = code >> 30, mat = code & 255u;
+                    for (;;) {
+                        const uint32_t live = __ballot_sync(kFull, m != 0u);
+                        if (!live) break;
+                        if (m) {
+                            const uint32_t v = __ffs(m) - 1;
+                            m &= m - 1u;
+                            const uint32_t p = at + v * step, bit = p & 31u;
+                            const uint64_t w = wordBase + (p >> 5);
+                            if (MODE != 1) {
+                                atomicOr(sink.bits + w, 0x80000000u >> bit);
+                                if (MODE == 0)
+                                    hits[staged + __popc(live & laneMaskLt())] =
+                                        ((w * 32u + bit) << 24) | (cls << 8) | mat;
+                            } else {
+                                const WordRank wr = sink.wordRank[w];
+                                const uint32_t r = wr.rank + (bit ? __popc(wr.bits >> (32u - bit)) : 0u);
+                                if (r < sink.keysCap) {
+                                    if (kWide) {
+                                        const unsigned long long key = ((unsigned long long)cls << 40) |
+                                                                       ((unsigned long long)mat << 32) |
+                                                                       __ldg(triOf + pos);
+                                        atomicMax(reinterpret_cast<unsigned long long*>(sink.keys) + r, key);
+                                        sink.positions[r] = w * 32u + bit;   // every hit of a voxel stores the same
+                                    } else {
+                                        atomicMax(reinterpret_cast<uint32_t*>(sink.keys) + r, (cls << 8) | mat);
+                                    }
+                                }
+                            }
+                        }
+                        if (MODE == 0) {
+                            staged += __popc(live);
+                            if (staged > kStageHits - 32u) flush();
+                        }
+                    }
+                }
+            } while (__any_sync(kFull, ++s < nSlices));
         }
     }
-    if (sink.mode == 0) sink.flush(ws, lane);
+    if (MODE == 0) flush();
 }
 
 // Exclusive popcount prefix over the surface words (ranks of surface voxels).
@@ -809,29 +935,28 @@ __global__ void mergeKeysKernel(const unsigned long long* __restrict__ list, con
 
 }  // namespace
 
-void launch_surface_prepare(const Batch& b, uint32_t nWork, uint32_t* codes, uint32_t* units, uint32_t* buckets,
-                            uint32_t* unitsP, void* recs, void* ovl, cudaStream_t s,
-                            uint32_t* launches) {
-    const uint32_t grid = gridFor(nWork, 256);
-    surfaceClassifyKernel<<<grid, 256, 0, s>>>(b, nWork, codes, units, buckets);
-    surfacePartitionKernel<<<grid, 256, 0, s>>>(b, codes, units, nWork, buckets, buckets + kSurfaceBuckets, unitsP,
-                                                static_cast<SurfRec*>(recs), static_cast<SurfOvl*>(ovl));
-    *launches += 2;
+void launch_surface_prepare(const Batch& b, uint32_t nWork, unsigned long long* cursor, unsigned long long* total,
+                            uint32_t* classes, uint32_t* offsets, uint32_t* triOf, void* recs, void* depth,
+                            cudaStream_t s, uint32_t* launches) {
+    surfacePrepareKernel<<<gridFor(nWork, kPrepThreads, 148u * 64u), kPrepThreads, 0, s>>>(
+        b, nWork, cursor, total, classes, offsets, triOf, static_cast<SurfRec*>(recs), static_cast<SurfDepth*>(depth));
+    *launches += 1;
 }
 
 template <int K>
-static void launchSurfaceWorkKind(uint32_t batch, uint32_t grid, const Sink& sink, const Batch& b, const SurfRec* R,
-                                  const SurfOvl* O, const uint32_t* offsets, uint32_t nWork, const uint32_t* total,
-                                  const uint32_t* buckets, uint32_t* queue, cudaStream_t s) {
-    if (batch == 8)
-        surfaceWorkKernel<8, K><<<grid, kBlock, 0, s>>>(sink, b, R, O, offsets, nWork, total, buckets, queue);
-    else if (batch == 32)
-        surfaceWorkKernel<32, K><<<grid, kBlock, 0, s>>>(sink, b, R, O, offsets, nWork, total, buckets, queue);
-    else surfaceWorkKernel<16, K><<<grid, kBlock, 0, s>>>(sink, b, R, O, offsets, nWork, total, buckets, queue);
+static void launchSurfaceWorkKind(int mode, uint32_t grid, const Sink& sink, const Batch& b, const SurfRec* R,
+                                  const SurfDepth* D, const uint32_t* triOf, const uint32_t* offsets,
+                                  const unsigned long long* cursor, const unsigned long long* total, uint32_t batch,
+                                  uint32_t* queue, cudaStream_t s) {
+    if (mode == 0)
+        surfaceWorkKernel<K, 0><<<grid, kBlock, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
+    else if (mode == 1)
+        surfaceWorkKernel<K, 1><<<grid, kBlock, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
+    else surfaceWorkKernel<K, 2><<<grid, kBlock, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
 }
 
-void launch_surface_work(int kind, int mode, int wide, const Batch& b, const void* recs, const void* ovl,
-                         const uint32_t* offsets, uint32_t nWork, const uint32_t* total, const uint32_t* buckets,
+void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, const void* depth, const uint32_t* triOf,
+                         const uint32_t* offsets, const unsigned long long* cursor, const unsigned long long* total,
                          uint32_t* surf, const WordRank* ranks, void* keys, uint32_t keysCap,
                          unsigned long long* positions, unsigned long long* list, uint32_t* listCount,
                          uint32_t listCap, uint32_t blocksPerSm, uint32_t batch, uint32_t* queue, cudaStream_t s,
@@ -846,24 +971,14 @@ void launch_surface_work(int kind, int mode, int wide, const Batch& b, const voi
     sink.list = list;
     sink.listCount = listCount;
     sink.listCap = listCap;
-    sink.mode = mode;
-    sink.wide = wide;
     const uint32_t grid = 148u * blocksPerSm;
     const SurfRec* R = static_cast<const SurfRec*>(recs);
-    const SurfOvl* O = static_cast<const SurfOvl*>(ovl);
-    switch (kind) {
-    case kShort: launchSurfaceWorkKind<kShort>(batch, grid, sink, b, R, O, offsets, nWork, total, buckets, queue, s); break;
-    case kLong: launchSurfaceWorkKind<kLong>(batch, grid, sink, b, R, O, offsets, nWork, total, buckets, queue, s); break;
-    case kPartial:
-        launchSurfaceWorkKind<kPartial>(batch, grid, sink, b, R, O, offsets, nWork, total, buckets, queue, s);
-        break;
-    case kShortFcc:
-        launchSurfaceWorkKind<kShortFcc>(batch, grid, sink, b, R, O, offsets, nWork, total, buckets, queue, s);
-        break;
-    default:
-        launchSurfaceWorkKind<kLongFcc>(batch, grid, sink, b, R, O, offsets, nWork, total, buckets, queue, s);
-        break;
-    }
+    const SurfDepth* D = static_cast<const SurfDepth*>(depth);
+    auto launch = kind == kShort ? launchSurfaceWorkKind<kShort>
+                : kind == kLong ? launchSurfaceWorkKind<kLong>
+                : kind == kPartial ? launchSurfaceWorkKind<kPartial>
+                : kind == kShortFcc ? launchSurfaceWorkKind<kShortFcc> : launchSurfaceWorkKind<kLongFcc>;
+    launch(mode, grid, sink, b, R, D, triOf, offsets, cursor, total, batch, queue, s);
     *launches += 1;
 }
 
