@@ -111,7 +111,8 @@ bool solid_may_list(const PassGeom& g, uint64_t nSplits, uint32_t nWork);
 void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, unsigned long long* big,
                          uint32_t* bigCount, uint32_t bigCap, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
                          cudaStream_t s, uint32_t* launches);
-void launch_row_fill(const Batch& b, uint64_t nRows, uint32_t* fill, cudaStream_t s, uint32_t* launches);
+void launch_row_fill(const Batch& b, uint64_t nRows, uint64_t totalWords, uint32_t* fill, cudaStream_t s,
+                     uint32_t* launches);
 
 // ---- Surface voxelization: src/voxelizer.cu:2358-2989, 3040-4201 ----
 // Triangles with surface work get consecutive positions (ordered by (class,
@@ -144,9 +145,12 @@ void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, c
                          uint32_t listCap, uint32_t blocksPerSm, uint32_t batch, uint32_t* queue, cudaStream_t s,
                          uint32_t* launches);
 // Exclusive popcount prefix over `words` surface words, stored beside each
-// word; *total = surface voxels.
-void launch_surface_rank(const uint32_t* bits, uint64_t words, WordRank* ranks, uint32_t* tileSums, uint32_t* total,
-                         cudaStream_t s, uint32_t* launches);
+// word (words of sectors without surface nodes are left out); *total = surface
+// voxels; the keys of all of them (at most keysCap) are zeroed.  *done is zero
+// on entry; `sums` has room for surface_rank_sums(words) entries.
+size_t surface_rank_sums(uint64_t words);
+void launch_surface_rank(const uint32_t* bits, uint64_t words, WordRank* ranks, uint32_t* sums, uint32_t* done,
+                         uint32_t* total, void* keys, uint32_t keysCap, int wide, cudaStream_t s, uint32_t* launches);
 // Zeroes min(*count, cap) keys.
 void launch_surface_keys_zero(void* keys, const uint32_t* count, uint32_t cap, int wide, cudaStream_t s,
                               uint32_t* launches);

@@ -276,7 +276,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     vxb::launch_solid_toggle(b, n_triangles, reinterpret_cast<unsigned long long*>(status),
                              vxb::solid_may_list(g, nSub, n_triangles) ? big : nullptr, status + 3, kBigChunks, grid, 3, nullptr,
                              s, &launches);
-    vxb::launch_row_fill(b, tab.rowBase[1], grid, s, &launches);
+    vxb::launch_row_fill(b, tab.rowBase[1], tab.wordBase[1], grid, s, &launches);
     e = cudaGetLastError();
     if (e != cudaSuccess) return failf(VXB_ECUDA, "%s", cudaGetErrorString(e));
     return VXB_OK;

@@ -23,7 +23,7 @@ namespace {
 // kSurfTotal and kSurfHigh likewise; kSurfCursor takes two words.
 enum : int { kSolidTotal = 0, kSolidHigh = 1, kSurfTotal = 2, kSurfHigh = 3, kSurfCursor = 4, kHitCount = 6,
              kSurfaceVoxels = 7, kSurfQueue = 8, kToggleQueue = 9, kBigCount = 10, kPruneOverflow = 11,
-             kSurfClasses = 12, kPruneCounts = 15 };
+             kSurfClasses = 12, kRankDone = 15, kPruneCounts = 16 };
 
 // The work counts take 32 bits: totals of 2^32 - 1 or more are refused.
 bool countOverflow(const uint32_t* h) { return h[1] || h[0] == 0xFFFFFFFFu; }
@@ -304,7 +304,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
         if (wide_ && (rc = triOf.ensure(4 * (size_t)nWork_))) return rc;
         if ((rc = surf.ensure(wordBytes))) return rc;
         if ((rc = ranks.ensure(2 * wordBytes))) return rc;
-        if ((rc = rankTiles.ensure(4 * ((size_t)totalWords_ / 2048 + 2)))) return rc;
+        if ((rc = rankTiles.ensure(4 * surface_rank_sums(totalWords_)))) return rc;
         if ((rc = recs.ensure(kSurfRecBytes * (size_t)nWork_))) return rc;
         if ((rc = depth.ensure(kSurfDepthBytes * (size_t)nWork_))) return rc;
         // Hit list: 8-byte entries (bit position << 24 | key).  PartialNode
@@ -377,12 +377,12 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         tuneMark(kKnobSurface, true, ss);
         if (timer) timer->mark(5, true, ss);
         VXB_CUDA(cudaEventRecord(evSurfBits_, ss));
+        // Ranks, and zeroed material keys by rank.
         launch_surface_rank(surf.as<uint32_t>(), totalWords_, ranks.as<WordRank>(), rankTiles.as<uint32_t>(),
-                            st + kSurfaceVoxels, ss, &launches);
+                            st + kRankDone, st + kSurfaceVoxels, keys.p, keysCap_, wide_ ? 1 : 0, ss, &launches);
         if (timer) timer->mark(1, true, ss);
         // Material keys by surface rank (independent of pruning).
         if (timer) timer->mark(4, false, ss);
-        launch_surface_keys_zero(keys.p, st + kSurfaceVoxels, keysCap_, wide_ ? 1 : 0, ss, &launches);
         if (!retraverse)
             launch_surface_merge(hitList.as<unsigned long long>(), st + kHitCount, listCap_, ranks.as<WordRank>(),
                                  keys.as<uint32_t>(), keysCap_, shape.mergeBlocksPerSm, mergeEntries_, ss, &launches);
@@ -402,7 +402,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
                         mayList_ ? bigList.as<unsigned long long>() : nullptr, st + kBigCount, kBigCap, fillP,
                         shape.toggleBlocksPerSm, shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
     tuneMark(kKnobToggle, true, s);
-    launch_row_fill(b, totalRows_, fillP, s, &launches);
+    launch_row_fill(b, totalRows_, totalWords_, fillP, s, &launches);
     mark(0, true);
     if (!nodes_) {
         if (!aliasFill_)

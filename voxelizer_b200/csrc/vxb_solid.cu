@@ -34,6 +34,8 @@
 #include "vxb_device.cuh"
 #include "vxb_kernels.cuh"
 
+#include <algorithm>
+
 namespace vxb {
 
 using namespace detail;
@@ -493,15 +495,20 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidBigKernel(Batch b, 
 // inverts it when the words before it in its row hold an odd number of
 // toggles.  That parity is a segmented XOR scan over the lanes (a ballot of
 // word parities, cut at the lanes that start a row) plus the parity carried
-// from the previous chunk for the row that continues into this one.
-constexpr uint32_t kFillRows = 16;
+// from the previous chunk for the row that continues into this one.  Bound by
+// the loads in flight: kFillAhead chunks are loaded before the first is
+// scanned, and a task holds about kFillWords words whatever the row length
+// (one chunk ahead and 16 rows a task: room, 13.5 M words, 50 us, duct, 130
+// words a row, 50, batch of 64 meshes 95; now 41, 28 and 69).
+constexpr uint32_t kFillAhead = 6;
+constexpr uint32_t kFillWords = 1152;  // words of a task, about
 
-__global__ void rowFillKernel(Batch b, uint64_t nRows, uint32_t* __restrict__ fill) {
+__global__ void rowFillKernel(Batch b, uint64_t nRows, uint32_t rowsPerTask, uint32_t* __restrict__ fill) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t nWarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * kFillRows < nRows; g += nWarps) {
-        uint64_t row = g * kFillRows;
-        const uint64_t rowEnd = min(row + kFillRows, nRows);
+    for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * rowsPerTask < nRows; g += nWarps) {
+        uint64_t row = g * rowsPerTask;
+        const uint64_t rowEnd = min(row + rowsPerTask, nRows);
         while (row < rowEnd) {
             // The rows of [row, rowEnd) in one unit.
             const uint32_t u = b.nUnits > 1 ? unitOf(b.rowBase, b.nUnits, row) : 0u;
@@ -509,29 +516,35 @@ __global__ void rowFillKernel(Batch b, uint64_t nRows, uint32_t* __restrict__ fi
             const uint64_t r1 = min(rowEnd, uRow1);
             const Unit& U = b.units[u];
             const uint32_t ipx = U.g.ipx;
+            const FastDiv divX = U.g.divX;
             uint32_t* words = fill + U.wordBase;
             const uint32_t w0 = (uint32_t)(row - uRow0) * ipx, w1 = (uint32_t)(r1 - uRow0) * ipx;
             uint32_t carry = 0u;
-            for (uint32_t cb = w0; cb < w1; cb += 32u) {
-                const uint32_t w = cb + lane;
-                const bool valid = w < w1;
-                const uint32_t x = valid ? words[w] : 0u;
-                const uint32_t starts = __ballot_sync(0xffffffffu, valid && (w - w0) % ipx == 0u);
-                const uint32_t odd = __ballot_sync(0xffffffffu, __popc(x) & 1u);
-                const uint32_t upTo = starts & ((2u << lane) - 1u);   // row starts at lanes <= lane
-                uint32_t below = (1u << lane) - 1u;                  // lanes < lane
-                uint32_t pre;
-                if (upTo) {
-                    below &= ~((1u << (31u - __clz(upTo))) - 1u);
-                    pre = __popc(odd & below) & 1u;
-                } else {
-                    pre = (__popc(odd & below) & 1u) ^ carry;
+            for (uint32_t cb = w0; cb < w1; cb += 32u * kFillAhead) {
+                uint32_t x[kFillAhead];
+#pragma unroll
+                for (uint32_t q = 0; q < kFillAhead; ++q) x[q] = cb + 32u * q + lane < w1 ? words[cb + 32u * q + lane] : 0u;
+#pragma unroll
+                for (uint32_t q = 0; q < kFillAhead; ++q) {
+                    const uint32_t w = cb + 32u * q + lane;
+                    const bool valid = w < w1;
+                    const uint32_t starts = __ballot_sync(0xffffffffu, valid && divX.div(w) * ipx == w);
+                    const uint32_t odd = __ballot_sync(0xffffffffu, __popc(x[q]) & 1u);
+                    const uint32_t upTo = starts & ((2u << lane) - 1u);   // row starts at lanes <= lane
+                    uint32_t below = (1u << lane) - 1u;                  // lanes < lane
+                    uint32_t pre;
+                    if (upTo) {
+                        below &= ~((1u << (31u - __clz(upTo))) - 1u);
+                        pre = __popc(odd & below) & 1u;
+                    } else {
+                        pre = (__popc(odd & below) & 1u) ^ carry;
+                    }
+                    uint32_t p = x[q];
+                    p ^= p >> 1; p ^= p >> 2; p ^= p >> 4; p ^= p >> 8; p ^= p >> 16;
+                    if (pre) p = ~p;
+                    if (valid && p != x[q]) words[w] = p;
+                    carry = __shfl_sync(0xffffffffu, pre ^ (__popc(x[q]) & 1u), 31);
                 }
-                uint32_t p = x;
-                p ^= p >> 1; p ^= p >> 2; p ^= p >> 4; p ^= p >> 8; p ^= p >> 16;
-                if (pre) p = ~p;
-                if (valid && p != x) words[w] = p;
-                carry = __shfl_sync(0xffffffffu, pre ^ (__popc(x) & 1u), 31);
             }
             row = r1;
         }
@@ -568,8 +581,13 @@ void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* tot
     }
 }
 
-void launch_row_fill(const Batch& b, uint64_t nRows, uint32_t* fill, cudaStream_t s, uint32_t* launches) {
-    rowFillKernel<<<gridFor((nRows + kFillRows - 1) / kFillRows * 32u, 256), 256, 0, s>>>(b, nRows, fill);
+void launch_row_fill(const Batch& b, uint64_t nRows, uint64_t totalWords, uint32_t* fill, cudaStream_t s,
+                     uint32_t* launches) {
+    // About kFillWords words a task (six rounds of loads), less where
+    // that leaves fewer than 16 warps per SM.
+    const uint64_t rows = std::min(kFillWords * nRows / std::max<uint64_t>(totalWords, 1), nRows / (148u * 16u));
+    const uint32_t perTask = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(rows, 1), 512);
+    rowFillKernel<<<gridFor((nRows + perTask - 1) / perTask * 32u, 256), 256, 0, s>>>(b, nRows, perTask, fill);
     *launches += 1;
 }
 

@@ -525,9 +525,12 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
     unsigned long long* const hits = stage[threadIdx.x >> 5];
     uint32_t staged = 0;
     const uint32_t chunks = (total + 31u) / 32u;
-    const uint32_t batches = (chunks + chunksPerBatch - 1) / chunksPerBatch;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
+    // A short work list goes to all warps, a chunk each, before a warp takes
+    // several (3,000 chunks: 30 us with 8 a warp, 15 so).
+    chunksPerBatch = min(chunksPerBatch, max(chunks / nWarps, 1u));
+    const uint32_t batches = (chunks + chunksPerBatch - 1) / chunksPerBatch;
     // Batches in a fixed grid-stride order, or (queue != NULL) taken from a
     // device work queue, one atomic per batch, so that warps that drew cheap
     // batches keep working while others finish expensive ones.
@@ -784,22 +787,47 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
     if (MODE == 0) flush();
 }
 
-// Exclusive popcount prefix over the surface words (ranks of surface voxels).
+// Exclusive popcount prefix over the surface words (ranks of surface voxels)
+// in two launches.  The first sums the tiles, and the block that finishes last
+// (a counter, nobody waits) turns the sums into their prefix; the second
+// writes the ranks (tile offset plus the block's exclusive scan) and zeroes the
+// tile's keys.  The words were just written by the surface pass and are read
+// from L2 where they stay.  Ranks are only read where there are surface nodes,
+// so sectors of four words without any are not written.
+//
+// Bounds: DRAM.  Sums, ranks and zeroed keys took four launches:
+// room (13.5 M words) 64 us, now 60; duct (8.7 M) 43, now 24; batch of 64
+// meshes (21 M) 90, now 59; 44,000 words 13, now 8.  With every word's rank
+// written by tiles of four steps the room's second launch takes 58 instead of
+// 46 us.
 constexpr int kRankItems = 8;
-constexpr uint32_t kRankTile = kBlock * kRankItems;
+constexpr uint32_t kRankStep = kBlock * kRankItems;   // words of a step; a tile has S steps
 
-// Two passes over the surface words, the second after the tile sums are
-// scanned: kApply false writes each tile's popcount sum, kApply true writes
-// the ranks (tile offset plus the block's exclusive scan).  The words were
-// just written by the surface pass and are read from L2 where they stay.
-template <bool kApply>
-__global__ void rankTileKernel(const uint32_t* __restrict__ words, uint64_t n, WordRank* __restrict__ ranks,
-                               uint32_t* __restrict__ tileSums) {
-    __shared__ uint32_t warpSums[33];
-    const uint64_t base = (uint64_t)blockIdx.x * kRankTile + (uint64_t)threadIdx.x * kRankItems;
-    const bool whole = base + kRankItems <= n;   // 32-byte aligned: kRankItems words per thread
-    uint32_t x[kRankItems], c[kRankItems];
-    if (whole) {
+// Exclusive scan of v over the block, its total in *sum.
+__device__ __forceinline__ uint32_t blockScan(uint32_t v, uint32_t* warpSums, uint32_t* sum) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= (uint32_t)o) incl += t;
+    }
+    if (lane == 31) warpSums[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kBlock / 32; ++k) {
+        if (k < warp) before += warpSums[k];
+        all += warpSums[k];
+    }
+    __syncthreads();
+    *sum = all;
+    return before + incl - v;
+}
+
+__device__ __forceinline__ void rankLoad(const uint32_t* __restrict__ words, uint64_t n, uint64_t base,
+                                         uint32_t x[kRankItems]) {
+    if (base + kRankItems <= n) {   // 32-byte aligned: kRankItems words per thread
         const uint4 a = __ldg(reinterpret_cast<const uint4*>(words + base));
         const uint4 b = __ldg(reinterpret_cast<const uint4*>(words + base) + 1);
         x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
@@ -808,86 +836,99 @@ __global__ void rankTileKernel(const uint32_t* __restrict__ words, uint64_t n, W
 #pragma unroll
         for (int i = 0; i < kRankItems; ++i) x[i] = base + i < n ? __ldg(words + base + i) : 0u;
     }
-#pragma unroll
-    for (int i = 0; i < kRankItems; ++i) c[i] = (uint32_t)__popc(x[i]);
-    uint32_t sum = 0;
-#pragma unroll
-    for (int i = 0; i < kRankItems; ++i) sum += c[i];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) warpSums[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t s = lane < (kBlock / 32) ? warpSums[lane] : 0u;
-        uint32_t si = s;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, si, o);
-            if (lane >= o) si += t;
-        }
-        if (lane < kBlock / 32) warpSums[lane] = si - s;
-        if (lane == 31) warpSums[32] = si;
-    }
-    __syncthreads();
-    if (!kApply) {
-        if (threadIdx.x == 0) tileSums[blockIdx.x] = warpSums[32];
-        return;
-    }
-    uint32_t r[kRankItems];
-    uint32_t ex = __ldg(tileSums + blockIdx.x) + warpSums[warp] + incl - sum;
-#pragma unroll
-    for (int i = 0; i < kRankItems; ++i) {
-        r[i] = ex;
-        ex += c[i];
-    }
-    if (whole) {
-        uint4* out = reinterpret_cast<uint4*>(ranks + base);
-#pragma unroll
-        for (int i = 0; i < kRankItems; i += 2) out[i / 2] = make_uint4(x[i], r[i], x[i + 1], r[i + 1]);
-    } else {
-#pragma unroll
-        for (int i = 0; i < kRankItems; ++i)
-            if (base + i < n) ranks[base + i] = WordRank{x[i], r[i]};
-    }
 }
 
-__global__ void rankSumsKernel(uint32_t* tileSums, uint32_t nTiles, uint32_t* total) {
-    __shared__ uint32_t warpSums[33];
+// done: zero on entry, the number of blocks that have written their sums.
+// stepSums[step]: the surface nodes of the tile's steps before it.
+template <int S>
+__global__ void __launch_bounds__(kBlock) rankSumKernel(const uint32_t* __restrict__ words, uint64_t n,
+                                                        uint32_t* tileSums, uint32_t* __restrict__ stepSums,
+                                                        uint32_t* done, uint32_t* total) {
+    __shared__ uint32_t warpSums[kBlock / 32], steps[S][kBlock / 32];
+    __shared__ bool last;
+    uint32_t x[S][kRankItems], all;
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+        rankLoad(words, n, ((uint64_t)blockIdx.x * S + k) * kRankStep + (uint64_t)threadIdx.x * kRankItems, x[k]);
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < kRankItems; ++i) sum += (uint32_t)__popc(x[k][i]);
+        sum = __reduce_add_sync(kFull, sum);
+        if ((threadIdx.x & 31u) == 0) steps[k][threadIdx.x >> 5] = sum;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t sum = 0;
+        for (int k = 0; k < S; ++k) {
+            stepSums[(uint64_t)blockIdx.x * S + k] = sum;
+            for (int w = 0; w < kBlock / 32; ++w) sum += steps[k][w];
+        }
+        tileSums[blockIdx.x] = sum;
+        __threadfence();
+        last = atomicAdd(done, 1u) + 1u == gridDim.x;
+    }
+    __syncthreads();
+    if (!last) return;
     uint32_t carry = 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t start = 0; start < nTiles; start += blockDim.x) {
-        const uint32_t i = start + threadIdx.x;
-        const uint32_t v = i < nTiles ? tileSums[i] : 0u;
-        uint32_t incl = v;
+    for (uint32_t start = 0; start < gridDim.x; start += kRankStep) {
+        const uint32_t i0 = start + threadIdx.x * kRankItems;
+        uint32_t v[kRankItems], s = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
+        for (int i = 0; i < kRankItems; ++i) {
+            v[i] = i0 + i < gridDim.x ? __ldcg(tileSums + i0 + i) : 0u;
+            s += v[i];
         }
-        if (lane == 31) warpSums[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            const uint32_t s = lane < (int)(blockDim.x >> 5) ? warpSums[lane] : 0u;
-            uint32_t si = s;
+        uint32_t ex = carry + blockScan(s, warpSums, &all);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, si, o);
-                if (lane >= o) si += t;
-            }
-            if (lane < (int)(blockDim.x >> 5)) warpSums[lane] = si - s;
-            if (lane == 31) warpSums[32] = si;
+        for (int i = 0; i < kRankItems; ++i) {
+            if (i0 + i < gridDim.x) tileSums[i0 + i] = ex;
+            ex += v[i];
         }
-        __syncthreads();
-        if (i < nTiles) tileSums[i] = carry + warpSums[warp] + incl - v;
-        carry += warpSums[32];
-        __syncthreads();
+        carry += all;
     }
     if (threadIdx.x == 0) *total = carry;
+}
+
+template <bool kWide>
+__global__ void __launch_bounds__(kBlock) rankWriteKernel(const uint32_t* __restrict__ words, uint64_t n,
+                                                          WordRank* __restrict__ ranks,
+                                                          const uint32_t* __restrict__ tileSums,
+                                                          const uint32_t* __restrict__ stepSums, uint32_t stepsPerTile,
+                                                          void* keys, uint32_t keysCap) {
+    __shared__ uint32_t warpSums[kBlock / 32];
+    const uint64_t base = (uint64_t)blockIdx.x * kRankStep + (uint64_t)threadIdx.x * kRankItems;
+    uint32_t x[kRankItems], sum = 0, all;
+    rankLoad(words, n, base, x);
+#pragma unroll
+    for (int i = 0; i < kRankItems; ++i) sum += (uint32_t)__popc(x[i]);
+    const uint32_t first = __ldg(tileSums + blockIdx.x / stepsPerTile) + __ldg(stepSums + blockIdx.x);
+    uint32_t ex = first + blockScan(sum, warpSums, &all);
+#pragma unroll
+    for (int h = 0; h < kRankItems; h += 4) {
+        uint32_t r[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            r[i] = ex;
+            ex += (uint32_t)__popc(x[h + i]);
+        }
+        if (ex == r[0]) continue;
+        if (base + h + 4 <= n) {
+            uint4* out = reinterpret_cast<uint4*>(ranks + base + h);
+            out[0] = make_uint4(x[h], r[0], x[h + 1], r[1]);
+            out[1] = make_uint4(x[h + 2], r[2], x[h + 3], r[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (base + h + i < n) ranks[base + h + i] = WordRank{x[h + i], r[i]};
+        }
+    }
+    const uint64_t end = min((uint64_t)first + all, (uint64_t)keysCap);
+    for (uint64_t i = (uint64_t)first + threadIdx.x; i < end; i += kBlock) {
+        if (kWide) reinterpret_cast<unsigned long long*>(keys)[i] = 0ull;
+        else reinterpret_cast<uint32_t*>(keys)[i] = 0u;
+    }
 }
 
 __global__ void zeroKeysKernel(void* keys, const uint32_t* __restrict__ countPtr, uint32_t cap, int wide) {
@@ -982,13 +1023,20 @@ void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, c
     *launches += 1;
 }
 
-void launch_surface_rank(const uint32_t* bits, uint64_t words, WordRank* ranks, uint32_t* tileSums, uint32_t* total,
-                         cudaStream_t s, uint32_t* launches) {
-    const uint32_t tiles = (uint32_t)((words + kRankTile - 1) / kRankTile);
-    rankTileKernel<false><<<tiles ? tiles : 1, kBlock, 0, s>>>(bits, words, ranks, tileSums);
-    rankSumsKernel<<<1, 1024, 0, s>>>(tileSums, tiles, total);
-    rankTileKernel<true><<<tiles ? tiles : 1, kBlock, 0, s>>>(bits, words, ranks, tileSums);
-    *launches += 3;
+size_t surface_rank_sums(uint64_t words) { return 2 * (size_t)(words / kRankStep + 8); }
+
+void launch_surface_rank(const uint32_t* bits, uint64_t words, WordRank* ranks, uint32_t* sums, uint32_t* done,
+                         uint32_t* total, void* keys, uint32_t keysCap, int wide, cudaStream_t s, uint32_t* launches) {
+    // Tiles of four steps once there are two blocks of them per SM: fewer sums
+    // for the last block to scan.
+    const uint32_t S = words >= 148ull * 2 * 4 * kRankStep ? 4u : 1u;
+    const uint32_t steps = std::max(1u, (uint32_t)((words + kRankStep - 1) / kRankStep)), tiles = (steps + S - 1) / S;
+    uint32_t* stepSums = sums + tiles;   // up to S - 1 entries past `steps` are written
+    if (S == 4) rankSumKernel<4><<<tiles, kBlock, 0, s>>>(bits, words, sums, stepSums, done, total);
+    else rankSumKernel<1><<<tiles, kBlock, 0, s>>>(bits, words, sums, stepSums, done, total);
+    if (wide) rankWriteKernel<true><<<steps, kBlock, 0, s>>>(bits, words, ranks, sums, stepSums, S, keys, keysCap);
+    else rankWriteKernel<false><<<steps, kBlock, 0, s>>>(bits, words, ranks, sums, stepSums, S, keys, keysCap);
+    *launches += 2;
 }
 
 void launch_surface_keys_zero(void* keys, const uint32_t* count, uint32_t cap, int wide, cudaStream_t s,
