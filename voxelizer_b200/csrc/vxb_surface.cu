@@ -62,6 +62,9 @@ template <int M> __device__ __forceinline__ F3 crossF(F3 a, F3 b) {
 
 struct IBox { int lo[3], hi[3]; };
 
+// The division where divByF does not apply.
+__device__ __noinline__ float divideF(float x, float d) { return __fdiv_rn(x, d); }
+
 // getTriangleBounds (float3, src/voxelizer.cu:2366-2390) and
 // getVoxelBoundsHalf (2471-2492).
 __device__ __forceinline__ IBox voxBoundsHalf(const F3* v, const PassGeom& g) {
@@ -75,14 +78,25 @@ __device__ __forceinline__ IBox voxBoundsHalf(const F3* v, const PassGeom& g) {
         if (v[i].y > mx.y) mx.y = v[i].y;
         if (v[i].z > mx.z) mx.z = v[i].z;
     }
-    const float d = g.df;
+    const float d = g.df, rd = g.rdf;
+    const float a[6] = {__fsub_rn(mn.x, g.mnf[0]), __fsub_rn(mn.y, g.mnf[1]), __fsub_rn(mn.z, g.mnf[2]),
+                        __fsub_rn(mx.x, g.mnf[0]), __fsub_rn(mx.y, g.mnf[1]), __fsub_rn(mx.z, g.mnf[2])};
+    bool ok = rd != 0.0f;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) ok &= divExactF(a[i]);
+    float q[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) q[i] = divByF(a[i], d, rd);
+    if (!ok) {
+#pragma unroll
+        for (int i = 0; i < 6; ++i) q[i] = divideF(a[i], d);
+    }
     IBox b;
-    b.lo[0] = __float2int_rz(ceilf(__fsub_rn(__fdiv_rn(__fsub_rn(mn.x, g.mnf[0]), d), 0.5f)));
-    b.lo[1] = __float2int_rz(ceilf(__fsub_rn(__fdiv_rn(__fsub_rn(mn.y, g.mnf[1]), d), 0.5f)));
-    b.lo[2] = __float2int_rz(ceilf(__fsub_rn(__fdiv_rn(__fsub_rn(mn.z, g.mnf[2]), d), 0.5f)));
-    b.hi[0] = __float2int_rz(floorf(__fadd_rn(__fdiv_rn(__fsub_rn(mx.x, g.mnf[0]), d), 0.5f)));
-    b.hi[1] = __float2int_rz(floorf(__fadd_rn(__fdiv_rn(__fsub_rn(mx.y, g.mnf[1]), d), 0.5f)));
-    b.hi[2] = __float2int_rz(floorf(__fadd_rn(__fdiv_rn(__fsub_rn(mx.z, g.mnf[2]), d), 0.5f)));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        b.lo[i] = __float2int_ru(__fsub_rn(q[i], 0.5f));
+        b.hi[i] = __float2int_rd(__fadd_rn(q[3 + i], 0.5f));
+    }
     return b;
 }
 
@@ -198,18 +212,14 @@ static_assert(site::DT_3DY == 3 && site::DT_3DZ == 5, "depth range form");
 __device__ __forceinline__ float sum2fm(int m, float a, float b, float c, float d) {
     return m == 0 ? sum2f<0>(a, b, c, d) : m == 1 ? sum2f<1>(a, b, c, d) : sum2f<2>(a, b, c, d);
 }
-// setupYZ / ZX / XYOverlapTest (src/voxelizer.cu:2675-2757).  A = 0: (y, z)
-// oriented by n.x; A = 1: (z, x) by n.y; A = 2: (x, y) by n.z.
-template <int A, int DE> __device__ __forceinline__ Overlap setupOverlap(const F3* t, F3 n, float d) {
+// setupYZ / ZX / XYOverlapTest (src/voxelizer.cu:2675-2757): edge functions
+// over the coordinates (a, b) of the vertices, oriented by the normal's third
+// component.
+template <int DE> __device__ __forceinline__ Overlap setupOverlap(const float* a, const float* b, float nn, float d) {
     Overlap o;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        const F3& p = t[i];
-        const F3& q = t[(i + 1) % 3];
-        float pa, pb, qa, qb, nn;
-        if (A == 0) { pa = p.y; pb = p.z; qa = q.y; qb = q.z; nn = n.x; }
-        else if (A == 1) { pa = p.z; pb = p.x; qa = q.z; qb = q.x; nn = n.y; }
-        else { pa = p.x; pb = p.y; qa = q.x; qb = q.y; nn = n.z; }
+        const float pa = a[i], pb = b[i], qa = a[(i + 1) % 3], qb = b[(i + 1) % 3];
         if (nn >= 0.0f) { o.nx[i] = __fsub_rn(pb, qb); o.ny[i] = __fsub_rn(qa, pa); }
         else { o.nx[i] = __fsub_rn(qb, pb); o.ny[i] = __fsub_rn(pa, qa); }
         const float s = sum2fm((DE >> (2 * i)) & 3, o.nx[i], pa, o.ny[i], pb);
@@ -218,76 +228,91 @@ template <int A, int DE> __device__ __forceinline__ Overlap setupOverlap(const F
     return o;
 }
 
-// Component of (x, y, z) along the inner, outer or depth axis.
-__device__ __forceinline__ float along(uint32_t axis, int role, float x, float y, float z) {
-    return role == 0 ? (axis == 0 ? y : x) : role == 1 ? (axis == 2 ? y : z) : axis == 0 ? x : axis == 1 ? y : z;
+// (x, y, z) turned so that the axis comes first: [0] depth, then the two
+// coordinates of the dominant projection in its order ((y, z), (z, x) or
+// (x, y)).  The inner axis is [1], but [2] for axis 1; the outer one the other.
+template <class T> __device__ __forceinline__ T turned(uint32_t axis, int k, T x, T y, T z) {
+    return k == 0 ? (axis == 0 ? x : axis == 1 ? y : z) : k == 1 ? (axis == 0 ? y : axis == 1 ? z : x)
+                                                                 : (axis == 0 ? z : axis == 1 ? x : y);
 }
 
-// Set-up records of a triangle at position pos.
+// Set-up records of a triangle (the second one for 3D boxes only).
 __device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32_t t, const F3* v, const IBox& box,
-                                            uint32_t code, uint32_t units, uint32_t pos, SurfRec* __restrict__ recs,
-                                            SurfDepth* __restrict__ depth) {
+                                            uint32_t code, uint32_t units, SurfRec* rec, SurfDepth* depth) {
     const uint32_t bb = code >> 30, axis = (code >> 28) & 3u;
     const float d = U.g.df;
+    const int in = 1, out = 2;   // swapped for axis 1
     SurfRec r;
+    int lo[3], hi[3];
+    float m[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
         r.cu[i] = r.cf[i] = r.de[i] = 0.0f;
-        r.m[i] = along(axis, i, U.g.mnf[0], U.g.mnf[1], U.g.mnf[2]);
+        lo[i] = turned(axis, i, box.lo[0], box.lo[1], box.lo[2]);
+        hi[i] = turned(axis, i, box.hi[0], box.hi[1], box.hi[2]);
+        m[i] = turned(axis, i, U.g.mnf[0], U.g.mnf[1], U.g.mnf[2]);
     }
-    r.lo[0] = axis == 0 ? box.lo[1] : box.lo[0];
-    r.lo[1] = axis == 2 ? box.lo[1] : box.lo[2];
-    r.dlo = axis == 0 ? box.lo[0] : axis == 1 ? box.lo[1] : box.lo[2];
-    r.hi = 0;
-    r.ext = (uint32_t)((axis == 0 ? box.hi[1] : box.hi[0]) - r.lo[0]) + 1u;
+    const bool turn = axis == 1;
+    r.lo[0] = turn ? lo[out] : lo[in];
+    r.lo[1] = turn ? lo[in] : lo[out];
+    r.m[0] = turn ? m[out] : m[in];
+    r.m[1] = turn ? m[in] : m[out];
+    r.m[2] = m[0];
+    r.dlo = lo[0];
+    r.hi = bb == 3 ? hi[0] : turn ? hi[in] : hi[out];
+    r.ext = (uint32_t)((turn ? hi[out] : hi[in]) - r.lo[0]) + 1u;
     r.rext = __fdividef(1.0f, (float)r.ext);
     r.code = code | (units >= (1u << 22) ? kLongUnits : 0u) | (U.M ? __ldg(U.M + t) : 0u);
     r.unit = unit;
     if (bb >= 2) {
-        const F3 e0 = subF(v[0], v[2]), e1 = subF(v[1], v[0]);
-        const F3 n = bb == 2 ? crossF<site::CRF_2D>(e0, e1) : crossF<site::CRF_3D>(e0, e1);
-        static_assert(site::DE_2D_YZ == site::DE_3D_YZ && site::DE_2D_ZX == site::DE_3D_ZX &&
-                          site::DE_2D_XY == site::DE_3D_XY, "one set-up form");
-        Overlap o[3];
-        o[0] = setupOverlap<0, site::DE_3D_YZ>(v, n, d);
-        o[1] = setupOverlap<1, site::DE_3D_ZX>(v, n, d);
-        o[2] = setupOverlap<2, site::DE_3D_XY>(v, n, d);
+        static_assert(site::CRF_2D == site::CRF_3D && site::DE_2D_YZ == site::DE_3D_YZ &&
+                          site::DE_3D_ZX == site::DE_3D_YZ && site::DE_3D_XY == site::DE_3D_YZ &&
+                          site::DE_2D_ZX == site::DE_3D_YZ && site::DE_2D_XY == site::DE_3D_YZ, "one set-up form");
+        const F3 nv = crossF<site::CRF_3D>(subF(v[0], v[2]), subF(v[1], v[0]));
+        float n[3], p[3][3];   // p[k]: coordinate k of the three vertices
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            n[k] = turned(axis, k, nv.x, nv.y, nv.z);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) p[k][i] = turned(axis, k, v[i].x, v[i].y, v[i].z);
+        }
+        const Overlap o = setupOverlap<site::DE_3D_YZ>(p[1], p[2], n[0], d);
         // 2D boxes: products of the inner coordinate unfused, of the outer one
-        // fused; 3D boxes: products of the first coordinate unfused.  The
-        // first coordinate of the (z, x) projection is the outer one.
-        const bool swap = bb == 2 && axis == 1;
+        // fused; 3D boxes: products of the first coordinate unfused.
+        const bool swap = bb == 2 && turn;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const float nx = axis == 0 ? o[0].nx[i] : axis == 1 ? o[1].nx[i] : o[2].nx[i];
-            const float ny = axis == 0 ? o[0].ny[i] : axis == 1 ? o[1].ny[i] : o[2].ny[i];
-            r.cu[i] = swap ? ny : nx;
-            r.cf[i] = swap ? nx : ny;
-            r.de[i] = axis == 0 ? o[0].de[i] : axis == 1 ? o[1].de[i] : o[2].de[i];
+            r.cu[i] = swap ? o.ny[i] : o.nx[i];
+            r.cf[i] = swap ? o.nx[i] : o.ny[i];
+            r.de[i] = o.de[i];
         }
-        if (bb == 2) {
-            r.hi = axis == 2 ? box.hi[1] : box.hi[2];
-        } else {
-            r.hi = axis == 0 ? box.hi[0] : axis == 1 ? box.hi[1] : box.hi[2];
+        if (bb == 3) {
+            // The other two projections, tested in this order: the second
+            // coordinate and the depth, the depth and the first coordinate.
+            const Overlap f = setupOverlap<site::DE_3D_YZ>(p[2], p[0], n[1], d);
+            const Overlap g = setupOverlap<site::DE_3D_YZ>(p[0], p[1], n[2], d);
             SurfDepth s;
+            s.v0[0] = turn ? p[out][0] : p[in][0];
+            s.v0[1] = turn ? p[in][0] : p[out][0];
+            s.v0[2] = p[0][0];
+            s.n[0] = turn ? n[out] : n[in];
+            s.n[1] = turn ? n[in] : n[out];
+            s.n[2] = n[0];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                s.v0[i] = along(axis, i, v[0].x, v[0].y, v[0].z);
-                s.n[i] = along(axis, i, n.x, n.y, n.z);
-                // First test: (column, depth) coordinates of zx, xy or yz;
-                // second: (depth, column) coordinates of xy, yz or zx.
-                s.cc1[i] = axis == 0 ? o[1].nx[i] : axis == 1 ? o[2].nx[i] : o[0].nx[i];
-                s.cd1[i] = axis == 0 ? o[1].ny[i] : axis == 1 ? o[2].ny[i] : o[0].ny[i];
-                s.de1[i] = axis == 0 ? o[1].de[i] : axis == 1 ? o[2].de[i] : o[0].de[i];
-                s.cd2[i] = axis == 0 ? o[2].nx[i] : axis == 1 ? o[0].nx[i] : o[1].nx[i];
-                s.cc2[i] = axis == 0 ? o[2].ny[i] : axis == 1 ? o[0].ny[i] : o[1].ny[i];
-                s.de2[i] = axis == 0 ? o[2].de[i] : axis == 1 ? o[0].de[i] : o[1].de[i];
+                s.cc1[i] = f.nx[i];
+                s.cd1[i] = f.ny[i];
+                s.de1[i] = f.de[i];
+                s.cd2[i] = g.nx[i];
+                s.cc2[i] = g.ny[i];
+                s.de2[i] = g.de[i];
             }
-            s.rn = divScaleF(s.n[2]) ? __frcp_rn(s.n[2]) : 0.0f;
+            s.rn = divScaleF(n[0]) ? __frcp_rn(n[0]) : 0.0f;
             s.pad = s.pad2[0] = s.pad2[1] = 0.0f;
-            depth[pos] = s;
+            *depth = s;
         }
     }
-    recs[pos] = r;
+    *rec = r;
 }
 
 // Classification, positions and set-up.  A block takes kPrepThreads
@@ -303,10 +328,10 @@ __device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32
 // Bounds: the triangle gathers and the records' stores.  In place of a
 // classification, a partition by global (class, axis) cursors that set up the
 // records and a three-launch scan of the units: PREP_FIGURES
-constexpr int kPrepThreads = 256;
+constexpr int kPrepThreads = 128;
 constexpr uint32_t kUnitBits = 33;
 
-__global__ void __launch_bounds__(kPrepThreads) surfacePrepareKernel(Batch b, uint32_t nWork,
+__global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b, uint32_t nWork,
                                                                      unsigned long long* cursor,
                                                                      unsigned long long* total, uint32_t* classes,
                                                                      uint32_t* __restrict__ offsets,
@@ -389,12 +414,11 @@ __global__ void __launch_bounds__(kPrepThreads) surfacePrepareKernel(Batch b, ui
         }
         __syncthreads();
         // Positions past the arrays are only possible after a carry.
-        const uint32_t pos0 = (uint32_t)(base >> kUnitBits);
-        if (threadIdx.x < n && pos0 + threadIdx.x < nWork)
-            offsets[pos0 + threadIdx.x] = (uint32_t)(base + before + incl - x);
-        if (u && pos0 + at < nWork) {
+        const uint32_t pos0 = (uint32_t)(base >> kUnitBits), room = pos0 < nWork ? min(n, nWork - pos0) : 0u;
+        if (threadIdx.x < room) offsets[pos0 + threadIdx.x] = (uint32_t)(base + before + incl - x);
+        if (u && at < room) {
             if (triOf) triOf[pos0 + at] = t;
-            setupRecord(b.units[unit], unit, t, v, box, code, u, pos0 + at, recs, depth);
+            setupRecord(b.units[unit], unit, t, v, box, code, u, recs + pos0 + at, depth + pos0 + at);
         }
         __syncthreads();
     }
