@@ -591,221 +591,220 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
             const uint32_t item = base + lane, pos = t0 + k;
             t0 += k31 + (nextOff == base + 32u ? 1u : 0u);
 
-            // The item's column and its depth range [dlo, dhi]; `deep` for
-            // the ranges of 3D boxes, which are clamped to [blo, bhi] and the
-            // slices below.
+            // The item's column and its depth range [a, z]; `deep` for 3D
+            // boxes, whose range comes from the plane.
             const Unit* U = b.units;
             uint32_t code = 0, nSlices = 0;
-            int inner = 0, outer = 0, dlo = 0, dhi = -1, blo = 0, bhi = -1;
+            int inner = 0, outer = 0, dlo = 0, dhi = -1, blo = 0, bhi = 0;
             float pi = 0.0f, po = 0.0f, mD = 0.0f, d = 0.0f;
             bool deep = false;
             if (item < total) {
-                const SurfRec& rec = recs[pos];
-                const float4 r0 = __ldg(reinterpret_cast<const float4*>(&rec)),
-                             r1 = __ldg(reinterpret_cast<const float4*>(&rec) + 1);
-                const uint4 r2 = __ldg(reinterpret_cast<const uint4*>(&rec) + 2),
-                            r3 = __ldg(reinterpret_cast<const uint4*>(&rec) + 3);
-                const float4 r4 = __ldg(reinterpret_cast<const float4*>(&rec) + 4);
-                const float cu[3] = {r0.x, r0.y, r0.z}, cf[3] = {r0.w, r1.x, r1.y},
-                            de[3] = {r1.z, r1.w, __uint_as_float(r2.x)};
-                const uint32_t ext = r2.w;
+                const uint4* rec = reinterpret_cast<const uint4*>(recs + pos);
+                const uint4 r2 = __ldg(rec + 2), r3 = __ldg(rec + 3), r0 = __ldg(rec), r1 = __ldg(rec + 1),
+                            r4 = __ldg(rec + 4);
                 code = r3.y;
                 U = b.units + r3.z;
+                const uint32_t ext = r2.w, axis = (code >> 28) & 3u, bb = code >> 30, u = item - ok;
                 inner = (int)r2.y;
                 outer = (int)r2.z;
-                dlo = (int)r3.w;
-                const int hi = __float_as_int(r4.x);
-                mD = r4.w;
-                const uint32_t axis = (code >> 28) & 3u, bb = code >> 30;
-                const uint32_t u = item - ok;
+                dlo = blo = (int)r3.w;
+                bhi = (int)r4.x;
+                mD = __uint_as_float(r4.w);
                 if (bb == 1) {
                     dlo += (int)u;
                     dhi = dlo;
                 } else {
                     // u / ext by the approximate reciprocal, which is off by
                     // one at the most below 2^22 columns.
-                    uint32_t q, m;
-                    if (code & kLongUnits) {
-                        q = u / ext;
-                        m = u - q * ext;
-                    } else {
-                        q = (uint32_t)((float)u * __uint_as_float(r3.x));
-                        m = u - q * ext;
-                        if ((int)m < 0) {
-                            m += ext;
-                            --q;
-                        }
-                        if (m >= ext) {
-                            m -= ext;
-                            ++q;
-                        }
+                    uint32_t q = (uint32_t)((float)u * __uint_as_float(r3.x));
+                    if (code & kLongUnits) q = u / ext;
+                    int m = (int)(u - q * ext);
+                    if (m < 0) {
+                        m += (int)ext;
+                        --q;
+                    }
+                    if ((uint32_t)m >= ext) {
+                        m -= (int)ext;
+                        ++q;
                     }
                     const int olo = outer;
-                    inner += (int)m;
+                    inner += m;
                     outer += (int)q;
                     d = U->g.df;
-                    pi = vbComp(inner, r4.y, d);
-                    po = vbComp(outer, r4.z, d);
+                    pi = vbComp(inner, __uint_as_float(r4.y), d);
+                    po = vbComp(outer, __uint_as_float(r4.z), d);
+                    const float cu[3] = {__uint_as_float(r0.x), __uint_as_float(r0.y), __uint_as_float(r0.z)},
+                                cf[3] = {__uint_as_float(r0.w), __uint_as_float(r1.x), __uint_as_float(r1.y)},
+                                de[3] = {__uint_as_float(r1.z), __uint_as_float(r1.w), __uint_as_float(r2.x)};
+                    const bool turn = bb == 3u && axis == 1u;
+                    const float pu = turn ? po : pi, pf = turn ? pi : po;
+                    bool hit = true;
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) hit &= sum2p1f<2>(cu[i], pu, cf[i], pf, de[i]) >= 0.0f;
                     if (bb == 2) {
                         constexpr int UN = site::UNR_2D[K];
-                        bool pro = false;
                         if (UN > 1) {
+                            // Outer iterations of the prolog are unfused.
                             const uint32_t oa = axis == 2 ? 1u : 2u;   // outer axis
-                            int lo = olo, ohi = hi;
+                            int lo = olo, ohi = bhi;
                             if (U->sliceN[oa] > 1u)
                                 subspaceRange(b.slices + 2 * (U->sliceBase + U->sliceN[0] + (oa == 2u ? U->sliceN[1] : 0u)),
                                               U->sliceN[oa], outer, lo, ohi);
-                            pro = inProlog<UN>(outer - lo, ohi - lo + 1);
-                        }
-                        bool hit = true;
+                            if (inProlog<UN>(outer - lo, ohi - lo + 1)) {
+                                hit = true;
 #pragma unroll
-                        for (int i = 0; i < 3; ++i)
-                            hit &= (pro ? sum2p1f<0>(cu[i], pi, cf[i], po, de[i])
-                                        : sum2p1f<2>(cu[i], pi, cf[i], po, de[i])) >= 0.0f;
+                                for (int i = 0; i < 3; ++i) hit &= sum2p1f<0>(cu[i], pi, cf[i], po, de[i]) >= 0.0f;
+                            }
+                        }
                         dhi = hit ? dlo : dlo - 1;
                     } else {
-                        const float pu = axis == 1 ? po : pi, pf = axis == 1 ? pi : po;
-                        bool hit = true;
-#pragma unroll
-                        for (int i = 0; i < 3; ++i) hit &= sum2p1f<2>(cu[i], pu, cf[i], pf, de[i]) >= 0.0f;
                         dhi = dlo - 1;
                         if (hit) {
                             const float4* s = reinterpret_cast<const float4*>(depth + pos);
                             deep = true;
-                            blo = dlo;
-                            bhi = hi;
-                            depthRange<K>(axis, pi, po, __ldg(s), __ldg(s + 1), mD, d, U->g.rdf, dlo, dhi);
                             nSlices = U->sliceN[axis];
+                            depthRange<K>(axis, pi, po, __ldg(s), __ldg(s + 1), mD, d, U->g.rdf, dlo, dhi);
                         }
                     }
                 }
             }
             const uint32_t axis = (code >> 28) & 3u;
-            // One slice of the depth axis at a time (a single one covers the
-            // grid, and the box is inside the grid).
-            uint32_t s = 0;
-            do {
-                int a = dlo, z = s == 0u ? dhi : dlo - 1;
-                if (deep) {
-                    int lo = blo, hi = bhi;
-                    if (nSlices > 1u) {
-                        const uint32_t* sl = b.slices + 2 * (U->sliceBase + (axis >= 1u ? U->sliceN[0] : 0u) +
-                                                             (axis == 2u ? U->sliceN[1] : 0u));
-                        if (s < nSlices) {
-                            lo = max(lo, (int)__ldg(sl + 2 * s));
-                            hi = min(hi, (int)__ldg(sl + 2 * s + 1) - 1);
-                        } else {
-                            hi = lo - 1;
-                        }
-                    } else if (s > 0u) {
-                        hi = lo - 1;
-                    }
-                    if (lo > hi || dlo > hi || dhi < lo) {
-                        a = 0;
-                        z = -1;
-                    } else {
-                        a = max(dlo, lo);
-                        z = min(dhi, hi);
-                    }
+            // The hits among voxels a + w0 .. a + w0 + 31 of a range of cnt.
+            auto test = [&](int a, uint32_t cnt, uint32_t w0) {
+                if (w0 >= cnt) return 0u;
+                if (!deep || cnt == 1u) return 1u;
+                float e[20];   // cc1 cd1 de1 cc2 cd2 de2
+                const float4* f = reinterpret_cast<const float4*>(depth + pos) + 2;
+#pragma unroll
+                for (int i = 0; i < 5; ++i) {
+                    const float4 q = __ldg(f + i);
+                    e[4 * i] = q.x; e[4 * i + 1] = q.y; e[4 * i + 2] = q.z; e[4 * i + 3] = q.w;
                 }
-                const uint32_t cnt = z >= a ? (uint32_t)(z - a) + 1u : 0u;
-                for (uint32_t w0 = 0; __any_sync(kFull, w0 < cnt); w0 += 32u) {
-                    // Hits of voxels a + w0 .. a + w0 + 31.
-                    uint32_t m = w0 < cnt ? 1u : 0u;
-                    if (deep && cnt > 1u && w0 < cnt) {
-                        float e[20];   // cc1 cd1 de1 cc2 cd2 de2
-                        const float4* f = reinterpret_cast<const float4*>(depth + pos) + 2;
+                const float p1 = axis == 1 ? pi : po, p2 = axis == 1 ? po : pi;
+                float k1[3], k2[3];
 #pragma unroll
-                        for (int i = 0; i < 5; ++i) {
-                            const float4 q = __ldg(f + i);
-                            e[4 * i] = q.x; e[4 * i + 1] = q.y; e[4 * i + 2] = q.z; e[4 * i + 3] = q.w;
-                        }
-                        const float p1 = axis == 1 ? pi : po, p2 = axis == 1 ? po : pi;
-                        float k1[3], k2[3];
+                for (int i = 0; i < 3; ++i) {
+                    k1[i] = __fmul_rn(e[i], p1);
+                    k2[i] = __fmul_rn(e[9 + i], p2);
+                }
+                const uint32_t last = min(cnt - w0, 32u);
+                uint32_t m = 0u;
+                for (uint32_t v = 0; v < last; ++v) {
+                    const float pd = vbComp(a + (int)(w0 + v), mD, d);
+                    bool hit = true;
 #pragma unroll
-                        for (int i = 0; i < 3; ++i) {
-                            k1[i] = __fmul_rn(e[i], p1);
-                            k2[i] = __fmul_rn(e[9 + i], p2);
-                        }
-                        const uint32_t last = min(cnt - w0, 32u);
-                        m = 0u;
-                        for (uint32_t v = 0; v < last; ++v) {
-                            const float pd = vbComp(a + (int)(w0 + v), mD, d);
-                            bool hit = true;
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) {
-                                hit &= __fadd_rn(__fmaf_rn(e[3 + i], pd, k1[i]), e[6 + i]) >= 0.0f;
-                                hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
-                            }
-                            m |= hit ? 1u << v : 0u;
-                        }
-                        constexpr int UL = site::UNR_3DL[K];
-                        static_assert(UL == 0 || UL == 2, "at most one prolog iteration");
-                        // The prolog iteration in its own form of the first
-                        // test (the x-dominant one differs by node type).
-                        if (UL == 2 && w0 == 0u && (cnt & 1u) && (kXProlog == 21 || axis != 0u)) {
-                            const float pd = vbComp(a, mD, d);
-                            bool hit = true;
-#pragma unroll
-                            for (int i = 0; i < 3; ++i) {
-                                hit &= __fadd_rn(__fmaf_rn(e[i], p1, __fmul_rn(e[3 + i], pd)), e[6 + i]) >= 0.0f;
-                                hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
-                            }
-                            m = (m & ~1u) | (hit ? 1u : 0u);
-                        }
+                    for (int i = 0; i < 3; ++i) {
+                        hit &= __fadd_rn(__fmaf_rn(e[3 + i], pd, k1[i]), e[6 + i]) >= 0.0f;
+                        hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
                     }
-                    if (!__any_sync(kFull, m != 0u)) continue;
-                    // Bit position in the unit of the column's voxel at depth
-                    // 0 and its step along the depth.  The allocation holds a
-                    // voxel one column further along x and padY / padZ rows
-                    // further along y / z.
-                    uint32_t at = 0, step = 0;
-                    uint64_t wordBase = 0;
+                    m |= hit ? 1u << v : 0u;
+                }
+                constexpr int UL = site::UNR_3DL[K];
+                static_assert(UL == 0 || UL == 2, "at most one prolog iteration");
+                // The prolog iteration in its own form of the first test (the
+                // x-dominant one differs by node type).
+                if (UL == 2 && w0 == 0u && (cnt & 1u) && (kXProlog == 21 || axis != 0u)) {
+                    const float pd = vbComp(a, mD, d);
+                    bool hit = true;
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) {
+                        hit &= __fadd_rn(__fmaf_rn(e[i], p1, __fmul_rn(e[3 + i], pd)), e[6 + i]) >= 0.0f;
+                        hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
+                    }
+                    m = (m & ~1u) | (hit ? 1u : 0u);
+                }
+                return m;
+            };
+            // Records the hits m of voxels first + 0 .. 31 along the depth
+            // (whole warp).
+            auto record = [&](uint32_t m, int first) {
+                uint32_t live = __ballot_sync(kFull, m != 0u);
+                if (!live) return;
+                // Bit position in the unit of the voxel at `first` and its
+                // step along the depth.  The allocation holds a voxel one
+                // column further along x and padY / padZ rows further along
+                // y / z.
+                uint32_t at = 0, step = 0;
+                uint32_t* bits = sink.bits;
+                unsigned long long entry = 0;
+                uint64_t wordBase = 0;
+                if (m) {
+                    const uint32_t X = U->g.X, AY = U->g.AY, pY = U->g.padY, pZ = U->g.padZ;
+                    wordBase = U->wordBase;
+                    bits += wordBase;
+                    entry = (wordBase << 29) | ((code >> 30) << 8) | (code & 255u);
+                    const uint32_t zr = axis == 2 ? pZ : (uint32_t)outer + pZ;
+                    const uint32_t yr = pY + (axis == 0 ? (uint32_t)inner : axis == 2 ? (uint32_t)outer : 0u);
+                    step = axis == 0 ? 1u : axis == 1 ? X : X * AY;
+                    at = (zr * AY + yr) * X + (axis == 0 ? 1u : (uint32_t)inner + 1u) + (uint32_t)first * step;
+                }
+                do {
                     if (m) {
-                        const uint32_t X = U->g.X, AY = U->g.AY, pY = U->g.padY, pZ = U->g.padZ;
-                        wordBase = U->wordBase;
-                        const uint32_t zr = axis == 2 ? pZ : (uint32_t)outer + pZ;
-                        const uint32_t yr = pY + (axis == 0 ? (uint32_t)inner : axis == 2 ? (uint32_t)outer : 0u);
-                        step = axis == 0 ? 1u : axis == 1 ? X : X * AY;
-                        at = (zr * AY + yr) * X + (axis == 0 ? 1u : (uint32_t)inner + 1u) + (uint32_t)(a + (int)w0) * step;
-                    }
-                    const uint32_t cls = code >> 30, mat = code & 255u;
-                    for (;;) {
-                        const uint32_t live = __ballot_sync(kFull, m != 0u);
-                        if (!live) break;
-                        if (m) {
-                            const uint32_t v = __ffs(m) - 1;
-                            m &= m - 1u;
-                            const uint32_t p = at + v * step, bit = p & 31u;
+                        const uint32_t v = __ffs(m) - 1;
+                        m &= m - 1u;
+                        const uint32_t p = at + v * step, bit = p & 31u;
+                        if (MODE != 1) {
+                            atomicOr(bits + (p >> 5), 0x80000000u >> bit);
+                            if (MODE == 0)
+                                hits[staged + __popc(live & laneMaskLt())] = entry + ((unsigned long long)p << 24);
+                        } else {
                             const uint64_t w = wordBase + (p >> 5);
-                            if (MODE != 1) {
-                                atomicOr(sink.bits + w, 0x80000000u >> bit);
-                                if (MODE == 0)
-                                    hits[staged + __popc(live & laneMaskLt())] =
-                                        ((w * 32u + bit) << 24) | (cls << 8) | mat;
-                            } else {
-                                const WordRank wr = sink.wordRank[w];
-                                const uint32_t r = wr.rank + (bit ? __popc(wr.bits >> (32u - bit)) : 0u);
-                                if (r < sink.keysCap) {
-                                    if (kWide) {
-                                        const unsigned long long key = ((unsigned long long)cls << 40) |
-                                                                       ((unsigned long long)mat << 32) |
-                                                                       __ldg(triOf + pos);
-                                        atomicMax(reinterpret_cast<unsigned long long*>(sink.keys) + r, key);
-                                        sink.positions[r] = w * 32u + bit;   // every hit of a voxel stores the same
-                                    } else {
-                                        atomicMax(reinterpret_cast<uint32_t*>(sink.keys) + r, (cls << 8) | mat);
-                                    }
+                            const WordRank wr = sink.wordRank[w];
+                            const uint32_t r = wr.rank + (bit ? __popc(wr.bits >> (32u - bit)) : 0u);
+                            if (r < sink.keysCap) {
+                                const uint32_t cls = code >> 30, mat = code & 255u;
+                                if (kWide) {
+                                    const unsigned long long key = ((unsigned long long)cls << 40) |
+                                                                   ((unsigned long long)mat << 32) | __ldg(triOf + pos);
+                                    atomicMax(reinterpret_cast<unsigned long long*>(sink.keys) + r, key);
+                                    sink.positions[r] = w * 32u + bit;   // every hit of a voxel stores the same
+                                } else {
+                                    atomicMax(reinterpret_cast<uint32_t*>(sink.keys) + r, (cls << 8) | mat);
                                 }
                             }
                         }
-                        if (MODE == 0) {
-                            staged += __popc(live);
-                            if (staged > kStageHits - 32u) flush();
-                        }
                     }
+                    if (MODE == 0) {
+                        staged += __popc(live);
+                        if (staged > kStageHits - 32u) flush();
+                    }
+                    live = __ballot_sync(kFull, m != 0u);
+                } while (live);
+            };
+            // One slice covers the grid, and the box is inside the grid.
+            if (!__any_sync(kFull, nSlices > 1u)) {
+                int a = dlo, z = dhi;
+                if (deep) {
+                    a = max(dlo, blo);
+                    z = min(dhi, bhi);
+                    if (dlo > bhi || dhi < blo) z = a - 1;
                 }
-            } while (__any_sync(kFull, ++s < nSlices));
+                const uint32_t cnt = z >= a ? (uint32_t)(z - a) + 1u : 0u;
+                record(test(a, cnt, 0u), a);
+                if (__any_sync(kFull, cnt > 32u))
+                    for (uint32_t w0 = 32u; __any_sync(kFull, w0 < cnt); w0 += 32u) record(test(a, cnt, w0), a + (int)w0);
+                continue;
+            }
+            // One slice of the depth axis at a time.
+            for (uint32_t s = 0; __any_sync(kFull, s == 0u || s < nSlices); ++s) {
+                int a = dlo, z = s == 0u ? dhi : dlo - 1;
+                if (deep) {
+                    int lo = blo, hi = bhi;
+                    if (s < nSlices) {
+                        const uint32_t* sl = b.slices + 2 * (U->sliceBase + (axis >= 1u ? U->sliceN[0] : 0u) +
+                                                             (axis == 2u ? U->sliceN[1] : 0u));
+                        lo = max(lo, (int)__ldg(sl + 2 * s));
+                        hi = min(hi, (int)__ldg(sl + 2 * s + 1) - 1);
+                    } else {
+                        hi = lo - 1;
+                    }
+                    a = max(dlo, lo);
+                    z = min(dhi, hi);
+                    if (lo > hi || dlo > hi || dhi < lo) z = a - 1;
+                }
+                const uint32_t cnt = z >= a ? (uint32_t)(z - a) + 1u : 0u;
+                for (uint32_t w0 = 0; __any_sync(kFull, w0 < cnt); w0 += 32u) record(test(a, cnt, w0), a + (int)w0);
+            }
         }
     }
     if (MODE == 0) flush();
