@@ -138,16 +138,23 @@ __device__ __forceinline__ IBox gridClamp(IBox b, const PassGeom& g) {
     return b;
 }
 
-// Work units: voxels along the axis for 1D boxes, columns of the dominant
-// projection otherwise; 0 for an empty (fully outside) box.
-__device__ __forceinline__ uint32_t surfUnits(const IBox& b, uint32_t code) {
+// Columns of the dominant projection (voxels along the axis for 1D boxes); 0
+// for an empty (fully outside) box.  *rows: work units, rows of up to 32
+// columns (a 1D line is one).
+__device__ __forceinline__ uint32_t surfColumns(const IBox& b, uint32_t code, uint32_t* rows) {
+    *rows = 0u;
     if (b.lo[0] > b.hi[0] || b.lo[1] > b.hi[1] || b.lo[2] > b.hi[2]) return 0u;
     const uint32_t bb = code >> 30, axis = (code >> 28) & 3u;
     const uint32_t ex = (uint32_t)(b.hi[0] - b.lo[0] + 1), ey = (uint32_t)(b.hi[1] - b.lo[1] + 1),
                    ez = (uint32_t)(b.hi[2] - b.lo[2] + 1);
     if (bb == 0) return 0u;
-    if (bb == 1) return axis == 0 ? ex : axis == 1 ? ey : ez;
-    return axis == 0 ? ey * ez : axis == 1 ? ex * ez : ex * ey;
+    if (bb == 1) {
+        *rows = 1u;
+        return axis == 0 ? ex : axis == 1 ? ey : ez;
+    }
+    const uint32_t in = axis == 0 ? ey : ex, out = axis == 2 ? ey : ez;
+    *rows = (in + 31u) / 32u * out;
+    return in * out;
 }
 
 // The unit and mesh triangle of work triangle wt.
@@ -171,13 +178,12 @@ struct __align__(16) SurfRec {
     float cu[3], cf[3], de[3];
     int lo[2];          // voxel box clamped to the grid: first inner, outer
     uint32_t ext;       // inner extent
-    float rext;         // about 1 / ext
-    uint32_t code;      // class << 30 | axis << 28 | kLongUnits | material
+    uint32_t segs;      // work units of a row: its 32-column segments
+    uint32_t code;      // class << 30 | axis << 28 | material
     uint32_t unit;      // unit of the batch
-    int dlo, hi;        // first depth; last depth (3D) or outer (2D)
+    int dlo, hi;        // first depth; last depth (1D, 3D) or outer (2D)
     float m[3];         // minimum corner along inner, outer, depth
 };
-constexpr uint32_t kLongUnits = 1u << 27;   // 2^22 or more columns
 // Second record (112 bytes) of 3D boxes, in (inner, outer, depth) order.
 struct __align__(16) SurfDepth {
     float v0[3], n[3];  // first vertex, normal
@@ -238,7 +244,7 @@ template <class T> __device__ __forceinline__ T turned(uint32_t axis, int k, T x
 
 // Set-up records of a triangle (the second one for 3D boxes only).
 __device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32_t t, const F3* v, const IBox& box,
-                                            uint32_t code, uint32_t units, SurfRec* rec, SurfDepth* depth) {
+                                            uint32_t code, SurfRec* rec, SurfDepth* depth) {
     const uint32_t bb = code >> 30, axis = (code >> 28) & 3u;
     const float d = U.g.df;
     const int in = 1, out = 2;   // swapped for axis 1
@@ -259,10 +265,10 @@ __device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32
     r.m[1] = turn ? m[in] : m[out];
     r.m[2] = m[0];
     r.dlo = lo[0];
-    r.hi = bb == 3 ? hi[0] : turn ? hi[in] : hi[out];
+    r.hi = bb != 2 ? hi[0] : turn ? hi[in] : hi[out];
     r.ext = (uint32_t)((turn ? hi[out] : hi[in]) - r.lo[0]) + 1u;
-    r.rext = __fdividef(1.0f, (float)r.ext);
-    r.code = code | (units >= (1u << 22) ? kLongUnits : 0u) | (U.M ? __ldg(U.M + t) : 0u);
+    r.segs = (r.ext + 31u) / 32u;
+    r.code = code | (U.M ? __ldg(U.M + t) : 0u);
     r.unit = unit;
     if (bb >= 2) {
         static_assert(site::CRF_2D == site::CRF_3D && site::DE_2D_YZ == site::DE_3D_YZ &&
@@ -321,13 +327,15 @@ __device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32
 // and their work units with one 64-bit atomic: *cursor counts triangles above
 // bit kUnitBits and units below, so that positions and unit offsets of all
 // blocks follow the same order.  offsets[pos] is the first unit of pos.
-// *total is the exact number of units: past 2^32 - 2 of them the cursor may
-// have carried and the work kernel does nothing.  classes[0..3): triangles per
+// *total is the number of columns: past 2^32 - 2 of them the cursor may have
+// carried and the work kernel does nothing.  classes[0..3): triangles per
 // class.
 //
 // Bounds: the triangle gathers and the records' stores.  In place of a
 // classification, a partition by global (class, axis) cursors that set up the
-// records and a three-launch scan of the units: PREP_FIGURES
+// records and a three-launch scan of the units, 140 us on the room and 455 on
+// a batch of 64 meshes (4.2 M triangles), now 73 and 245 us.  Records staged in
+// shared memory and stored in order took 76 and 297 us.
 constexpr int kPrepThreads = 128;
 constexpr uint32_t kUnitBits = 33;
 
@@ -345,7 +353,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint64_t b0 = (uint64_t)blockIdx.x * kPrepThreads; b0 < nWork; b0 += (uint64_t)gridDim.x * kPrepThreads) {
         const uint64_t wt = b0 + threadIdx.x;
-        uint32_t t = 0, unit = 0, code = 0, u = 0;
+        uint32_t t = 0, unit = 0, code = 0, u = 0, columns = 0;
         F3 v[3];
         IBox box;
         if (wt < nWork) {
@@ -356,7 +364,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
                 const IBox full = voxBoundsHalf(v, U.g);
                 code = classifyTri(v, full);
                 box = gridClamp(full, U.g);
-                u = surfUnits(box, code);
+                columns = surfColumns(box, code, &u);
             }
         }
         const uint32_t bucket = u ? ((code >> 30) - 1u) * 3u + ((code >> 28) & 3u) : kNone;
@@ -406,8 +414,11 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
         }
         if (threadIdx.x == 0 && n) {
             base = atomicAdd(cursor, ((unsigned long long)n << kUnitBits) + sum);
-            atomicAdd(total, sum);
         }
+        unsigned long long all = columns;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) all += __shfl_down_sync(kFull, all, o);
+        if (lane == 0 && all) atomicAdd(total, all);
         if (threadIdx.x < 3) {
             const uint32_t c = cnt[(threadIdx.x + 1u) * 3u * kW] - cnt[threadIdx.x * 3u * kW];
             if (c) atomicAdd(classes + threadIdx.x, c);
@@ -418,7 +429,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
         if (threadIdx.x < room) offsets[pos0 + threadIdx.x] = (uint32_t)(base + before + incl - x);
         if (u && at < room) {
             if (triOf) triOf[pos0 + at] = t;
-            setupRecord(b.units[unit], unit, t, v, box, code, u, recs + pos0 + at, depth + pos0 + at);
+            setupRecord(b.units[unit], unit, t, v, box, code, recs + pos0 + at, depth + pos0 + at);
         }
         __syncthreads();
     }
@@ -506,19 +517,30 @@ struct Sink {
 // Hits of one warp are staged in shared memory before they go to the global
 // hit list, so that the list takes one atomic per flush.
 constexpr uint32_t kStageHits = 256;
+constexpr int kWorkThreads = 128;
 
-// The work list.  Warps take batches of `chunksPerBatch` consecutive 32-item
-// chunks; within a batch the owner of each chunk's first item follows from
-// the previous chunk.  Every listed triangle has at least one unit, so a
-// chunk's 32 items belong to at most 32 consecutive positions: lane l loads
-// off[t0 + l] and a bit mask of the triangle starts inside the chunk gives
-// every lane its owner.
+// The rows of a warp's last two chunks, and the warp's queue of columns that
+// pass (slot of the row << 5 | column).
+struct SurfWarp {
+    int4 a[64];     // inner of the first column, outer, position, code
+    int4 b[64];     // unit, first and last depth, minimum corner along the depth
+    float2 c[64];   // minimum corner along the inner axis, the row's corner along the outer axis
+    uint16_t queue[1024 + 32];
+};
+
+// The work list: rows of up to 32 columns of the dominant projection.  Warps
+// take batches of `chunksPerBatch` consecutive chunks of 32 rows; within a
+// batch the owner of each chunk's first row follows from the previous chunk.
+// Every listed triangle has at least one row, so a chunk's rows belong to at
+// most 32 consecutive positions: lane l loads off[t0 + l] and a bit mask of
+// the triangle starts inside the chunk gives every lane its owner.
 //
-// A lane takes one item: a voxel of a 1D line, a column of a 2D box
-// (process2DTriangles, src/voxelizer.cu:3418-3596: the dominant projection
-// only) or of a 3D box (process3DTriangles, 3603-3955: dominant projection,
+// A lane takes one row and tests its columns against the dominant projection
+// (all of process2DTriangles, src/voxelizer.cu:3418-3596, and the first test
+// of process3DTriangles, 3603-3955), about ten operations a column.  The
+// columns that pass, about half, are queued and worked 32 at a time, a lane each: a
 // depth range from the plane, then per material subspace slice of the depth
-// axis either the single voxel or the other two projections per voxel).  The
+// axis either the single voxel or the other two projections per voxel.  The
 // products of the column's coordinate do not change along the depth, so a
 // depth voxel costs six fused edge values.  The depth loop only marks hits
 // (32 voxels at a time in a mask); they are recorded afterwards, one per lane
@@ -529,9 +551,19 @@ constexpr uint32_t kStageHits = 256;
 // hit list; mode 1: merge the key at the voxel's rank (surface bits are
 // complete); mode 2: set the bit only.  PartialNodes have 64-bit keys.
 //
-// Bounds: issue.  WORK_FIGURES
+// Bounds: issue (about two thirds of the slots) and the latency of the record
+// and edge gathers.  With a column per lane, 303 of 570 instructions of a
+// chunk of 32 columns found the owner and loaded its record, and half of the
+// lanes idled through the rest.  Alone on a B200, a column per lane with hits
+// recorded inside the depth loop / marked first / by rows: room (22.3 M
+// columns, 19.2 M hits) 582 / 527 / 450 us, stress FCC mesh (slivers) 193 /
+// 163 / 73 us, duct 120 / 103 / 95 us.  A list of 5,120 triangles takes 18-22
+// instead of 14 us.  The stage must hold several steps' hits: with 128 or 64
+// entries instead of 256 the waits for the list's counter make it 676 and
+// 967 us; prefetching the next chunk's records and larger batches gave
+// nothing (508-540 us with 8 chunks a batch).
 template <int K, int MODE>
-__global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch b, const SurfRec* __restrict__ recs,
+__global__ void __launch_bounds__(kWorkThreads, 8) surfaceWorkKernel(Sink sink, Batch b, const SurfRec* __restrict__ recs,
                                                                const SurfDepth* __restrict__ depth,
                                                                const uint32_t* __restrict__ triOf,
                                                                const uint32_t* __restrict__ off,
@@ -541,18 +573,22 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
     constexpr bool kWide = K == kPartial;
     constexpr int kXProlog = site::OT_3DXP_ZX[K];
     static_assert(kXProlog == site::OT_3DX_ZX || kXProlog == 21, "x-dominant prolog form");
-    __shared__ unsigned long long stage[kBlock / 32][MODE == 0 ? kStageHits : 1];
-    const unsigned long long exact = *totalPtr;
-    if (exact >= 0xFFFFFFFFull) return;   // refused by the host
-    const uint32_t n = (uint32_t)(*cursor >> kUnitBits), total = (uint32_t)exact;
+    __shared__ unsigned long long stage[kWorkThreads / 32][MODE == 0 ? kStageHits : 1];
+    __shared__ SurfWarp shared[kWorkThreads / 32];
+    if (*totalPtr >= 0xFFFFFFFFull) return;   // refused by the host
+    const unsigned long long listed = *cursor;
+    const uint32_t n = (uint32_t)(listed >> kUnitBits), total = (uint32_t)listed;
     const uint32_t lane = threadIdx.x & 31u;
     unsigned long long* const hits = stage[threadIdx.x >> 5];
+    SurfWarp& sw = shared[threadIdx.x >> 5];
     uint32_t staged = 0;
-    const uint32_t chunks = (total + 31u) / 32u;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
-    // A short work list goes to all warps, a chunk each, before a warp takes
-    // several (3,000 chunks: 30 us with 8 a warp, 15 so).
+    // A short list goes to the warps that fit the device, in chunks of fewer
+    // rows and a chunk each, before a warp takes several.
+    uint32_t rows = 32u;   // per chunk, a power of two
+    while (rows > 1u && total / rows < 148u * 32u) rows >>= 1;
+    const uint32_t chunks = (total + rows - 1u) / rows;
     chunksPerBatch = min(chunksPerBatch, max(chunks / nWarps, 1u));
     const uint32_t batches = (chunks + chunksPerBatch - 1) / chunksPerBatch;
     // Batches in a fixed grid-stride order, or (queue != NULL) taken from a
@@ -574,105 +610,178 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
         __syncwarp();
         staged = 0;
     };
-    for (uint32_t bt = queue ? nextBatch(0) : warp; bt < batches; bt = nextBatch(bt)) {
-        const uint32_t c1 = min((bt + 1) * chunksPerBatch, chunks);
-        uint32_t t0 = warpFindOwner(off, n, bt * chunksPerBatch * 32u, lane);
-        for (uint32_t c = bt * chunksPerBatch; c < c1; ++c) {
-            const uint32_t base = c * 32u;
+    uint32_t bt = queue ? nextBatch(0) : warp, c = 0, c1 = 0, t0 = 0;   // batch, its chunks left, first position
+    uint32_t half = 0, head = 0, tail = 0;   // row slots to fill next, queue entries
+    bool drain = false;
+    for (;;) {
+        // Full groups of columns first; a partial one only when its row slots
+        // are needed or nothing is left.
+        if (tail - head < 32u && !(drain && tail != head)) {
+            drain = false;
+            if (c == c1) {
+                if (bt >= batches) {
+                    if (tail == head) break;
+                    drain = true;
+                    continue;
+                }
+                c = bt * chunksPerBatch;
+                c1 = min(c + chunksPerBatch, chunks);
+                t0 = warpFindOwner(off, n, c * rows, lane);
+                bt = nextBatch(bt);
+            }
+            // What is left moves to the front of the queue.
+            const uint32_t left = tail - head;
+            const uint32_t entry = lane < left ? sw.queue[head + lane] : 0u;
+            if (__any_sync(kFull, lane < left && (entry >> 10) == half)) {
+                drain = true;
+                continue;
+            }
+            __syncwarp();
+            if (lane < left) sw.queue[lane] = (uint16_t)entry;
+            head = 0;
+            const uint32_t base = c * rows;
             const uint32_t ol = t0 + lane < n ? __ldg(off + t0 + lane) : total;
             const uint32_t o32 = t0 + 32u < n ? __ldg(off + t0 + 32u) : total;
             const uint32_t starts =
-                __reduce_or_sync(kFull, (t0 + lane < n && lane >= 1u && ol < base + 32u) ? 1u << (ol - base) : 0u);
+                __reduce_or_sync(kFull, (t0 + lane < n && lane >= 1u && ol < base + rows) ? 1u << (ol - base) : 0u);
             const uint32_t k = __popc(starts & ((2u << lane) - 1u));
             const uint32_t ok = __shfl_sync(kFull, ol, k);
             const uint32_t k31 = __popc(starts);
             const uint32_t next = __shfl_sync(kFull, ol, (k31 + 1u) & 31u);
             const uint32_t nextOff = k31 < 31u ? next : o32;
             const uint32_t item = base + lane, pos = t0 + k;
-            t0 += k31 + (nextOff == base + 32u ? 1u : 0u);
-
-            // The item's column and its depth range [a, z]; `deep` for 3D
-            // boxes, whose range comes from the plane.
+            t0 += k31 + (nextOff == base + rows ? 1u : 0u);
+            ++c;
+            // The columns of the row that pass the dominant projection.
+            uint32_t pass = 0;
+            if (lane < rows && item < total) {
+                const uint4* rec = reinterpret_cast<const uint4*>(recs + pos);
+                const uint4 r2 = __ldg(rec + 2), r3 = __ldg(rec + 3), r4 = __ldg(rec + 4), r0 = __ldg(rec),
+                            r1 = __ldg(rec + 1);
+                const uint32_t code = r3.y, ext = r2.w, segs = r3.x, axis = (code >> 28) & 3u, bb = code >> 30;
+                int inner = (int)r2.y, outer = (int)r2.z;
+                float po = 0.0f;
+                if (bb == 1) {
+                    pass = 1u;
+                } else {
+                    const Unit* U = b.units + r3.z;
+                    uint32_t row = item - ok, cols = ext;
+                    if (segs > 1u) {
+                        const uint32_t u = row;
+                        row = u / segs;
+                        const uint32_t seg = u - row * segs;
+                        inner += (int)(32u * seg);
+                        cols = min(ext - 32u * seg, 32u);
+                    }
+                    outer += (int)row;
+                    const float d = U->g.df, mI = __uint_as_float(r4.y);
+                    po = vbComp(outer, __uint_as_float(r4.z), d);
+                    const float cu[3] = {__uint_as_float(r0.x), __uint_as_float(r0.y), __uint_as_float(r0.z)},
+                                de[3] = {__uint_as_float(r1.z), __uint_as_float(r1.w), __uint_as_float(r2.x)};
+                    float cf[3] = {__uint_as_float(r0.w), __uint_as_float(r1.x), __uint_as_float(r1.y)};
+                    if (bb == 3u && axis == 1u) {
+                        // Products of the outer coordinate unfused.
+                        float k[3];
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) k[i] = __fmul_rn(cu[i], po);
+                        for (uint32_t c2 = 0; c2 < cols; ++c2) {
+                            const float pi = vbComp(inner + (int)c2, mI, d);
+                            bool hit = true;
+#pragma unroll
+                            for (int i = 0; i < 3; ++i) hit &= __fadd_rn(__fmaf_rn(cf[i], pi, k[i]), de[i]) >= 0.0f;
+                            pass |= hit ? 1u << c2 : 0u;
+                        }
+                    } else {
+                        float pf = po;
+                        if (bb == 2) {
+                            constexpr int UN = site::UNR_2D[K];
+                            if (UN > 1) {
+                                const uint32_t oa = axis == 2 ? 1u : 2u;   // outer axis
+                                int lo = (int)r2.z, hi = (int)r4.x;
+                                if (U->sliceN[oa] > 1u)
+                                    subspaceRange(b.slices + 2 * (U->sliceBase + U->sliceN[0] + (oa == 2u ? U->sliceN[1] : 0u)),
+                                                  U->sliceN[oa], outer, lo, hi);
+                                if (inProlog<UN>(outer - lo, hi - lo + 1)) {
+                                    // Prolog rows are unfused: the outer
+                                    // product rounded, then added (times 1).
+#pragma unroll
+                                    for (int i = 0; i < 3; ++i) cf[i] = __fmul_rn(cf[i], po);
+                                    pf = 1.0f;
+                                }
+                            }
+                        }
+                        for (uint32_t c2 = 0; c2 < cols; ++c2) {
+                            const float pi = vbComp(inner + (int)c2, mI, d);
+                            bool hit = true;
+#pragma unroll
+                            for (int i = 0; i < 3; ++i)
+                                hit &= __fadd_rn(__fmaf_rn(cf[i], pf, __fmul_rn(cu[i], pi)), de[i]) >= 0.0f;
+                            pass |= hit ? 1u << c2 : 0u;
+                        }
+                    }
+                }
+                const uint32_t slot = half * 32u + lane;
+                sw.a[slot] = make_int4(inner, outer, (int)pos, (int)code);
+                sw.b[slot] = make_int4((int)r3.z, (int)r3.w, (int)r4.x, (int)r4.w);
+                sw.c[slot] = make_float2(__uint_as_float(r4.y), po);
+            }
+            const uint32_t cnt = __popc(pass);
+            uint32_t incl = cnt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t q = __shfl_up_sync(kFull, incl, o);
+                if (lane >= (uint32_t)o) incl += q;
+            }
+            uint32_t at = left + incl - cnt;
+            while (pass) {
+                sw.queue[at++] = (uint16_t)((half << 10) | (lane << 5) | (__ffs(pass) - 1));
+                pass &= pass - 1u;
+            }
+            tail = left + __shfl_sync(kFull, incl, 31);
+            half ^= 1u;
+            __syncwarp();
+            continue;
+        }
+        {
+            const uint32_t q0 = head, queued = tail;
+            head += min(tail - head, 32u);
+            // The lane's column and its depth range; `deep` for 3D boxes, whose
+            // range comes from the plane.
             const Unit* U = b.units;
-            uint32_t code = 0, nSlices = 0;
+            uint32_t code = 0, nSlices = 0, pos = 0;
             int inner = 0, outer = 0, dlo = 0, dhi = -1, blo = 0, bhi = 0;
             float pi = 0.0f, po = 0.0f, mD = 0.0f, d = 0.0f;
             bool deep = false;
-            if (item < total) {
-                const uint4* rec = reinterpret_cast<const uint4*>(recs + pos);
-                const uint4 r2 = __ldg(rec + 2), r3 = __ldg(rec + 3), r0 = __ldg(rec), r1 = __ldg(rec + 1),
-                            r4 = __ldg(rec + 4);
-                code = r3.y;
-                U = b.units + r3.z;
-                const uint32_t ext = r2.w, axis = (code >> 28) & 3u, bb = code >> 30, u = item - ok;
-                inner = (int)r2.y;
-                outer = (int)r2.z;
-                dlo = blo = (int)r3.w;
-                bhi = (int)r4.x;
-                mD = __uint_as_float(r4.w);
-                if (bb == 1) {
-                    dlo += (int)u;
-                    dhi = dlo;
-                } else {
-                    // u / ext by the approximate reciprocal, which is off by
-                    // one at the most below 2^22 columns.
-                    uint32_t q = (uint32_t)((float)u * __uint_as_float(r3.x));
-                    if (code & kLongUnits) q = u / ext;
-                    int m = (int)(u - q * ext);
-                    if (m < 0) {
-                        m += (int)ext;
-                        --q;
-                    }
-                    if ((uint32_t)m >= ext) {
-                        m -= (int)ext;
-                        ++q;
-                    }
-                    const int olo = outer;
-                    inner += m;
-                    outer += (int)q;
+            if (q0 + lane < queued) {
+                const uint32_t e = sw.queue[q0 + lane], src = e >> 5;
+                const int4 ra = sw.a[src], rb = sw.b[src];
+                const float2 rc = sw.c[src];
+                code = (uint32_t)ra.w;
+                pos = (uint32_t)ra.z;
+                U = b.units + rb.x;
+                inner = ra.x + (int)(e & 31u);
+                outer = ra.y;
+                dlo = blo = rb.y;
+                bhi = rb.z;
+                mD = __int_as_float(rb.w);
+                const uint32_t bb = code >> 30, axis = (code >> 28) & 3u;
+                dhi = bb == 1u ? bhi : dlo;
+                if (bb == 3u) {
                     d = U->g.df;
-                    pi = vbComp(inner, __uint_as_float(r4.y), d);
-                    po = vbComp(outer, __uint_as_float(r4.z), d);
-                    const float cu[3] = {__uint_as_float(r0.x), __uint_as_float(r0.y), __uint_as_float(r0.z)},
-                                cf[3] = {__uint_as_float(r0.w), __uint_as_float(r1.x), __uint_as_float(r1.y)},
-                                de[3] = {__uint_as_float(r1.z), __uint_as_float(r1.w), __uint_as_float(r2.x)};
-                    const bool turn = bb == 3u && axis == 1u;
-                    const float pu = turn ? po : pi, pf = turn ? pi : po;
-                    bool hit = true;
-#pragma unroll
-                    for (int i = 0; i < 3; ++i) hit &= sum2p1f<2>(cu[i], pu, cf[i], pf, de[i]) >= 0.0f;
-                    if (bb == 2) {
-                        constexpr int UN = site::UNR_2D[K];
-                        if (UN > 1) {
-                            // Outer iterations of the prolog are unfused.
-                            const uint32_t oa = axis == 2 ? 1u : 2u;   // outer axis
-                            int lo = olo, ohi = bhi;
-                            if (U->sliceN[oa] > 1u)
-                                subspaceRange(b.slices + 2 * (U->sliceBase + U->sliceN[0] + (oa == 2u ? U->sliceN[1] : 0u)),
-                                              U->sliceN[oa], outer, lo, ohi);
-                            if (inProlog<UN>(outer - lo, ohi - lo + 1)) {
-                                hit = true;
-#pragma unroll
-                                for (int i = 0; i < 3; ++i) hit &= sum2p1f<0>(cu[i], pi, cf[i], po, de[i]) >= 0.0f;
-                            }
-                        }
-                        dhi = hit ? dlo : dlo - 1;
-                    } else {
-                        dhi = dlo - 1;
-                        if (hit) {
-                            const float4* s = reinterpret_cast<const float4*>(depth + pos);
-                            deep = true;
-                            nSlices = U->sliceN[axis];
-                            depthRange<K>(axis, pi, po, __ldg(s), __ldg(s + 1), mD, d, U->g.rdf, dlo, dhi);
-                        }
-                    }
+                    pi = vbComp(inner, rc.x, d);
+                    po = rc.y;
+                    const float4* s = reinterpret_cast<const float4*>(depth + pos);
+                    deep = true;
+                    nSlices = U->sliceN[axis];
+                    depthRange<K>(axis, pi, po, __ldg(s), __ldg(s + 1), mD, d, U->g.rdf, dlo, dhi);
                 }
             }
             const uint32_t axis = (code >> 28) & 3u;
             // The hits among voxels a + w0 .. a + w0 + 31 of a range of cnt.
             auto test = [&](int a, uint32_t cnt, uint32_t w0) {
                 if (w0 >= cnt) return 0u;
-                if (!deep || cnt == 1u) return 1u;
+                const uint32_t last = min(cnt - w0, 32u);
+                if (!deep || cnt == 1u) return kFull >> (32u - last);
                 float e[20];   // cc1 cd1 de1 cc2 cd2 de2
                 const float4* f = reinterpret_cast<const float4*>(depth + pos) + 2;
 #pragma unroll
@@ -687,7 +796,6 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
                     k1[i] = __fmul_rn(e[i], p1);
                     k2[i] = __fmul_rn(e[9 + i], p2);
                 }
-                const uint32_t last = min(cnt - w0, 32u);
                 uint32_t m = 0u;
                 for (uint32_t v = 0; v < last; ++v) {
                     const float pd = vbComp(a + (int)(w0 + v), mD, d);
@@ -771,40 +879,33 @@ __global__ void __launch_bounds__(kBlock, 4) surfaceWorkKernel(Sink sink, Batch 
                     live = __ballot_sync(kFull, m != 0u);
                 } while (live);
             };
-            // One slice covers the grid, and the box is inside the grid.
-            if (!__any_sync(kFull, nSlices > 1u)) {
-                int a = dlo, z = dhi;
-                if (deep) {
-                    a = max(dlo, blo);
-                    z = min(dhi, bhi);
-                    if (dlo > bhi || dhi < blo) z = a - 1;
-                }
-                const uint32_t cnt = z >= a ? (uint32_t)(z - a) + 1u : 0u;
-                record(test(a, cnt, 0u), a);
-                if (__any_sync(kFull, cnt > 32u))
-                    for (uint32_t w0 = 32u; __any_sync(kFull, w0 < cnt); w0 += 32u) record(test(a, cnt, w0), a + (int)w0);
-                continue;
+            // The range clamped to the box, one piece per material subspace
+            // slice (most ranges lie in one).
+            int a = dlo, z = dhi;
+            if (deep) {
+                a = max(dlo, blo);
+                z = min(dhi, bhi);
             }
-            // One slice of the depth axis at a time.
-            for (uint32_t s = 0; __any_sync(kFull, s == 0u || s < nSlices); ++s) {
-                int a = dlo, z = s == 0u ? dhi : dlo - 1;
-                if (deep) {
-                    int lo = blo, hi = bhi;
-                    if (s < nSlices) {
-                        const uint32_t* sl = b.slices + 2 * (U->sliceBase + (axis >= 1u ? U->sliceN[0] : 0u) +
-                                                             (axis == 2u ? U->sliceN[1] : 0u));
-                        lo = max(lo, (int)__ldg(sl + 2 * s));
-                        hi = min(hi, (int)__ldg(sl + 2 * s + 1) - 1);
-                    } else {
-                        hi = lo - 1;
+            do {
+                int end = z;
+                if (nSlices > 1u && a <= z) {
+                    const uint32_t* sl = b.slices + 2 * (U->sliceBase + (axis >= 1u ? U->sliceN[0] : 0u) +
+                                                         (axis == 2u ? U->sliceN[1] : 0u)) + 1;
+                    uint32_t e = __ldg(sl);
+                    while ((uint32_t)a >= e) {
+                        sl += 2;
+                        e = __ldg(sl);
                     }
-                    a = max(dlo, lo);
-                    z = min(dhi, hi);
-                    if (lo > hi || dlo > hi || dhi < lo) z = a - 1;
+                    end = min(z, (int)e - 1);
                 }
-                const uint32_t cnt = z >= a ? (uint32_t)(z - a) + 1u : 0u;
-                for (uint32_t w0 = 0; __any_sync(kFull, w0 < cnt); w0 += 32u) record(test(a, cnt, w0), a + (int)w0);
-            }
+                const uint32_t cnt = end >= a ? (uint32_t)(end - a) + 1u : 0u;
+                uint32_t w0 = 0;
+                do {
+                    record(test(a, cnt, w0), a + (int)w0);
+                    w0 += 32u;
+                } while (__any_sync(kFull, w0 < cnt));
+                a = end + 1;
+            } while (__any_sync(kFull, a <= z));
         }
     }
     if (MODE == 0) flush();
@@ -1013,10 +1114,10 @@ static void launchSurfaceWorkKind(int mode, uint32_t grid, const Sink& sink, con
                                   const unsigned long long* cursor, const unsigned long long* total, uint32_t batch,
                                   uint32_t* queue, cudaStream_t s) {
     if (mode == 0)
-        surfaceWorkKernel<K, 0><<<grid, kBlock, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
+        surfaceWorkKernel<K, 0><<<grid, kWorkThreads, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
     else if (mode == 1)
-        surfaceWorkKernel<K, 1><<<grid, kBlock, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
-    else surfaceWorkKernel<K, 2><<<grid, kBlock, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
+        surfaceWorkKernel<K, 1><<<grid, kWorkThreads, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
+    else surfaceWorkKernel<K, 2><<<grid, kWorkThreads, 0, s>>>(sink, b, R, D, triOf, offsets, cursor, total, batch, queue);
 }
 
 void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, const void* depth, const uint32_t* triOf,
@@ -1035,14 +1136,16 @@ void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, c
     sink.list = list;
     sink.listCount = listCount;
     sink.listCap = listCap;
-    const uint32_t grid = 148u * blocksPerSm;
+    const uint32_t grid = 148u * blocksPerSm * (256u / kWorkThreads);   // shapes count blocks of 256 threads
     const SurfRec* R = static_cast<const SurfRec*>(recs);
     const SurfDepth* D = static_cast<const SurfDepth*>(depth);
     auto launch = kind == kShort ? launchSurfaceWorkKind<kShort>
                 : kind == kLong ? launchSurfaceWorkKind<kLong>
                 : kind == kPartial ? launchSurfaceWorkKind<kPartial>
                 : kind == kShortFcc ? launchSurfaceWorkKind<kShortFcc> : launchSurfaceWorkKind<kLongFcc>;
-    launch(mode, grid, sink, b, R, D, triOf, offsets, cursor, total, batch, queue, s);
+    // The shapes count chunks of 32 columns; four of them make about one of 32
+    // rows.
+    launch(mode, grid, sink, b, R, D, triOf, offsets, cursor, total, std::max(batch / 4u, 1u), queue, s);
     *launches += 1;
 }
 
