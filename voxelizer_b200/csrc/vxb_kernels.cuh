@@ -173,8 +173,8 @@ int meshCheck(const float* dV, uint32_t nV, const uint32_t* dI, uint64_t nIdx, u
 // Pruning of every unit (Cartesian node grids): `solid` from fill | surf
 // (surf may be NULL).  counts[p], p < passes, is the length of pass p's
 // change list and *overflow a flag, all zero on entry.  Pass 0 goes over all
-// words, pass 1 over the words it changed (list0), the others in one block
-// with alternating lists of at most `cap` (unit << 32 | word) entries.  The
+// words, pass 1 over the words it changed (list0), the others in one cluster
+// with alternating lists of at most `cap` (unit << 32 | word) entries.
 // blockBase: exclusive prefix over the units of prune_blocks (nUnits + 1
 // entries) for `planes` = prune_planes(totalWords); `blocks` is their sum.  The
 // grid is pruned unless counts[passes - 1] or *overflow is set (a list longer

@@ -350,11 +350,16 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     for (bool& u : tuneUsed_) u = false;
     // Work counts, hit count and pruning counts.
     VXB_CUDA(cudaMemsetAsync(st, 0, 4 * (kPruneCounts + (size_t)kPasses), s));
-    // Surface voxelization, hit list and surface ranks on the side stream,
-    // beside the solid pass (they share no buffer).
+    // The surface pass runs on the side stream beside the solid pass (they
+    // share no buffer).  The solid pass is queued behind the surface work, which
+    // covers the host time of its launches, and before the ranks.
     cudaStream_t ss = s;
     const bool serial = timer && timer->enabled && timer->serial;
-    if (anyMaterials_) {
+    // Without a hit list (PartialNode keys, or the tuned strategy) the first
+    // traversal sets surface bits only and a second one merges every hit at its
+    // rank.
+    const bool retraverse = wide_ || shape.surfMerge != 0;
+    auto surfaceBits = [&]() -> int {
         if (!serial) {
             ss = side_;
             VXB_CUDA(cudaEventRecord(evFork_, s));
@@ -366,10 +371,6 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
                                reinterpret_cast<unsigned long long*>(st + kSurfTotal), st + kSurfClasses,
                                sOffsets.as<uint32_t>(), wide_ ? triOf.as<uint32_t>() : nullptr, recs.p, depth.p, ss,
                                &launches);
-        // Without a hit list (PartialNode keys, or the tuned strategy) the
-        // first traversal sets surface bits only and a second one merges
-        // every hit at its rank.
-        const bool retraverse = wide_ || shape.surfMerge != 0;
         if (timer) timer->mark(5, false, ss);
         tuneMark(kKnobSurfaceSpan, false, ss);
         tuneMark(kKnobSurface, false, ss);
@@ -377,6 +378,9 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         tuneMark(kKnobSurface, true, ss);
         if (timer) timer->mark(5, true, ss);
         VXB_CUDA(cudaEventRecord(evSurfBits_, ss));
+        return 0;
+    };
+    auto surfaceKeys = [&]() -> int {
         // Ranks, and zeroed material keys by rank.
         launch_surface_rank(surf.as<uint32_t>(), totalWords_, ranks.as<WordRank>(), rankTiles.as<uint32_t>(),
                             st + kRankDone, st + kSurfaceVoxels, keys.p, keysCap_, wide_ ? 1 : 0, ss, &launches);
@@ -393,6 +397,12 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
         tuneMark(kKnobSurfaceSpan, true, ss);
         if (timer) timer->mark(4, true, ss);
         VXB_CUDA(cudaEventRecord(evSurfDone_, ss));
+        return 0;
+    };
+    if (anyMaterials_) {
+        if (int rc = surfaceBits()) return rc;
+        if (serial)
+            if (int rc = surfaceKeys()) return rc;
     }
     // Solid voxelization.
     mark(0, false);
@@ -404,6 +414,8 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     tuneMark(kKnobToggle, true, s);
     launch_row_fill(b, totalRows_, totalWords_, fillP, s, &launches);
     mark(0, true);
+    if (anyMaterials_ && !serial)
+        if (int rc = surfaceKeys()) return rc;
     if (!nodes_) {
         if (!aliasFill_)
             for (const Unit& u : units_)
@@ -416,7 +428,9 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     // bits (pruning runs beside the merge) to the join with the merged keys:
     // the merge's cost on the way to emission, not its own duration.
     bool mergeSpan = false;
-    if (anyMaterials_ && !serial) {
+    // Small grids do not fill the device, so the priority is not worth two
+    // event pairs (5 us of a 100 us call).
+    if (anyMaterials_ && !serial && totalWords_ >= kPriorityWords) {
         VXB_CUDA(cudaEventRecord(evSolid_, s));
         VXB_CUDA(cudaStreamWaitEvent(hi_, evSolid_, 0));
         ps = hi_;
