@@ -334,8 +334,11 @@ __device__ __forceinline__ void setupRecord(const Unit& U, uint32_t unit, uint32
 // Bounds: the triangle gathers and the records' stores.  In place of a
 // classification, a partition by global (class, axis) cursors that set up the
 // records and a three-launch scan of the units, 140 us on the room and 455 on
-// a batch of 64 meshes (4.2 M triangles), now 73 and 245 us.  Records staged in
-// shared memory and stored in order took 76 and 297 us.
+// a batch of 64 meshes (4.2 M triangles), now 70 and 215 us.  Records staged in
+// shared memory and stored in order took 20% more.  Atomics on the shared
+// counters are about 1 ns each, so blocks add theirs up over their triangles
+// (added per 128 triangles: 245 us) and take 32 sets per SM at the most (64: 5
+// us more).
 constexpr int kPrepThreads = 128;
 constexpr uint32_t kUnitBits = 33;
 
@@ -351,6 +354,8 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
     __shared__ uint32_t sorted[kPrepThreads];               // units in order of position
     __shared__ unsigned long long warpSum[kW], base;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned long long allColumns = 0;   // of the thread's triangles
+    uint32_t ofClass = 0;                // the block's triangles of class threadIdx.x + 1
     for (uint64_t b0 = (uint64_t)blockIdx.x * kPrepThreads; b0 < nWork; b0 += (uint64_t)gridDim.x * kPrepThreads) {
         const uint64_t wt = b0 + threadIdx.x;
         uint32_t t = 0, unit = 0, code = 0, u = 0, columns = 0;
@@ -415,14 +420,8 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
         if (threadIdx.x == 0 && n) {
             base = atomicAdd(cursor, ((unsigned long long)n << kUnitBits) + sum);
         }
-        unsigned long long all = columns;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) all += __shfl_down_sync(kFull, all, o);
-        if (lane == 0 && all) atomicAdd(total, all);
-        if (threadIdx.x < 3) {
-            const uint32_t c = cnt[(threadIdx.x + 1u) * 3u * kW] - cnt[threadIdx.x * 3u * kW];
-            if (c) atomicAdd(classes + threadIdx.x, c);
-        }
+        allColumns += columns;
+        if (threadIdx.x < 3) ofClass += cnt[(threadIdx.x + 1u) * 3u * kW] - cnt[threadIdx.x * 3u * kW];
         __syncthreads();
         // Positions past the arrays are only possible after a carry.
         const uint32_t pos0 = (uint32_t)(base >> kUnitBits), room = pos0 < nWork ? min(n, nWork - pos0) : 0u;
@@ -433,6 +432,10 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
         }
         __syncthreads();
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) allColumns += __shfl_down_sync(kFull, allColumns, o);
+    if (lane == 0 && allColumns) atomicAdd(total, allColumns);
+    if (threadIdx.x < 3 && ofClass) atomicAdd(classes + threadIdx.x, ofClass);
 }
 
 // getSingleVoxelBoundsComponent, src/voxelizer.cu:2575-2586.
@@ -1103,7 +1106,7 @@ __global__ void mergeKeysKernel(const unsigned long long* __restrict__ list, con
 void launch_surface_prepare(const Batch& b, uint32_t nWork, unsigned long long* cursor, unsigned long long* total,
                             uint32_t* classes, uint32_t* offsets, uint32_t* triOf, void* recs, void* depth,
                             cudaStream_t s, uint32_t* launches) {
-    surfacePrepareKernel<<<gridFor(nWork, kPrepThreads, 148u * 64u), kPrepThreads, 0, s>>>(
+    surfacePrepareKernel<<<gridFor(nWork, kPrepThreads, 148u * 32u), kPrepThreads, 0, s>>>(
         b, nWork, cursor, total, classes, offsets, triOf, static_cast<SurfRec*>(recs), static_cast<SurfDepth*>(depth));
     *launches += 1;
 }
