@@ -501,11 +501,19 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
 
 void Pipeline::surfaceWork(int mode, cudaStream_t s) {
     uint32_t* st = status.as<uint32_t>();
+    // Few triangles in a small grid: a single wave of blocks (4 per SM of 256
+    // threads) instead of four, of which three find no work (128^3: 17.4 us,
+    // four waves 22.6).  On large grids the few triangles have many rows, and a
+    // wave that stays resident holds up the solid pass (4096 x 256 x 256: 377
+    // us a call, with four waves 370).
+    const uint32_t blocksPerSm = nWork_ <= kFewTriangles && totalWords_ < kPriorityWords
+                                     ? std::min(shape.surfBlocksPerSm, 4u)
+                                     : shape.surfBlocksPerSm;
     launch_surface_work(nodeKind_, mode, batch(), recs.p, depth.p, triOf.as<uint32_t>(), sOffsets.as<uint32_t>(),
                         reinterpret_cast<unsigned long long*>(st + kSurfCursor),
                         reinterpret_cast<unsigned long long*>(st + kSurfTotal), surf.as<uint32_t>(),
                         ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(),
-                        hitList.as<unsigned long long>(), st + kHitCount, listCap_, shape.surfBlocksPerSm,
+                        hitList.as<unsigned long long>(), st + kHitCount, listCap_, blocksPerSm,
                         shape.surfBatch, shape.surfQueue ? st + kSurfQueue : nullptr, s, &launches);
 }
 
