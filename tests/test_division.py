@@ -47,6 +47,35 @@ def test_quotient_is_correctly_rounded(scale):
     assert _div_by(0.0, ds[0]) == 0.0
 
 
+def _round32(x):
+    """A rational rounded to FP32 (nearest, ties to even), exactly."""
+    f = np.float32(float(x))
+    near = [f, np.nextafter(f, np.float32(np.inf)), np.nextafter(f, np.float32(-np.inf))]
+    return min(near, key=lambda c: (abs(Fraction(float(c)) - x), int(c.view(np.uint32)) & 1))
+
+
+def _div_by_f(x, d):
+    fx, fd = Fraction(float(x)), Fraction(float(d))
+    r = Fraction(float(_round32(1 / fd)))
+    q = Fraction(float(_round32(fx * r)))
+    for _ in range(2):
+        e = Fraction(float(_round32(fx - q * fd)))
+        q = Fraction(float(_round32(q + e * r)))
+    return np.float32(float(q))
+
+
+@pytest.mark.parametrize("scale", [0, 20, -25])
+def test_float_quotient_is_correctly_rounded(scale):
+    rng = random.Random(scale)
+    last = np.float32(2.0 ** -23)
+    ms = [np.float32(1.0 + rng.getrandbits(23) * 2.0 ** -23) for _ in range(60)]
+    ms += [np.float32(1.0) + k * last for k in range(4)] + [np.float32(2.0) - k * last for k in range(1, 5)]
+    for d in ms:
+        for x in rng.sample(ms, 24):
+            for sx in (x, -x * np.float32(2.0 ** scale)):
+                assert _div_by_f(sx, d) == _round32(Fraction(float(sx)) / Fraction(float(d)))
+
+
 def test_division_by_multiplication():
     """FastDiv (csrc/vxb_kernels.cuh) restated: n * m >> (27 + L) is n // d for
     every n below 2^27, with m << 4 in 32 bits."""
