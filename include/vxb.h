@@ -90,10 +90,12 @@ vxb_status vxb_create(vxb_voxelizer** out, int node_type, const float* vertices,
 /* ~Voxelizer(): frees the instance.  Its device buffers go to a
  * process-wide cache of idle blocks (at most 16 GiB) that later instances
  * draw from, so that creating one voxelizer per mesh does not pay cudaMalloc
- * / cudaFree every time.  (Calls return with their work complete; after a
- * failed call this waits for the device first.) */
+ * / cudaFree every time; its streams go to a list of at most 64 idle ones.
+ * (Calls return with their work complete; after a failed call this waits for
+ * the device first.) */
 vxb_status vxb_destroy(vxb_voxelizer* v);
-/* No reference counterpart: returns every idle cached block to the driver. */
+/* No reference counterpart: returns every idle cached block and stream to the
+ * driver. */
 vxb_status vxb_trim_cache(void);
 
 /* setMaterials(materials, nrOfUniqueMaterials), include/voxelizer.h:862,

@@ -45,10 +45,7 @@ struct vxb_voxelizer {
     bool meshOnDevice = false, matsOnDevice = false;
     bool hasMaterials = false;   // setMaterials was called (materials live on the host or the device)
     vxb::DevBuf dV, dI, dM, outStage, dCheck;
-    cudaStream_t copyStream = nullptr;   // device-to-host copies of streamed output
-    ~vxb_voxelizer() {
-        if (copyStream) cudaStreamDestroy(copyStream);
-    }
+    vxb::PoolStream copyStream;   // device-to-host copies of streamed output
     // Slices along x: the rotated mesh (made on the first such call) and the
     // rotated slice's node array before the boundary ids.
     vxb::DevBuf dVrot, xStage, xFlag;
@@ -466,7 +463,7 @@ struct vxb_batch {
     std::vector<Entry> entries;
     bool prepared = false;       // pipeline tables match `entries`
     vxb::Pipeline pipe;
-    cudaStream_t own = nullptr;  // capture stream when the caller passes the legacy default stream
+    vxb::PoolStream own;         // capture stream when the caller passes the legacy default stream
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t graphStream = nullptr;
@@ -480,10 +477,7 @@ struct vxb_batch {
         graph = nullptr;
         graphKernels = 0;
     }
-    ~vxb_batch() {
-        dropGraph();
-        if (own) cudaStreamDestroy(own);
-    }
+    ~vxb_batch() { dropGraph(); }
 };
 
 // ---------------------------------------------------------------------------
@@ -829,13 +823,13 @@ vxb_status vxb_voxelize_to_host(vxb_voxelizer* v, int nodes, const vxb_request* 
     cudaPointerAttributes pa;
     const bool pinned = cudaPointerGetAttributes(&pa, host_out) == cudaSuccess && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();
-    if (pinned && !v->copyStream) VXB_CUDA(cudaStreamCreateWithFlags(&v->copyStream, cudaStreamNonBlocking));
-    v->pipe.streamOutput(pinned && nodes ? host_out : nullptr, gi.bytes, v->copyStream);
+    if (pinned && (rc = v->copyStream.ensure(false))) return rc;
+    v->pipe.streamOutput(pinned && nodes ? host_out : nullptr, gi.bytes, v->copyStream.s);
     rc = v->run(nodes, req, v->outStage.p, gi.bytes, 0, info);
     const bool copied = v->pipe.hostCopied();
     v->pipe.streamOutput(nullptr, 0, nullptr);
     if (copied) {
-        cudaError_t e = cudaStreamSynchronize(v->copyStream);
+        cudaError_t e = cudaStreamSynchronize(v->copyStream.s);
         if (rc == 0 && e != cudaSuccess) rc = failf(VXB_ECUDA, "%s", cudaGetErrorString(e));
     } else if (rc == 0) {
         cudaError_t e = cudaMemcpy(host_out, v->outStage.p, gi.bytes, cudaMemcpyDeviceToHost);
@@ -958,9 +952,9 @@ vxb_status vxb_batch_run(vxb_batch* b, void* stream, int flags) {
     if (useGraph && s == nullptr) {
         // The legacy default stream cannot be captured: run on the batch's
         // own stream, ordered after the caller's default-stream work.
-        if (!b->own) VXB_CUDA(cudaStreamCreateWithFlags(&b->own, cudaStreamNonBlocking));
+        if (int orc = b->own.ensure(false)) return orc;
         VXB_CUDA(cudaStreamSynchronize(nullptr));
-        s = b->own;
+        s = b->own.s;
     }
     int rc;
     b->busy = true;

@@ -1,4 +1,5 @@
-// Error reporting and the process-wide device block cache.
+// Error reporting and the process-wide lists of idle device blocks and
+// streams.
 
 #include "vxb.h"
 #include "vxb_host.h"
@@ -8,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <vector>
 
 namespace vxb {
 
@@ -29,6 +31,24 @@ struct BlockCache {
 
 BlockCache& blockCache() {
     static BlockCache* c = new BlockCache;   // never destroyed: blocks outlive static destructors
+    return *c;
+}
+
+// Idle streams with their device and priority.  A stream that is given back
+// past the limit is destroyed; vxb_trim_cache destroys them all.
+struct StreamCache {
+    struct Idle {
+        cudaStream_t s;
+        int dev;
+        bool high;
+    };
+    std::mutex mu;
+    std::vector<Idle> idle;
+    static constexpr size_t kStreams = 64;
+};
+
+StreamCache& streamCache() {
+    static StreamCache* c = new StreamCache;
     return *c;
 }
 
@@ -97,6 +117,46 @@ int DevBuf::ensure(size_t bytes) {
     return 0;
 }
 
+PoolStream::~PoolStream() {
+    if (!s) return;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+        cudaStreamQuery(s) == cudaSuccess) {
+        StreamCache& c = streamCache();
+        std::lock_guard<std::mutex> lock(c.mu);
+        if (c.idle.size() < StreamCache::kStreams) {
+            c.idle.push_back(StreamCache::Idle{s, dev, high});
+            return;
+        }
+    }
+    cudaGetLastError();
+    cudaStreamDestroy(s);
+}
+
+int PoolStream::ensure(bool greatestPriority) {
+    if (s) return 0;
+    VXB_CUDA(cudaGetDevice(&dev));
+    high = greatestPriority;
+    {
+        StreamCache& c = streamCache();
+        std::lock_guard<std::mutex> lock(c.mu);
+        for (size_t i = c.idle.size(); i-- > 0;) {
+            if (c.idle[i].dev != dev || c.idle[i].high != high) continue;
+            s = c.idle[i].s;
+            c.idle[i] = c.idle.back();
+            c.idle.pop_back();
+            return 0;
+        }
+    }
+    int least = 0, greatest = 0;
+    if (high) VXB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    const cudaError_t e = high ? cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest)
+                               : cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) s = nullptr;
+    VXB_CUDA(e);
+    return 0;
+}
+
 }  // namespace vxb
 
 extern "C" {
@@ -116,6 +176,16 @@ vxb_status vxb_trim_cache(void) {
     for (auto& e : idle) {
         cudaSetDevice(e.second.first);
         cudaFree(e.second.second);
+    }
+    vxb::StreamCache& sc = vxb::streamCache();
+    std::vector<vxb::StreamCache::Idle> streams;
+    {
+        std::lock_guard<std::mutex> lock(sc.mu);
+        streams.swap(sc.idle);
+    }
+    for (auto& e : streams) {
+        cudaSetDevice(e.dev);
+        cudaStreamDestroy(e.s);
     }
     cudaSetDevice(cur);
     return VXB_OK;

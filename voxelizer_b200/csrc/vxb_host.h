@@ -1,5 +1,6 @@
 // Host-side support shared by the engine files: error reporting for
-// vxb_last_error, and device buffers backed by a process-wide block cache.
+// vxb_last_error, and device buffers and streams backed by process-wide lists
+// of idle ones.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -51,6 +52,22 @@ struct DevBuf {
     // before it queues any.
     int ensure(size_t bytes);
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
+};
+
+// A non-blocking stream of the current device from a process-wide list of
+// idle ones: making and destroying a stream takes 105 us, and a voxelizer per
+// mesh needs two.  `high`: of the greatest priority.
+struct PoolStream {
+    cudaStream_t s = nullptr;
+    int dev = 0;
+    bool high = false;
+    PoolStream() = default;
+    PoolStream(const PoolStream&) = delete;
+    PoolStream& operator=(const PoolStream&) = delete;
+    // Gives the stream back if its work is complete and it is in no capture
+    // (it is destroyed otherwise).
+    ~PoolStream();
+    int ensure(bool greatestPriority);
 };
 
 }  // namespace vxb

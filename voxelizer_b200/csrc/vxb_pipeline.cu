@@ -286,14 +286,11 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     mergeEntries_ = 0;
     keysCap_ = 0;
     if (anyMaterials_) {
-        if (!side_) {
+        if (!evHiDone_) {
             // Pruning and emission (on the way to the result) run on a stream
             // of the greatest priority, so that their blocks are placed
             // before the merge's when both wait for room on the SMs.
-            int least = 0, greatest = 0;
-            VXB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-            VXB_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
-            VXB_CUDA(cudaStreamCreateWithPriority(&hi_, cudaStreamNonBlocking, greatest));
+            if ((rc = side_.ensure(false)) || (rc = hi_.ensure(true))) return rc;
             VXB_CUDA(cudaEventCreateWithFlags(&evFork_, cudaEventDisableTiming));
             VXB_CUDA(cudaEventCreateWithFlags(&evSurfBits_, cudaEventDisableTiming));
             VXB_CUDA(cudaEventCreateWithFlags(&evSurfDone_, cudaEventDisableTiming));
@@ -361,7 +358,7 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     const bool retraverse = wide_ || shape.surfMerge != 0;
     auto surfaceBits = [&]() -> int {
         if (!serial) {
-            ss = side_;
+            ss = side_.s;
             VXB_CUDA(cudaEventRecord(evFork_, s));
             VXB_CUDA(cudaStreamWaitEvent(ss, evFork_, 0));
         }
@@ -432,8 +429,8 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     // event pairs (5 us of a 100 us call).
     if (anyMaterials_ && !serial && totalWords_ >= kPriorityWords) {
         VXB_CUDA(cudaEventRecord(evSolid_, s));
-        VXB_CUDA(cudaStreamWaitEvent(hi_, evSolid_, 0));
-        ps = hi_;
+        VXB_CUDA(cudaStreamWaitEvent(hi_.s, evSolid_, 0));
+        ps = hi_.s;
     }
     // Split-ordered pruning (src/host_side.cpp:1183-1206).
     if (anyCartesian_ && !raw_) {
@@ -543,8 +540,6 @@ int Pipeline::pruneUntilStable(cudaStream_t s) {
 Pipeline::~Pipeline() {
     for (cudaEvent_t e : {evFork_, evSurfBits_, evSurfDone_, evSolid_, evHiDone_})
         if (e) cudaEventDestroy(e);
-    if (side_) cudaStreamDestroy(side_);
-    if (hi_) cudaStreamDestroy(hi_);
     for (cudaEvent_t& e : tuneEv_)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t& e : outEv_)

@@ -141,7 +141,7 @@ private:
     DevBuf recs, depth, sOffsets, triOf, hitList, keys, values;
     // The surface pass runs on a second stream beside the solid pass, joined
     // before pruning (surface bits) and before emission (merged keys).
-    cudaStream_t side_ = nullptr, hi_ = nullptr;
+    PoolStream side_, hi_;
     cudaEvent_t evFork_ = nullptr, evSurfBits_ = nullptr, evSurfDone_ = nullptr, evSolid_ = nullptr,
                 evHiDone_ = nullptr;
 };
