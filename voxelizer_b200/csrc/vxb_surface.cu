@@ -443,6 +443,16 @@ __device__ __forceinline__ float vbComp(int c, float m, float d) {
     return linf<1>(__fsub_rn((float)c, 0.5f), d, m);
 }
 
+// Two values per operation, each rounded as by itself: two columns of a row, or
+// the two projections of a voxel of the depth range.  It halves the edge
+// functions' instructions; the stress FCC mesh, whose rows are long, takes 71
+// instead of 76 us (a call 173 -> 171), the room 447 instead of 450.
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 vbComp2(int c, float m, float d) {
+    const float2 x = __fadd2_rn(make_float2((float)c, (float)(c + 1)), both(-0.5f));
+    return __ffma2_rn(x, both(d), both(m));
+}
+
 // determineDepthRange{X,Y,Z} (src/voxelizer.cu:3994-4119) with
 // intersectWithPlane* and boundsCheck, in (inner, outer, depth) coordinates:
 // p the column's corner, t0 the first vertex, n the normal.
@@ -560,11 +570,12 @@ struct SurfWarp {
 // lanes idled through the rest.  Alone on a B200, a column per lane with hits
 // recorded inside the depth loop / marked first / by rows: room (22.3 M
 // columns, 19.2 M hits) 582 / 527 / 450 us, stress FCC mesh (slivers) 193 /
-// 163 / 73 us, duct 120 / 103 / 95 us.  A list of 5,120 triangles takes 18-22
-// instead of 14 us.  The stage must hold several steps' hits: with 128 or 64
-// entries instead of 256 the waits for the list's counter make it 676 and
-// 967 us; prefetching the next chunk's records and larger batches gave
-// nothing (508-540 us with 8 chunks a batch).
+// 163 / 76 us, duct 120 / 103 / 95 us; with two columns per operation 447, 71
+// and 93 us.  A list of 5,120 triangles takes 18 instead of 14 us.  The stage
+// must hold several steps' hits: with 128 or 64 entries instead of 256 the
+// waits for the list's counter make it 676 and 967 us; prefetching the next
+// chunk's records and larger batches gave nothing (508-540 us with 8 chunks a
+// batch).
 template <int K, int MODE>
 __global__ void __launch_bounds__(kWorkThreads, 8) surfaceWorkKernel(Sink sink, Batch b, const SurfRec* __restrict__ recs,
                                                                const SurfDepth* __restrict__ depth,
@@ -687,12 +698,16 @@ __global__ void __launch_bounds__(kWorkThreads, 8) surfaceWorkKernel(Sink sink, 
                         float k[3];
 #pragma unroll
                         for (int i = 0; i < 3; ++i) k[i] = __fmul_rn(cu[i], po);
-                        for (uint32_t c2 = 0; c2 < cols; ++c2) {
-                            const float pi = vbComp(inner + (int)c2, mI, d);
-                            bool hit = true;
+                        for (uint32_t c2 = 0; c2 < cols; c2 += 2u) {
+                            const float2 pi = vbComp2(inner + (int)c2, mI, d);
+                            bool h0 = true, h1 = true;
 #pragma unroll
-                            for (int i = 0; i < 3; ++i) hit &= __fadd_rn(__fmaf_rn(cf[i], pi, k[i]), de[i]) >= 0.0f;
-                            pass |= hit ? 1u << c2 : 0u;
+                            for (int i = 0; i < 3; ++i) {
+                                const float2 e = __fadd2_rn(__ffma2_rn(both(cf[i]), pi, both(k[i])), both(de[i]));
+                                h0 &= e.x >= 0.0f;
+                                h1 &= e.y >= 0.0f;
+                            }
+                            pass |= ((h0 ? 1u : 0u) | (h1 ? 2u : 0u)) << c2;
                         }
                     } else {
                         float pf = po;
@@ -713,15 +728,20 @@ __global__ void __launch_bounds__(kWorkThreads, 8) surfaceWorkKernel(Sink sink, 
                                 }
                             }
                         }
-                        for (uint32_t c2 = 0; c2 < cols; ++c2) {
-                            const float pi = vbComp(inner + (int)c2, mI, d);
-                            bool hit = true;
+                        for (uint32_t c2 = 0; c2 < cols; c2 += 2u) {
+                            const float2 pi = vbComp2(inner + (int)c2, mI, d);
+                            bool h0 = true, h1 = true;
 #pragma unroll
-                            for (int i = 0; i < 3; ++i)
-                                hit &= __fadd_rn(__fmaf_rn(cf[i], pf, __fmul_rn(cu[i], pi)), de[i]) >= 0.0f;
-                            pass |= hit ? 1u << c2 : 0u;
+                            for (int i = 0; i < 3; ++i) {
+                                const float2 e = __fadd2_rn(
+                                    __ffma2_rn(both(cf[i]), both(pf), __fmul2_rn(both(cu[i]), pi)), both(de[i]));
+                                h0 &= e.x >= 0.0f;
+                                h1 &= e.y >= 0.0f;
+                            }
+                            pass |= ((h0 ? 1u : 0u) | (h1 ? 2u : 0u)) << c2;
                         }
                     }
+                    pass &= kFull >> (32u - cols);
                 }
                 const uint32_t slot = half * 32u + lane;
                 sw.a[slot] = make_int4(inner, outer, (int)pos, (int)code);
@@ -805,8 +825,12 @@ __global__ void __launch_bounds__(kWorkThreads, 8) surfaceWorkKernel(Sink sink, 
                     bool hit = true;
 #pragma unroll
                     for (int i = 0; i < 3; ++i) {
-                        hit &= __fadd_rn(__fmaf_rn(e[3 + i], pd, k1[i]), e[6 + i]) >= 0.0f;
-                        hit &= __fadd_rn(__fmaf_rn(e[12 + i], pd, k2[i]), e[15 + i]) >= 0.0f;
+                        // Both projections at once.
+                        const float2 q = __fadd2_rn(__ffma2_rn(make_float2(e[3 + i], e[12 + i]), both(pd),
+                                                               make_float2(k1[i], k2[i])),
+                                                    make_float2(e[6 + i], e[15 + i]));
+                        hit &= q.x >= 0.0f;
+                        hit &= q.y >= 0.0f;
                     }
                     m |= hit ? 1u << v : 0u;
                 }
