@@ -762,13 +762,12 @@ def main():
 
     # Algorithmic bytes per launch of the two heaviest kernels.
     #  emit: the node grid written once, the pruned and surface bit grids read once.
-    #  surface work: every partitioned triangle's record (64 B) and the edge
-    #  functions its class tests (36 B for 2D boxes, 108 B for 3D boxes), and
-    #  per hit an 8-byte hit-list entry and a 4-byte surface-word update
-    #  (read and write).
+    #  surface work: every listed triangle's record (80 B), for 3D boxes the
+    #  depth record (112 B), and per hit an 8-byte hit-list entry and a 4-byte
+    #  surface-word update (read and write).
     emit_bytes = n_nodes * 2 + 2 * n_nodes / 8
     st_tris = stats["surface_triangles"]
-    surf_bytes = 64 * sum(st_tris) + 36 * st_tris[1] + 108 * st_tris[2] + 16 * stats["surface_hits"]
+    surf_bytes = 80 * sum(st_tris) + 112 * st_tris[2] + 16 * stats["surface_hits"]
     kernels = [("emitNarrowKernel<LongNode>", emit_bytes, median("emit"), "emit_cartesian_long_room1024_bytes"),
                ("surfaceWorkKernel", surf_bytes, median("surface_work"), "surface_work_room1024_bytes")]
     roofs = []

@@ -211,7 +211,7 @@ typedef struct {
     uint32_t units;                 /* meshes x lattices */
     uint32_t work_triangles;        /* triangles x lattices */
     uint32_t solid_candidates;      /* (triangle, subspace, 4x4 tile) candidates of the solid pass */
-    uint32_t surface_columns;       /* work items of the surface pass */
+    uint32_t surface_columns;       /* columns of the surface pass */
     uint32_t surface_hits;          /* surface voxel hits (with repeats); 0 when no hit list was kept */
     uint32_t surface_voxels;        /* distinct surface voxels */
     uint32_t surface_triangles[3];  /* triangles with surface work by class: 1D, 2D, 3D boxes */
@@ -293,12 +293,10 @@ vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const uint32_t* 
 vxb_status vxb_noalloc_status(void);
 
 /* No counterpart in the reference (the reference sums its tile counts on the
- * host).  The exclusive scan that sizes every work list, exported so that
- * its overflow detection can be tested without a work list of 2^32
- * entries: scans n device counts into offsets (n + 1 device entries) on
- * `stream`, waits, and writes the 32-bit total and the overflow flag (1 when
- * the sum is 2^32 - 1 or more, and the offsets are then not valid).
- * Allocates its tile sums. */
+ * host).  An exclusive scan of work counts with overflow detection: scans n
+ * device counts into offsets (n + 1 device entries) on `stream`, waits, and
+ * writes the 32-bit total and the overflow flag (1 when the sum is 2^32 - 1 or
+ * more, and the offsets are then not valid).  Allocates its tile sums. */
 vxb_status vxb_scan_counts(const uint32_t* counts, uint32_t n, uint32_t* offsets, uint32_t* total,
                            uint32_t* overflow, void* stream);
 

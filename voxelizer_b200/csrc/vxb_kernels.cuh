@@ -92,7 +92,8 @@ struct Batch {
     const uint8_t* later;
 };
 
-// Work-list scan: exclusive offsets (n + 1 entries) and the grand total.
+// Exclusive offsets (n + 1 entries) and the grand total of n counts
+// (vxb_scan_counts).
 void launch_scan(const uint32_t* in, uint32_t* offsets, uint32_t n, uint32_t* blockSums, uint32_t* total,
                  uint32_t* overflow, cudaStream_t s, uint32_t* launches);
 
@@ -124,19 +125,20 @@ constexpr size_t kSurfDepthBytes = 112;
 
 // Classification and set-up of the work triangles of units with materials:
 // records, first work unit per position (offsets), mesh triangle per position
-// (triOf, may be NULL).  *cursor, *total (the exact number of work units) and
+// (triOf, may be NULL).  *cursor, *total (the exact number of columns) and
 // classes[0..3) (triangles per class) are zero on entry.
 void launch_surface_prepare(const Batch& b, uint32_t nWork, unsigned long long* cursor, unsigned long long* total,
                             uint32_t* classes, uint32_t* offsets, uint32_t* triOf, void* recs, void* depth,
                             cudaStream_t s, uint32_t* launches);
-// Surface work over what launch_surface_prepare wrote, one thread per column.
+// Surface work over what launch_surface_prepare wrote, a lane per row of up to
+// 32 columns and then a lane per column that passes.
 // mode 0: set bits in the `surf` arena and append (bit position << 24 | key)
 // to `list` (entries past listCap are counted, not stored); mode 1: merge
 // every hit's key at its rank (needs complete bits and their `ranks`) and, for
 // PartialNodes (64-bit keys), store its arena position in `positions`; mode 2:
 // set bits only.  kind: the node type, whose instantiation of the class
-// kernels the arithmetic follows.  batch: 32-item chunks a warp takes at a
-// time.  queue: as for launch_solid_toggle.  Nothing is done when *total is
+// kernels the arithmetic follows.  batch: chunks of 32 columns a warp takes at
+// a time (four make a chunk of 32 rows).  queue: as for launch_solid_toggle.  Nothing is done when *total is
 // 2^32 - 1 or more.
 void launch_surface_work(int kind, int mode, const Batch& b, const void* recs, const void* depth, const uint32_t* triOf,
                          const uint32_t* offsets, const unsigned long long* cursor, const unsigned long long* total,

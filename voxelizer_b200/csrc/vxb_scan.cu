@@ -1,4 +1,4 @@
-// Work-list scan kernels.
+// Exclusive scan of counts (vxb_scan_counts).
 #include "vxb_common.cuh"
 #include "vxb_device.cuh"
 #include "vxb_kernels.cuh"

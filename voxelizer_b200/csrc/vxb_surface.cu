@@ -6,10 +6,10 @@
 // to the grid, work units), gives the triangles with work consecutive
 // positions, ordered by class and axis inside a block, and writes one set-up
 // record per position together with the prefix of its work units.  The work
-// list runs over that prefix: one thread per column of the dominant projection
-// (per voxel of a 1D line).  Warps find the triangle of each of their 32 items
-// with one coalesced load of 32 offsets, so the work kernel has no block-wide
-// barrier.
+// list runs over that prefix: rows of up to 32 columns of the dominant
+// projection (a 1D line is one row).  Warps find the triangle of each of their
+// 32 rows with one coalesced load of 32 offsets, so the work kernel has no
+// block-wide barrier.
 //
 // The reference runs the surface kernels once per material subspace on
 // boxes clamped to it.  Subspaces tile the grid, so the columns of the

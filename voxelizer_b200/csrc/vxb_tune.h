@@ -15,14 +15,14 @@
 namespace vxb {
 
 struct LaunchShape {
-    uint32_t surfBlocksPerSm = 16;   // surfaceWorkKernel blocks per SM
-    uint32_t surfBatch = 8;          // surfaceWorkKernel 32-item chunks per owner search
+    uint32_t surfBlocksPerSm = 16;   // surfaceWorkKernel blocks of 256 threads (two of its own) per SM
+    uint32_t surfBatch = 8;          // surfaceWorkKernel chunks of 32 columns per owner search (4: one of 32 rows)
     // mergeKeysKernel (timed from the surface-bits join to the keys join);
     // 0: one block per 1,024 expected list entries instead of a persistent
     // grid (its blocks retire as they finish, so pruning's blocks get room).
     uint32_t mergeBlocksPerSm = 0;
-    uint32_t emitBlocksPerSm = 16;   // emitNarrowKernel
-    uint32_t toggleBlocksPerSm = 3;  // solidToggleKernel
+    uint32_t emitBlocksPerSm = 16;   // emitNarrowKernel: half the blocks per SM that share the grid's planes
+    uint32_t toggleBlocksPerSm = 3;  // solidToggleKernel: groups of 8 blocks per SM at the most
     // Work distribution of surfaceWorkKernel / solidToggleKernel: 0 a fixed
     // grid-stride order, 1 a device work queue (persistent warps / blocks
     // take the next batch of items with one atomic each).
