@@ -396,6 +396,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) surfacePrepareKernel(Batch b,
         }
         __syncthreads();
         const uint32_t n = cnt[kSurfaceBuckets * kW];
+        if (n == 0) continue;   // as for most sets of a slice (a call on 1 M triangles 138 -> 133 us)
         uint32_t at = 0;
         if (u) {
             at = cnt[bucket * kW + warp] + __popc(peers & laneMaskLt());
