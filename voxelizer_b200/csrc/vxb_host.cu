@@ -9,7 +9,6 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <vector>
 
 namespace vxb {
 
@@ -43,8 +42,9 @@ struct StreamCache {
         bool high;
     };
     std::mutex mu;
-    std::vector<Idle> idle;
     static constexpr size_t kStreams = 64;
+    Idle idle[kStreams];
+    size_t n = 0;
 };
 
 StreamCache& streamCache() {
@@ -124,8 +124,8 @@ PoolStream::~PoolStream() {
         cudaStreamQuery(s) == cudaSuccess) {
         StreamCache& c = streamCache();
         std::lock_guard<std::mutex> lock(c.mu);
-        if (c.idle.size() < StreamCache::kStreams) {
-            c.idle.push_back(StreamCache::Idle{s, dev, high});
+        if (c.n < StreamCache::kStreams) {
+            c.idle[c.n++] = StreamCache::Idle{s, dev, high};
             return;
         }
     }
@@ -140,11 +140,10 @@ int PoolStream::ensure(bool greatestPriority) {
     {
         StreamCache& c = streamCache();
         std::lock_guard<std::mutex> lock(c.mu);
-        for (size_t i = c.idle.size(); i-- > 0;) {
+        for (size_t i = c.n; i-- > 0;) {
             if (c.idle[i].dev != dev || c.idle[i].high != high) continue;
             s = c.idle[i].s;
-            c.idle[i] = c.idle.back();
-            c.idle.pop_back();
+            c.idle[i] = c.idle[--c.n];
             return 0;
         }
     }
@@ -178,14 +177,16 @@ vxb_status vxb_trim_cache(void) {
         cudaFree(e.second.second);
     }
     vxb::StreamCache& sc = vxb::streamCache();
-    std::vector<vxb::StreamCache::Idle> streams;
+    vxb::StreamCache::Idle streams[vxb::StreamCache::kStreams];
+    size_t n = 0;
     {
         std::lock_guard<std::mutex> lock(sc.mu);
-        streams.swap(sc.idle);
+        for (; n < sc.n; ++n) streams[n] = sc.idle[n];
+        sc.n = 0;
     }
-    for (auto& e : streams) {
-        cudaSetDevice(e.dev);
-        cudaStreamDestroy(e.s);
+    for (size_t i = 0; i < n; ++i) {
+        cudaSetDevice(streams[i].dev);
+        cudaStreamDestroy(streams[i].s);
     }
     cudaSetDevice(cur);
     return VXB_OK;
