@@ -453,6 +453,10 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch 
             uint32_t at = 0;
             if (lane == 0) at = atomicAdd(bigCount, more);
             at = __shfl_sync(kFull, at, 0);
+            // The batches that reserved 2^26 entries have 2^32 candidates: the
+            // host refuses the call, and the rest would be in vain.
+            static_assert((unsigned long long)kChunk << 26 == 1ull << 32, "candidates of 2^26 chunks");
+            if (at >= 1u << 26) break;
             // A list without room for all of them leaves the batch to this
             // warp; the entries it reserved are marked as empty.
             const bool fits = at < bigCap && more <= bigCap - at;
