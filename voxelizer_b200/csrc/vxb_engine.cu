@@ -587,6 +587,7 @@ vxb_status vxb_destroy(vxb_voxelizer* v) {
     int cur = 0;
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
+    const vxb::CaptureRelaxed relaxed;
     if (v->busy) cudaDeviceSynchronize();
     delete v;
     if (cur != dev) cudaSetDevice(cur);
@@ -906,6 +907,7 @@ vxb_status vxb_batch_destroy(vxb_batch* b) {
     int cur = 0;
     cudaGetDevice(&cur);
     if (cur != dev) cudaSetDevice(dev);
+    const vxb::CaptureRelaxed relaxed;
     if (b->busy) cudaDeviceSynchronize();
     delete b;
     if (cur != dev) cudaSetDevice(cur);

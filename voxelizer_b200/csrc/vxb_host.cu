@@ -119,8 +119,9 @@ int DevBuf::ensure(size_t bytes) {
 
 PoolStream::~PoolStream() {
     if (!s) return;
+    const CaptureRelaxed relaxed;   // for the query
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+    if (relaxed.ok && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
         cudaStreamQuery(s) == cudaSuccess) {
         StreamCache& c = streamCache();
         std::lock_guard<std::mutex> lock(c.mu);

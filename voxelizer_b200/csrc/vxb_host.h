@@ -54,6 +54,21 @@ struct DevBuf {
     template <class T> T* as() const { return reinterpret_cast<T*>(p); }
 };
 
+// While it lives, this thread may make the calls that a graph capture in any
+// thread forbids although they have no part in it (stream queries, cudaFree,
+// cudaGraphExecDestroy) without invalidating that capture: an instance may be
+// destroyed at any time, as by garbage collection in the middle of one.
+struct CaptureRelaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool ok = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    CaptureRelaxed() = default;
+    CaptureRelaxed(const CaptureRelaxed&) = delete;
+    CaptureRelaxed& operator=(const CaptureRelaxed&) = delete;
+    ~CaptureRelaxed() {
+        if (ok) cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+};
+
 // A non-blocking stream of the current device from a process-wide list of
 // idle ones: making and destroying a stream takes 105 us, and a voxelizer per
 // mesh needs two.  `high`: of the greatest priority.
