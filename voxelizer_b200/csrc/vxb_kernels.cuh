@@ -218,14 +218,20 @@ void launch_fcc_boundaries(void* nodes, uint32_t X, uint32_t Y, uint32_t Z, uint
 void launch_partial_values(const Batch& b, const void* keys, const uint32_t* count, uint32_t cap,
                            unsigned long long* values, cudaStream_t s, uint32_t* launches);
 // Keys (PartialNodes: values) at ranks >= keysCap read as 0.
-// Planes [zBegin, zEnd) of every unit.  spanBase: exclusive prefix over the
-// units of emit_spans (nUnits + 1 entries), `spans` their sum.
-uint32_t emit_spans(const PassGeom& g);
-void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* spanBase, uint32_t spans,
-                           uint32_t zBegin, uint32_t zEnd, const uint32_t* finalSolid, const uint32_t* fill,
-                           const uint32_t* surf, const WordRank* ranks, const void* keys, uint32_t keysCap,
-                           const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s,
-                           uint32_t* launches);
+// Planes [zBegin, zEnd) of every unit.  1- and 2-byte nodes: a task is a span of
+// a plane's words (emit_tasks in a plane; packed: of one warp, else of a block)
+// over `planes` planes, at most 64; emit_planes gives that number from the tasks
+// of all single planes of all units, emit_packed the kind of task from those of
+// both kinds.  `tasks` is the number of tasks and taskBase their exclusive prefix
+// over the units (nUnits + 1 entries; NULL for one unit).
+constexpr uint32_t kEmitLevels = 7;   // planes 1, 2, .. 64
+uint32_t emit_tasks(const PassGeom& g, bool packed);
+bool emit_packed(uint64_t chunkPlanes, uint64_t blockPlanes);
+uint32_t emit_planes(uint64_t taskPlanes, bool packed, uint32_t blocksPerSm);
+void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* taskBase, uint32_t tasks,
+                           bool packed, uint32_t planes, uint32_t zBegin, uint32_t zEnd, const uint32_t* finalSolid,
+                           const uint32_t* fill, const uint32_t* surf, const WordRank* ranks, const void* keys,
+                           uint32_t keysCap, const unsigned long long* values, cudaStream_t s, uint32_t* launches);
 
 // An FCC mesh: its four sub-lattice units are units [unit0, unit0 + 4).
 struct FccMesh {

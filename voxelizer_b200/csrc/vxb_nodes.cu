@@ -549,10 +549,25 @@ __device__ __forceinline__ void emitWords(const EmitArgs& args, const EmitSlots&
     __syncwarp();
 }
 
-template <int K>
-__global__ void __launch_bounds__(kEmitWarps * 32, 4) emitNarrowKernel(EmitArgs a, const uint32_t* __restrict__ spanBase,
-                                                                       uint32_t planes, uint32_t zBegin,
-                                                                       uint32_t zEnd) {
+// A task covers a chunk of 32 words (kPacked, one warp) or kEmitWarps of them
+// (one block) over `planes` planes.  Tasks are numbered through: along a plane,
+// groups of planes, units (taskBase), so that no block of a batch is without
+// work whatever its units' shapes.  Where planes are so thin that the warps of a
+// block would idle (emit_packed), tasks are warps': 60,000 planes of 7 words
+// 29 us, 189 with a block a plane; 2,000 meshes of 16-24 voxels 590 us a batch
+// instead of 698.  One unit of wide planes (kUnit) has its groups of planes
+// along the grid's y, which keeps z out of the vector registers: 1-3% of a call
+// (room, duct) against a division of the block's number.  They are fewer than
+// the 65,535 blocks that y takes: emit_planes leaves at most twice as many tasks
+// as blocks share the grid (2 * 148 * 2 * 32 with the widest launch shape), or
+// groups of 64 planes, and 65,535 of those with planes this wide (more than five
+// chunks) are more words than a grid may have.
+enum EmitTasks { kUnit, kBlocks, kPacked };
+
+template <int K, EmitTasks T>
+__global__ void __launch_bounds__(kEmitWarps * 32, 4) emitNarrowKernel(EmitArgs a, const uint32_t* __restrict__ taskBase,
+                                                                       uint32_t tasks, uint32_t planes,
+                                                                       uint32_t zBegin, uint32_t zEnd) {
     typedef NodeT<K> NT;
     static_assert(NT::bytes <= 2, "narrow nodes only");
     constexpr uint32_t NB = NT::bytes;
@@ -561,11 +576,21 @@ __global__ void __launch_bounds__(kEmitWarps * 32, 4) emitNarrowKernel(EmitArgs 
     __shared__ __align__(16) uint32_t stageAll[kEmitWarps][32 * (8 * NB + 4)];
     __shared__ EmitSlots slotsAll[kEmitWarps];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t u = a.b.nUnits > 1 ? unitOf(spanBase, a.b.nUnits, blockIdx.x) : 0u;
+    const uint32_t task = T == kPacked ? blockIdx.x * kEmitWarps + warp : blockIdx.x;
+    if (task >= tasks) return;   // whole warp
+    const uint32_t u = T != kUnit && taskBase ? unitOf(taskBase, a.b.nUnits, task) : 0u;
     const Unit& U = a.b.units[u];
     const uint32_t ipx = U.g.ipx, AY = U.g.AY, AZ = U.g.AZ, plane = ipx * AY;
-    const uint32_t z0 = zBegin + blockIdx.y * planes, z1 = min(z0 + planes, min(AZ, zEnd));
-    const uint32_t first = ((blockIdx.x - (a.b.nUnits > 1 ? __ldg(spanBase + u) : 0u)) * kEmitWarps + warp) * 32u;
+    constexpr uint32_t kSpan = T == kPacked ? 32u : 32u * kEmitWarps;
+    uint32_t span = task, group = blockIdx.y;
+    if (T != kUnit) {
+        const uint32_t perPlane = (plane + kSpan - 1u) / kSpan;
+        span -= taskBase ? __ldg(taskBase + u) : 0u;
+        group = span / perPlane;
+        span -= group * perPlane;
+    }
+    const uint32_t z0 = zBegin + group * planes, z1 = min(z0 + planes, min(AZ, zEnd));
+    const uint32_t first = span * kSpan + (T == kPacked ? 0u : warp * 32u);
     if (z0 >= z1 || first >= plane) return;   // whole warp
     EmitSlots& slots = slotsAll[warp];
     uint32_t* const stage = stageAll[warp];
@@ -1010,13 +1035,29 @@ void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, con
     *launches += 1;
 }
 
-uint32_t emit_spans(const PassGeom& g) { return (g.ipx * g.AY + kEmitWarps * 32u - 1) / (kEmitWarps * 32u); }
+uint32_t emit_tasks(const PassGeom& g, bool packed) {
+    const uint32_t span = packed ? 32u : 32u * kEmitWarps;
+    return (g.ipx * g.AY + span - 1) / span;
+}
 
-void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* spanBase, uint32_t spans,
-                           uint32_t zBegin, uint32_t zEnd, const uint32_t* finalSolid, const uint32_t* fill,
-                           const uint32_t* surf, const WordRank* ranks, const void* keys, uint32_t keysCap,
-                           const unsigned long long* values, uint32_t blocksPerSm, cudaStream_t s,
-                           uint32_t* launches) {
+bool emit_packed(uint64_t chunkPlanes, uint64_t blockPlanes) {
+    // At 128^3 (17 chunks a plane, 24 warps: 1.4) both take the same time.
+    return 2 * kEmitWarps * blockPlanes > 3 * chunkPlanes;
+}
+
+uint32_t emit_planes(uint64_t taskPlanes, bool packed, uint32_t blocksPerSm) {
+    // Planes per task: 2 * blocksPerSm blocks per SM share the grid (their work
+    // differs, so more of them balance better), but a warp's set-up pays for 8
+    // planes where 8 blocks per SM remain.
+    const uint64_t blocks = packed ? taskPlanes / kEmitWarps : taskPlanes;
+    const uint64_t share = blocks / (148u * 2u * (uint64_t)blocksPerSm), least = std::min<uint64_t>(8, blocks / (148u * 8u));
+    return (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(1, std::max(share, least)));
+}
+
+void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, const uint32_t* taskBase, uint32_t tasks,
+                           bool packed, uint32_t planes, uint32_t zBegin, uint32_t zEnd, const uint32_t* finalSolid,
+                           const uint32_t* fill, const uint32_t* surf, const WordRank* ranks, const void* keys,
+                           uint32_t keysCap, const unsigned long long* values, cudaStream_t s, uint32_t* launches) {
     EmitArgs a;
     a.keysCap = keysCap;
     a.b = b;
@@ -1029,16 +1070,16 @@ void launch_emit_cartesian(int nodeKind, const Batch& b, uint64_t totalWords, co
     if (nodeKind == kPartial) {
         emitPartialKernel<<<gridFor(totalWords, 256, 148u * 64u), 256, 0, s>>>(a, totalWords, zBegin, zEnd);
     } else {
-        // Planes per warp: 2 * blocksPerSm blocks per SM share the grid (their
-        // work differs, so more of them balance better), but a warp's set-up
-        // pays for 8 planes where 8 blocks per SM remain.
-        const uint64_t chunks = totalWords / (32u * kEmitWarps);
-        const uint64_t share = chunks / (148u * 2u * blocksPerSm), least = std::min<uint64_t>(8, chunks / (148u * 8u));
-        const uint32_t planes = (uint32_t)std::min<uint64_t>(64, std::max<uint64_t>(1, std::max(share, least)));
-        const dim3 grid(spans, (zEnd - zBegin + planes - 1) / planes);
-        if (nodeKind == kShort)
-            emitNarrowKernel<kShort><<<grid, kEmitWarps * 32, 0, s>>>(a, spanBase, planes, zBegin, zEnd);
-        else emitNarrowKernel<kLong><<<grid, kEmitWarps * 32, 0, s>>>(a, spanBase, planes, zBegin, zEnd);
+        dim3 grid(packed ? (tasks + kEmitWarps - 1) / kEmitWarps : tasks);
+        auto kernel = nodeKind == kShort ? emitNarrowKernel<kShort, kBlocks> : emitNarrowKernel<kLong, kBlocks>;
+        if (packed) {
+            kernel = nodeKind == kShort ? emitNarrowKernel<kShort, kPacked> : emitNarrowKernel<kLong, kPacked>;
+        } else if (!taskBase) {
+            const uint32_t groups = (zEnd - zBegin + planes - 1) / planes;
+            grid = dim3(tasks /= groups, groups);
+            kernel = nodeKind == kShort ? emitNarrowKernel<kShort, kUnit> : emitNarrowKernel<kLong, kUnit>;
+        }
+        kernel<<<grid, kEmitWarps * 32, 0, s>>>(a, taskBase, tasks, planes, zBegin, zEnd);
     }
     *launches += 1;
 }

@@ -243,14 +243,28 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
             pruneBase.push_back((uint32_t)blocks);
         }
     pruneBlocks_ = pruneBase.back();
-    // Blocks of a plane and planes of the emission.
-    std::vector<uint32_t> spanBase{0};
+    // Tasks of the emission.  The planes of a task follow from the launch shape
+    // of each run; one unit takes any number, several units a power of two,
+    // whose prefixes over the units are laid out here.
+    std::vector<uint32_t> emitBase;
+    uint64_t taskPlanes[2] = {0, 0};
     maxPlanes_ = 0;
     for (const Unit& u : units_) {
-        spanBase.push_back(spanBase.back() + emit_spans(u.g));
+        for (int k = 0; k < 2; ++k) taskPlanes[k] += (uint64_t)emit_tasks(u.g, k != 0) * u.g.AZ;
         maxPlanes_ = std::max(maxPlanes_, u.g.AZ);
     }
-    emitSpans_ = spanBase.back();
+    emitPacked_ = emit_packed(taskPlanes[1], taskPlanes[0]);
+    taskPlanes_ = taskPlanes[emitPacked_];
+    if (anyCartesian_ && units_.size() > 1)
+        for (uint32_t level = 0; level < kEmitLevels; ++level) {
+            uint64_t tasks = 0;
+            for (const Unit& u : units_) {
+                emitBase.push_back((uint32_t)tasks);
+                tasks += (uint64_t)emit_tasks(u.g, emitPacked_) * ((u.g.AZ + (1u << level) - 1u) >> level);
+            }
+            emitBase.push_back((uint32_t)tasks);
+            emitTasks_[level] = tasks <= 0x7FFFFFFFull ? (uint32_t)tasks : 0u;   // 0: too many for this level
+        }
     // A single plain voxelization writes its solid grid straight into the
     // caller's buffer.
     aliasFill_ = !nodes_ && jobs.size() == 1;
@@ -264,7 +278,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     oSlices_ = append(blob_, slices);
     oLater_ = append(blob_, later);
     oPrune_ = append(blob_, pruneBase);
-    oSpans_ = append(blob_, spanBase);
+    oEmit_ = append(blob_, emitBase);
     oFcc_ = append(blob_, fccMeshes);
     oPairBase_ = append(blob_, pairBase);
     // Buffers.
@@ -515,10 +529,20 @@ void Pipeline::surfaceWork(int mode, cudaStream_t s) {
 }
 
 void Pipeline::emitCartesian(uint32_t zBegin, uint32_t zEnd, cudaStream_t s) {
-    launch_emit_cartesian(nodeKind_, batch(), totalWords_, reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oSpans_),
-                          emitSpans_, zBegin, zEnd, fin.as<uint32_t>(), fill.as<uint32_t>(), surf.as<uint32_t>(),
-                          ranks.as<WordRank>(), keys.p, keysCap_, values.as<unsigned long long>(),
-                          shape.emitBlocksPerSm, s, &launches);
+    uint32_t planes = emit_planes(taskPlanes_, emitPacked_, shape.emitBlocksPerSm), tasks;
+    const uint32_t* base = nullptr;
+    if (units_.size() == 1) {
+        tasks = emit_tasks(units_[0].g, emitPacked_) * ((zEnd - zBegin + planes - 1) / planes);
+    } else {
+        uint32_t level = 0;
+        while (level + 1 < kEmitLevels && ((2u << level) <= planes || !emitTasks_[level])) ++level;
+        planes = 1u << level;
+        tasks = emitTasks_[level];
+        base = reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oEmit_) + level * (units_.size() + 1);
+    }
+    launch_emit_cartesian(nodeKind_, batch(), totalWords_, base, tasks, emitPacked_, planes, zBegin, zEnd,
+                          fin.as<uint32_t>(), fill.as<uint32_t>(), surf.as<uint32_t>(), ranks.as<WordRank>(), keys.p,
+                          keysCap_, values.as<unsigned long long>(), s, &launches);
 }
 
 // Full passes until nothing changes, with a host check after each.
