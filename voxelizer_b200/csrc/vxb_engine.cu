@@ -1002,6 +1002,7 @@ vxb_status vxb_batch_run(vxb_batch* b, void* stream, int flags) {
         rc = b->pipe.finish(s);
         b->launches = b->pipe.launches;
     }
+    if (b->pipe.keysMoved()) b->dropGraph();
     if (rc == 0) {
         b->busy = false;
         for (const vxb_batch::Entry& e : b->entries) e.v->busy = false;

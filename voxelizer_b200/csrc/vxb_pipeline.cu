@@ -599,6 +599,7 @@ void Pipeline::tuneFinish() {
 }
 
 int Pipeline::finish(cudaStream_t s) {
+    keysMoved_ = false;
     if (!nodes_) {
         VXB_CUDA(cudaStreamSynchronize(s));
         tuneFinish();
@@ -633,6 +634,10 @@ int Pipeline::finish(cudaStream_t s) {
             // Merge every hit straight at its rank (second traversal).
             int rc;
             if ((uint64_t)surfaceVoxels + 1 > keysCap_) {
+                // Without room (cap 0) until both buffers are there: a run
+                // after a failed one then stores no keys.
+                keysMoved_ = true;
+                keysCap_ = 0;
                 if ((rc = keys.ensure(((size_t)surfaceVoxels + 1) * (wide_ ? 8 : 4)))) return rc;
                 if (wide_ && (rc = values.ensure(((size_t)surfaceVoxels + 1) * 8))) return rc;
                 keysCap_ = surfaceVoxels + 1;

@@ -76,6 +76,9 @@ public:
     // work: a hit list that overflowed, or a pruning subspace that needed
     // more passes than were queued.
     int finish(cudaStream_t s);
+    // Whether the last finish gave the key buffers another size and place: a
+    // graph captured before holds the old ones.
+    bool keysMoved() const { return keysMoved_; }
     // Kernels launched by the last enqueue + finish.
     uint32_t launches = 0;
     // Node output of a one-mesh Cartesian run copied to pinned host memory
@@ -130,7 +133,7 @@ private:
     uint64_t taskPlanes_ = 0, totalWords_ = 0, totalRows_ = 0, totalPairs_ = 0;
     int nodeKind_ = 0, nodes_ = 1;
     bool anyMaterials_ = false, anyCartesian_ = false, wide_ = false, aliasFill_ = false, raw_ = false,
-         mayList_ = false, emitPacked_ = false;
+         mayList_ = false, emitPacked_ = false, keysMoved_ = false;
     uint32_t listCap_ = 0, keysCap_ = 0, pruneCap_ = 0, mergeEntries_ = 0;
     // table offsets (bytes) in `tables`
     size_t oUnits_ = 0, oWork_ = 0, oRow_ = 0, oWord_ = 0, oSplits_ = 0, oSlices_ = 0, oLater_ = 0,
