@@ -265,7 +265,7 @@ vxb_status vxb_batch_last_launch_count(vxb_batch* b, uint32_t* launches);
  * cannot let cudaFree / cudaMalloc synchronize the device mid-step.  It
  * allocates nothing: the mesh (dev_vertices: 3 floats per vertex,
  * dev_indices: 3 indices per triangle) and dev_out are the caller's device
- * buffers, and its work lists live in a fixed device array of 20,990,720
+ * buffers, and its work lists live in a fixed device array of 12,862,464
  * bytes inside the library, which every GPU that loads the library holds
  * until exit.  min_vertex / max_vertex: the mesh's bounding box, the
  * component-wise min / max of the vertices (vxb_plan reports it).

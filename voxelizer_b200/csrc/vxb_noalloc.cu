@@ -6,7 +6,7 @@
 // times cudaMalloc) synchronizes the whole device, which a caller that keeps
 // several streams busy cannot afford in the middle of a time step.  The
 // caller passes the mesh and the output already in device memory; the work
-// lists this path needs (a range-checked copy of the indices, the chunks of
+// lists this path needs (a range-checked copy of the indices, the batches of
 // triangles with very many candidates, the yz subspace table and the unit
 // table) live in a fixed, statically sized array in device memory instead of
 // buffers allocated per call.  The call itself allocates nothing, on the
@@ -54,7 +54,7 @@ namespace {
 
 constexpr uint32_t kMaxTriangles = 1u << 20;  // 1,048,576
 constexpr uint32_t kMaxSubspaces = 1024;
-constexpr uint32_t kBigChunks = 1u << 20;     // chunks of big triangles (launch_solid_toggle)
+constexpr uint32_t kMaxBatches = kMaxTriangles / 32;   // of launch_solid_toggle, for any number of triangles
 constexpr int kMaxDevices = 64;
 
 constexpr size_t roundUp(size_t v) { return (v + 255) / 256 * 256; }
@@ -69,18 +69,18 @@ struct UnitTables {
 };
 
 // Layout of the scratch array (byte offsets).
-constexpr size_t kStatusOff = 0;  // [0, 1] candidate total, [2] index out of range, [3] big chunks
+constexpr size_t kStatusOff = 0;  // [0, 1] candidate total, [2] index out of range, [4, 5] cursor of the batches
 constexpr size_t kTablesOff = kStatusOff + 256;
 constexpr size_t kSubspaceOff = kTablesOff + 768;
 static_assert(sizeof(UnitTables) <= 768, "tables region");
 constexpr size_t kBigOff = kSubspaceOff + roundUp(kMaxSubspaces * sizeof(vxb::SplitYZ));
-constexpr size_t kIndexOff = kBigOff + roundUp(8 * (size_t)kBigChunks + 1792);
+constexpr size_t kIndexOff = kBigOff + roundUp(8 * (size_t)kMaxBatches);
 constexpr size_t kScratchBytes = kIndexOff + roundUp(12 * (size_t)kMaxTriangles);
-static_assert(kScratchBytes == 20990720, "scratch layout changed: update the stated size");
+static_assert(kScratchBytes == 12862464, "scratch layout changed: update the stated size");
 
 }  // namespace
 
-// 20,990,720 bytes (about 20.0 MiB) of device memory, held by every GPU that
+// 12,862,464 bytes (about 12.3 MiB) of device memory, held by every GPU that
 // loads this library until the process exits.
 static __device__ __align__(256) unsigned char g_noallocScratch[kScratchBytes];
 
@@ -125,7 +125,7 @@ __global__ void noallocSetupKernel(UnitTables tab, uint32_t resY, uint32_t resZ,
                                    UnitTables* dtab, vxb::SplitYZ* dsub, uint32_t* status) {
     if (threadIdx.x == 0) {
         *dtab = tab;
-        status[0] = status[1] = status[2] = status[3] = 0u;
+        for (int k = 0; k < 6; ++k) status[k] = 0u;
     }
     const uint32_t ny = (resY + splitY - 1) / splitY, nz = (resZ + splitZ - 1) / splitZ;
     for (uint32_t k = threadIdx.x; k < ny * nz; k += blockDim.x) {
@@ -251,7 +251,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     uint32_t* status = reinterpret_cast<uint32_t*>(scratch + kStatusOff);
     UnitTables* dtab = reinterpret_cast<UnitTables*>(scratch + kTablesOff);
     vxb::SplitYZ* dsub = reinterpret_cast<vxb::SplitYZ*>(scratch + kSubspaceOff);
-    unsigned long long* big = reinterpret_cast<unsigned long long*>(scratch + kBigOff);
+    uint32_t* big = reinterpret_cast<uint32_t*>(scratch + kBigOff);
     uint32_t* grid = static_cast<uint32_t*>(dev_out);
     vxb::Batch b;
     memset(&b, 0, sizeof(b));
@@ -274,8 +274,8 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
         dev_indices, nIdx, n_vertices, checkedIdx, status);
     launches += 2;
     vxb::launch_solid_toggle(b, n_triangles, reinterpret_cast<unsigned long long*>(status),
-                             vxb::solid_may_list(g, nSub, n_triangles) ? big : nullptr, status + 3, kBigChunks, grid, 3, nullptr,
-                             s, &launches);
+                             vxb::solid_may_list(g, nSub, n_triangles) ? big : nullptr,
+                             reinterpret_cast<unsigned long long*>(status + 4), grid, 3, nullptr, s, &launches);
     vxb::launch_row_fill(b, tab.rowBase[1], tab.wordBase[1], grid, s, &launches);
     e = cudaGetLastError();
     if (e != cudaSuccess) return failf(VXB_ECUDA, "%s", cudaGetErrorString(e));

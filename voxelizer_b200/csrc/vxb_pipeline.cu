@@ -20,10 +20,10 @@ namespace {
 
 // Slots of the status buffer; pruning flags follow at kFlags.
 // kSolidTotal and kSolidHigh are the low and high word of one 64-bit count.
-// kSurfTotal and kSurfHigh likewise; kSurfCursor takes two words.
+// kSurfTotal and kSurfHigh likewise; the cursors take two words.
 enum : int { kSolidTotal = 0, kSolidHigh = 1, kSurfTotal = 2, kSurfHigh = 3, kSurfCursor = 4, kHitCount = 6,
-             kSurfaceVoxels = 7, kSurfQueue = 8, kToggleQueue = 9, kBigCount = 10, kPruneOverflow = 11,
-             kSurfClasses = 12, kRankDone = 15, kPruneCounts = 16 };
+             kSurfaceVoxels = 7, kSurfQueue = 8, kToggleQueue = 9, kBigCursor = 10,
+             kSurfClasses = 12, kRankDone = 15, kPruneOverflow = 16, kPruneCounts = 17 };
 
 // The work counts take 32 bits: totals of 2^32 - 1 or more are refused.
 bool countOverflow(const uint32_t* h) { return h[1] || h[0] == 0xFFFFFFFFu; }
@@ -288,7 +288,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     if ((rc = status.ensure(4 * (kPruneCounts + (size_t)kPasses)))) return rc;
     mayList_ = false;
     for (const Unit& u : units_) mayList_ |= solid_may_list(u.g, u.nSplits, nWork_);
-    if (mayList_ && (rc = bigList.ensure(8 * (size_t)kBigCap))) return rc;
+    if (mayList_ && (rc = bigList.ensure(8 * (size_t)solid_batches(nWork_)))) return rc;
     if (!aliasFill_ && (rc = fill.ensure(wordBytes))) return rc;
     if (anyCartesian_ && (rc = fin.ensure(wordBytes))) return rc;
     // Change lists of the pruning passes: the first pass lists every word it
@@ -420,8 +420,9 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     VXB_CUDA(cudaMemsetAsync(fillP, 0, wordBytes, s));
     tuneMark(kKnobToggle, false, s);
     launch_solid_toggle(b, nWork_, reinterpret_cast<unsigned long long*>(st + kSolidTotal),
-                        mayList_ ? bigList.as<unsigned long long>() : nullptr, st + kBigCount, kBigCap, fillP,
-                        shape.toggleBlocksPerSm, shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
+                        mayList_ ? bigList.as<uint32_t>() : nullptr,
+                        reinterpret_cast<unsigned long long*>(st + kBigCursor), fillP, shape.toggleBlocksPerSm,
+                        shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
     tuneMark(kKnobToggle, true, s);
     launch_row_fill(b, totalRows_, totalWords_, fillP, s, &launches);
     mark(0, true);

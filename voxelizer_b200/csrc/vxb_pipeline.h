@@ -99,7 +99,6 @@ public:
     static constexpr uint32_t kLoopListMax = 32768;   // longest list the one-cluster passes take
     static constexpr uint64_t kPriorityWords = 1u << 20;   // grids from here on finish on the high-priority stream
     static constexpr uint32_t kFewTriangles = 1u << 15;
-    static constexpr uint32_t kBigCap = 1u << 19;       // candidate chunks listed by the solid pass
     static constexpr uint32_t kOutChunks = 4;         // emit / host-copy ranges of streamed output
 
     // Launch shape of the last enqueue (the autotuner's choice).

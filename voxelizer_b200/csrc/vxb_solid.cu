@@ -17,8 +17,9 @@
 // included) and walks their candidates 32 at a time over a prefix of those
 // counts, so nothing is counted, scanned or searched in global memory first
 // and no block-wide barrier holds a warp.  A batch with more than kSplit
-// candidates keeps its first chunk and lists the others, which a second
-// launch spreads over all warps (a box wall alone has tens of thousands).
+// candidates keeps its first chunk and is listed with the number of the others,
+// which a second launch spreads over all warps (a box wall alone has tens of
+// thousands).  The list has room for every batch.
 //
 // Bounds: FP64 issue at half rate (48 edge values a candidate) and the latency
 // of its chains.  Solid pass alone on a B200 (memset, toggles, row fill), with
@@ -47,6 +48,7 @@ constexpr int kWarps = 4;                     // warps per block of the toggle k
 constexpr int kBlocks = 5;                    // resident blocks per SM
 constexpr uint32_t kSplit = 256;              // candidates of a batch before its chunks are listed
 constexpr uint32_t kChunk = 64;               // candidates of one listed chunk
+constexpr uint32_t kChunkBits = 33;           // low bits of the list's cursor: chunks; above: batches
 constexpr uint32_t kFull = 0xffffffffu;
 
 __device__ __forceinline__ void loadTriD(const float* __restrict__ V, const uint32_t* __restrict__ I, uint32_t t,
@@ -424,13 +426,15 @@ __device__ __forceinline__ void solidCandidates(SolidSlots& st, const Batch& b, 
 
 // Toggles of every work triangle.  A warp takes batches of `perWarp` (a
 // power of two up to 32) triangles in a fixed grid-stride order or (queue !=
-// NULL) from a device work queue, one atomic per batch.  The chunks after the
-// first of a batch with more than kSplit candidates are appended to `big`
-// (batch << 32 | chunk).  *total counts the candidates.
+// NULL) from a device work queue, one atomic per batch.  A batch with more than
+// kSplit candidates is listed for its chunks after the first: big[k] is the
+// number of the first of them among all listed chunks, big[bigCap + k] the
+// batch.  One atomic on *cursor gives both k and that number, so the numbers
+// ascend.  *total counts the candidates.
 __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch b, uint32_t nWork, uint32_t perWarp,
-                                                                          unsigned long long* total,
-                                                                          unsigned long long* big, uint32_t* bigCount,
-                                                                          uint32_t bigCap, uint32_t* __restrict__ fill,
+                                                                          unsigned long long* total, uint32_t* big,
+                                                                          unsigned long long* cursor, uint32_t bigCap,
+                                                                          uint32_t* __restrict__ fill,
                                                                           uint32_t* queue) {
     __shared__ SolidSlots slots[kWarps];
     const uint32_t lane = threadIdx.x & 31u;
@@ -450,19 +454,20 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch 
         uint32_t n = solidBatch(st, b, bt, perWarp, nWork, lane, &mine, &off);
         if (n > kSplit && big) {
             const uint32_t more = (n - 1u) / kChunk;   // chunks 1 .. more
-            uint32_t at = 0;
-            if (lane == 0) at = atomicAdd(bigCount, more);
+            unsigned long long at = 0;
+            if (lane == 0) at = atomicAdd(cursor, (1ull << kChunkBits) + more);
             at = __shfl_sync(kFull, at, 0);
-            // The batches that reserved 2^26 entries have 2^32 candidates: the
-            // host refuses the call, and the rest would be in vain.
+            const uint32_t entry = (uint32_t)(at >> kChunkBits);
+            // The batches that reserved 2^26 chunks have 2^32 candidates: the
+            // host refuses the call, and the rest would be in vain.  (Past that
+            // the chunks may carry into the number of batches.)
             static_assert((unsigned long long)kChunk << 26 == 1ull << 32, "candidates of 2^26 chunks");
-            if (at >= 1u << 26) break;
-            // A list without room for all of them leaves the batch to this
-            // warp; the entries it reserved are marked as empty.
-            const bool fits = at < bigCap && more <= bigCap - at;
-            for (uint32_t k = lane; k < more && at < bigCap && k < bigCap - at; k += 32u)
-                big[at + k] = fits ? ((unsigned long long)bt << 32) | (k + 1u) : ~0ull;
-            if (fits) n = kChunk;
+            if ((at & ((1ull << kChunkBits) - 1u)) >= 1u << 26 || entry >= bigCap) break;
+            if (lane == 0) {
+                big[entry] = (uint32_t)at;
+                big[bigCap + entry] = bt;
+            }
+            n = kChunk;
         }
         solidCandidates(st, b, off, 0u, n, lane, fill);
         bt = queue ? take() : bt + nWarps;
@@ -474,20 +479,22 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch 
 
 // The listed chunks, one warp each.
 __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidBigKernel(Batch b, uint32_t nWork, uint32_t perWarp,
-                                                                       const unsigned long long* __restrict__ big,
-                                                                       const uint32_t* __restrict__ bigCount,
+                                                                       const unsigned long long* __restrict__ total,
+                                                                       const uint32_t* __restrict__ big,
+                                                                       const unsigned long long* __restrict__ cursor,
                                                                        uint32_t bigCap, uint32_t* __restrict__ fill) {
     __shared__ SolidSlots slots[kWarps];
+    if (*total >= 0xFFFFFFFFull) return;   // refused by the host
     const uint32_t lane = threadIdx.x & 31u;
     SolidSlots& st = slots[threadIdx.x >> 5];
-    const uint32_t entries = min(*bigCount, bigCap);
-    for (uint32_t e = blockIdx.x * kWarps + (threadIdx.x >> 5); e < entries; e += gridDim.x * kWarps) {
-        const unsigned long long ent = big[e];
-        if (ent == ~0ull) continue;
+    const unsigned long long listed = *cursor;
+    const uint32_t entries = (uint32_t)(listed >> kChunkBits), chunks = (uint32_t)listed;
+    for (uint32_t c = blockIdx.x * kWarps + (threadIdx.x >> 5); c < chunks; c += gridDim.x * kWarps) {
+        const uint32_t e = warpFindOwner(big, entries, c, lane);
         unsigned long long mine = 0;
         uint32_t off;
-        const uint32_t n = solidBatch(st, b, (uint32_t)(ent >> 32), perWarp, nWork, lane, &mine, &off);
-        const uint32_t first = (uint32_t)ent * kChunk;
+        const uint32_t n = solidBatch(st, b, __ldg(big + bigCap + e), perWarp, nWork, lane, &mine, &off);
+        const uint32_t first = (c - __ldg(big + e) + 1u) * kChunk;
         solidCandidates(st, b, off, first, min(n - first, kChunk) + first, lane, fill);
     }
 }
@@ -571,16 +578,21 @@ bool solid_may_list(const PassGeom& g, uint64_t nSplits, uint32_t nWork) {
     return ((g.resY + 3ull) / 4 + nSplits) * ((g.resZ + 3ull) / 4 + nSplits) * solidPerWarp(nWork) > kSplit;
 }
 
-void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, unsigned long long* big,
-                         uint32_t* bigCount, uint32_t bigCap, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
+uint32_t solid_batches(uint32_t nWork) {
+    const uint32_t perWarp = solidPerWarp(nWork);
+    return (nWork + perWarp - 1) / perWarp;
+}
+
+void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, uint32_t* big,
+                         unsigned long long* cursor, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
                          cudaStream_t s, uint32_t* launches) {
-    const uint32_t perWarp = solidPerWarp(nWork), batches = (nWork + perWarp - 1) / perWarp;
+    const uint32_t perWarp = solidPerWarp(nWork), batches = solid_batches(nWork);
     if (queue) cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
     const uint32_t grid = gridFor(batches, kWarps, 148u * 8u * blocksPerSm);
-    solidToggleKernel<<<grid, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, big, bigCount, bigCap, fill, queue);
+    solidToggleKernel<<<grid, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, big, cursor, batches, fill, queue);
     *launches += 1;
     if (big) {
-        solidBigKernel<<<148 * kBlocks, kWarps * 32, 0, s>>>(b, nWork, perWarp, big, bigCount, bigCap, fill);
+        solidBigKernel<<<148 * kBlocks, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, big, cursor, batches, fill);
         *launches += 1;
     }
 }
