@@ -62,8 +62,8 @@ struct Unit {
     const uint32_t* I;    // indices into V (3 per triangle),
     const uint8_t* M;     // material per triangle (NULL without materials)
     uint32_t nT;          // triangles of the mesh
-    uint32_t splitBase;   // solid yz subspaces: SplitYZ entries [splitBase, splitBase + nSplits)
-    uint32_t nSplits;
+    uint32_t splitBase;   // solid yz subspaces: splitN[0] * splitN[1] SplitYZ entries, y inner
+    uint32_t splitN[2];   // subspaces along y, along z
     uint32_t sliceBase;   // material subspace slices: (lo, hi) pairs, x then y then z
     uint32_t sliceN[3];
     uint32_t laterBase;   // AY + AZ flags: row y + 1 / plane z + 1 starts a later pruning subspace

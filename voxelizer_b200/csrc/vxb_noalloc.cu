@@ -241,7 +241,8 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     tab.unit.V = dev_vertices;
     tab.unit.I = checkedIdx;
     tab.unit.nT = n_triangles;
-    tab.unit.nSplits = nSub;
+    tab.unit.splitN[0] = (uint32_t)ny;
+    tab.unit.splitN[1] = (uint32_t)nz;
     tab.unit.out = dev_out;
     tab.workBase[1] = n_triangles;
     tab.rowBase[1] = (uint64_t)g.AY * g.AZ;

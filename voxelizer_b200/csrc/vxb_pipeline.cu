@@ -195,7 +195,8 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
             u.splitBase = (uint32_t)splits.size();
             for (const auto& z : p.zSplitsExt)
                 for (const auto& y : p.ySplitsExt) splits.push_back(SplitYZ{y.lo, y.hi, z.lo, z.hi});
-            u.nSplits = (uint32_t)splits.size() - u.splitBase;
+            u.splitN[0] = (uint32_t)p.ySplitsExt.size();
+            u.splitN[1] = (uint32_t)p.zSplitsExt.size();
             u.sliceBase = (uint32_t)(slices.size() / 2);
             const std::vector<Range>* axes[3] = {&p.xMat, &p.yMat, &p.zMat};
             for (int a = 0; a < 3; ++a) {
@@ -287,7 +288,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     if ((rc = tables.ensure(blob_.size() + 64))) return rc;
     if ((rc = status.ensure(4 * (kPruneCounts + (size_t)kPasses)))) return rc;
     mayList_ = false;
-    for (const Unit& u : units_) mayList_ |= solid_may_list(u.g, u.nSplits, nWork_);
+    for (const Unit& u : units_) mayList_ |= solid_may_list(u.g, (uint64_t)u.splitN[0] * u.splitN[1], nWork_);
     if (mayList_ && (rc = bigList.ensure(8 * (size_t)solid_batches(nWork_)))) return rc;
     if (!aliasFill_ && (rc = fill.ensure(wordBytes))) return rc;
     if (anyCartesian_ && (rc = fin.ensure(wordBytes))) return rc;
