@@ -100,19 +100,19 @@ void launch_scan(const uint32_t* in, uint32_t* offsets, uint32_t n, uint32_t* bl
 // ---- Solid (parity) voxelization: src/voxelizer.cu:840-1617 ----
 // The toggles of every candidate into the `fill` arena, then the row prefix
 // XOR over all rows of the batch.  *total (zero on entry) receives the number
-// of candidates.  `big` lists the batches of triangles with very many candidates
-// (2 * solid_batches entries, *cursor zero on entry); it may be NULL where
-// solid_may_list answers false for every unit, and the call then takes one
-// launch instead of two.
+// of candidates.  `big` (solid_big_bytes; *cursor zero on entry) lists the batches
+// of triangles with very many candidates, and the first listCap chunks of them
+// one by one; it may be NULL where solid_may_list answers false for every unit,
+// and the call then takes one launch instead of two.
 // blocksPerSm: launch shape (the autotuner's choice; results do not depend
 // on it), here and in the launchers below that take one.  queue: NULL for
 // a fixed grid-stride order, else a device word the launcher zeroes and the
 // kernel's warps take batches of work from.
 bool solid_may_list(const PassGeom& g, uint64_t nSplits, uint32_t nWork);
-uint32_t solid_batches(uint32_t nWork);
-void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, uint32_t* big,
-                         unsigned long long* cursor, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
-                         cudaStream_t s, uint32_t* launches);
+size_t solid_big_bytes(uint32_t nWork, uint32_t listCap);
+void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, void* big,
+                         unsigned long long* cursor, uint32_t listCap, uint32_t* fill, uint32_t blocksPerSm,
+                         uint32_t* queue, cudaStream_t s, uint32_t* launches);
 void launch_row_fill(const Batch& b, uint64_t nRows, uint64_t totalWords, uint32_t* fill, cudaStream_t s,
                      uint32_t* launches);
 

@@ -252,7 +252,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     uint32_t* status = reinterpret_cast<uint32_t*>(scratch + kStatusOff);
     UnitTables* dtab = reinterpret_cast<UnitTables*>(scratch + kTablesOff);
     vxb::SplitYZ* dsub = reinterpret_cast<vxb::SplitYZ*>(scratch + kSubspaceOff);
-    uint32_t* big = reinterpret_cast<uint32_t*>(scratch + kBigOff);
+    void* big = scratch + kBigOff;
     uint32_t* grid = static_cast<uint32_t*>(dev_out);
     vxb::Batch b;
     memset(&b, 0, sizeof(b));
@@ -276,7 +276,7 @@ extern "C" vxb_status vxb_voxelize_bits_noalloc(const float* dev_vertices, const
     launches += 2;
     vxb::launch_solid_toggle(b, n_triangles, reinterpret_cast<unsigned long long*>(status),
                              vxb::solid_may_list(g, nSub, n_triangles) ? big : nullptr,
-                             reinterpret_cast<unsigned long long*>(status + 4), grid, 3, nullptr, s, &launches);
+                             reinterpret_cast<unsigned long long*>(status + 4), 0, grid, 3, nullptr, s, &launches);
     vxb::launch_row_fill(b, tab.rowBase[1], tab.wordBase[1], grid, s, &launches);
     e = cudaGetLastError();
     if (e != cudaSuccess) return failf(VXB_ECUDA, "%s", cudaGetErrorString(e));

@@ -289,7 +289,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     if ((rc = status.ensure(4 * (kPruneCounts + (size_t)kPasses)))) return rc;
     mayList_ = false;
     for (const Unit& u : units_) mayList_ |= solid_may_list(u.g, (uint64_t)u.splitN[0] * u.splitN[1], nWork_);
-    if (mayList_ && (rc = bigList.ensure(8 * (size_t)solid_batches(nWork_)))) return rc;
+    if (mayList_ && (rc = bigList.ensure(solid_big_bytes(nWork_, kBigChunks)))) return rc;
     if (!aliasFill_ && (rc = fill.ensure(wordBytes))) return rc;
     if (anyCartesian_ && (rc = fin.ensure(wordBytes))) return rc;
     // Change lists of the pruning passes: the first pass lists every word it
@@ -421,9 +421,8 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
     VXB_CUDA(cudaMemsetAsync(fillP, 0, wordBytes, s));
     tuneMark(kKnobToggle, false, s);
     launch_solid_toggle(b, nWork_, reinterpret_cast<unsigned long long*>(st + kSolidTotal),
-                        mayList_ ? bigList.as<uint32_t>() : nullptr,
-                        reinterpret_cast<unsigned long long*>(st + kBigCursor), fillP, shape.toggleBlocksPerSm,
-                        shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
+                        mayList_ ? bigList.p : nullptr, reinterpret_cast<unsigned long long*>(st + kBigCursor),
+                        kBigChunks, fillP, shape.toggleBlocksPerSm, shape.toggleQueue ? st + kToggleQueue : nullptr, s, &launches);
     tuneMark(kKnobToggle, true, s);
     launch_row_fill(b, totalRows_, totalWords_, fillP, s, &launches);
     mark(0, true);

@@ -99,6 +99,7 @@ public:
     static constexpr uint32_t kLoopListMax = 32768;   // longest list the one-cluster passes take
     static constexpr uint64_t kPriorityWords = 1u << 20;   // grids from here on finish on the high-priority stream
     static constexpr uint32_t kFewTriangles = 1u << 15;
+    static constexpr uint32_t kBigChunks = 1u << 17;   // candidate chunks that the solid pass writes out
     static constexpr uint32_t kOutChunks = 4;         // emit / host-copy ranges of streamed output
 
     // Launch shape of the last enqueue (the autotuner's choice).

@@ -19,7 +19,9 @@
 // and no block-wide barrier holds a warp.  A batch with more than kSplit
 // candidates keeps its first chunk and is listed with the number of the others,
 // which a second launch spreads over all warps (a box wall alone has tens of
-// thousands).  The list has room for every batch.
+// thousands).  The list has room for every batch.  The first listCap chunks are
+// also written out one by one: the search of a chunk's batch costs a call whose
+// solid pass is mostly chunks 1-1.5% (stress mesh, 171 us).
 //
 // Bounds: FP64 issue at half rate (48 edge values a candidate) and the latency
 // of its chains.  Solid pass alone on a B200 (memset, toggles, row fill), with
@@ -461,16 +463,25 @@ __device__ __forceinline__ void solidCandidates(SolidSlots& st, const Batch& b, 
     }
 }
 
+// The listed batches and their chunks (launch_solid_toggle).
+struct BigList {
+    unsigned long long* cursor;   // NULL: nothing is listed
+    uint32_t* first;
+    uint32_t* batch;
+    uint32_t cap;                 // batches
+    uint2* list;                  // batch and chunk, for the first listCap chunks
+    uint32_t listCap;
+};
+
 // Toggles of every work triangle.  A warp takes batches of `perWarp` (a
 // power of two up to 32) triangles in a fixed grid-stride order or (queue !=
 // NULL) from a device work queue, one atomic per batch.  A batch with more than
-// kSplit candidates is listed for its chunks after the first: big[k] is the
-// number of the first of them among all listed chunks, big[bigCap + k] the
-// batch.  One atomic on *cursor gives both k and that number, so the numbers
-// ascend.  *total counts the candidates.
+// kSplit candidates is listed for its chunks after the first: big.first[k] is the
+// number of the first of them among all listed chunks, big.batch[k] the batch.
+// One atomic on *cursor gives both k and that number, so the numbers ascend.
+// *total counts the candidates.
 __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch b, uint32_t nWork, uint32_t perWarp,
-                                                                          unsigned long long* total, uint32_t* big,
-                                                                          unsigned long long* cursor, uint32_t bigCap,
+                                                                          unsigned long long* total, BigList big,
                                                                           uint32_t* __restrict__ fill,
                                                                           uint32_t* queue) {
     __shared__ SolidSlots slots[kWarps];
@@ -489,21 +500,23 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch 
     while (bt < batches) {
         uint32_t off;
         uint32_t n = solidBatch(st, b, bt, perWarp, nWork, lane, &mine, &off);
-        if (n > kSplit && big) {
+        if (n > kSplit && big.cursor) {
             const uint32_t more = (n - 1u) / kChunk;   // chunks 1 .. more
             unsigned long long at = 0;
-            if (lane == 0) at = atomicAdd(cursor, (1ull << kChunkBits) + more);
+            if (lane == 0) at = atomicAdd(big.cursor, (1ull << kChunkBits) + more);
             at = __shfl_sync(kFull, at, 0);
             const uint32_t entry = (uint32_t)(at >> kChunkBits);
             // The batches that reserved 2^26 chunks have 2^32 candidates: the
             // host refuses the call, and the rest would be in vain.  (Past that
             // the chunks may carry into the number of batches.)
             static_assert((unsigned long long)kChunk << 26 == 1ull << 32, "candidates of 2^26 chunks");
-            if ((at & ((1ull << kChunkBits) - 1u)) >= 1u << 26 || entry >= bigCap) break;
+            if ((at & ((1ull << kChunkBits) - 1u)) >= 1u << 26 || entry >= big.cap) break;
             if (lane == 0) {
-                big[entry] = (uint32_t)at;
-                big[bigCap + entry] = bt;
+                big.first[entry] = (uint32_t)at;
+                big.batch[entry] = bt;
             }
+            for (uint32_t k = lane; k < more && (uint32_t)at + k < big.listCap; k += 32u)
+                big.list[(uint32_t)at + k] = make_uint2(bt, k + 1u);
             n = kChunk;
         }
         solidCandidates(st, b, off, 0u, n, lane, fill);
@@ -517,21 +530,25 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidToggleKernel(Batch 
 // The listed chunks, one warp each.
 __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidBigKernel(Batch b, uint32_t nWork, uint32_t perWarp,
                                                                        const unsigned long long* __restrict__ total,
-                                                                       const uint32_t* __restrict__ big,
-                                                                       const unsigned long long* __restrict__ cursor,
-                                                                       uint32_t bigCap, uint32_t* __restrict__ fill) {
+                                                                       BigList big, uint32_t* __restrict__ fill) {
     __shared__ SolidSlots slots[kWarps];
     if (*total >= 0xFFFFFFFFull) return;   // refused by the host
     const uint32_t lane = threadIdx.x & 31u;
     SolidSlots& st = slots[threadIdx.x >> 5];
-    const unsigned long long listed = *cursor;
+    const unsigned long long listed = *big.cursor;
     const uint32_t entries = (uint32_t)(listed >> kChunkBits), chunks = (uint32_t)listed;
     for (uint32_t c = blockIdx.x * kWarps + (threadIdx.x >> 5); c < chunks; c += gridDim.x * kWarps) {
-        const uint32_t e = warpFindOwner(big, entries, c, lane);
+        uint2 at;   // batch, chunk of it
+        if (c < big.listCap) {
+            at = big.list[c];
+        } else {
+            const uint32_t e = warpFindOwner(big.first, entries, c, lane);
+            at = make_uint2(big.batch[e], c - big.first[e] + 1u);
+        }
         unsigned long long mine = 0;
         uint32_t off;
-        const uint32_t n = solidBatch(st, b, __ldg(big + bigCap + e), perWarp, nWork, lane, &mine, &off);
-        const uint32_t first = (c - __ldg(big + e) + 1u) * kChunk;
+        const uint32_t n = solidBatch(st, b, at.x, perWarp, nWork, lane, &mine, &off);
+        const uint32_t first = at.y * kChunk;
         solidCandidates(st, b, off, first, min(n - first, kChunk) + first, lane, fill);
     }
 }
@@ -615,21 +632,32 @@ bool solid_may_list(const PassGeom& g, uint64_t nSplits, uint32_t nWork) {
     return ((g.resY + 3ull) / 4 + nSplits) * ((g.resZ + 3ull) / 4 + nSplits) * solidPerWarp(nWork) > kSplit;
 }
 
-uint32_t solid_batches(uint32_t nWork) {
+static uint32_t solidBatches(uint32_t nWork) {
     const uint32_t perWarp = solidPerWarp(nWork);
     return (nWork + perWarp - 1) / perWarp;
 }
 
-void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, uint32_t* big,
-                         unsigned long long* cursor, uint32_t* fill, uint32_t blocksPerSm, uint32_t* queue,
-                         cudaStream_t s, uint32_t* launches) {
-    const uint32_t perWarp = solidPerWarp(nWork), batches = solid_batches(nWork);
+size_t solid_big_bytes(uint32_t nWork, uint32_t listCap) { return 8 * ((size_t)solidBatches(nWork) + listCap); }
+
+void launch_solid_toggle(const Batch& b, uint32_t nWork, unsigned long long* total, void* big,
+                         unsigned long long* cursor, uint32_t listCap, uint32_t* fill, uint32_t blocksPerSm,
+                         uint32_t* queue, cudaStream_t s, uint32_t* launches) {
+    const uint32_t perWarp = solidPerWarp(nWork), batches = solidBatches(nWork);
+    BigList l{};
+    if (big) {
+        l.cursor = cursor;
+        l.list = static_cast<uint2*>(big);
+        l.listCap = listCap;
+        l.first = reinterpret_cast<uint32_t*>(l.list + listCap);
+        l.batch = l.first + batches;
+        l.cap = batches;
+    }
     if (queue) cudaMemsetAsync(queue, 0, sizeof(uint32_t), s);
     const uint32_t grid = gridFor(batches, kWarps, 148u * 8u * blocksPerSm);
-    solidToggleKernel<<<grid, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, big, cursor, batches, fill, queue);
+    solidToggleKernel<<<grid, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, l, fill, queue);
     *launches += 1;
     if (big) {
-        solidBigKernel<<<148 * kBlocks, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, big, cursor, batches, fill);
+        solidBigKernel<<<148 * kBlocks, kWarps * 32, 0, s>>>(b, nWork, perWarp, total, l, fill);
         *launches += 1;
     }
 }
