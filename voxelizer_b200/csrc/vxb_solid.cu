@@ -52,6 +52,7 @@ constexpr uint32_t kSplit = 256;              // candidates of a batch before it
 constexpr uint32_t kChunk = 64;               // candidates of one listed chunk
 constexpr uint32_t kChunkBits = 33;           // low bits of the list's cursor: chunks; above: batches
 constexpr uint32_t kFull = 0xffffffffu;
+constexpr uint32_t kSeveral = 0x80000000u;    // a triangle in several subspaces
 
 __device__ __forceinline__ void loadTriD(const float* __restrict__ V, const uint32_t* __restrict__ I, uint32_t t,
                                          D3* v) {
@@ -155,8 +156,7 @@ struct SolidSlots {
     uint32_t wt[32], unit[32];
     uint32_t flags[32];   // bits 0-2: top-left generation edges; bit 3: binning edges are the same
     uint32_t off[32];     // first candidate
-    uint32_t tilesY[32];  // tiles along y of all subspaces
-    uint32_t sub[32];     // the only subspace of the triangle (~0: several)
+    uint32_t sub[32];     // the triangle's only subspace, or its tiles along y of all of them | kSeveral
     uint16_t queue[512];
 };
 
@@ -167,7 +167,7 @@ struct SolidSlots {
 // of candidates made the solid pass of a box 7.6 ms, now 2.0.  A triangle within
 // one subspace keeps its number.
 __device__ __forceinline__ uint32_t solidCount(const Batch& b, uint32_t wt, BinTri& bt, uint32_t* unit,
-                                               uint32_t* tilesY, uint32_t* sub) {
+                                               uint32_t* sub) {
     uint32_t t;
     *unit = workUnit(b, wt, &t);
     const Unit& U = b.units[*unit];
@@ -175,24 +175,27 @@ __device__ __forceinline__ uint32_t solidCount(const Batch& b, uint32_t wt, BinT
     if (binRejected(bt)) return 0u;
     const SplitYZ* __restrict__ splits = b.splits + U.splitBase;
     const uint32_t ny = U.splitN[0], nz = U.splitN[1];
-    uint32_t cy = 0, cz = 0, sy = 0, sz = 0, lo, hi;
+    uint32_t lo, hi;
+    const SplitYZ q0 = splits[0];
+    uint32_t cy = commonTiles(bt.vlo[0], bt.vhi[0], q0.y0, q0.y1, &lo, &hi);
+    uint32_t cz = commonTiles(bt.vlo[1], bt.vhi[1], q0.z0, q0.z1, &lo, &hi);
+    uint32_t sy = 0, sz = 0;
     bool several = false;
-    for (uint32_t s = 0; s < ny; ++s) {
+    for (uint32_t s = 1; s < ny; ++s) {
         const uint32_t n = commonTiles(bt.vlo[0], bt.vhi[0], splits[s].y0, splits[s].y1, &lo, &hi);
         if (!n) continue;
         several |= cy != 0u;
         cy += n;
         sy = s;
     }
-    for (uint32_t s = 0; s < nz; ++s) {
+    for (uint32_t s = 1; s < nz; ++s) {
         const uint32_t n = commonTiles(bt.vlo[1], bt.vhi[1], splits[s * ny].z0, splits[s * ny].z1, &lo, &hi);
         if (!n) continue;
         several |= cz != 0u;
         cz += n;
         sz = s;
     }
-    *tilesY = cy;
-    *sub = several ? ~0u : sz * ny + sy;
+    *sub = several ? kSeveral | cy : sz * ny + sy;
     return cy * cz;
 }
 
@@ -240,8 +243,8 @@ __device__ __forceinline__ uint32_t solidBatch(SolidSlots& st, const Batch& b, u
                                                uint32_t nWork, uint32_t lane, unsigned long long* mine, uint32_t* off) {
     const uint32_t wt = batch * perWarp + lane;
     BinTri bt;
-    uint32_t unit = 0, tilesY = 0, sub = 0;
-    const uint32_t c = lane < perWarp && wt < nWork ? solidCount(b, wt, bt, &unit, &tilesY, &sub) : 0u;
+    uint32_t unit = 0, sub = 0;
+    const uint32_t c = lane < perWarp && wt < nWork ? solidCount(b, wt, bt, &unit, &sub) : 0u;
     *mine += c;
     uint32_t incl = c;
 #pragma unroll
@@ -253,7 +256,6 @@ __device__ __forceinline__ uint32_t solidBatch(SolidSlots& st, const Batch& b, u
     if (c) {
         const uint32_t slot = __popc(used & laneMaskLt());
         st.off[slot] = incl - c;
-        st.tilesY[slot] = tilesY;
         st.sub[slot] = sub;
         solidStage(st, slot, bt, unit, wt);
     }
@@ -311,12 +313,12 @@ __device__ __forceinline__ uint32_t solidCandidate(const SolidSlots& st, uint32_
     uint32_t lo[2] = {0, 0}, hi[2] = {1, 1}, nty = 1;
     const int vlo[2] = {st.lo[0][slot], st.lo[1][slot]}, vhi[2] = {st.hi[0][slot], st.hi[1][slot]};
     const uint32_t sub = st.sub[slot];
-    SplitYZ sp = splits[sub != ~0u ? sub : 0u];
-    if (sub != ~0u) {
+    SplitYZ sp = splits[sub & kSeveral ? 0u : sub];
+    if (!(sub & kSeveral)) {
         nty = commonTiles(vlo[0], vhi[0], sp.y0, sp.y1, &lo[0], &hi[0]);
         commonTiles(vlo[1], vhi[1], sp.z0, sp.z1, &lo[1], &hi[1]);
     } else {
-        const uint32_t ny = U.splitN[0], nz = U.splitN[1], tilesY = st.tilesY[slot];
+        const uint32_t ny = U.splitN[0], nz = U.splitN[1], tilesY = sub & ~kSeveral;
         uint32_t ntz = 1;
         for (uint32_t s = 0; s < nz; ++s) {
             const SplitYZ q = splits[s * ny];
@@ -532,10 +534,10 @@ __global__ void __launch_bounds__(kWarps * 32, kBlocks) solidBigKernel(Batch b, 
                                                                        const unsigned long long* __restrict__ total,
                                                                        BigList big, uint32_t* __restrict__ fill) {
     __shared__ SolidSlots slots[kWarps];
-    if (*total >= 0xFFFFFFFFull) return;   // refused by the host
+    const unsigned long long listed = *big.cursor, all = *total;   // both in flight
+    if (all >= 0xFFFFFFFFull) return;   // refused by the host
     const uint32_t lane = threadIdx.x & 31u;
     SolidSlots& st = slots[threadIdx.x >> 5];
-    const unsigned long long listed = *big.cursor;
     const uint32_t entries = (uint32_t)(listed >> kChunkBits), chunks = (uint32_t)listed;
     for (uint32_t c = blockIdx.x * kWarps + (threadIdx.x >> 5); c < chunks; c += gridDim.x * kWarps) {
         uint2 at;   // batch, chunk of it
