@@ -178,15 +178,15 @@ int meshCheck(const float* dV, uint32_t nV, const uint32_t* dI, uint64_t nIdx, u
 // change list and *overflow a flag, all zero on entry.  Pass 0 goes over all
 // words, pass 1 over the words it changed (list0), the others in one cluster
 // with alternating lists of at most `cap` (unit << 32 | word) entries.
-// blockBase: exclusive prefix over the units of prune_blocks (nUnits + 1
-// entries) for `planes` = prune_planes(totalWords); `blocks` is their sum.  The
-// grid is pruned unless counts[passes - 1] or *overflow is set (a list longer
-// than cap or, after pass 1, than escapeAt): then launch_prune_full passes,
+// blockBase[k]: exclusive prefix over the units of prune_blocks for thin = k
+// (nUnits + 1 entries) and `planes` = prune_planes(totalWords); blocks[k] is their
+// sum.  The grid is pruned unless counts[passes - 1] or *overflow is set (a list
+// longer than cap or, after pass 1, than escapeAt): then launch_prune_full passes,
 // which set *changed, finish it.
 uint32_t prune_planes(uint64_t totalWords);
-uint32_t prune_blocks(const PassGeom& g, uint32_t planes);
-void launch_prune(const Batch& b, uint64_t totalWords, const uint32_t* blockBase, uint32_t blocks, uint32_t planes,
-                  uint32_t* solid, const uint32_t* fill, const uint32_t* surf, uint32_t passes,
+uint32_t prune_blocks(const PassGeom& g, uint32_t planes, bool thin);
+void launch_prune(const Batch& b, uint64_t totalWords, const uint32_t* const blockBase[2], const uint32_t blocks[2],
+                  uint32_t planes, uint32_t* solid, const uint32_t* fill, const uint32_t* surf, uint32_t passes,
                   unsigned long long* list0, unsigned long long* list1, uint32_t* counts, uint32_t cap,
                   uint32_t escapeAt, uint32_t* overflow, cudaStream_t s, uint32_t* launches);
 void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, const uint32_t* fill,

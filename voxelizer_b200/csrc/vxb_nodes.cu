@@ -99,12 +99,21 @@ __device__ __forceinline__ uint32_t prunedWord(uint32_t w, uint32_t prev, uint32
 // outside the span are read again from memory.  So each word of the two
 // arenas is loaded once per block instead of seven times, and the positions
 // are divided out once per block.
+//
+// A unit whose planes are thin (kPruneThin words at the most) would leave most
+// of such a block idle.  In a launch of its own, its threads take one word each,
+// across planes, and load its neighbours: pruning of a rod of 60,002 planes of 7
+// words 256 us walking planes, 15 this way; 4,002 planes of 512 words 34 and 27;
+// a batch of 2,000 meshes of 16-24 voxels 434 and 137 us.
 constexpr int kPruneThreads = 512;
 constexpr int kPruneWords = 2;   // words per thread and plane
 constexpr uint32_t kPruneSpan = kPruneThreads * kPruneWords;
+constexpr uint32_t kPruneThin = kPruneSpan / 2;
+constexpr uint32_t kThinThreads = 256;
 constexpr uint32_t kPruneKeep = 512;   // changed words a block collects before it lists them one by one
 
-__global__ void __launch_bounds__(kPruneThreads) pruneFirstKernel(Batch b, const uint32_t* __restrict__ blockBase,
+template <bool kThin>
+__global__ void __launch_bounds__(kThin ? kThinThreads : kPruneThreads) pruneFirstKernel(Batch b, const uint32_t* __restrict__ blockBase,
                                                                   uint32_t planes, uint32_t* __restrict__ solid,
                                                                   const uint32_t* __restrict__ fill,
                                                                   const uint32_t* __restrict__ surf,
@@ -117,7 +126,48 @@ __global__ void __launch_bounds__(kPruneThreads) pruneFirstKernel(Batch b, const
     const uint32_t u = b.nUnits > 1 ? unitOf(blockBase, b.nUnits, blockIdx.x) : 0u;
     const PruneView v = pruneView(b, u, solid, fill, surf);
     const uint32_t plane = v.ipx * v.AY, spans = (plane + kPruneSpan - 1) / kPruneSpan;
-    const uint32_t t = blockIdx.x - __ldg(blockBase + u), zc = t / spans;
+    const uint32_t t = blockIdx.x - __ldg(blockBase + u);
+    // Lists a changed word.
+    auto keep = [&](uint32_t idx) {
+        const uint32_t k = atomicAdd(&nKept, 1u);
+        if (k < kPruneKeep) {
+            kept[k] = idx;
+            return;
+        }
+        const uint32_t g = atomicAdd(count, 1u);
+        if (g < cap) list[g] = ((unsigned long long)u << 32) | idx;
+        else *overflow = 1u;
+    };
+    // The block's collected words go to the list together (whole block).
+    auto listKept = [&]() {
+        __syncthreads();
+        const uint32_t nList = min(nKept, kPruneKeep);
+        if (threadIdx.x == 0 && nList) listAt = atomicAdd(count, nList);
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < nList; k += kThin ? kThinThreads : kPruneThreads) {
+            if (listAt + k < cap) list[listAt + k] = ((unsigned long long)u << 32) | kept[k];
+            else *overflow = 1u;
+        }
+    };
+    if (kThin) {
+        __syncthreads();   // nKept
+        const uint32_t idx = t * kThinThreads + threadIdx.x;
+        if (idx < v.nWords) {
+            const uint32_t w = unpruned(v, idx);
+            uint32_t nw = 0u;
+            if (w) {
+                const uint32_t row = v.divX.div(idx), k = idx - row * v.ipx, z = v.divY.div(row), y = row - z * v.AY;
+                auto at = [&](bool there, uint32_t i) { return there ? unpruned(v, i) : 0u; };
+                nw = prunedWord(w, at(k > 0, idx - 1), at(k + 1 < v.ipx, idx + 1), at(y > 0, idx - v.ipx),
+                                at(y + 1 < v.AY, idx + v.ipx), at(z > 0, idx - plane), at(z + 1 < v.AZ, idx + plane));
+                if (nw != w) keep(idx);
+            }
+            v.S[idx] = nw;
+        }
+        listKept();
+        return;
+    }
+    const uint32_t zc = t / spans;
     const uint32_t s0 = (t - zc * spans) * kPruneSpan;
     const uint32_t z0 = zc * planes, z1 = min(z0 + planes, v.AZ), n = min(kPruneSpan, plane - s0);
     uint32_t sides[kPruneWords];   // bits 0-3: a neighbour at x - 1, x + 1, y - 1, y + 1
@@ -167,16 +217,7 @@ __global__ void __launch_bounds__(kPruneThreads) pruneFirstKernel(Batch b, const
                 };
                 nw = prunedWord(w, at(0, l > 0, -1), at(1, l + 1 < n, 1), at(2, l >= v.ipx, -(int)v.ipx),
                                 at(3, l + v.ipx < n, (int)v.ipx), below[q], up[q]);
-                if (nw != w) {
-                    const uint32_t k = atomicAdd(&nKept, 1u);
-                    if (k < kPruneKeep) {
-                        kept[k] = base + l;
-                    } else {
-                        const uint32_t g = atomicAdd(count, 1u);
-                        if (g < cap) list[g] = ((unsigned long long)u << 32) | (base + l);
-                        else *overflow = 1u;
-                    }
-                }
+                if (nw != w) keep(base + l);
             }
             v.S[base + l] = nw;
             below[q] = w;
@@ -184,14 +225,7 @@ __global__ void __launch_bounds__(kPruneThreads) pruneFirstKernel(Batch b, const
 #pragma unroll
         for (int q = 0; q < kPruneWords; ++q) mid[q] = up[q];
     }
-    __syncthreads();
-    const uint32_t nList = min(nKept, kPruneKeep);
-    if (threadIdx.x == 0 && nList) listAt = atomicAdd(count, nList);
-    __syncthreads();
-    for (uint32_t k = threadIdx.x; k < nList; k += kPruneThreads) {
-        if (listAt + k < cap) list[listAt + k] = ((unsigned long long)u << 32) | kept[k];
-        else *overflow = 1u;
-    }
+    listKept();
 }
 
 // Clears `dead` of word idx and lists the word when that took a bit.
@@ -1004,16 +1038,23 @@ uint32_t prune_planes(uint64_t totalWords) {
     return (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, totalWords / kPruneSpan / (148u * 8u)));
 }
 
-uint32_t prune_blocks(const PassGeom& g, uint32_t planes) {
-    return ((g.ipx * g.AY + kPruneSpan - 1) / kPruneSpan) * ((g.AZ + planes - 1) / planes);
+uint32_t prune_blocks(const PassGeom& g, uint32_t planes, bool thin) {
+    const uint32_t plane = g.ipx * g.AY, spans = (plane + kPruneSpan - 1) / kPruneSpan;
+    if (thin != (plane <= kPruneThin)) return 0u;
+    return thin ? (plane * g.AZ + kThinThreads - 1) / kThinThreads : spans * ((g.AZ + planes - 1) / planes);
 }
 
-void launch_prune(const Batch& b, uint64_t totalWords, const uint32_t* blockBase, uint32_t blocks, uint32_t planes,
-                  uint32_t* solid, const uint32_t* fill, const uint32_t* surf, uint32_t passes,
+void launch_prune(const Batch& b, uint64_t totalWords, const uint32_t* const blockBase[2], const uint32_t blocks[2],
+                  uint32_t planes, uint32_t* solid, const uint32_t* fill, const uint32_t* surf, uint32_t passes,
                   unsigned long long* list0, unsigned long long* list1, uint32_t* counts, uint32_t cap,
                   uint32_t escapeAt, uint32_t* overflow, cudaStream_t s, uint32_t* launches) {
-    pruneFirstKernel<<<blocks, kPruneThreads, 0, s>>>(b, blockBase, planes, solid, fill, surf, list0, counts, cap,
-                                                      overflow);
+    for (int thin = 0; thin < 2; ++thin) {
+        if (!blocks[thin]) continue;
+        auto kernel = thin ? pruneFirstKernel<true> : pruneFirstKernel<false>;
+        kernel<<<blocks[thin], thin ? kThinThreads : kPruneThreads, 0, s>>>(b, blockBase[thin], planes, solid, fill,
+                                                                            surf, list0, counts, cap, overflow);
+        *launches += 1;
+    }
     // Few words change.  Up to 64 K words one cluster takes every list (a launch
     // less: 11.6 us of pruning instead of 13.6 at 128^3); larger grids take
     // pass 1 on the whole device, a thread per 16 words at the most.
@@ -1026,7 +1067,7 @@ void launch_prune(const Batch& b, uint64_t totalWords, const uint32_t* blockBase
     }
     pruneListLoopKernel<<<kLoopBlocks, kLoopThreads, 0, s>>>(b, solid, fill, surf, passes, first, list0, list1,
                                                              counts, cap, escapeAt, overflow);
-    *launches += 2;
+    *launches += 1;
 }
 
 void launch_prune_full(const Batch& b, uint64_t totalWords, uint32_t* solid, const uint32_t* fill,

@@ -234,16 +234,20 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     totalRows_ = rowBase.back();
     nFcc_ = (uint32_t)fccMeshes.size();
     totalPairs_ = pairBase.back();
-    // Blocks of the first pruning pass.
-    std::vector<uint32_t> pruneBase{0};
+    // Blocks of the first pruning pass, of wide and of thin units.
+    std::vector<uint32_t> pruneBase[2];
     prunePlanes_ = prune_planes(totalWords_);
-    if (anyCartesian_)
-        for (const Unit& u : units_) {
-            const uint64_t blocks = (uint64_t)pruneBase.back() + prune_blocks(u.g, prunePlanes_);
-            if (blocks > 0x7FFFFFFFull) return failf(VXB_EOVERFLOW, "pruning launch of more than 2^31 blocks");
-            pruneBase.push_back((uint32_t)blocks);
-        }
-    pruneBlocks_ = pruneBase.back();
+    for (int thin = 0; thin < 2; ++thin) {
+        uint64_t blocks = 0;
+        if (anyCartesian_)
+            for (const Unit& u : units_) {
+                pruneBase[thin].push_back((uint32_t)blocks);
+                blocks += prune_blocks(u.g, prunePlanes_, thin != 0);
+                if (blocks > 0x7FFFFFFFull) return failf(VXB_EOVERFLOW, "pruning launch of more than 2^31 blocks");
+            }
+        pruneBase[thin].push_back((uint32_t)blocks);
+        pruneBlocks_[thin] = (uint32_t)blocks;
+    }
     // Tasks of the emission.  The planes of a task follow from the launch shape
     // of each run; one unit takes any number, several units a power of two,
     // whose prefixes over the units are laid out here.
@@ -278,7 +282,7 @@ int Pipeline::prepare(const std::vector<MeshJob>& jobs, cudaStream_t s) {
     oSplits_ = append(blob_, splits);
     oSlices_ = append(blob_, slices);
     oLater_ = append(blob_, later);
-    oPrune_ = append(blob_, pruneBase);
+    for (int thin = 0; thin < 2; ++thin) oPrune_[thin] = append(blob_, pruneBase[thin]);
     oEmit_ = append(blob_, emitBase);
     oFcc_ = append(blob_, fccMeshes);
     oPairBase_ = append(blob_, pairBase);
@@ -455,10 +459,12 @@ int Pipeline::enqueue(cudaStream_t s, StageTimer* timer) {
             mergeSpan = true;
         }
         mark(2, false);
-        launch_prune(b, totalWords_, reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oPrune_), pruneBlocks_,
-                     prunePlanes_, fin.as<uint32_t>(), fillP, anyMaterials_ ? surf.as<uint32_t>() : nullptr, kPasses,
-                     pruneLists.as<unsigned long long>(), pruneLists.as<unsigned long long>() + pruneCap_,
-                     st + kPruneCounts, pruneCap_, kLoopListMax, st + kPruneOverflow, ps, &launches);
+        const uint32_t* const blockBase[2] = {reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oPrune_[0]),
+                                              reinterpret_cast<const uint32_t*>(tables.as<uint8_t>() + oPrune_[1])};
+        launch_prune(b, totalWords_, blockBase, pruneBlocks_, prunePlanes_, fin.as<uint32_t>(), fillP,
+                     anyMaterials_ ? surf.as<uint32_t>() : nullptr, kPasses, pruneLists.as<unsigned long long>(),
+                     pruneLists.as<unsigned long long>() + pruneCap_, st + kPruneCounts, pruneCap_, kLoopListMax,
+                     st + kPruneOverflow, ps, &launches);
         mark(2, true);
     }
     // Join: emission reads the merged keys.

@@ -128,7 +128,7 @@ private:
 
     std::vector<MeshJob> jobs_;
     std::vector<Unit> units_;
-    uint32_t nWork_ = 0, nFcc_ = 0, prunePlanes_ = 0, pruneBlocks_ = 0, maxPlanes_ = 0;
+    uint32_t nWork_ = 0, nFcc_ = 0, prunePlanes_ = 0, pruneBlocks_[2] = {}, maxPlanes_ = 0;
     uint32_t emitTasks_[kEmitLevels] = {};
     uint64_t taskPlanes_ = 0, totalWords_ = 0, totalRows_ = 0, totalPairs_ = 0;
     int nodeKind_ = 0, nodes_ = 1;
@@ -137,7 +137,7 @@ private:
     uint32_t listCap_ = 0, keysCap_ = 0, pruneCap_ = 0, mergeEntries_ = 0;
     // table offsets (bytes) in `tables`
     size_t oUnits_ = 0, oWork_ = 0, oRow_ = 0, oWord_ = 0, oSplits_ = 0, oSlices_ = 0, oLater_ = 0,
-           oPrune_ = 0, oEmit_ = 0, oFcc_ = 0, oPairBase_ = 0;
+           oPrune_[2] = {}, oEmit_ = 0, oFcc_ = 0, oPairBase_ = 0;
     std::vector<uint8_t> blob_;   // host copy of the tables (alive while the upload runs)
 
     DevBuf tables, status, bigList;
