@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(128) partialValuesKernel(Batch b, const unsign
 __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t totalWords, uint32_t zBegin, uint32_t zEnd) {
     typedef NodeT<kPartial> NT;
     __shared__ uint32_t ids[8][32][9];          // 32 ids a word, padded
-    __shared__ uint32_t masks[8][32][4];        // surface, surface less cleared nodes, fill, rank
+    __shared__ uint4 masks[8][32];              // surface, surface less cleared nodes, fill, rank
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint64_t gbase = ((uint64_t)blockIdx.x * 8u + warp) * 32u; gbase < totalWords;
          gbase += (uint64_t)gridDim.x * 8u * 32u) {
@@ -827,14 +827,13 @@ __global__ void __launch_bounds__(256) emitPartialKernel(EmitArgs a, uint64_t to
 #pragma unroll
             for (int i = 0; i < 8; ++i) ids[warp][lane][i] = N[i];
         }
-        *reinterpret_cast<uint4*>(masks[warp][lane]) =
-            make_uint4(n.s0, sm, fm, sm ? a.ranks[U.wordBase + w].rank : 0u);
+        masks[warp][lane] = make_uint4(n.s0, sm, fm, sm ? a.ranks[U.wordBase + w].rank : 0u);
         __syncwarp();
 #pragma unroll 4
         for (uint32_t i = wbeg * 16u + lane; i < wend * 16u; i += 32u) {
             const uint32_t l = i >> 4, p = (i & 15u) * 2u;   // word and its first node
             const uint32_t id2 = reinterpret_cast<const uint16_t*>(ids[warp][l])[p >> 1];
-            const uint4 m = *reinterpret_cast<const uint4*>(masks[warp][l]);
+            const uint4 m = masks[warp][l];
             uint64_t v[2];
 #pragma unroll
             for (uint32_t j = 0; j < 2; ++j) {
