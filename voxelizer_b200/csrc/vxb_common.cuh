@@ -17,17 +17,6 @@ __device__ __forceinline__ uint32_t laneMaskLt() {
     return m;
 }
 
-// Largest t with offsets[t] <= item (offsets: n + 1 non-decreasing entries).
-__device__ __forceinline__ uint32_t findOwner(const uint32_t* __restrict__ offsets, uint32_t n, uint32_t item) {
-    uint32_t lo = 0, hi = n;  // invariant: offsets[lo] <= item < offsets[hi]
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(offsets + mid) <= item) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 // Unit of element x: the largest u < n with base[u] <= x (base[0] = 0).
 template <class T>
 __device__ __forceinline__ uint32_t unitOf(const T* __restrict__ base, uint32_t n, T x) {

@@ -60,12 +60,6 @@ template <int M> __device__ __forceinline__ double lin(double i, double d, doubl
 }
 
 // ---- FP32 forms ----
-template <int M> __device__ __forceinline__ float sum2p1f(float a, float b, float c, float d, float e) {
-    if (M == 0) return __fadd_rn(__fadd_rn(__fmul_rn(a, b), __fmul_rn(c, d)), e);
-    if (M == 1) return __fadd_rn(__fmaf_rn(a, b, __fmul_rn(c, d)), e);
-    if (M == 2) return __fadd_rn(__fmaf_rn(c, d, __fmul_rn(a, b)), e);
-    return __fmaf_rn(a, b, __fmaf_rn(c, d, e));
-}
 template <int M> __device__ __forceinline__ float sum2f(float a, float b, float c, float d) {
     if (M == 0) return __fadd_rn(__fmul_rn(a, b), __fmul_rn(c, d));
     if (M == 1) return __fmaf_rn(a, b, __fmul_rn(c, d));
@@ -89,80 +83,40 @@ template <int M> __device__ __forceinline__ float linf(float a, float d, float m
 }
 
 // ---------------------------------------------------------------------------
-// Node layouts (byte-identical to the reference's include/node_types.h) and
-// the surface key each layout stores in its own slot while the surface pass
-// runs.  A key orders the triangles that touched a node: triangle class
-// (1D < 2D < 3D) first, then material; the largest key wins.
+// Node layouts (byte-identical to the reference's include/node_types.h) and the
+// material of a merged surface key.  A key orders the triangles that touched a
+// node: triangle class (1D < 2D < 3D) first, then material (class << 8 | material;
+// PartialNodes class << 40 | material << 32 | triangle); the largest key wins.
 enum NodeKind { kShort = 0, kLong = 1, kPartial = 2, kShortFcc = 3, kLongFcc = 4 };
 
 template <int K> struct NodeT;
 template <> struct NodeT<kShort> {
-    typedef uint8_t slot_t;
     static constexpr int bytes = 1;
-    static constexpr bool fcc = false;
-    __device__ static slot_t key(uint32_t cls, uint32_t mat, uint32_t) { return (slot_t)((cls << 3) | (mat & 7u)); }
     __device__ static uint32_t keyMat(uint64_t k) { return (uint32_t)k & 7u; }
     __device__ static uint64_t pack(uint32_t bid, uint32_t mat, float) { return (uint64_t)(((mat << 5) | (bid & 31u)) & 0xFFu); }
 };
 template <> struct NodeT<kLong> {
-    typedef uint16_t slot_t;
     static constexpr int bytes = 2;
-    static constexpr bool fcc = false;
-    __device__ static slot_t key(uint32_t cls, uint32_t mat, uint32_t) { return (slot_t)((cls << 8) | (mat & 255u)); }
     __device__ static uint32_t keyMat(uint64_t k) { return (uint32_t)k & 255u; }
     __device__ static uint64_t pack(uint32_t bid, uint32_t mat, float) { return (uint64_t)((bid & 255u) | ((mat & 255u) << 8)); }
 };
 template <> struct NodeT<kPartial> {
-    typedef unsigned long long slot_t;
     static constexpr int bytes = 8;
-    static constexpr bool fcc = false;
-    __device__ static slot_t key(uint32_t cls, uint32_t mat, uint32_t tri) {
-        return ((slot_t)cls << 40) | ((slot_t)(mat & 255u) << 32) | (slot_t)tri;
-    }
     __device__ static uint32_t keyMat(uint64_t k) { return (uint32_t)(k >> 32) & 255u; }
     __device__ static uint64_t pack(uint32_t bid, uint32_t mat, float r) {
         return (uint64_t)(bid & 255u) | ((uint64_t)(mat & 255u) << 8) | ((uint64_t)__float_as_uint(r) << 32);
     }
 };
 template <> struct NodeT<kShortFcc> {
-    typedef uint16_t slot_t;
     static constexpr int bytes = 2;
-    static constexpr bool fcc = true;
-    __device__ static slot_t key(uint32_t cls, uint32_t mat, uint32_t) { return (slot_t)((cls << 4) | (mat & 15u)); }
     __device__ static uint32_t keyMat(uint64_t k) { return (uint32_t)k & 15u; }
     __device__ static uint64_t pack(uint32_t bid, uint32_t mat, float) { return (uint64_t)(((mat << 12) | (bid & 4095u)) & 0xFFFFu); }
 };
 template <> struct NodeT<kLongFcc> {
-    typedef uint32_t slot_t;
     static constexpr int bytes = 4;
-    static constexpr bool fcc = true;
-    __device__ static slot_t key(uint32_t cls, uint32_t mat, uint32_t) { return (slot_t)((cls << 8) | (mat & 255u)); }
     __device__ static uint32_t keyMat(uint64_t k) { return (uint32_t)k & 255u; }
     __device__ static uint64_t pack(uint32_t bid, uint32_t mat, float) { return (uint64_t)((bid & 0xFFFFu) | ((mat & 255u) << 16)); }
 };
-
-// Atomic max of a node-sized key inside the 32-bit (or 64-bit) word that
-// holds it.  Slots never straddle words: nodes are 1, 2, 4 or 8 bytes.
-template <class S> __device__ __forceinline__ void slotMax(S* slot, S key);
-template <> __device__ __forceinline__ void slotMax<unsigned long long>(unsigned long long* slot, unsigned long long key) {
-    atomicMax(slot, key);
-}
-template <> __device__ __forceinline__ void slotMax<uint32_t>(uint32_t* slot, uint32_t key) { atomicMax(slot, key); }
-template <class S> __device__ __forceinline__ void slotMax(S* slot, S key) {
-    uintptr_t a = reinterpret_cast<uintptr_t>(slot);
-    uint32_t* w = reinterpret_cast<uint32_t*>(a & ~uintptr_t(3));
-    const uint32_t shift = (uint32_t)(a & 3u) * 8u;
-    const uint32_t mask = (sizeof(S) == 1 ? 0xFFu : 0xFFFFu) << shift;
-    uint32_t old = *reinterpret_cast<volatile uint32_t*>(w);
-    for (;;) {
-        uint32_t cur = (old & mask) >> shift;
-        if ((uint32_t)key <= cur) return;
-        uint32_t nv = (old & ~mask) | ((uint32_t)key << shift);
-        uint32_t prev = atomicCAS(w, old, nv);
-        if (prev == old) return;
-        old = prev;
-    }
-}
 
 // Boundary ids by 6-neighbour permutation (bits -x 1, +x 2, -y 4, +y 8,
 // -z 16, +z 32), the numbering of the reference's getOrientation

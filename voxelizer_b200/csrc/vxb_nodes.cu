@@ -1,14 +1,14 @@
 // Node classification kernels: packed-bit pruning and node emission.
 //
 // Emission reads three bit grids (final solid, unpruned fill, surface) and
-// writes the node grid once.  One thread owns one 32-bit word (32 nodes of a
-// row): it forms the six neighbour masks of its word with shifts of the word
-// and of the words around it, so a whole word of boundary ids costs a few
-// bitwise operations when the word is uniform (all empty, or all solid with
-// all six neighbours solid: id 27).  The ids of a mixed word are computed
-// bit-sliced (a plane per id bit) and transposed to bytes.  A warp's 32 words
-// are staged in shared memory and stored as contiguous 512-byte rows with
-// 16-byte vector stores.
+// writes the node grid once, from 32-bit words (32 nodes of a row).  The
+// neighbour masks of a word are shifts of it and of the words around it, so a
+// word of one id (all empty, or all solid with all six neighbours solid: id 27)
+// costs a few bitwise operations; the ids of the others are computed bit-sliced
+// (a plane per id bit) and transposed to bytes.  1- and 2-byte nodes: warps walk
+// planes along z, store words of one id at once and collect the others until 32
+// are there.  PartialNodes and FCC nodes: a lane forms the ids of a word, and the
+// warp stores its words' nodes in order, 16 bytes a lane.
 //
 // Grids of one unit hold fewer than 2^32 voxels, so word indices inside a
 // unit fit 32 bits; arena offsets (unit word bases) are 64-bit.
