@@ -92,7 +92,8 @@ vxb_status vxb_create(vxb_voxelizer** out, int node_type, const float* vertices,
  * draw from, so that creating one voxelizer per mesh does not pay cudaMalloc
  * / cudaFree every time; its streams go to a list of at most 64 idle ones.
  * (Calls return with their work complete; after a failed call this waits for
- * the device first.) */
+ * the device first.)  A CUDA graph capture that is under way in this or another
+ * thread stays valid. */
 vxb_status vxb_destroy(vxb_voxelizer* v);
 /* No reference counterpart: returns every idle cached block and stream to the
  * driver. */

@@ -26,9 +26,9 @@
 // Bounds: FP64 issue at half rate (48 edge values a candidate) and the latency
 // of its chains.  Solid pass alone on a B200 (memset, toggles, row fill), with
 // a candidate list staged per block and with this split: room of 1,049,868
-// triangles at 1024 voxels 364 -> 196 us, 81,920 triangles at 701 voxels
-// 87 -> 52 us, 576 triangles at 32 voxels 48 -> 17 us.  Chunks of 32 / 64 /
-// 128 candidates on the room: 204 / 196 / 232 us; 32 costs scenes with many
+// triangles at 1024 voxels 364 -> 192 us, 81,920 triangles at 701 voxels
+// 87 -> 52 us, 576 triangles at 32 voxels 48 -> 17 us.  Chunks of 32 or
+// 128 candidates took 8 and 36 us more on the room; 32 costs scenes with many
 // medium triangles (stress mesh 54 against 45 us) because every chunk sets
 // its batch up again.  Five resident blocks of 96 registers: six (80) and
 // seven (72) spill and are equal or up to 8% slower.
