@@ -48,12 +48,13 @@ def test_long_lines_are_shared_out():
     for mats in (None, m.materials):
         with Voxelizer(m.vertices, m.indices, mats, 8, node_type=LONG) as vx:
             out = torch.empty(int(vx.plan(1, 60_000).bytes), dtype=torch.uint8, device="cuda")
-            for _ in range(3):
+            best = 1.0
+            for _ in range(5):
                 torch.cuda.synchronize()
                 start = time.perf_counter()
                 vx.voxelize_device(1, 60_000, out)
                 torch.cuda.synchronize()
-                t = time.perf_counter() - start
-        took.append(t)
+                best = min(best, time.perf_counter() - start)
+        took.append(best)
     # One lane that takes a line of 60,000 voxels: 50 times as long.
     assert took[1] < 10 * took[0]

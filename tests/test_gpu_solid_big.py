@@ -31,17 +31,18 @@ def test_few_triangles_many_candidates():
     v, boxes = _nested()
 
     def run(f):
-        """The grid and the seconds of a call (the second one).  All grids have
+        """The grid and the seconds of the fastest call.  All grids have
         all vertices, so they have the same bounding box."""
         with Voxelizer(v, f, node_type=LONG) as vx:
             out = torch.empty(int(vx.plan(0, 8192).count), dtype=torch.int32, device="cuda")
-            for _ in range(2):
+            best = 100.0
+            for _ in range(3):
                 torch.cuda.synchronize()
                 start = time.perf_counter()
                 vx.voxelize_device(0, 8192, out)
                 torch.cuda.synchronize()
-                took = time.perf_counter() - start
-        return out, took
+                best = min(best, time.perf_counter() - start)
+        return out, best
 
     all_boxes, took = run(np.concatenate(boxes))
     alone = [run(f) for f in boxes]

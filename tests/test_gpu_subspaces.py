@@ -40,12 +40,13 @@ def test_many_subspaces_cost_little():
     with Voxelizer(v, f, node_type=LONG) as vx:
         for vox in ((1024, 512, 512), (1024, 64, 64)):
             out = torch.empty(int(vx.plan(0, 4096, vox).count), dtype=torch.int32, device="cuda")
-            for _ in range(2):
+            best = 1.0
+            for _ in range(4):
                 torch.cuda.synchronize()
                 start = time.perf_counter()
                 vx.voxelize_device(0, 4096, out, vox)
                 torch.cuda.synchronize()
-                t = time.perf_counter() - start
-            took.append(t)
+                best = min(best, time.perf_counter() - start)
+            took.append(best)
     # With each subspace looked at per candidate, 50 times as long.
     assert took[1] < 12 * took[0]
