@@ -586,11 +586,13 @@ __device__ __forceinline__ void emitWords(const EmitArgs& args, const EmitSlots&
 // A task covers a chunk of 32 words (kPacked, one warp) or kEmitWarps of them
 // (one block) over `planes` planes.  Tasks are numbered through: along a plane,
 // groups of planes, units (taskBase), so that no block of a batch is without
-// work whatever its units' shapes.  Where planes are so thin that the warps of a
-// block would idle (emit_packed), tasks are warps': 60,000 planes of 7 words
-// 29 us, 189 with a block a plane; 2,000 meshes of 16-24 voxels 590 us a batch
-// instead of 698.  One unit of wide planes (kUnit) has its groups of planes
-// along the grid's y, which keeps z out of the vector registers: 1-3% of a call
+// work whatever its units' shapes (1,000 meshes of 36 planes beside one of 4,098:
+// 1,250 us a call with the tallest unit's planes for all, now 227).  Where planes
+// are so thin that the warps of a block would idle (emit_packed), tasks are
+// warps': 60,002 planes of 7 words 27 us, 58 with blocks; 2,000 meshes of 16-24
+// voxels 142 us a call and 178.  One unit of wide planes (kUnit) has its groups
+// of planes along the grid's y, which keeps z out of the vector registers: 1-3%
+// of a call
 // (room, duct) against a division of the block's number.  They are fewer than
 // the 65,535 blocks that y takes: emit_planes leaves at most twice as many tasks
 // as blocks share the grid (2 * 148 * 2 * 32 with the widest launch shape), or
@@ -1081,7 +1083,9 @@ uint32_t emit_tasks(const PassGeom& g, bool packed) {
 }
 
 bool emit_packed(uint64_t chunkPlanes, uint64_t blockPlanes) {
-    // At 128^3 (17 chunks a plane, 24 warps: 1.4) both take the same time.
+    // Half again as many warps as chunks.  The same within 2-4 us for 13 chunks
+    // on 16 warps (54 us packed, 56 in blocks), 10 on 16 (52, 56) and 4 on 8 (31,
+    // 29); 1 on 8 is 27 and 58.
     return 2 * kEmitWarps * blockPlanes > 3 * chunkPlanes;
 }
 
