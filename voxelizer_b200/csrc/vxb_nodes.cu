@@ -592,12 +592,11 @@ __device__ __forceinline__ void emitWords(const EmitArgs& args, const EmitSlots&
 // warps': 60,002 planes of 7 words 27 us, 58 with blocks; 2,000 meshes of 16-24
 // voxels 142 us a call and 178.  One unit of wide planes (kUnit) has its groups
 // of planes along the grid's y, which keeps z out of the vector registers: 1-3%
-// of a call
-// (room, duct) against a division of the block's number.  They are fewer than
-// the 65,535 blocks that y takes: emit_planes leaves at most twice as many tasks
-// as blocks share the grid (2 * 148 * 2 * 32 with the widest launch shape), or
-// groups of 64 planes, and 65,535 of those with planes this wide (more than five
-// chunks) are more words than a grid may have.
+// of a call (room, duct) against a division of the block's number.  They are
+// fewer than the 65,535 blocks that y takes: emit_planes leaves at most twice as
+// many tasks as blocks share the grid (2 * 148 * 2 * 32 with the widest launch
+// shape), or groups of 64 planes, and 65,535 of those with planes this wide (more
+// than five chunks) are more words than a grid may have.
 enum EmitTasks { kUnit, kBlocks, kPacked };
 
 template <int K, EmitTasks T>
